@@ -18,8 +18,16 @@ h(x) = exp(-x^2) (2x/sqrt(pi) + erfcx(x)) with erfcx(x) = exp(x^2) erfc(x)
 ~ t P(t), t = 1/(1 + x/2), P of degree EW32_DEG, fitted here by least
 squares in relative error on Chebyshev nodes of [0, EW32_XFIT].
 
+The FP64 forms' double-float kernels (xmd_ewald_df.cu) use finer tables of
+degree 4 (DF_W = 1/256), a row of eight floats an interval: c0, c1 and c2 as
+FP32 pairs (high and low part), c3 and c4 as single floats, so that a row is
+two 16-byte loads and the polynomial runs in FP32 with error-free products.
+
 Run:  python gen_ewald_tables.py > xmd_ewald_tables.h   (needs mpmath, numpy)
+      python gen_ewald_tables.py --df > xmd_ewald_df_tables.h
 """
+import sys
+
 import mpmath as mp
 import numpy as np
 
@@ -86,6 +94,40 @@ def erfcx_fit():
     return [float(v) for v in c], float(np.max(np.abs(fit - ye) / ye))
 
 
+DF_W, DF_DEG = 0.00390625, 4
+DF_NINT = {"H": 1340, "ERFC": 1494}  # up to x = 5.23 (forces) and 5.83 (energies)
+
+
+def split(c):
+    """c as an FP32 pair (high, low)"""
+    hi = np.float32(float(c))
+    return hi, np.float32(float(c - mp.mpf(float(hi))))
+
+
+def df_table(f, nint):
+    """rows of eight floats and the largest error of their exact sum"""
+    rows, worst = [], 0.0
+    for i in range(nint):
+        a, b = (mp.mpf(i) - mp.mpf(1) / 2) * DF_W, (mp.mpf(i) + mp.mpf(1) / 2) * DF_W
+        c = interpolant(f, a, b, DF_DEG)
+        row = [*split(c[0]), *split(c[1]), *split(c[2]), np.float32(float(c[3])), np.float32(float(c[4]))]
+        v = [mp.mpf(float(x)) for x in row]
+        p = [v[0] + v[1], v[2] + v[3], v[4] + v[5], v[6], v[7]]
+        for s in range(41):
+            t = -1 + 2 * mp.mpf(s) / 40
+            worst = max(worst, abs(horner(p, t) - f((a + b) / 2 + (b - a) / 2 * t)))
+        rows.append(row)
+    return rows, float(worst)
+
+
+def emit_df(name, rows):
+    out = [f"#define {name}_INIT {{ \\"]
+    for r in rows:
+        out.append("    " + ", ".join(f"{c!s}f" for c in r) + ", \\")
+    out.append("  }")
+    return "\n".join(out)
+
+
 def emit(name, rows):
     """An initializer macro, usable for host arrays and __constant__ arrays."""
     out = [f"#define {name}_INIT {{ \\"]
@@ -95,7 +137,25 @@ def emit(name, rows):
     return "\n".join(out)
 
 
-if __name__ == "__main__":
+def main_df():
+    dh, dhe = df_table(h, DF_NINT["H"])
+    de, dee = df_table(e, DF_NINT["ERFC"])
+    print(f"""// xmd_ewald_df_tables.h -- generated by gen_ewald_tables.py --df; do not edit.
+//
+// FP32-pair tables of h(x) = erfc(x) + 2 x exp(-x^2)/sqrt(pi) and erfc(x):
+// intervals of width {DF_W} centred at i w, t = 2 (x - i w)/w, rows
+// (c0 hi, c0 lo, c1 hi, c1 lo, c2 hi, c2 lo, c3, c4); max |error| of the
+// rows' exact sums {dhe:.2e} (h), {dee:.2e} (erfc)
+#pragma once
+#define EWD_INV_W {1 / DF_W!r}f
+#define EWD_H_NINT {DF_NINT["H"]}
+#define EWD_ERFC_NINT {DF_NINT["ERFC"]}
+""")
+    print(emit_df("EWD_H", dh))
+    print(emit_df("EWD_ERFC", de))
+
+
+def main():
     th, eh = table(h)
     te, ee = table(e)
     print(f"""// xmd_ewald_tables.h -- generated by gen_ewald_tables.py; do not edit.
@@ -123,3 +183,7 @@ if __name__ == "__main__":
 #define EW32_DEG {EW32_DEG}
 #define EW32_XFIT {EW32_XFIT!r}
 #define EW32_ERFCX_INIT {{ {", ".join(repr(v) for v in c32)} }}""")
+
+
+if __name__ == "__main__":
+    main_df() if "--df" in sys.argv else main()

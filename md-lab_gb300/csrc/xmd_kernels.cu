@@ -2043,6 +2043,8 @@ size_t pair_scratch_doubles(const Geo &g) {
   // partial slots (doubles, or float2 in the FP32 form), then room for the
   // FP32 form's copies of the positions and inverse masses
   size_t a = (size_t)T * g.slots() + (g.slots() + (size_t)g.P * g.Ns + 1) / 2 + 1;
+  const size_t d = g.D == 3 ? (size_t)T * g.slots() + 1 + ewd_pos_doubles(g) : 0;
+  if (d > a) a = d;
   size_t b = jobs * g.P;
   return a > b ? a : b;
 }
@@ -2159,6 +2161,7 @@ static cudaError_t pair_launch(const Geo &g, const PairPrm &p_in, const double *
 
 cudaError_t pair_force(const Geo &g, const PairPrm &p, const double *x, const double *m,
                        double *f, double *scratch, cudaStream_t st) {
+  if (p.inv_mass > 0 && ewd_applies(g, p, false)) return ewd_force(g, p, x, f, scratch, st);
   const int T = (g.N + 31) / 32;
   const int jobs = T * (T + 1) / 2;
   cudaError_t e;
@@ -2176,7 +2179,13 @@ cudaError_t pair_energy(const Geo &g, const PairPrm &p, const double *x, double 
   const int T = (g.N + 31) / 32;
   const int jobs = T * (T + 1) / 2;
   cudaError_t e;
-  DISPATCH_D(g.D, e = (pair_launch<D, true>(g, p, x, nullptr, scratch, T, jobs, st)));
+  double unit = 1.0;
+  if (ewd_applies(g, p, true)) {
+    e = ewd_energy_tiles(g, p, x, scratch, st);
+    unit = p.qs * p.alpha;
+  } else {
+    DISPATCH_D(g.D, e = (pair_launch<D, true>(g, p, x, nullptr, scratch, T, jobs, st)));
+  }
   if (e != cudaSuccess) return e;
   // the Ewald energy carries -pi/(alpha^2 V) per pair (md_statistics_x.c:385)
   double add = 0;
@@ -2184,12 +2193,13 @@ cudaError_t pair_energy(const Geo &g, const PairPrm &p, const double *x, double 
     const double V = g.box[0] * g.box[1] * g.box[2];
     add = -p.qs * M_PI / (p.alpha * p.alpha * V) * ((double)g.N * (g.N - 1) / 2);
   }
-  return reduce_into(scratch, jobs * g.P, 1.0 / g.P, add, acc, st);
+  return reduce_into(scratch, jobs * g.P, unit / g.P, add, acc, st);
 }
 
 size_t pair2_scratch_doubles(const Geo &ga, const Geo &gb) {
   const int TA = (ga.N + 31) / 32, TB = (gb.N + 31) / 32;
-  const size_t forces = (size_t)TB * ga.slots() + (size_t)TA * gb.slots();
+  size_t forces = (size_t)TB * ga.slots() + (size_t)TA * gb.slots();
+  if (ga.D == 3) forces += 1 + ewd_pos_doubles(ga) + ewd_pos_doubles(gb);
   const size_t energy = (size_t)TA * TB * ga.P;
   return forces > energy ? forces : energy;
 }
@@ -2230,8 +2240,10 @@ static cudaError_t cross_dispatch(const Geo &ga, const Geo &gb, const PairPrm &p
 
 cudaError_t pair_force_2(const Geo &ga, const Geo &gb, const PairPrm &p, const double *xa, const double *ma,
                          const double *xb, const double *mb, double *fa, double *fb, double *scratch,
-                         cudaStream_t st) {
+                         cudaStream_t st, double inv_ma, double inv_mb) {
   if (ga.D != gb.D || ga.P != gb.P) return cudaErrorInvalidValue;
+  if (inv_ma > 0 && inv_mb > 0 && ewd_applies(ga, p, false))
+    return ewd_force_2(ga, gb, p, xa, inv_ma, xb, inv_mb, fa, fb, scratch, st);
   const int TA = (ga.N + 31) / 32, TB = (gb.N + 31) / 32;
   double *outa = scratch, *outb = scratch + (size_t)TB * ga.slots();
   cudaError_t e;

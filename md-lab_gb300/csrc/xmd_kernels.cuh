@@ -207,6 +207,16 @@ void set_tuning(int what, int kind, int D, int N, int P, int v);
 int tuning(int what, int kind, int D, int N, int P);
 cudaError_t pair_energy(const Geo &g, const PairPrm &p, const double *x, double *acc,
                         double *scratch, cudaStream_t st);
+// real-space Ewald in double-float (xmd_ewald_df.cu): whether a call takes
+// it (forces also need one mass a species), the space its positions need in
+// the scratch, and the launches pair_force and pair_force_2 hand over
+bool ewd_applies(const Geo &g, const PairPrm &p, bool energy);
+size_t ewd_pos_doubles(const Geo &g);
+cudaError_t ewd_force(const Geo &g, const PairPrm &p, const double *x, double *f, double *scratch, cudaStream_t st);
+// the real-space energies of the tile jobs, in units of s alpha, into scratch
+cudaError_t ewd_energy_tiles(const Geo &g, const PairPrm &p, const double *x, double *scratch, cudaStream_t st);
+cudaError_t ewd_force_2(const Geo &ga, const Geo &gb, const PairPrm &p, const double *xa, double inv_ma,
+                        const double *xb, double inv_mb, double *fa, double *fb, double *scratch, cudaStream_t st);
 
 // Pair forces (not Ewald) with the per-tile partials in a fixed array of
 // NOALLOC_SCRATCH_DOUBLES doubles inside the library (4 MiB): no allocation.
@@ -219,12 +229,13 @@ cudaError_t pair_force_noalloc(const Geo &g, const PairPrm &p, const double *x, 
 
 // two species with the same P and box (md_pimd_x.c:3282-3632): cross pairs
 // only, every bead of species a with every bead of species b in its slice;
-// f_a += F/(m_a P), f_b -= F/(m_b P), with a's box.  scratch: at least
+// f_a += F/(m_a P), f_b -= F/(m_b P), with a's box.  inv_ma, inv_mb: the
+// species' inverse masses where each has one, else 0.  scratch: at least
 // pair2_scratch_doubles(ga, gb) doubles.
 size_t pair2_scratch_doubles(const Geo &ga, const Geo &gb);
 cudaError_t pair_force_2(const Geo &ga, const Geo &gb, const PairPrm &p, const double *xa, const double *ma,
                          const double *xb, const double *mb, double *fa, double *fb, double *scratch,
-                         cudaStream_t st);
+                         cudaStream_t st, double inv_ma = 0, double inv_mb = 0);
 // sum over slices and cross pairs of V/P (plus -pi/(alpha^2 V) per pair for Ewald), added to *acc
 cudaError_t pair_energy_2(const Geo &ga, const Geo &gb, const PairPrm &p, const double *xa, const double *xb,
                           double *acc, double *scratch, cudaStream_t st);

@@ -568,7 +568,8 @@ int md_pimd_calc_pair_force_2_x(md_pimd_t_x *pimd, md_pimd_t_x *pimd2, md_pair_f
                                1.0 / (sb->mass0 * pimd2->P), sb->f.as<double>(), st));
   }
   XMD_CUDA(xk::pair_force_2(sa->geo, sb->geo, prm, sa->x.as<double>(), sa->m.as<double>(), sb->x.as<double>(),
-                            sb->m.as<double>(), sa->f.as<double>(), sb->f.as<double>(), scr, st));
+                            sb->m.as<double>(), sa->f.as<double>(), sb->f.as<double>(), scr, st,
+                            sa->uniform_mass ? 1.0 / sa->mass0 : 0.0, sb->uniform_mass ? 1.0 / sb->mass0 : 0.0));
   return 0;
 }
 
@@ -685,6 +686,7 @@ int md_gb300_autotune_fp64_x(md_pimd_t_x *pimd, md_pair_force_t_x pf, int repeat
       return fail(MD_GB_ERR_UNSUPPORTED, "Ewald alpha*L below %.1f (images beyond the neighbouring boxes)",
                   2 * EWALD_XCUT / 3);
     prm.rcut = EWALD_XCUT_FORCE / prm.alpha;
+    prm.inv_mass = 1.0 / sd->mass0;
     XMD_TRY(ewald_tables(pimd, sd, pd));
   }
   const xk::Geo &g = sd->geo;
