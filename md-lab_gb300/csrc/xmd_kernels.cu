@@ -2551,7 +2551,7 @@ __global__ void k_recip_energy(Geo g, const double2 *__restrict__ S, const doubl
 }
 
 static int ncols(int ns) { return ns * (2 * ns + 1) + ns + 1; }
-static size_t recip_split_at(int ns) { return (5 * (size_t)ncols(ns) + 1 + 3) & ~(size_t)3; }
+size_t recip_df_off(int ns) { return (5 * (size_t)ncols(ns) + 1 + 3) & ~(size_t)3; }
 
 cudaError_t recip_setup(const Geo &g, int ns, double alpha, double qs, Recip &r,
                         cudaStream_t st) {
@@ -2594,29 +2594,8 @@ cudaError_t recip_setup(const Geo &g, int ns, double alpha, double qs, Recip &r,
   // compact table offsets of the kept columns (4 nzmax + 1 entries each)
   std::vector<int> toff(kept.size() + 1, 0);
   for (size_t i = 0; i < kept.size(); ++i) toff[i + 1] = toff[i] + 4 * kept[i].first + 1;
-  // the split for the FP64 forces: the columns whose largest force weight
-  // is below RECIP_SPLIT of the largest go to the FP32 kernels (after the
-  // FP64 ones in the split list, both parts longest first)
-  std::vector<int4> split_in, split_out;
-  std::vector<int> toff_in(1, 0);
-  for (size_t i = 0; i < kept.size(); ++i) {
-    const int4 c = kept[i].second;
-    const int nzmax = kept[i].first;
-    double wc = 0;
-    for (int nz = c.z; nz <= nzmax; ++nz) {
-      const int k = c.w + nz - c.z;
-      wc = wgt[k] > wc ? wgt[k] : wc;
-    }
-    if (wc < RECIP_SPLIT * wmax) {
-      split_out.push_back(c);
-    } else {
-      split_in.push_back(c);
-      toff_in.push_back(toff_in.back() + 4 * nzmax + 1);
-    }
-  }
-  r.ncol_in = (int)split_in.size();
-  r.ncol_out = (int)split_out.size();
-  r.tsz_in = toff_in.back();
+  std::vector<int> dft;
+  recip_df_tables(ns, cd, wgt, wmax, r, dft);
   r.nsum = ns;
   r.nk = nk;
   r.ncol = (int)cd.size();
@@ -2636,41 +2615,25 @@ cudaError_t recip_setup(const Geo &g, int ns, double alpha, double qs, Recip &r,
   e = cudaMemcpyAsync(r.kvec + 4 * (size_t)(ns * (2 * ns + 1) + ns + 1), toff.data(), sizeof(int) * toff.size(),
                       cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return e;
-  split_in.insert(split_in.end(), split_out.begin(), split_out.end());
-  if (!split_in.empty()) {
-    e = cudaMemcpyAsync(r.kvec + recip_split_at(ns), split_in.data(), sizeof(int4) * split_in.size(),
-                        cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return e;
-  }
-  e = cudaMemcpyAsync(r.kvec + recip_split_at(ns) + 4 * (size_t)ncols(ns), toff_in.data(),
-                      sizeof(int) * toff_in.size(), cudaMemcpyHostToDevice, st);
+  e = cudaMemcpyAsync(r.kvec + recip_df_off(ns), dft.data(), sizeof(int) * dft.size(), cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return e;
   // dropped vectors keep S = 0 (their c(n) = 0 multiplies them in the energies)
   if (r.S) {
     e = cudaMemsetAsync(r.S, 0, sizeof(double2) * (size_t)nk * g.P, st);
     if (e != cudaSuccess) return e;
   }
-  if (r.S32) {
-    e = cudaMemsetAsync(r.S32, 0, sizeof(float2) * (size_t)nk * g.P, st);
-    if (e != cudaSuccess) return e;
-  }
   return cudaStreamSynchronize(st);
 }
 
 // kvec: the kept columns (int4, longest first) and their compact table
-// offsets, then, from recip_split_at (16-byte aligned), the split list (the
-// FP64 columns, then the FP32 ones) and the FP64 columns' table offsets
-size_t recip_cols_ints(int ns) { return recip_split_at(ns) + 5 * (size_t)ncols(ns) + 1; }
+// offsets, then, from recip_df_off (16-byte aligned), the double-float
+// kernels' tables
+size_t recip_cols_ints(int ns) { return recip_df_off(ns) + recip_df_ints(ns); }
 
 // compact table offsets behind the column table in the same buffer
 static const int *recip_toff(const Recip &r) {
   return r.kvec + 4 * (size_t)(r.nsum * (2 * r.nsum + 1) + r.nsum + 1);
 }
-static const int4 *recip_split_cols(const Recip &r) { return (const int4 *)(r.kvec + recip_split_at(r.nsum)); }
-static const int *recip_split_toff(const Recip &r) {
-  return r.kvec + recip_split_at(r.nsum) + 4 * (size_t)ncols(r.nsum);
-}
-
 #define DISPATCH_NS(nsv, ...)                                         \
   switch (nsv) {                                                      \
     case 1: { constexpr int NS = 1; __VA_ARGS__; } break;             \
@@ -2688,10 +2651,10 @@ static const int *recip_split_toff(const Recip &r) {
     default: return cudaErrorInvalidValue;                            \
   }
 
-// FP64 structure factors of the columns cols[0, nc) (all kept columns by default)
-static cudaError_t structure_factors(const Geo &g, const Recip &r, const double *x,
-                                     cudaStream_t st, const int4 *cols = nullptr, int nc = -1) {
-  if (!cols) cols = (const int4 *)r.kvec, nc = r.ncol;
+// FP64 structure factors of the kept columns
+static cudaError_t structure_factors(const Geo &g, const Recip &r, const double *x, cudaStream_t st) {
+  const int4 *cols = (const int4 *)r.kvec;
+  const int nc = r.ncol;
   const size_t n = (size_t)g.P * 3 * g.Ns;
   {
     XK_PROF("phase");
@@ -2726,49 +2689,50 @@ static cudaError_t structure_factors(const Geo &g, const Recip &r, const double 
 
 size_t recip_table_doubles(const Geo &g, int ns) { return (size_t)g.P * ncols(ns) * (4 * ns + 1) * 2; }
 
-static cudaError_t recip_cols32(const Geo &g, const Recip &r, const double *x, double inv_mP, double *f,
-                                cudaStream_t st, const int4 *cols, int nc, float2 *S32, float2 *T32);
+static cudaError_t recip_tables_of(const Geo &g, const Recip &r, cudaStream_t st) {
+  const int nc = r.ncol;
+  dim3 tgrid((nc + 7) / 8, g.P), tblk(r.nsum + 1, 8);
+  DISPATCH_NS(r.nsum, {
+    XK_PROF("recip_tables");
+    k_recip_tables<NS><<<tgrid, tblk, 0, st>>>((const int4 *)r.kvec, nc, (const double2 *)r.S, r.coef, r.nk,
+                                               (double2 *)r.T);
+  });
+  return XK_LAUNCHED();
+}
+
+static cudaError_t recip_force_from(const Geo &g, const Recip &own, const double *T_other, double scale, double *f,
+                                    cudaStream_t st) {
+  const int nc = own.ncol;
+  const size_t smem = sizeof(double2) * own.tsz;
+  dim3 grid((g.N + 127) / 128, g.P);
+  DISPATCH_NS(own.nsum, {
+    auto kf = k_recip_force<NS>;
+    static bool opted = false;
+    if (!opted) {
+      cudaError_t ea = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      if (ea != cudaSuccess) return ea;
+      opted = true;
+    }
+    XK_PROF("recip_force");
+    kf<<<grid, 128, smem, st>>>(g, (const double2 *)own.phase, (const int4 *)own.kvec, recip_toff(own), nc,
+                                (const double2 *)T_other, scale, f, nullptr, 0.0);
+  });
+  return XK_LAUNCHED();
+}
 
 cudaError_t recip_force(const Geo &g, const Recip &r, const double *x, double inv_mP, double *f,
-                        cudaStream_t st, bool fp32_outer) {
+                        cudaStream_t st, bool df) {
   if (g.D != 3) return cudaErrorInvalidValue;
-  // the split: the FP64 columns here, the small-weight ones by the FP32 kernels
-  const bool split = fp32_outer && r.S32 && r.ncol_out > 0;
-  const int4 *cols = split ? recip_split_cols(r) : (const int4 *)r.kvec;
-  const int *toff = split ? recip_split_toff(r) : recip_toff(r);
-  const int nc = split ? r.ncol_in : r.ncol;
-  cudaError_t e = structure_factors(g, r, x, st, cols, nc);
-  if (e != cudaSuccess) return e;
-  const size_t smem = sizeof(double2) * (split ? r.tsz_in : r.tsz);
-  dim3 tgrid((nc + 7) / 8, g.P), tblk(r.nsum + 1, 8);
-  dim3 grid((g.N + 127) / 128, g.P);
-  if (nc > 0) {
-    DISPATCH_NS(r.nsum, {
-      {
-        XK_PROF("recip_tables");
-        k_recip_tables<NS><<<tgrid, tblk, 0, st>>>(cols, nc, (const double2 *)r.S, r.coef, r.nk, (double2 *)r.T);
-      }
-      auto kf = k_recip_force<NS>;
-      // opt in to the largest dynamic shared memory once per instantiation
-      static bool opted = false;
-      if (!opted) {
-        cudaError_t ea = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-        if (ea != cudaSuccess) return ea;
-        opted = true;
-      }
-      {
-        XK_PROF("recip_force");
-        kf<<<grid, 128, smem, st>>>(g, (const double2 *)r.phase, cols, toff, nc, (const double2 *)r.T,
-                                    4 * M_PI * inv_mP, f, nullptr, 0.0);
-      }
-    });
-    e = XK_LAUNCHED();
-    if (e != cudaSuccess) return e;
+  if (df) {
+    cudaError_t e = recip_df_sk(g, r, x, st);
+    if (e == cudaSuccess) e = recip_df_tables_of(g, r, st);
+    if (e == cudaSuccess) e = recip_df_force_from(g, r, r.T, 4 * M_PI * inv_mP, f, st);
+    return e;
   }
-  if (!split) return cudaSuccess;
-  // the FP32 columns' tables go behind the FP64 columns' ones
-  float2 *T32 = (float2 *)(r.T + 2 * (size_t)g.P * r.ncol_in * (4 * r.nsum + 1));
-  return recip_cols32(g, r, x, inv_mP, f, st, cols + r.ncol_in, r.ncol_out, (float2 *)r.S32, T32);
+  cudaError_t e = structure_factors(g, r, x, st);
+  if (e == cudaSuccess) e = recip_tables_of(g, r, st);
+  if (e == cudaSuccess) e = recip_force_from(g, r, r.T, 4 * M_PI * inv_mP, f, st);
+  return e;
 }
 
 cudaError_t recip_force_energy(const Geo &g, const Recip &r, const double *x, double scale, double *f,
@@ -2814,8 +2778,13 @@ cudaError_t recip_force_energy(const Geo &g, const Recip &r, const double *x, do
 }
 
 cudaError_t recip_energy(const Geo &g, const Recip &r, const double *x, double *acc,
-                         double *scratch, cudaStream_t st) {
+                         double *scratch, cudaStream_t st, bool df) {
   if (g.D != 3) return cudaErrorInvalidValue;
+  if (df) {
+    cudaError_t e = recip_df_sk(g, r, x, st);
+    if (e == cudaSuccess) e = recip_df_energy(g, r, scratch, st);
+    return e == cudaSuccess ? reduce_into(scratch, g.P, 1.0 / g.P, 0.0, acc, st) : e;
+  }
   cudaError_t e = structure_factors(g, r, x, st);
   if (e != cudaSuccess) return e;
   {
@@ -2834,45 +2803,23 @@ cudaError_t recip_energy(const Geo &g, const Recip &r, const double *x, double *
 // cross energy of slice j is sum_{n in H} 2 c(n) Re(S_a,j(n) S_b,j(n)*).
 // Each species keeps its own phases, structure factors and tables (T from
 // its own S); a's forces read b's tables and b's read a's.
-static cudaError_t recip_tables_of(const Geo &g, const Recip &r, cudaStream_t st) {
-  const int nc = r.ncol;
-  dim3 tgrid((nc + 7) / 8, g.P), tblk(r.nsum + 1, 8);
-  DISPATCH_NS(r.nsum, {
-    XK_PROF("recip_tables");
-    k_recip_tables<NS><<<tgrid, tblk, 0, st>>>((const int4 *)r.kvec, nc, (const double2 *)r.S, r.coef, r.nk,
-                                               (double2 *)r.T);
-  });
-  return XK_LAUNCHED();
-}
-
-static cudaError_t recip_force_from(const Geo &g, const Recip &own, const double *T_other, double scale, double *f,
-                                    cudaStream_t st) {
-  const int nc = own.ncol;
-  const size_t smem = sizeof(double2) * own.tsz;
-  dim3 grid((g.N + 127) / 128, g.P);
-  DISPATCH_NS(own.nsum, {
-    auto kf = k_recip_force<NS>;
-    static bool opted = false;
-    if (!opted) {
-      cudaError_t ea = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-      if (ea != cudaSuccess) return ea;
-      opted = true;
-    }
-    XK_PROF("recip_force");
-    kf<<<grid, 128, smem, st>>>(g, (const double2 *)own.phase, (const int4 *)own.kvec, recip_toff(own), nc,
-                                (const double2 *)T_other, scale, f, nullptr, 0.0);
-  });
-  return XK_LAUNCHED();
-}
-
 static bool recip_pair_ok(const Geo &ga, const Recip &ra, const Geo &gb, const Recip &rb) {
   return ga.D == 3 && gb.D == 3 && ga.P == gb.P && ra.nsum == rb.nsum && ra.nk == rb.nk && ra.ncol == rb.ncol;
 }
 
 cudaError_t recip_force_2(const Geo &ga, const Recip &ra, const double *xa, double inv_mPa, double *fa,
                           const Geo &gb, const Recip &rb, const double *xb, double inv_mPb, double *fb,
-                          cudaStream_t st) {
+                          cudaStream_t st, bool df) {
   if (!recip_pair_ok(ga, ra, gb, rb)) return cudaErrorInvalidValue;
+  if (df) {
+    cudaError_t e = recip_df_sk(ga, ra, xa, st);
+    if (e == cudaSuccess) e = recip_df_sk(gb, rb, xb, st);
+    if (e == cudaSuccess) e = recip_df_tables_of(ga, ra, st);
+    if (e == cudaSuccess) e = recip_df_tables_of(gb, rb, st);
+    if (e == cudaSuccess) e = recip_df_force_from(ga, ra, rb.T, 4 * M_PI * inv_mPa, fa, st);
+    if (e == cudaSuccess) e = recip_df_force_from(gb, rb, ra.T, 4 * M_PI * inv_mPb, fb, st);
+    return e;
+  }
   cudaError_t e = structure_factors(ga, ra, xa, st);
   if (e == cudaSuccess) e = structure_factors(gb, rb, xb, st);
   if (e == cudaSuccess) e = recip_tables_of(ga, ra, st);
@@ -3810,17 +3757,14 @@ __global__ void __launch_bounds__(2 * RF_PB) k_recip_force32(Geo g, const float2
   f[sidx(j, 2, l, 3, g.Ns)] += scale * fz * g.inv_box[2];
 }
 
+// phases, structure factors, tables and forces in FP32 for all kept columns
 cudaError_t recip_force32(const Geo &g, const Recip &r, const double *x, double inv_mP, double *f,
                           cudaStream_t st) {
   if (g.D != 3) return cudaErrorInvalidValue;
+  const int4 *cols = (const int4 *)r.kvec;
+  const int nc = r.ncol;
   // the FP32 structure factors and tables use the FP64 form's buffers
-  return recip_cols32(g, r, x, inv_mP, f, st, (const int4 *)r.kvec, r.ncol, (float2 *)r.S, (float2 *)r.T);
-}
-
-// phases, structure factors, tables and forces in FP32 for the columns
-// cols[0, nc): all kept columns (the mixed form) or the FP64 form's split
-static cudaError_t recip_cols32(const Geo &g, const Recip &r, const double *x, double inv_mP, double *f,
-                                cudaStream_t st, const int4 *cols, int nc, float2 *S32, float2 *T32) {
+  float2 *S32 = (float2 *)r.S, *T32 = (float2 *)r.T;
   const size_t n = (size_t)g.P * 3 * g.Ns;
   // FP32 phases live behind the FP64 ones in the same buffer
   float2 *ph32 = (float2 *)(r.phase + recip_phase_doubles(g, r.nsum));

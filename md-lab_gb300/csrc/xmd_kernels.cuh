@@ -247,28 +247,28 @@ cudaError_t pair_energy_2(const Geo &ga, const Geo &gb, const PairPrm &p, const 
 // only because it is a cube (at alpha L = 5.6, nsum = 10 the kept ones are
 // the 52% inside |n|^2 <= 111).
 constexpr double RECIP_KEEP = 1e-17;
-// The FP64 forces (recip_force with fp32_outer) take the columns whose
-// every vector has a force weight below RECIP_SPLIT of the largest through
-// the FP32 kernels (at alpha L = 5.6 the columns with nx^2 + ny^2 >= 49: 45%
-// of the vectors); their FP32 rounding of a few 1e-7 then leaves below
-// 1e-13 of the reciprocal force.
-constexpr double RECIP_SPLIT = 1e-7;
+// The FP64 form's double-float kernels (xmd_recip_df.cu) sum the vectors
+// with a force weight of at least RECIP_DF_SPLIT of the largest in
+// double-float and the smaller ones in FP32, whose rounding of a few 1e-7
+// then leaves below 1e-14 of the reciprocal force (at alpha L = 5.6 the
+// line lies at |n|^2 = 52, 30% of the kept vectors inside).
+constexpr double RECIP_DF_SPLIT = 1e-8;
 struct Recip {
   int nsum;
   int nk;              // half-space wave vectors of the cube
   int ncol;            // kept columns (set by recip_setup)
   int tsz;             // entries of the kept columns' force tables (compact, set by recip_setup)
-  int ncol_in, ncol_out;  // of those, the FP64 and the FP32 columns of the split (set by recip_setup)
-  int tsz_in;          // entries of the FP64 columns' compact force tables (set by recip_setup)
-  double *S32;         // [P][nk] FP32 complex structure factors of the split's FP32 columns, or NULL
+  int df_items, items; // structure-factor items of the double-float kernels: with double-float harmonics, all
+  int tdf;             // float4 entries of their compact force tables (all three set by recip_setup)
   double *coef;        // [nk] s * exp(-pi^2 G^2/alpha^2) / (pi V G^2), 0 for a dropped vector;
                        // then the same nk values in FP32 (recip_coef_bytes(nk) bytes in all)
   int *kvec;           // kept columns, longest first: int4 (nx | nzmax << 8, ny, first nz,
-                       // offset of its first k), then compact table offsets;
-                       // recip_cols_ints(nsum) ints
-  double *phase;       // [P][3][nsum+1][Ns] complex
-  double *S;           // [P][nk] complex
-  double *T;           // [P][columns][2 nsum + 1] complex force tables
+                       // offset of its first k), then compact table offsets, then
+                       // from recip_df_off(nsum) the double-float kernels' columns,
+                       // table offsets and items; recip_cols_ints(nsum) ints
+  double *phase;       // [P][3][nsum+1][Ns] complex (FP64, or four floats a number)
+  double *S;           // [P][nk] complex, likewise
+  double *T;           // [P][columns][2 nsum + 1] complex force tables, likewise
   double csum;         // sum of coef (host value, set by recip_setup)
 };
 size_t recip_phase_doubles(const Geo &g, int nsum);
@@ -278,18 +278,30 @@ size_t recip_cols_ints(int nsum);
 size_t recip_table_doubles(const Geo &g, int nsum);
 cudaError_t recip_setup(const Geo &g, int nsum, double alpha, double qs, Recip &r,
                         cudaStream_t st);
-// fp32_outer (with r.S32 set): the split columns through the FP32 kernels
+// df: through the double-float kernels
 cudaError_t recip_force(const Geo &g, const Recip &r, const double *x, double inv_mP,
-                        double *f, cudaStream_t st, bool fp32_outer = false);
+                        double *f, cudaStream_t st, bool df = false);
 cudaError_t recip_energy(const Geo &g, const Recip &r, const double *x, double *acc,
-                         double *scratch, cudaStream_t st);
+                         double *scratch, cudaStream_t st, bool df = false);
+// the double-float kernels (xmd_recip_df.cu): their host tables (from the
+// kept columns, nx | nzmax << 8 in x, and the vectors' force weights),
+// phases and structure factors, tables, forces from tables, slice energies
+size_t recip_df_off(int nsum);
+size_t recip_df_ints(int nsum);
+void recip_df_tables(int nsum, const std::vector<int4> &kept, const std::vector<double> &wgt, double wmax, Recip &r,
+                     std::vector<int> &out);
+cudaError_t recip_df_sk(const Geo &g, const Recip &r, const double *x, cudaStream_t st);
+cudaError_t recip_df_tables_of(const Geo &g, const Recip &r, cudaStream_t st);
+cudaError_t recip_df_force_from(const Geo &g, const Recip &r, const double *T, double scale, double *f,
+                                cudaStream_t st);
+cudaError_t recip_df_energy(const Geo &g, const Recip &r, double *part, cudaStream_t st);
 
 // two species (same P, box and Ewald parameters): a's forces from b's
 // structure factors and b's from a's (both Recip's phase, S and T are
 // rewritten); the cross energy sum_j sum_{n in H} 2 c(n) Re(S_a S_b*) / P
 cudaError_t recip_force_2(const Geo &ga, const Recip &ra, const double *xa, double inv_mPa, double *fa,
                           const Geo &gb, const Recip &rb, const double *xb, double inv_mPb, double *fb,
-                          cudaStream_t st);
+                          cudaStream_t st, bool df = false);
 cudaError_t recip_energy_2(const Geo &ga, const Recip &ra, const double *xa, const Geo &gb, const Recip &rb,
                            const double *xb, double *acc, double *scratch, cudaStream_t st);
 

@@ -395,21 +395,18 @@ int xmd::ewald_tables(md_pimd_t_x *pimd, SimDev *sd, PimdDev *pd) {
   XMD_TRY(reserve(pd->rc_cols, sizeof(int) * xk::recip_cols_ints(ns)));
   // FP64 phases, then their FP32 copy for the mixed form
   XMD_TRY(reserve(pd->rc_phase, sizeof(double) * xk::recip_phase_doubles(g, ns) * 3 / 2));
-  // FP64 structure factors, then the FP32 ones of the FP64 form's split
-  XMD_TRY(reserve(pd->rc_S, sizeof(double) * 3 * (size_t)nk * g.P));
+  XMD_TRY(reserve(pd->rc_S, sizeof(double) * 2 * (size_t)nk * g.P));
   XMD_TRY(reserve(pd->rc_T, sizeof(double) * xk::recip_table_doubles(g, ns)));
   xk::Recip r{};
   r.coef = pd->rc_coef.as<double>();
   r.kvec = pd->rc_cols.as<int>();
   r.S = pd->rc_S.as<double>();
-  r.S32 = r.S + 2 * (size_t)nk * g.P;
   XMD_CUDA(xk::recip_setup(g, ns, a, qs, r, stream()));
   pd->rc_ncol = r.ncol;
   pd->rc_tsz = r.tsz;
-  pd->rc_ncol_in = r.ncol_in;
-  pd->rc_ncol_out = r.ncol_out;
-  pd->rc_tsz_in = r.tsz_in;
-  pd->rc_s32_off = 2 * (size_t)nk * g.P;
+  pd->rc_df_items = r.df_items;
+  pd->rc_items = r.items;
+  pd->rc_tdf = r.tdf;
   pd->rc_nsum = ns;
   pd->rc_alpha = a;
   pd->rc_qs = qs;
@@ -429,10 +426,9 @@ xk::Recip xmd::recip_of(PimdDev *pd) {
   r.nk = pd->rc_nk;
   r.ncol = pd->rc_ncol;
   r.tsz = pd->rc_tsz;
-  r.ncol_in = pd->rc_ncol_in;
-  r.ncol_out = pd->rc_ncol_out;
-  r.tsz_in = pd->rc_tsz_in;
-  r.S32 = pd->rc_S.as<double>() + pd->rc_s32_off;
+  r.df_items = pd->rc_df_items;
+  r.items = pd->rc_items;
+  r.tdf = pd->rc_tdf;
   r.coef = pd->rc_coef.as<double>();
   r.kvec = pd->rc_cols.as<int>();
   r.phase = pd->rc_phase.as<double>();
@@ -565,7 +561,8 @@ int md_pimd_calc_pair_force_2_x(md_pimd_t_x *pimd, md_pimd_t_x *pimd2, md_pair_f
       return fail(MD_GB_ERR_UNSUPPORTED, "structure-factor Ewald needs equal bead masses within each species");
     XMD_CUDA(xk::recip_force_2(sa->geo, recip_of(pa), sa->x.as<double>(), 1.0 / (sa->mass0 * pimd->P),
                                sa->f.as<double>(), sb->geo, recip_of(pb), sb->x.as<double>(),
-                               1.0 / (sb->mass0 * pimd2->P), sb->f.as<double>(), st));
+                               1.0 / (sb->mass0 * pimd2->P), sb->f.as<double>(), st,
+                               g_precision != MD_GB_PRECISION_FP64_STRICT));
   }
   XMD_CUDA(xk::pair_force_2(sa->geo, sb->geo, prm, sa->x.as<double>(), sa->m.as<double>(), sb->x.as<double>(),
                             sb->m.as<double>(), sa->f.as<double>(), sb->f.as<double>(), scr, st,
@@ -1062,7 +1059,8 @@ int md_pimd_calc_pair_energy_x(md_pimd_t_x *pimd, md_pair_energy_t_x pe, md_stat
     if (learned_mode(pimd, false) == 1) {
       XMD_TRY(learned_recip_energy(pimd, sd, acc, scr));
     } else {
-      XMD_CUDA(xk::recip_energy(sd->geo, recip_of(pd), sd->x.as<double>(), acc, scr, st));
+      XMD_CUDA(xk::recip_energy(sd->geo, recip_of(pd), sd->x.as<double>(), acc, scr, st,
+                                g_precision != MD_GB_PRECISION_FP64_STRICT));
     }
   }
   xk::PairPrm prm = pair_params(kind);

@@ -106,3 +106,19 @@ def test_close_pair_keeps_its_relative_accuracy(lib):
         assert np.abs(f[0, :, 0] * 2 * sep * sep - 1.0).max() < 1e-12
     finally:
         s.free()
+
+
+@pytest.mark.parametrize("N,P,nsum", [(2, 2, 1), (7, 3, 4), (64, 2, 6), (65, 5, 11), (300, 2, 9)])
+def test_reciprocal_sums_alone(lib, N, P, nsum):
+    """a large alpha L makes the real-space part vanish beside the reciprocal one; every wave vector of the cube is
+    kept then, most of them double-float"""
+    box = (6.0, 6.5, 7.0)
+    xmd_x.set_potentials(lib, coul_s=1.0, alpha=9.0 / 6.0, nsum=nsum)
+    s = _system(lib, N, P, box, 3 * N + P, 1.7)
+    try:
+        f, f0 = _forces(lib, [s], 0), _forces(lib, [s], 2)
+        assert np.abs(f - f0).max() <= TOL_F * np.abs(f0).max()
+        e, e0 = _energy(lib, s, 0), _energy(lib, s, 2)
+        assert abs(e - e0) <= TOL_E * (abs(e0) + N * N / 2 / 6.0)
+    finally:
+        s.free()
