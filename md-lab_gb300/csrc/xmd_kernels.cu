@@ -2608,6 +2608,11 @@ cudaError_t recip_setup(const Geo &g, int ns, double alpha, double qs, Recip &r,
   std::vector<float> coef32(coef.begin(), coef.end());
   e = cudaMemcpyAsync(r.coef + nk, coef32.data(), sizeof(float) * nk, cudaMemcpyHostToDevice, st);
   if (e != cudaSuccess) return e;
+  // and as FP32 pairs for the double-float ones
+  std::vector<float2> pairs(nk);
+  for (int k = 0; k < nk; ++k) pairs[k] = make_float2(coef32[k], (float)(coef[k] - (double)coef32[k]));
+  e = cudaMemcpyAsync(r.coef + recip_coef_pairs_at(nk), pairs.data(), sizeof(float2) * nk, cudaMemcpyHostToDevice, st);
+  if (e != cudaSuccess) return e;
   if (!cd.empty()) {
     e = cudaMemcpyAsync(r.kvec, cd.data(), sizeof(int4) * cd.size(), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return e;

@@ -261,7 +261,7 @@ struct Recip {
   int df_items, items; // structure-factor items of the double-float kernels: with double-float harmonics, all
   int tdf;             // float4 entries of their compact force tables (all three set by recip_setup)
   double *coef;        // [nk] s * exp(-pi^2 G^2/alpha^2) / (pi V G^2), 0 for a dropped vector;
-                       // then the same nk values in FP32 (recip_coef_bytes(nk) bytes in all)
+                       // then the same nk values in FP32 and as FP32 pairs (recip_coef_bytes(nk) in all)
   int *kvec;           // kept columns, longest first: int4 (nx | nzmax << 8, ny, first nz,
                        // offset of its first k), then compact table offsets, then
                        // from recip_df_off(nsum) the double-float kernels' columns,
@@ -272,7 +272,9 @@ struct Recip {
   double csum;         // sum of coef (host value, set by recip_setup)
 };
 size_t recip_phase_doubles(const Geo &g, int nsum);
-inline size_t recip_coef_bytes(int nk) { return (sizeof(double) + sizeof(float)) * (size_t)nk; }
+inline size_t recip_coef_pairs_at(int nk) { return nk + ((size_t)nk + 1) / 2; }  // in doubles
+inline size_t recip_coef_bytes(int nk) { return sizeof(double) * (recip_coef_pairs_at(nk) + nk); }
+inline const float2 *recip_coef_pairs(const Recip &r) { return (const float2 *)(r.coef + recip_coef_pairs_at(r.nk)); }
 int recip_count(int nsum);
 size_t recip_cols_ints(int nsum);
 size_t recip_table_doubles(const Geo &g, int nsum);

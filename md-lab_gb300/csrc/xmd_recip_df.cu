@@ -59,7 +59,7 @@ __host__ __device__ inline int dc_nx(int4 c) { return c.x & 255; }
 __host__ __device__ inline int dc_nz(int4 c) { return (c.x >> 8) & 255; }
 __host__ __device__ inline int dc_nzs(int4 c) { return (c.x >> 16) - 1; }
 
-constexpr int DF_NG = 4;  // harmonics of one structure-factor item
+constexpr int DF_NG = 8;  // harmonics of one structure-factor item
 
 // ints of the double-float tables: columns, table offsets, items
 static int ncols_of(int ns) { return ns * (2 * ns + 1) + ns + 1; }
@@ -138,89 +138,117 @@ __global__ void __launch_bounds__(128) k_df_phase(Geo g, int ns, const double *_
   }
 }
 
-// Structure factors: GR threads share an item (column and DF_NG harmonics)
-// of a slice, particles interleaved; phases staged DF_CH particles at a
-// time.  With P = sum e_xy cos(nz theta_z), Q = sum e_xy sin(nz theta_z):
-// S(+nz) = P + iQ, S(-nz) = P - iQ.  The FP32 items add their products in
-// FP32 over 16 particles and those sums in double-float.
-// Bound: FP32 issue of the double-float items (about 230 instructions a
-// particle and item).
+// Structure factors: DF_GR threads share an item (column and DF_NG harmonics)
+// of a slice, particles interleaved; phases staged DF_CH particles at a time,
+// the next chunk copied asynchronously while one is summed.  With
+// P = sum e_xy cos(nz theta_z), Q = sum e_xy sin(nz theta_z):
+// S(+nz) = P + iQ, S(-nz) = P - iQ.  FP32 harmonics add their products in
+// FP32, 8 particles at a time, into the accumulator's low part, which then
+// joins the high part exactly.
+// Bound: FP32 issue of the double-float harmonics (48 instructions a
+// particle and pair, 60 for e_xy).  Eight harmonics an item and not four:
+// inside the sphere a column has at most seven, so e_xy is formed once a
+// column, and no group is padded (142 -> 83 us at 512 x 64 with the
+// asynchronous copies).  Blocks of the double-float items, the longest, start
+// first.
 constexpr int DF_CH = 64, DF_SK_T = 512, DF_GR = 8;
+
+__device__ __forceinline__ void copy16(float4 *dst, const float4 *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
 template <int NS>
 __global__ void __launch_bounds__(DF_SK_T, 1)
     k_df_sk(int N, int Ns, const float4 *__restrict__ ph, const int4 *__restrict__ cols, const int *__restrict__ items,
             int ndf, int nitems, float4 *__restrict__ S, int nk) {
-  constexpr int LD = DF_CH + 1;
-  extern __shared__ __align__(16) float4 df_sp[];  // [3][NS + 1][LD]
-  const int j = blockIdx.y, gq = threadIdx.x % DF_GR;
-  const int it = blockIdx.x * (DF_SK_T / DF_GR) + threadIdx.x / DF_GR;
-  const bool live = it < nitems, isdf = it < ndf;
+  constexpr int LD = DF_CH + 1, STAGE = 3 * (NS + 1) * LD, NG = NS < DF_NG ? NS : DF_NG;
+  extern __shared__ __align__(16) float4 df_sp[];  // two stages of [3][NS + 1][LD]
+  const int j = blockIdx.x, gq = threadIdx.x % DF_GR;
+  const int it = blockIdx.y * (DF_SK_T / DF_GR) + threadIdx.x / DF_GR;
+  const bool live = it < nitems;
   const int item = live ? items[it] : 0;
   const int4 c = cols[item & 0xffff];
-  const int n0 = (item >> 16) * DF_NG, nzmax = live ? dc_nz(c) : 0;
-  const float4 *px = df_sp + dc_nx(c) * LD, *py = df_sp + (NS + 1 + abs(c.y)) * LD, *pz = df_sp + 2 * (NS + 1) * LD;
+  const int n0 = (item >> 16) * DF_NG;
+  const int top = live ? min(dc_nz(c) - n0, NG) : 0;           // harmonics of this item
+  const int nd = live && it < ndf ? max(dc_nzs(c) - n0, 0) : -1;  // of those, double-float (-1: e_xy in FP32 too)
+  const int ox = dc_nx(c) * LD, oy = (NS + 1 + abs(c.y)) * LD, oz = (2 * (NS + 1) + n0 + 1) * LD;
   const float sy = c.y < 0 ? -1.f : 1.f;
-  df s0r = {0.f, 0.f}, s0i = {0.f, 0.f}, Pr[DF_NG], Pi[DF_NG], Qr[DF_NG], Qi[DF_NG];
+  df s0r = {0.f, 0.f}, s0i = {0.f, 0.f}, Pr[NG], Pi[NG], Qr[NG], Qi[NG];
 #pragma unroll
-  for (int u = 0; u < DF_NG; ++u) Pr[u] = Pi[u] = Qr[u] = Qi[u] = {0.f, 0.f};
+  for (int u = 0; u < NG; ++u) Pr[u] = Pi[u] = Qr[u] = Qi[u] = {0.f, 0.f};
   const float4 *base = ph + (size_t)j * 3 * (NS + 1) * Ns;
-  for (int l0 = 0; l0 < N; l0 += DF_CH) {
-    const int cnt = N - l0 < DF_CH ? N - l0 : DF_CH;
-    __syncthreads();
+  const int chunks = (N + DF_CH - 1) / DF_CH;
+  auto stage = [&](int k) {
+    float4 *to = df_sp + (k & 1) * STAGE;
+    const int l0 = k * DF_CH, cnt = min(N - l0, DF_CH);
     for (int q = threadIdx.x; q < 3 * (NS + 1) * DF_CH; q += DF_SK_T) {
       const int l = q % DF_CH, row = q / DF_CH;
-      if (l < cnt) df_sp[row * LD + l] = base[(size_t)row * Ns + l0 + l];
+      if (l < cnt) copy16(to + row * LD + l, base + (size_t)row * Ns + l0 + l);
     }
-    __syncthreads();
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  stage(0);
+  for (int k = 0; k < chunks; ++k) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // chunk k is there, and nobody reads the other stage any more
+    if (k + 1 < chunks) stage(k + 1);
     if (!live) continue;
-    if (isdf) {
+    const float4 *sp = df_sp + (k & 1) * STAGE;
+    const int cnt = min(N - k * DF_CH, DF_CH);
+    if (nd >= 0) {
       for (int l = gq; l < cnt; l += DF_GR) {
-        const dfc ex = unpack(px[l]);
-        dfc ey = unpack(py[l]);
+        const dfc ex = unpack(sp[ox + l]);
+        dfc ey = unpack(sp[oy + l]);
         ey.i.h *= sy, ey.i.l *= sy;
         const dfc e = mul(ex, ey);
         s0r = df_add(s0r, e.r);
         s0i = df_add(s0i, e.i);
 #pragma unroll
-        for (int u = 0; u < DF_NG; ++u) {
-          if (n0 + u + 1 > nzmax) break;
-          const dfc ez = unpack(pz[(n0 + u + 1) * LD + l]);
-          fma_to(Pr[u], e.r, ez.r);
-          fma_to(Pi[u], e.i, ez.r);
-          fma_to(Qr[u], e.r, ez.i);
-          fma_to(Qi[u], e.i, ez.i);
+        for (int u = 0; u < NG; ++u) {
+          if (u >= top) break;
+          const float4 v = sp[oz + u * LD + l];
+          if (u < nd) {
+            const dfc ez = unpack(v);
+            fma_to(Pr[u], e.r, ez.r);
+            fma_to(Pi[u], e.i, ez.r);
+            fma_to(Qr[u], e.r, ez.i);
+            fma_to(Qi[u], e.i, ez.i);
+          } else {
+            Pr[u].l = fmaf(e.r.h, v.x, Pr[u].l);
+            Pi[u].l = fmaf(e.i.h, v.x, Pi[u].l);
+            Qr[u].l = fmaf(e.r.h, v.y, Qr[u].l);
+            Qi[u].l = fmaf(e.i.h, v.y, Qi[u].l);
+          }
         }
       }
     } else {
-      // at most DF_CH / DF_GR = 8 terms a chunk, in FP32
-      float a0 = 0.f, a1 = 0.f, p[DF_NG][4];
-#pragma unroll
-      for (int u = 0; u < DF_NG; ++u) p[u][0] = p[u][1] = p[u][2] = p[u][3] = 0.f;
       for (int l = gq; l < cnt; l += DF_GR) {
-        const float4 ex = px[l], ey = py[l];
+        const float4 ex = sp[ox + l], ey = sp[oy + l];
         const float yi = sy * ey.y;
         const float er = fmaf(ex.x, ey.x, -ex.y * yi), ei = fmaf(ex.x, yi, ex.y * ey.x);
-        a0 += er;
-        a1 += ei;
+        s0r.l += er;
+        s0i.l += ei;
 #pragma unroll
-        for (int u = 0; u < DF_NG; ++u) {
-          if (n0 + u + 1 > nzmax) break;
-          const float4 ez = pz[(n0 + u + 1) * LD + l];
-          p[u][0] = fmaf(er, ez.x, p[u][0]);
-          p[u][1] = fmaf(ei, ez.x, p[u][1]);
-          p[u][2] = fmaf(er, ez.y, p[u][2]);
-          p[u][3] = fmaf(ei, ez.y, p[u][3]);
+        for (int u = 0; u < NG; ++u) {
+          if (u >= top) break;
+          const float4 v = sp[oz + u * LD + l];
+          Pr[u].l = fmaf(er, v.x, Pr[u].l);
+          Pi[u].l = fmaf(ei, v.x, Pi[u].l);
+          Qr[u].l = fmaf(er, v.y, Qr[u].l);
+          Qi[u].l = fmaf(ei, v.y, Qi[u].l);
         }
       }
-      s0r = df_add(s0r, {a0, 0.f});
-      s0i = df_add(s0i, {a1, 0.f});
+      s0r = two_sum(s0r.h, s0r.l);
+      s0i = two_sum(s0i.h, s0i.l);
+    }
 #pragma unroll
-      for (int u = 0; u < DF_NG; ++u) {
-        Pr[u] = df_add(Pr[u], {p[u][0], 0.f});
-        Pi[u] = df_add(Pi[u], {p[u][1], 0.f});
-        Qr[u] = df_add(Qr[u], {p[u][2], 0.f});
-        Qi[u] = df_add(Qi[u], {p[u][3], 0.f});
-      }
+    for (int u = 0; u < NG; ++u) {
+      if (u >= top) break;
+      if (u < nd) continue;
+      Pr[u] = two_sum(Pr[u].h, Pr[u].l);
+      Pi[u] = two_sum(Pi[u].h, Pi[u].l);
+      Qr[u] = two_sum(Qr[u].h, Qr[u].l);
+      Qi[u] = two_sum(Qi[u].h, Qi[u].l);
     }
   }
 #pragma unroll
@@ -228,7 +256,7 @@ __global__ void __launch_bounds__(DF_SK_T, 1)
     s0r = df_add(s0r, shfl_xor(ALL, s0r, o));
     s0i = df_add(s0i, shfl_xor(ALL, s0i, o));
 #pragma unroll
-    for (int u = 0; u < DF_NG; ++u) {
+    for (int u = 0; u < NG; ++u) {
       Pr[u] = df_add(Pr[u], shfl_xor(ALL, Pr[u], o));
       Pi[u] = df_add(Pi[u], shfl_xor(ALL, Pi[u], o));
       Qr[u] = df_add(Qr[u], shfl_xor(ALL, Qr[u], o));
@@ -239,95 +267,91 @@ __global__ void __launch_bounds__(DF_SK_T, 1)
   float4 *o = S + (size_t)j * nk + c.w - c.z;  // o[nz]
   if (n0 == 0 && c.z <= 0) o[0] = pack(s0r, s0i);
 #pragma unroll
-  for (int u = 0; u < DF_NG; ++u) {
+  for (int u = 0; u < NG; ++u) {
+    if (u >= top) break;
     const int n = n0 + u + 1;
-    if (n > nzmax) break;
     o[n] = pack(df_sub(Pr[u], Qi[u]), df_add(Pi[u], Qr[u]));
     if (c.z < 0) o[-n] = pack(df_add(Pr[u], Qi[u]), df_sub(Pi[u], Qr[u]));
   }
 }
 
-__device__ __forceinline__ float4 pack64(double r, double i) {
-  const float rh = (float)r, ih = (float)i;
-  return make_float4(rh, ih, (float)(r - rh), (float)(i - ih));
-}
-
 // Force tables of a slice, compact: per column W(0), then A, B, n A, n B (as
 // in k_recip_tables) per double-float harmonic, then (A, B) in FP32 per
-// remaining one.
+// remaining one.  coef: c(n) as FP32 pairs.
 template <int NS>
-__global__ void k_df_tables(const int4 *__restrict__ cols, const int *__restrict__ toff, int ncol,
-                            const float4 *__restrict__ S, const double *__restrict__ coef, int nk, int tdf,
-                            float4 *__restrict__ T) {
+__global__ void __launch_bounds__(8 * (NS + 1))
+    k_df_tables(const int4 *__restrict__ cols, const int *__restrict__ toff, int ncol, const float4 *__restrict__ S,
+                const float2 *__restrict__ coef, int nk, int tdf, float4 *__restrict__ T) {
   const int j = blockIdx.y, ci = blockIdx.x * blockDim.y + threadIdx.y, n = threadIdx.x;
   if (ci >= ncol) return;
   const int4 c = cols[ci];
   if (n > dc_nz(c)) return;
-  auto W = [&](int nz) {
-    if (nz < c.z) return make_double2(0.0, 0.0);
+  auto W = [&](int nz) -> dfc {  // c(n) conj(S(n))
+    if (nz < c.z) return {{0.f, 0.f}, {0.f, 0.f}};
     const int k = c.w + (nz - c.z);
-    const float4 s = S[(size_t)j * nk + k];
-    return make_double2(coef[k] * ((double)s.x + s.z), -coef[k] * ((double)s.y + s.w));
+    const float2 ck = coef[k];
+    const dfc s = unpack(S[(size_t)j * nk + k]);
+    return {df_mul({ck.x, ck.y}, s.r), df_mul({-ck.x, -ck.y}, s.i)};
   };
   float4 *o = T + (size_t)j * tdf + toff[ci];
-  const int nzs = dc_nzs(c) > 0 ? dc_nzs(c) : 0;
+  const int nzs = max(dc_nzs(c), 0);
   if (n == 0) {
-    const double2 w = W(0);
-    o[0] = pack64(w.x, w.y);
+    const dfc w = W(0);
+    o[0] = pack(w.r, w.i);
     return;
   }
-  const double2 wp = W(n), wm = W(-n);
-  const double2 A = make_double2(wp.x + wm.x, wp.y + wm.y), B = make_double2(wp.x - wm.x, wp.y - wm.y);
+  const dfc wp = W(n), wm = W(-n);
+  const df Ar = df_add(wp.r, wm.r), Ai = df_add(wp.i, wm.i), Br = df_sub(wp.r, wm.r), Bi = df_sub(wp.i, wm.i);
   if (n <= nzs) {
-    o[4 * n - 3] = pack64(A.x, A.y);
-    o[4 * n - 2] = pack64(B.x, B.y);
-    o[4 * n - 1] = pack64(n * A.x, n * A.y);
-    o[4 * n] = pack64(n * B.x, n * B.y);
+    const float m = (float)n;
+    o[4 * n - 3] = pack(Ar, Ai);
+    o[4 * n - 2] = pack(Br, Bi);
+    o[4 * n - 1] = pack(times(m, Ar), times(m, Ai));
+    o[4 * n] = pack(times(m, Br), times(m, Bi));
   } else {
-    o[4 * nzs + (n - nzs)] = make_float4((float)A.x, (float)A.y, (float)B.x, (float)B.y);
+    o[4 * nzs + (n - nzs)] = make_float4(Ar.h + Ar.l, Ai.h + Ai.l, Br.h + Br.l, Bi.h + Bi.l);
   }
 }
 
-// Forces: TPP threads share a particle, thread h taking columns h, h + TPP,
-// ... (sorted by length, so that neighbours run alike); tables, columns and
-// the block's x and y phase factors in shared memory, the z factors in
-// registers.  Per column, with U = sum_nz e_z W and V = sum_nz nz e_z W:
-// F_x, F_y from Im(e_xy U), F_z from Im(e_xy V).
+// Forces: a block of W warps has 32 particles of a slice, one a lane; warp w
+// takes columns w, w + W, ..., so that its lanes run alike and read each
+// table entry at one address, and the warps' sums meet in shared memory
+// (4 or 16 lanes a particle, each on its own column, waited for their
+// scattered table reads: 126 -> 98 us at 512 x 64, 29 -> 18 us at 128 x 32).
+// Tables, columns and the particles' x and y phase factors are staged, the z
+// factors in registers.  Per column, with U = sum_nz e_z W and
+// V = sum_nz nz e_z W: F_x, F_y from Im(e_xy U), F_z from Im(e_xy V).
 // Bound: FP32 issue (eight double-float multiply-adds a harmonic, 96
 // instructions).
-constexpr int DF_RF_T = 256;
-template <int NS, int TPP>
-__global__ void __launch_bounds__(DF_RF_T, 2)
+template <int NS, int NW>
+__global__ void __launch_bounds__(32 * NW, 16 / NW)
     k_df_force(Geo g, const float4 *__restrict__ ph, const int4 *__restrict__ cols, const int *__restrict__ toff,
                int ncol, const float4 *__restrict__ T, int tdf, double scale, double *__restrict__ f) {
-  constexpr int PPB = DF_RF_T / TPP;
   extern __shared__ __align__(16) float4 df_sm[];
-  float4 *sT = df_sm, *pxy = df_sm + tdf;                // [tdf], [2 (NS + 1)][PPB]
-  int4 *sc = (int4 *)(pxy + 2 * (NS + 1) * PPB);         // [ncol]
-  int *so = (int *)(sc + ncol);                          // [ncol]
-  const int j = blockIdx.y, l0 = blockIdx.x * PPB;
+  float4 *sT = df_sm, *pxy = df_sm + tdf;        // [tdf], [2 (NS + 1)][32]
+  int4 *sc = (int4 *)(pxy + 2 * (NS + 1) * 32);  // [ncol]
+  int *so = (int *)(sc + ncol);                  // [ncol]
+  const int j = blockIdx.y, l0 = blockIdx.x * 32, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const float4 *Tj = T + (size_t)j * tdf, *pj = ph + (size_t)j * 3 * (NS + 1) * g.Ns;
-  for (int q = threadIdx.x; q < tdf; q += DF_RF_T) sT[q] = Tj[q];
-  for (int q = threadIdx.x; q < ncol; q += DF_RF_T) sc[q] = cols[q], so[q] = toff[q];
-  for (int q = threadIdx.x; q < 2 * (NS + 1) * PPB; q += DF_RF_T) {
-    const int r = q / PPB, l = l0 + q % PPB;
-    if (l < g.N) pxy[q] = pj[(size_t)r * g.Ns + l];
-  }
-  __syncthreads();
-  const int li = threadIdx.x / TPP, h = threadIdx.x % TPP, l = l0 + li;
-  if (l >= g.N) return;  // a particle's TPP lanes leave together
+  const int l = min(l0 + lane, g.N - 1);  // (lanes past the end repeat the last particle)
+  for (int q = threadIdx.x; q < tdf; q += 32 * NW) copy16(sT + q, Tj + q);
+  for (int r = w; r < 2 * (NS + 1); r += NW) copy16(pxy + r * 32 + lane, pj + (size_t)r * g.Ns + l);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int q = threadIdx.x; q < ncol; q += 32 * NW) sc[q] = cols[q], so[q] = toff[q];
   dfc ez[NS];
 #pragma unroll
   for (int n = 1; n <= NS; ++n) ez[n - 1] = unpack(pj[((size_t)2 * (NS + 1) + n) * g.Ns + l]);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
   df F[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) F[d] = {0.f, 0.f};
-  for (int ci = h; ci < ncol; ci += TPP) {
+  for (int ci = w; ci < ncol; ci += NW) {
     const int4 c = sc[ci];
     const int nzs = dc_nzs(c), nzc = dc_nz(c);
     const float4 *t = sT + so[ci];
-    const float4 vx = pxy[dc_nx(c) * PPB + li];
-    float4 vy = pxy[(NS + 1 + abs(c.y)) * PPB + li];
+    const float4 vx = pxy[dc_nx(c) * 32 + lane];
+    float4 vy = pxy[(NS + 1 + abs(c.y)) * 32 + lane];
     if (c.y < 0) vy.y = -vy.y, vy.w = -vy.w;
     const float4 w0 = t[0];
     // the FP32 harmonics
@@ -378,14 +402,20 @@ __global__ void __launch_bounds__(DF_RF_T, 2)
     fma_to(F[2], e.r, Vi);
     fma_to(F[2], e.i, Vr);
   }
-  const unsigned gm = TPP >= 32 ? ALL : ((1u << TPP) - 1u) << ((threadIdx.x & 31) & ~(TPP - 1));
+  // the warps' sums, in order (the tables are no longer read)
+  __syncthreads();
+  float2 *sum = (float2 *)df_sm;  // [NW][3][32]
 #pragma unroll
-  for (int o = 1; o < TPP; o <<= 1)
-#pragma unroll
-    for (int d = 0; d < 3; ++d) F[d] = df_add(F[d], shfl_xor(gm, F[d], o));
-  if (h != 0) return;
-#pragma unroll
-  for (int d = 0; d < 3; ++d) f[sidx(j, d, l, 3, g.Ns)] += scale * df_value(F[d]) * g.inv_box[d];
+  for (int d = 0; d < 3; ++d) sum[(w * 3 + d) * 32 + lane] = make_float2(F[d].h, F[d].l);
+  __syncthreads();
+  if (w >= 3 || l0 + lane >= g.N) return;
+  df t = {0.f, 0.f};
+  for (int v = 0; v < NW; ++v) {
+    const float2 p = sum[(v * 3 + w) * 32 + lane];
+    t = df_add(t, {p.x, p.y});
+  }
+  const double ib = w == 0 ? g.inv_box[0] : (w == 1 ? g.inv_box[1] : g.inv_box[2]);
+  f[sidx(j, w, l, 3, g.Ns)] += scale * df_value(t) * ib;
 }
 
 // slice energies sum_n c(n) (|S|^2 - N), and the cross form 2 c(n) Re(S_a S_b*)
@@ -433,7 +463,7 @@ static const int *df_toff(const Recip &r) { return df_base(r) + toff_at(r.nsum);
 
 template <int NS>
 constexpr size_t sk_smem() {
-  return sizeof(float4) * 3 * (NS + 1) * (DF_CH + 1);
+  return 2 * sizeof(float4) * 3 * (NS + 1) * (DF_CH + 1);
 }
 
 cudaError_t recip_df_sk(const Geo &g, const Recip &r, const double *x, cudaStream_t st) {
@@ -444,7 +474,7 @@ cudaError_t recip_df_sk(const Geo &g, const Recip &r, const double *x, cudaStrea
   cudaError_t e = XK_LAUNCHED();
   if (e != cudaSuccess || r.items <= 0) return e;
   XK_PROF("sk");
-  const dim3 grid(cdivz(r.items, DF_SK_T / DF_GR), g.P);
+  const dim3 grid(g.P, cdivz(r.items, DF_SK_T / DF_GR));
   DF_NS(r.nsum, {
     static bool opted = false;
     if (!opted) {
@@ -463,24 +493,24 @@ cudaError_t recip_df_tables_of(const Geo &g, const Recip &r, cudaStream_t st) {
   if (r.items <= 0) return cudaSuccess;
   XK_PROF("recip_tables");
   const dim3 grid((r.ncol + 7) / 8, g.P), blk(r.nsum + 1, 8);
-  DF_NS(r.nsum, (k_df_tables<NS><<<grid, blk, 0, st>>>(df_cols(r), df_toff(r), r.ncol, (const float4 *)r.S, r.coef,
-                                                       r.nk, r.tdf, (float4 *)r.T)));
+  DF_NS(r.nsum, (k_df_tables<NS><<<grid, blk, 0, st>>>(df_cols(r), df_toff(r), r.ncol, (const float4 *)r.S,
+                                                       recip_coef_pairs(r), r.nk, r.tdf, (float4 *)r.T)));
   return XK_LAUNCHED();
 }
 
-template <int NS, int TPP>
+template <int NS, int NW>
 static cudaError_t launch_force(const Geo &g, const Recip &r, const double *T, double scale, double *f,
                                 cudaStream_t st) {
   static bool opted = false;
   if (!opted) {
     const cudaError_t e =
-        cudaFuncSetAttribute(k_df_force<NS, TPP>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+        cudaFuncSetAttribute(k_df_force<NS, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
     opted = true;
   }
-  constexpr int PPB = DF_RF_T / TPP;
-  const size_t smem = sizeof(float4) * (r.tdf + 2 * (NS + 1) * PPB) + (sizeof(int4) + sizeof(int)) * r.ncol;
-  k_df_force<NS, TPP><<<dim3((g.N + PPB - 1) / PPB, g.P), DF_RF_T, smem, st>>>(
+  size_t smem = sizeof(float4) * (r.tdf + 2 * (NS + 1) * 32) + (sizeof(int4) + sizeof(int)) * r.ncol;
+  smem = std::max(smem, sizeof(float2) * 3 * 32 * NW);
+  k_df_force<NS, NW><<<dim3((g.N + 31) / 32, g.P), 32 * NW, smem, st>>>(
       g, (const float4 *)r.phase, df_cols(r), df_toff(r), r.ncol, (const float4 *)T, r.tdf, scale, f);
   return XK_LAUNCHED();
 }
@@ -490,10 +520,10 @@ cudaError_t recip_df_force_from(const Geo &g, const Recip &r, const double *T, d
                                 cudaStream_t st) {
   if (r.items <= 0) return cudaSuccess;
   XK_PROF("recip_force");
-  // threads a particle: 4 once that fills the SMs with 16 warps each, else 16
-  const bool big = (size_t)g.N * g.P * 4 >= (size_t)152 * 512;
+  // 16 warps a block when blocks of 8 would not give every SM two
+  const bool few = (size_t)((g.N + 31) / 32) * g.P < 2 * 152;
   DF_NS(r.nsum, {
-    return big ? launch_force<NS, 4>(g, r, T, scale, f, st) : launch_force<NS, 16>(g, r, T, scale, f, st);
+    return few ? launch_force<NS, 16>(g, r, T, scale, f, st) : launch_force<NS, 8>(g, r, T, scale, f, st);
   });
   return cudaSuccess;
 }
