@@ -528,9 +528,60 @@ __device__ inline void ext_warp_sum(bool nz, double pm, int pe, double &sum, int
   E = Em;
 }
 
-// B_c column s for every chunk c: grid (chunks x 4 column groups, directions),
-// 8 warps per block, warp w of group g takes column s = 8 g + w.  Lane t
-// holds B[t][s]; step r adds row r: B[r][s] = sum_{s<=t<r} A[r][t] B[t][s].
+// ---- extended range on the integer pipe --------------------------------
+// A non-negative number m 2^(e-62) with a 62-bit integer mantissa (2^61 <= m
+// < 2^62, or m = 0 with e = XI_NONE): nine bits more than a double's, and no
+// FP64 instruction, which on GB300 holds its pipe for 64 cycles a warp.  The
+// unsigned solves and the diagonal blocks' inverses work on these; every
+// truncation is below 2^-60 of the value.
+struct XI {
+  long long m;
+  int e;
+};
+constexpr int XI_NONE = -(1 << 29);
+
+// v 2^e of a non-negative double v
+__device__ __forceinline__ XI xi_from(double v, int e) {
+  const long long b = __double_as_longlong(v);
+  const int ex = (int)(b >> 52);
+  XI r{((b & 0xFFFFFFFFFFFFFLL) | (1LL << 52)) << 9, e + ex - 1022};
+  if (ex == 0) r = {0, XI_NONE};
+  return r;
+}
+// a mantissa in [0.5, 1) and its power of two (zero: 0 and 0)
+__device__ __forceinline__ void xi_split(XI a, double &m, int &e) {
+  m = __longlong_as_double(a.m == 0 ? 0LL : (((a.m >> 9) & 0xFFFFFFFFFFFFFLL) | (1022LL << 52)));
+  e = a.m == 0 ? 0 : a.e;
+}
+__device__ __forceinline__ XI xi_mul(XI a, XI b) {
+  XI r{(long long)__umul64hi((unsigned long long)a.m << 2, (unsigned long long)b.m), a.e + b.e};
+  if (r.m < (1LL << 61)) r.m <<= 1, r.e -= 1;
+  return r;
+}
+__device__ __forceinline__ XI xi_add(XI a, XI b) {
+  XI r;
+  r.e = a.e > b.e ? a.e : b.e;
+  r.m = (a.m >> min(r.e - a.e, 63)) + (b.m >> min(r.e - b.e, 63));
+  if (r.m >= (1LL << 62)) r.m >>= 1, r.e += 1;
+  return r;
+}
+__device__ __forceinline__ XI xi_shfl(XI a, int src) {
+  return {__shfl_sync(FULL, a.m, src), __shfl_sync(FULL, a.e, src)};
+}
+// the warp's sum in every lane: aligned to the largest exponent with 57 bits,
+// in three 19-bit parts (a warp-wide integer reduction is one instruction)
+__device__ __forceinline__ XI xi_warp_sum(XI a) {
+  const int em = __reduce_max_sync(FULL, a.e);
+  const long long q = (a.m >> min(em - a.e, 63)) >> 5;
+  const unsigned p0 = __reduce_add_sync(FULL, (unsigned)q & 0x7ffffu);
+  const unsigned p1 = __reduce_add_sync(FULL, (unsigned)(q >> 19) & 0x7ffffu);
+  const unsigned p2 = __reduce_add_sync(FULL, (unsigned)(q >> 38));
+  const long long t = (long long)p0 + ((long long)p1 << 19) + ((long long)p2 << 38);
+  if (t == 0) return {0, XI_NONE};
+  const int sh = __clzll(t) - 2;
+  return {t << sh, em + 5 - sh};
+}
+
 // weight M_{i,j} of direction dir (0 forward, 1 backward) from ENk, the same
 // expression k_weights evaluates (so the same number)
 __device__ inline Ext weight_at(int N, double beta, double vi, double lnvi, const double *__restrict__ ENk,
@@ -542,31 +593,23 @@ __device__ inline Ext weight_at(int N, double beta, double vi, double lnvi, cons
 }
 
 // Column s of B(c) for direction dir, one warp; the chunk's block
-// A[r][t] = M_{i0+r, i0+t} (t < r) is staged in Am/Ae.
+// A[r][t] = M_{i0+r, i0+t} (t < r) is staged in Am/Ae as XI (zero elsewhere).
+// Lane r holds row r; step t takes the finished B[t][s] to the later rows:
+// one shuffle and one integer multiply-add a step, where a sum over the lanes
+// for each row took ten shuffles and FP64 products.
 __device__ inline void block_inv_column(int N, const TriJob &job, int dir, int c, int s,
-                                        const double (*Am)[TS_LD], const int (*Ae)[TS_LD]) {
+                                        const long long (*Am)[TS_LD], const int (*Ae)[TS_LD]) {
   const int lane = threadIdx.x & 31;
-  const int i0 = 1 + c * TS_CHUNK;
-  double bm = lane == s ? 0.5 : 0.0;  // B[s][s] = 1 = 0.5 * 2^1
-  int be = lane == s ? 1 : 0;
-  for (int r = s + 1; r < TS_CHUNK && i0 + r <= N; ++r) {
-    const bool in = lane >= s && lane < r;
-    const double am = in ? Am[r][lane] : 0.0;
-    const int ae = in ? Ae[r][lane] : 0;
-    const bool nz = in && __double_as_longlong(am) != 0 && __double_as_longlong(bm) != 0;
-    double sm;
-    int se;
-    ext_warp_sum(nz, am * bm, ae + be, sm, se);
-    if (lane == r) {
-      bm = se == EXT_NONE ? 0.0 : sm;
-      be = se == EXT_NONE ? 0 : se;
-      norm2(bm, be);
-    }
+  const int rows = min(TS_CHUNK, N - c * TS_CHUNK);
+  XI b = lane == s ? XI{1LL << 61, 1} : XI{0, XI_NONE};  // B[s][s] = 1
+  for (int t = s; t + 1 < rows; ++t) {
+    const XI x = xi_shfl(b, t);
+    if (lane > t) b = xi_add(b, xi_mul({Am[lane][t], Ae[lane][t]}, x));
   }
-  double *Bm = job.Bm[dir] + (size_t)c * TS_CHUNK * TS_CHUNK;
+  long long *Bm = (long long *)job.Bm[dir] + (size_t)c * TS_CHUNK * TS_CHUNK;
   int *Be = job.Be[dir] + (size_t)c * TS_CHUNK * TS_CHUNK;
-  Bm[lane * TS_CHUNK + s] = lane >= s ? bm : 0.0;
-  Be[lane * TS_CHUNK + s] = lane >= s ? be : 0;
+  Bm[lane * TS_CHUNK + s] = b.m;
+  Be[lane * TS_CHUNK + s] = b.e;
 }
 
 // m 2^e for 0 <= m < 4 (a product of normalised mantissas) and e <= 1021:
@@ -787,6 +830,37 @@ __device__ inline float2 cmulf(float2 a, float2 b) {
 // each) and outputs VBN / tmpV (host)
 TriJob tri_job(int N, double *rs_f, double *rs_b, double *VBN, double *tmpV);
 
+// out[] and the kept unknowns of a solve from X_0..X_N in shared memory, by
+// the calling block
+__device__ inline void tri_solve_out(int N, double beta, const TriJob &job, int backward, const long long *Xm,
+                                     const int *Xe) {
+  double *__restrict__ out = job.out[backward];
+  for (int i = threadIdx.x; i <= N; i += blockDim.x) {
+    double m;
+    int e;
+    xi_split({Xm[i], Xe[i]}, m, e);
+    if (i > 0) {
+      const double lnx = log(m) + e * LN2_HI + e * LN2_LO;
+      out[backward ? N - i : i] = -lnx / beta;
+    } else {
+      out[backward ? N : 0] = 0.0;
+    }
+    if (job.Xm[backward]) {
+      job.Xm[backward][i] = m;
+      job.Xe[backward][i] = e;
+    }
+  }
+}
+
+// row i's sum over the unknowns 0 <= j < j1, by the warp
+__device__ inline XI xi_dot(const double *__restrict__ Mm, const int *__restrict__ Me, const long long *Xm,
+                            const int *Xe, int i, int j1, int lane) {
+  XI a{0, XI_NONE};
+  for (int j = lane; j < j1; j += 32)
+    a = xi_add(a, xi_mul(xi_from(Mm[moff(i, j)], Me[moff(i, j)]), {Xm[j], Xe[j]}));
+  return xi_warp_sum(a);
+}
+
 // The block solve of direction `backward` by the calling thread block (any
 // whole number of warps; rows of a chunk go round-robin over the warps, each
 // row's sums inside one warp, so the result does not depend on the count).
@@ -794,14 +868,13 @@ TriJob tri_job(int N, double *rs_f, double *rs_b, double *VBN, double *tmpV);
 __device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, int backward, double *sh) {
   const double *__restrict__ Mm = job.Mm[backward];
   const int *__restrict__ Me = job.Me[backward];
-  const double *__restrict__ Bgm = job.Bm[backward];
+  const long long *__restrict__ Bgm = (const long long *)job.Bm[backward];
   const int *__restrict__ Bge = job.Be[backward];
-  double *__restrict__ out = job.out[backward];
-  double *Um = sh;                          // [TS_CHUNK][TS_LD] next chunk vs the chunk before it
-  double *Bsm = Um + TS_CHUNK * TS_LD;      // [TS_CHUNK][TS_LD] the chunk's B block
-  double *Pm = Bsm + TS_CHUNK * TS_LD;      // [TS_CHUNK] sums over the unknowns before the previous chunk
-  double *Rm = Pm + TS_CHUNK;               // [TS_CHUNK] right-hand sides of the chunk
-  double *Xm = Rm + TS_CHUNK;               // N+1
+  long long *Um = (long long *)sh;          // [TS_CHUNK][TS_LD] next chunk vs the chunk before it
+  long long *Bsm = Um + TS_CHUNK * TS_LD;   // [TS_CHUNK][TS_LD] the chunk's B block
+  long long *Pm = Bsm + TS_CHUNK * TS_LD;   // [TS_CHUNK] sums over the unknowns before the previous chunk
+  long long *Rm = Pm + TS_CHUNK;            // [TS_CHUNK] right-hand sides of the chunk
+  long long *Xm = Rm + TS_CHUNK;            // N+1
   int *Ue = (int *)(Xm + N + 1);            // [TS_CHUNK][TS_LD]
   int *Bse = Ue + TS_CHUNK * TS_LD;         // [TS_CHUNK][TS_LD]
   int *Pe = Bse + TS_CHUNK * TS_LD;         // [TS_CHUNK]
@@ -811,115 +884,69 @@ __device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, in
   // stage chunk n0's B block and its rows' weights against columns c0..c0+31
   auto stage = [&](int n0, int c0) {
     const int cc = (n0 - 1) / TS_CHUNK;
-    for (int q = threadIdx.x; q < 2 * TS_CHUNK * TS_CHUNK; q += blockDim.x) {
-      const int which = q / (TS_CHUNK * TS_CHUNK), rs = q % (TS_CHUNK * TS_CHUNK);
-      const int r = rs / TS_CHUNK, k = rs % TS_CHUNK, i = n0 + r;
-      const size_t o = (size_t)r * TS_LD + k;
-      if (which == 0) {
-        const bool in = i <= N && c0 >= 0;
-        Um[o] = in ? Mm[moff(i, c0 + k)] : 0.0;
-        Ue[o] = in ? Me[moff(i, c0 + k)] : 0;
-      } else {
-        Bsm[o] = i <= N ? Bgm[(size_t)cc * TS_CHUNK * TS_CHUNK + rs] : 0.0;
-        Bse[o] = i <= N ? Bge[(size_t)cc * TS_CHUNK * TS_CHUNK + rs] : 0;
-      }
+    for (int q = threadIdx.x; q < TS_CHUNK * TS_CHUNK; q += blockDim.x) {
+      const int r = q / TS_CHUNK, k = q % TS_CHUNK, i = n0 + r, o = r * TS_LD + k;
+      const bool in = i <= N;
+      const XI u = in && c0 >= 0 ? xi_from(Mm[moff(i, c0 + k)], Me[moff(i, c0 + k)]) : XI{0, XI_NONE};
+      Um[o] = u.m;
+      Ue[o] = u.e;
+      Bsm[o] = in ? Bgm[(size_t)cc * TS_CHUNK * TS_CHUNK + q] : 0;
+      Bse[o] = in ? Bge[(size_t)cc * TS_CHUNK * TS_CHUNK + q] : XI_NONE;
     }
   };
   if (threadIdx.x == 0) {
-    Xm[0] = 0.5;
+    Xm[0] = 1LL << 61;  // X_0 = 1
     Xe[0] = 1;
   }
   stage(1, -1);
-  __syncthreads();
-  // chunk 0: its rows against column 0 (X_0 = 1)
-  for (int r = w; r < TS_CHUNK; r += nw) {
-    const int i = 1 + r;
-    double am = 0.0;
-    int E = 0;
-    if (i <= N) ext_dot(Mm + moff(i, 0), Me + moff(i, 0), Xm, Xe, 0, 1, lane, am, E);
-    if (lane == 0) {
-      double pm = 0.0;
-      int pe = 0;
-      if (i <= N) ext_acc(pm, pe, am, E);
-      Pm[r] = pm;
-      Pe[r] = pe;
-    }
+  // chunk 0: its rows against column 0
+  for (int r = threadIdx.x; r < TS_CHUNK; r += blockDim.x) {
+    const XI p = 1 + r <= N ? xi_from(Mm[moff(1 + r, 0)], Me[moff(1 + r, 0)]) : XI{0, XI_NONE};
+    Pm[r] = p.m;
+    Pe[r] = p.e;
   }
   __syncthreads();
   for (int i0 = 1, c = 0; i0 <= N; i0 += TS_CHUNK, ++c) {
     // U: right-hand sides
     for (int r = w; r < TS_CHUNK; r += nw) {
-      if (i0 + r > N) continue;  // warp-uniform
-      double pm = Pm[r];
-      int pe = Pe[r];
+      XI p{Pm[r], Pe[r]};
       if (c > 0) {
-        const int col = i0 - TS_CHUNK + lane;
-        const size_t o = (size_t)r * TS_LD + lane;
-        const double mv = Um[o];
-        const bool nz = __double_as_longlong(mv) != 0 && __double_as_longlong(Xm[col]) != 0;
-        double sm;
-        int se;
-        ext_warp_sum(nz, mv * Xm[col], Ue[o] + Xe[col], sm, se);
-        if (lane == 0 && se != EXT_NONE) ext_acc(pm, pe, sm, se);
+        const int col = i0 - TS_CHUNK + lane, o = r * TS_LD + lane;
+        p = xi_add(p, xi_warp_sum(xi_mul({Um[o], Ue[o]}, {Xm[col], Xe[col]})));
       }
       if (lane == 0) {
-        norm2(pm, pe);
-        Rm[r] = pm;
-        Re[r] = pe;
+        Rm[r] = p.m;
+        Re[r] = p.e;
       }
     }
     __syncthreads();
     // B: the chunk's unknowns
     for (int r = w; r < TS_CHUNK; r += nw) {
-      const int i = i0 + r;
-      if (i > N) continue;  // warp-uniform
-      const size_t o = (size_t)r * TS_LD + lane;
-      const double bv = Bsm[o], rv = Rm[lane];
-      const bool nz = lane <= r && __double_as_longlong(bv) != 0 && __double_as_longlong(rv) != 0;
-      double sm;
-      int se;
-      ext_warp_sum(nz, bv * rv, Bse[o] + Re[lane], sm, se);
+      const int i = i0 + r, o = r * TS_LD + lane;
+      if (i > N) break;  // warp-uniform
+      const XI x = xi_warp_sum(xi_mul({Bsm[o], Bse[o]}, {Rm[lane], Re[lane]}));
       if (lane == 0) {
-        double xm = se == EXT_NONE ? 0.0 : sm;
-        int xe = se == EXT_NONE ? 0 : se;
-        norm2(xm, xe);
-        Xm[i] = xm;
-        Xe[i] = xe;
+        Xm[i] = x.m;
+        Xe[i] = x.e;
       }
     }
     __syncthreads();
     // next chunk: its weights against this chunk, its B block, and its rows'
     // sums over the unknowns before this chunk
     const int n0 = i0 + TS_CHUNK;
-    if (n0 <= N) {
-      stage(n0, i0);
-      for (int r = w; r < TS_CHUNK; r += nw) {
-        const int i = n0 + r;
-        if (i > N) break;  // warp-uniform; later rows are out of range too
-        double am;
-        int E;
-        ext_dot(Mm + moff(i, 0), Me + moff(i, 0), Xm, Xe, 0, i0, lane, am, E);
-        if (lane == 0) {
-          double pm = 0.0;
-          int pe = 0;
-          ext_acc(pm, pe, am, E);
-          Pm[r] = pm;
-          Pe[r] = pe;
-        }
+    if (n0 > N) break;
+    stage(n0, i0);
+    for (int r = w; r < TS_CHUNK; r += nw) {
+      const int i = n0 + r;
+      const XI p = i <= N ? xi_dot(Mm, Me, Xm, Xe, i, i0, lane) : XI{0, XI_NONE};
+      if (lane == 0) {
+        Pm[r] = p.m;
+        Pe[r] = p.e;
       }
     }
     __syncthreads();
   }
-  for (int i = threadIdx.x + 1; i <= N; i += blockDim.x) {
-    const double lnx = log(fabs(Xm[i])) + Xe[i] * LN2_HI + Xe[i] * LN2_LO;
-    out[backward ? N - i : i] = -lnx / beta;
-  }
-  if (threadIdx.x == 0) out[backward ? N : 0] = 0.0;
-  if (job.Xm[backward])
-    for (int i = threadIdx.x; i <= N; i += blockDim.x) {
-      job.Xm[backward][i] = Xm[i];
-      job.Xe[backward][i] = Xe[i];
-    }
+  tri_solve_out(N, beta, job, backward, Xm, Xe);
 }
 
 

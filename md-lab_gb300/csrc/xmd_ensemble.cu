@@ -442,8 +442,8 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
     }
   }
   {
-    double(*Am)[TS_LD] = (double(*)[TS_LD])ens_sh;
-    int(*Ae)[TS_LD] = (int(*)[TS_LD])(ens_sh + sizeof(double) * TS_CHUNK * TS_LD);
+    long long(*Am)[TS_LD] = (long long(*)[TS_LD])ens_sh;
+    int(*Ae)[TS_LD] = (int(*)[TS_LD])(ens_sh + sizeof(long long) * TS_CHUNK * TS_LD);
     for (int i = i0; i < i1; ++i) {
       const EnsSys &E = sys[i];
       const EnsSysDesc &d = E.d;
@@ -455,8 +455,9 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
           const int r = e / TS_CHUNK, t = e % TS_CHUNK;
           Ext wv{0.0, 0};
           if (t < r && i0 + r <= N) wv = weight_at(N, d.beta, d.vi, E.lnvi, d.ENk, d.lnn, dir, i0 + r, i0 + t);
-          Am[r][t] = wv.m;
-          Ae[r][t] = wv.e;
+          const XI q = xi_from(wv.m, wv.e);
+          Am[r][t] = q.m;
+          Ae[r][t] = q.e;
         }
         __syncthreads();
         for (int sc = w; sc < TS_CHUNK; sc += ENS_W) block_inv_column(N, E.job, dir, c, sc, Am, Ae);

@@ -879,7 +879,7 @@ __global__ void __launch_bounds__(128) k_weights_inv(int N, double beta, double 
                                                      const double *__restrict__ ENk,
                                                      const double *__restrict__ lnn, TriJob job, int first,
                                                      int both, int nblk) {
-  __shared__ double Am[TS_CHUNK][TS_LD];
+  __shared__ long long Am[TS_CHUNK][TS_LD];
   __shared__ int Ae[TS_CHUNK][TS_LD];
   if ((int)blockIdx.x < N) {
     weights_row(N, beta, vi, lnvi, ENk, lnn, (double *)job.Mm[0], (int *)job.Me[0], (double *)job.Mm[1],
@@ -895,8 +895,9 @@ __global__ void __launch_bounds__(128) k_weights_inv(int N, double beta, double 
     const int r = e / TS_CHUNK, t = e % TS_CHUNK;
     Ext w{0.0, 0};
     if (t < r && t >= s0 && i0 + r <= N) w = weight_at(N, beta, vi, lnvi, ENk, lnn, dir, i0 + r, i0 + t);
-    Am[r][t] = w.m;
-    Ae[r][t] = w.e;
+    const XI q = xi_from(w.m, w.e);
+    Am[r][t] = q.m;
+    Ae[r][t] = q.e;
   }
   __syncthreads();
   block_inv_column(N, job, dir, c, s, Am, Ae);
@@ -922,17 +923,24 @@ __global__ void __launch_bounds__(TSB_WARPS * 32) k_tri_solve_b(int N, double be
 // over everything before, (B) X = B R.  The other blocks own the later rows'
 // running sums (chunk k >= 1 belongs to block 1 + (k-1) mod (TSC_CL-1)): in
 // iteration c each adds chunk c-1's unknowns, which block 0 wrote into its
-// shared memory, to the rows of its chunks after c, and the owner of chunk
-// c+1 writes that chunk's completed sums into block 0's shared memory.  So
-// the long sums, which held most of the FP64 work and the L2 loads, run on
-// seven more SMs beside block 0's solve, one cluster barrier per chunk, and
-// block 0 loads only the next chunk's two 32 x 32 blocks (issued before the
-// chunk's solve, stored after it).
+// shared memory, to the rows of its chunks after c, one column a lane, and
+// the owner of chunk c+1 adds up those rows' lanes and writes the completed
+// sums into block 0's shared memory.  So the long sums run on seven more SMs
+// beside block 0's solve, one cluster barrier per chunk; every block loads
+// its next weights before that barrier.
+// Bound: the chain of N/32 chunks, two warp sums and a cluster barrier each.
+// All sums are on the integer pipe (XI): with FP64 products and a warp sum per
+// row and chunk the FP64 pipes of the summing blocks set the pace.
 constexpr int TSC_CL = 8;      // blocks per cluster (the portable cluster size)
 constexpr int TSC_WARPS = 16;  // warps per block; warp w takes rows w and w + 16 of a chunk
-constexpr int TSC_HB = 4;      // rows a summing warp loads before it reduces them
+constexpr int TSC_HB = 8;      // rows whose weights a summing warp loads ahead
 
-__device__ inline int tsc_slots(int nch) { return (nch - 1 + TSC_CL - 2) / (TSC_CL - 1); }
+__host__ __device__ inline int tsc_slots(int nch) { return (nch - 1 + TSC_CL - 2) / (TSC_CL - 1); }
+static size_t tsc_smem(int N) {
+  const size_t b0 = N + 1 + 3 * TS_CHUNK + 4 * TS_CHUNK * TS_LD;
+  const size_t h = 2 * TS_CHUNK + (size_t)tsc_slots((N + TS_CHUNK - 1) / TS_CHUNK) * TS_CHUNK * 32;
+  return (sizeof(long long) + sizeof(int)) * (b0 > h ? b0 : h) + 16;
+}
 
 __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
     k_tri_solve_c(int N, double beta, TriJob job, int first) {
@@ -942,7 +950,7 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
   const int backward = first + blockIdx.y;
   const double *__restrict__ Mm = job.Mm[backward];
   const int *__restrict__ Me = job.Me[backward];
-  const double *__restrict__ Bgm = job.Bm[backward];
+  const long long *__restrict__ Bgm = (const long long *)job.Bm[backward];
   const int *__restrict__ Bge = job.Be[backward];
   const int nch = (N + TS_CHUNK - 1) / TS_CHUNK;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -950,54 +958,66 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
   constexpr int CC = TS_CHUNK * TS_CHUNK;
   extern __shared__ double sh[];
   // block 0
-  double *Um = sh;                 // [2][TS_CHUNK][TS_LD] a chunk's weights against the chunk before it
-  double *Bsm = Um + 2 * BLK;      // [2][TS_CHUNK][TS_LD] a chunk's B block
-  double *Pm = Bsm + 2 * BLK;      // [2][TS_CHUNK] rows' sums over the unknowns before the previous chunk
-  double *Rm = Pm + 2 * TS_CHUNK;  // [TS_CHUNK] right-hand sides of the chunk being solved
-  double *Xm = Rm + TS_CHUNK;      // N+1
-  int *Ue = (int *)(Xm + N + 1);   // [2][TS_CHUNK][TS_LD]
-  int *Bse = Ue + 2 * BLK;         // [2][TS_CHUNK][TS_LD]
-  int *Pe = Bse + 2 * BLK;         // [2][TS_CHUNK]
-  int *Re = Pe + 2 * TS_CHUNK;     // [TS_CHUNK]
-  int *Xe = Re + TS_CHUNK;         // N+1
+  long long *Um = (long long *)sh;     // [2][TS_CHUNK][TS_LD] a chunk's weights against the chunk before it
+  long long *Bsm = Um + 2 * BLK;       // [2][TS_CHUNK][TS_LD] a chunk's B block
+  long long *Pm = Bsm + 2 * BLK;       // [2][TS_CHUNK] rows' sums over the unknowns before the previous chunk
+  long long *Rm = Pm + 2 * TS_CHUNK;   // [TS_CHUNK] right-hand sides of the chunk being solved
+  long long *Xm = Rm + TS_CHUNK;       // N+1
+  int *Ue = (int *)(Xm + N + 1);       // [2][TS_CHUNK][TS_LD]
+  int *Bse = Ue + 2 * BLK;             // [2][TS_CHUNK][TS_LD]
+  int *Pe = Bse + 2 * BLK;             // [2][TS_CHUNK]
+  int *Re = Pe + 2 * TS_CHUNK;         // [TS_CHUNK]
+  int *Xe = Re + TS_CHUNK;             // N+1
   // blocks 1..TSC_CL-1
   const int slots = tsc_slots(nch);
-  double *Hxm = sh;                  // [2][TS_CHUNK] the last solved chunk's unknowns
-  double *Hpm = Hxm + 2 * TS_CHUNK;  // [slots][TS_CHUNK] running sums of the owned chunks' rows
-  int *Hxe = (int *)(Hpm + slots * TS_CHUNK);
-  int *Hpe = Hxe + 2 * TS_CHUNK;
+  long long *Hxm = (long long *)sh;            // [2][TS_CHUNK] the last solved chunk's unknowns
+  long long *Ham = Hxm + 2 * TS_CHUNK;         // [slots][TS_CHUNK][32] the owned chunks' rows, a partial sum a lane
+  int *Hxe = (int *)(Ham + slots * TS_CHUNK * 32);
+  int *Hae = Hxe + 2 * TS_CHUNK;
+  // summing blocks: rows q = 0, 1, ... of the chunks after c, two a slot from
+  // slot t0(c) on; their weights against the columns from j0 on
+  auto first_slot = [&](int c) { return c + 1 > rank ? (c + 1 - rank + TSC_CL - 2) / (TSC_CL - 1) : 0; };
+  auto row_of = [&](int t0, int q) {
+    const int k = rank + (t0 + q / 2) * (TSC_CL - 1);
+    return 1 + k * TS_CHUNK + w + (q & 1) * TSC_WARPS;
+  };
+  double mv[TSC_HB];
+  int me[TSC_HB];
+  auto load = [&](int t0, int qb, int j0) {
+#pragma unroll
+    for (int u = 0; u < TSC_HB; ++u) {
+      const int i = row_of(t0, qb + u);
+      const bool ok = qb + u < 2 * (slots - t0) && i <= N;
+      mv[u] = ok ? Mm[moff(i, j0 + lane)] : 0.0;
+      me[u] = ok ? Me[moff(i, j0 + lane)] : 0;
+    }
+  };
   if (rank == 0) {
     if (threadIdx.x == 0) {
-      Xm[0] = 0.5;
+      Xm[0] = 1LL << 61;  // X_0 = 1
       Xe[0] = 1;
     }
-    // chunk 0: no chunk before it; its rows' sums over column 0 (X_0 = 1)
+    // chunk 0: no chunk before it; its rows' sums over column 0
     for (int q = threadIdx.x; q < CC; q += blockDim.x) {
-      const int r = q / TS_CHUNK, k = q % TS_CHUNK;
-      const size_t o = (size_t)r * TS_LD + k;
+      const int r = q / TS_CHUNK, o = r * TS_LD + q % TS_CHUNK;
       const bool in = 1 + r <= N;
-      Um[o] = 0.0;
-      Ue[o] = 0;
-      Bsm[o] = in ? Bgm[q] : 0.0;
-      Bse[o] = in ? Bge[q] : 0;
+      Um[o] = 0;
+      Ue[o] = XI_NONE;
+      Bsm[o] = in ? Bgm[q] : 0;
+      Bse[o] = in ? Bge[q] : XI_NONE;
     }
     if (threadIdx.x < TS_CHUNK) {
       const int i = 1 + threadIdx.x;
-      double pm = i <= N ? Mm[moff(i, 0)] : 0.0;
-      int pe = i <= N ? Me[moff(i, 0)] : 0;
-      norm2(pm, pe);
-      Pm[threadIdx.x] = pm;
-      Pe[threadIdx.x] = pe;
+      const XI p = i <= N ? xi_from(Mm[moff(i, 0)], Me[moff(i, 0)]) : XI{0, XI_NONE};
+      Pm[threadIdx.x] = p.m;
+      Pe[threadIdx.x] = p.e;
     }
   } else {
-    for (int q = threadIdx.x; q < slots * TS_CHUNK; q += blockDim.x) {
-      const int k = rank + (q / TS_CHUNK) * (TSC_CL - 1), i = 1 + k * TS_CHUNK + q % TS_CHUNK;
-      const bool in = k < nch && i <= N;
-      double pm = in ? Mm[moff(i, 0)] : 0.0;
-      int pe = in ? Me[moff(i, 0)] : 0;
-      norm2(pm, pe);
-      Hpm[q] = pm;
-      Hpe[q] = pe;
+    for (int q = threadIdx.x; q < slots * TS_CHUNK * 32; q += blockDim.x) {
+      const int k = rank + (q / (TS_CHUNK * 32)) * (TSC_CL - 1), i = 1 + k * TS_CHUNK + q / 32 % TS_CHUNK;
+      const XI p = q % 32 == 0 && i <= N ? xi_from(Mm[moff(i, 0)], Me[moff(i, 0)]) : XI{0, XI_NONE};
+      Ham[q] = p.m;
+      Hae[q] = p.e;
     }
   }
   cl.sync();  // every block has started and holds its initial sums
@@ -1006,7 +1026,8 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
     if (rank == 0) {
       // chunk c+1's blocks: loads issued now, stored after this chunk's solve
       const int n0 = i0 + TS_CHUNK;
-      double su[2], sb[2];
+      double su[2];
+      long long sb[2];
       int seu[2], seb[2];
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
@@ -1015,125 +1036,86 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
         const bool in = c + 1 < nch && i <= N;
         su[t] = in ? Mm[moff(i, i0 + k)] : 0.0;
         seu[t] = in ? Me[moff(i, i0 + k)] : 0;
-        sb[t] = in ? Bgm[(size_t)(c + 1) * CC + rs] : 0.0;
-        seb[t] = in ? Bge[(size_t)(c + 1) * CC + rs] : 0;
+        sb[t] = in ? Bgm[(size_t)(c + 1) * CC + rs] : 0;
+        seb[t] = in ? Bge[(size_t)(c + 1) * CC + rs] : XI_NONE;
       }
       // U: right-hand sides
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int r = w + h * TSC_WARPS;
-        if (i0 + r > N) continue;  // warp-uniform
-        double pm = Pm[buf * TS_CHUNK + r];
-        int pe = Pe[buf * TS_CHUNK + r];
+        const int r = w + h * TSC_WARPS, o = buf * BLK + r * TS_LD + lane;
+        XI p{Pm[buf * TS_CHUNK + r], Pe[buf * TS_CHUNK + r]};
         if (c > 0) {
           const int col = i0 - TS_CHUNK + lane;
-          const size_t o = (size_t)buf * BLK + (size_t)r * TS_LD + lane;
-          const double mv = Um[o];
-          const bool nz = __double_as_longlong(mv) != 0 && __double_as_longlong(Xm[col]) != 0;
-          double sm;
-          int se;
-          ext_warp_sum(nz, mv * Xm[col], Ue[o] + Xe[col], sm, se);
-          if (lane == 0 && se != EXT_NONE) ext_acc(pm, pe, sm, se);
+          p = xi_add(p, xi_warp_sum(xi_mul({Um[o], Ue[o]}, {Xm[col], Xe[col]})));
         }
         if (lane == 0) {
-          norm2(pm, pe);
-          Rm[r] = pm;
-          Re[r] = pe;
+          Rm[r] = p.m;
+          Re[r] = p.e;
         }
       }
       __syncthreads();
       // B: the chunk's unknowns, also into every other block's shared memory
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int r = w + h * TSC_WARPS, i = i0 + r;
+        const int r = w + h * TSC_WARPS, i = i0 + r, o = buf * BLK + r * TS_LD + lane;
         if (i > N) continue;  // warp-uniform
-        const size_t o = (size_t)buf * BLK + (size_t)r * TS_LD + lane;
-        const double bv = Bsm[o], rv = Rm[lane];
-        const bool nz = lane <= r && __double_as_longlong(bv) != 0 && __double_as_longlong(rv) != 0;
-        double sm;
-        int se;
-        ext_warp_sum(nz, bv * rv, Bse[o] + Re[lane], sm, se);  // (sm, se) reach every lane
-        double xm = se == EXT_NONE ? 0.0 : sm;
-        int xe = se == EXT_NONE ? 0 : se;
-        norm2(xm, xe);
+        const XI x = xi_warp_sum(xi_mul({Bsm[o], Bse[o]}, {Rm[lane], Re[lane]}));
         if (lane == 0) {
-          Xm[i] = xm;
-          Xe[i] = xe;
+          Xm[i] = x.m;
+          Xe[i] = x.e;
         } else if (lane < TSC_CL) {
-          *cl.map_shared_rank(Hxm + buf * TS_CHUNK + r, lane) = xm;
-          *cl.map_shared_rank(Hxe + buf * TS_CHUNK + r, lane) = xe;
+          *cl.map_shared_rank(Hxm + buf * TS_CHUNK + r, lane) = x.m;
+          *cl.map_shared_rank(Hxe + buf * TS_CHUNK + r, lane) = x.e;
         }
       }
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         const int rs = threadIdx.x + t * TSC_WARPS * 32;
-        const size_t o = (size_t)(buf ^ 1) * BLK + (size_t)(rs / TS_CHUNK) * TS_LD + rs % TS_CHUNK;
-        Um[o] = su[t];
-        Ue[o] = seu[t];
+        const int o = (buf ^ 1) * BLK + rs / TS_CHUNK * TS_LD + rs % TS_CHUNK;
+        const XI u = xi_from(su[t], seu[t]);
+        Um[o] = u.m;
+        Ue[o] = u.e;
         Bsm[o] = sb[t];
         Bse[o] = seb[t];
       }
     } else {
       if (c >= 1) {
         // chunk c-1's unknowns into the rows of the owned chunks after c
-        const int j0 = i0 - TS_CHUNK, pb = (c - 1) & 1;
-        const double xv = Hxm[pb * TS_CHUNK + lane];
-        const int xe = Hxe[pb * TS_CHUNK + lane];
-        const int t0 = c + 1 > rank ? (c + 1 - rank + TSC_CL - 2) / (TSC_CL - 1) : 0;
-        const int nq = 2 * (slots - t0);
+        const int j0 = i0 - TS_CHUNK, pb = (c - 1) & 1, t0 = first_slot(c), nq = 2 * (slots - t0);
+        const XI x{Hxm[pb * TS_CHUNK + lane], Hxe[pb * TS_CHUNK + lane]};
         for (int qb = 0; qb < nq; qb += TSC_HB) {
-          double mv[TSC_HB];
-          int me[TSC_HB];
+          if (qb > 0) load(t0, qb, j0);
 #pragma unroll
           for (int u = 0; u < TSC_HB; ++u) {
-            const int q = qb + u, t = t0 + q / 2, k = rank + t * (TSC_CL - 1);
-            const int i = 1 + k * TS_CHUNK + w + (q & 1) * TSC_WARPS;
-            const bool ok = q < nq && k < nch && i <= N;
-            mv[u] = ok ? Mm[moff(i, j0 + lane)] : 0.0;
-            me[u] = ok ? Me[moff(i, j0 + lane)] : 0;
-          }
-#pragma unroll
-          for (int u = 0; u < TSC_HB; ++u) {
-            const int q = qb + u, t = t0 + q / 2, k = rank + t * (TSC_CL - 1);
-            const int r = w + (q & 1) * TSC_WARPS, i = 1 + k * TS_CHUNK + r;
-            if (!(q < nq && k < nch && i <= N)) continue;  // warp-uniform
-            const bool nz = __double_as_longlong(mv[u]) != 0 && __double_as_longlong(xv) != 0;
-            double sm;
-            int se;
-            ext_warp_sum(nz, mv[u] * xv, me[u] + xe, sm, se);
-            if (lane == 0 && se != EXT_NONE) ext_acc(Hpm[t * TS_CHUNK + r], Hpe[t * TS_CHUNK + r], sm, se);
+            const int q = qb + u;
+            if (q >= nq || row_of(t0, q) > N) break;  // warp-uniform
+            const int o = ((t0 + q / 2) * TS_CHUNK + w + (q & 1) * TSC_WARPS) * 32 + lane;
+            const XI a = xi_add({Ham[o], Hae[o]}, xi_mul(xi_from(mv[u], me[u]), x));
+            Ham[o] = a.m;
+            Hae[o] = a.e;
           }
         }
       }
       // the owner of chunk c+1 hands its rows' sums (now over the unknowns
       // before chunk c) to block 0
       const int kn = c + 1;
-      if (kn < nch && 1 + (kn - 1) % (TSC_CL - 1) == rank && lane == 0) {
+      if (kn < nch && 1 + (kn - 1) % (TSC_CL - 1) == rank) {
         const int t = (kn - 1) / (TSC_CL - 1);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int r = w + h * TSC_WARPS;
-          if (1 + kn * TS_CHUNK + r > N) continue;
-          *cl.map_shared_rank(Pm + (kn & 1) * TS_CHUNK + r, 0) = Hpm[t * TS_CHUNK + r];
-          *cl.map_shared_rank(Pe + (kn & 1) * TS_CHUNK + r, 0) = Hpe[t * TS_CHUNK + r];
+          const int r = w + h * TSC_WARPS, o = (t * TS_CHUNK + r) * 32 + lane;
+          const XI p = xi_warp_sum({Ham[o], Hae[o]});
+          if (lane == 0) {
+            *cl.map_shared_rank(Pm + (kn & 1) * TS_CHUNK + r, 0) = p.m;
+            *cl.map_shared_rank(Pe + (kn & 1) * TS_CHUNK + r, 0) = p.e;
+          }
         }
       }
+      if (c + 1 < nch) load(first_slot(c + 1), 0, i0);
     }
     cl.sync();
   }
-  if (rank == 0) {
-    double *__restrict__ out = job.out[backward];
-    for (int i = threadIdx.x + 1; i <= N; i += blockDim.x) {
-      const double lnx = log(fabs(Xm[i])) + Xe[i] * LN2_HI + Xe[i] * LN2_LO;
-      out[backward ? N - i : i] = -lnx / beta;
-    }
-    if (threadIdx.x == 0) out[backward ? N : 0] = 0.0;
-    if (job.Xm[backward])
-      for (int i = threadIdx.x; i <= N; i += blockDim.x) {
-        job.Xm[backward][i] = Xm[i];
-        job.Xe[backward][i] = Xe[i];
-      }
-  }
+  if (rank == 0) tri_solve_out(N, beta, job, backward, Xm, Xe);
 }
 
 // whether a cluster of the block solve fits on this device with `smem`
@@ -1195,7 +1177,7 @@ static cudaError_t tri_solve(int N, double beta, const TriJob &job, int first, i
   if (!job.sign) {
     // unsigned weights: the block solve (the diagonal-block inverses came
     // with the weights, k_weights_inv)
-    const size_t smem_c = (sizeof(double) + sizeof(int)) * (N + 1 + 3 * TS_CHUNK + 4 * TS_CHUNK * TS_LD) + 16;
+    const size_t smem_c = tsc_smem(N);
     const int path = solve_choice(N);
     if (path == SOLVE_CLUSTER && !cluster_solve_fits(smem_c) && g_solve_force == SOLVE_CLUSTER)
       return cudaErrorInvalidConfiguration;  // forced, but no cluster of this size fits
