@@ -94,28 +94,49 @@ __device__ inline void chain_forces(const ChainState<L> &c, double kin, double c
 }
 
 
+// exp(r) 2^62 for |r| < 1/2 on the integer pipe: the Taylor series through
+// r^13/13! by Horner's rule on 64-bit fixed-point numbers, the terms from r^8
+// on, 1 + r/9 (1 + r/10 (...)) times r^8/8!, with 32 bits (their rounding and
+// the first omitted term are below 1e-17 of the result for |r| <= 0.35, a
+// tenth of a double's half ulp).  About 110 integer instructions, where
+// thirteen FP64 multiply-adds hold the FP64 pipe for 830 cycles a warp.
+__device__ __forceinline__ long long exp_q62(double r) {
+  const long long b = __double_as_longlong(r);
+  const int sh = (int)((b >> 52) & 0x7ff) - 1011;  // |r| = sig 2^(sh - 64)
+  const long long sig = (b & 0xFFFFFFFFFFFFFLL) | (1LL << 52);
+  long long R = sh >= 0 ? sig << min(sh, 10) : sig >> min(-sh, 63);
+  R = b < 0 ? -R : R;  // r 2^64
+  const int r32 = (int)(R >> 32);
+  constexpr unsigned ONE = 1u << 30;
+  unsigned t = ONE + __mulhi(r32, (int)__umulhi(ONE, 330382099u));  // 2^32 / 13
+  t = ONE + __mulhi(r32, (int)__umulhi(t, 357913941u));             // 2^32 / 12
+  t = ONE + __mulhi(r32, (int)__umulhi(t, 390451572u));
+  t = ONE + __mulhi(r32, (int)__umulhi(t, 429496729u));
+  t = ONE + __mulhi(r32, (int)__umulhi(t, 477218588u));  // 2^32 / 9
+  constexpr unsigned long long C8 = 114377133393536ULL;  // 2^62 / 8!
+  long long p = (long long)__umul64hi(C8 << 16, (unsigned long long)t << 18);
+  p = 915017067148291LL + __mul64hi(R, p);  // 2^62 / 7!
+  p = 6405119470038039LL + __mul64hi(R, p);
+  p = 38430716820228233LL + __mul64hi(R, p);
+  p = 192153584101141163LL + __mul64hi(R, p);
+  p = 768614336404564651LL + __mul64hi(R, p);
+  p = (1LL << 61) + __mul64hi(R, p);
+  p = (1LL << 62) + __mul64hi(R, p);
+  return (1LL << 62) + __mul64hi(R, p);
+}
+// p 2^-62 rounded to a double, 2^60 <= p < 2^63
+__device__ __forceinline__ double q62_double(long long p) {
+  const int z = __clzll(p);  // 1..3
+  const unsigned long long m = ((unsigned long long)p << (z - 1)) + (1ULL << 9);  // half an ulp of bit 10 added
+  return __longlong_as_double((long long)((m >> 10) + ((unsigned long long)(1023 - z) << 52)));
+}
+
 // exp(x) for the thermostat factors exp(-h v_eta / 4) and exp(-h v_eta / 2):
-// for |x| < 1/4, the usual case with a small step, its Taylor series through
-// x^12/12! by Horner's rule (the first omitted term is below 3e-18
-// relative, a fortieth of the FP64 rounding unit: twelve FMAs instead of a
-// general exponential's range reduction and longer polynomial), otherwise
-// exp().  The range test reads the bit pattern, off the FP64 pipe.
+// on the integer pipe for |x| < 1/4, the usual case with a small step,
+// otherwise exp().  The range test reads the bit pattern, off the FP64 pipe.
 __device__ inline double nhc_exp(double x) {
-  if ((__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFLL) < 0x3FD0000000000000LL) {  // |x| < 2^-2
-    double p = 1.0 / 479001600.0;
-    p = fma(p, x, 1.0 / 39916800.0);
-    p = fma(p, x, 1.0 / 3628800.0);
-    p = fma(p, x, 1.0 / 362880.0);
-    p = fma(p, x, 1.0 / 40320.0);
-    p = fma(p, x, 1.0 / 5040.0);
-    p = fma(p, x, 1.0 / 720.0);
-    p = fma(p, x, 1.0 / 120.0);
-    p = fma(p, x, 1.0 / 24.0);
-    p = fma(p, x, 1.0 / 6.0);
-    p = fma(p, x, 0.5);
-    p = fma(p, x, 1.0);
-    return fma(p, x, 1.0);
-  }
+  if ((__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFLL) < 0x3FD0000000000000LL)  // |x| < 2^-2
+    return q62_double(exp_q62(x));
   return exp(x);
 }
 
@@ -259,28 +280,15 @@ struct Ext {
   int e;     // value = m * 2^e
 };
 
-// exp(x) in extended range for any finite x: 2^e * exp(r), |r| <= ln2/2
+// exp(x) in extended range for any finite x: 2^e exp(r), |r| <= ln2/2 (the
+// reduction in FP64, the exponential on the integer pipe)
 __device__ inline Ext ext_exp(double x) {
-  const double q = rint(x * LOG2E);
+  constexpr double MAGIC = 6755399441055744.0;  // 1.5 2^52: adding rounds to an integer, in the low word
+  const double tq = fma(x, LOG2E, MAGIC), q = tq - MAGIC;
   double r = fma(-q, LN2_HI, x);
   r = fma(-q, LN2_LO, r);
-  // exp(r) for |r| <= ln2/2 by its Taylor series through r^13/13! (Horner):
-  // the first omitted term is below 5e-18 relative; thirteen FMAs, where a
-  // general exponential would reduce the argument a second time
-  double p = 1.0 / 6227020800.0;
-  p = fma(p, r, 1.0 / 479001600.0);
-  p = fma(p, r, 1.0 / 39916800.0);
-  p = fma(p, r, 1.0 / 3628800.0);
-  p = fma(p, r, 1.0 / 362880.0);
-  p = fma(p, r, 1.0 / 40320.0);
-  p = fma(p, r, 1.0 / 5040.0);
-  p = fma(p, r, 1.0 / 720.0);
-  p = fma(p, r, 1.0 / 120.0);
-  p = fma(p, r, 1.0 / 24.0);
-  p = fma(p, r, 1.0 / 6.0);
-  p = fma(p, r, 0.5);
-  p = fma(p, r, 1.0);
-  return {fma(p, r, 1.0), (int)q};
+  const bool large = (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFLL) >= 0x41D0000000000000LL;  // |x| >= 2^30
+  return {q62_double(exp_q62(r)), large ? (int)q : __double2loint(tq)};
 }
 
 // exp(x) through ext_exp, the power of two put into the exponent field by
@@ -386,8 +394,13 @@ struct TriJob {
   const int *Me[2];
   double *out[2];
   double *sign;  // optional: sign of X_i (signed weights), forward direction only
-  double *Bm[2];  // inverses of the 32 x 32 diagonal blocks (unsigned weights):
-  int *Be[2];     // [chunk][32][32] mantissas and exponents
+  // unsigned weights, [chunk][32][32] XI mantissas and exponents each: the
+  // inverses B of the diagonal blocks, and W = B U with U the chunk's weights
+  // against the chunk before it
+  double *Bm[2];
+  int *Be[2];
+  double *Wm[2];
+  int *We[2];
   double *Xm[2];  // optional: the unknowns X_0..X_N in extended range (unsigned
   int *Xe[2];     // solves), kept for the connection probabilities
 };
@@ -592,24 +605,30 @@ __device__ inline Ext weight_at(int N, double beta, double vi, double lnvi, cons
   return w;
 }
 
-// Column s of B(c) for direction dir, one warp; the chunk's block
-// A[r][t] = M_{i0+r, i0+t} (t < r) is staged in Am/Ae as XI (zero elsewhere).
-// Lane r holds row r; step t takes the finished B[t][s] to the later rows:
-// one shuffle and one integer multiply-add a step, where a sum over the lanes
-// for each row took ten shuffles and FP64 products.
-__device__ inline void block_inv_column(int N, const TriJob &job, int dir, int c, int s,
-                                        const long long (*Am)[TS_LD], const int (*Ae)[TS_LD]) {
+// One column of B(c) = (I - A)^-1 or W(c) = (I - A)^-1 U for direction dir,
+// by a warp: the forward substitution from right-hand side b (lane r holds row
+// r; a unit vector, or U's column).  The chunk's block A[r][t] =
+// M_{i0+r, i0+t} (t < r) is staged in Am/Ae as XI (zero elsewhere).  Step t
+// takes the finished row t to the later rows: one shuffle and one integer
+// multiply-add a step, where a sum over the lanes for each row took ten
+// shuffles and FP64 products.
+__device__ __forceinline__ XI block_solve_column(XI b, int t0, int rows, const long long (*Am)[TS_LD],
+                                                 const int (*Ae)[TS_LD]) {
   const int lane = threadIdx.x & 31;
-  const int rows = min(TS_CHUNK, N - c * TS_CHUNK);
-  XI b = lane == s ? XI{1LL << 61, 1} : XI{0, XI_NONE};  // B[s][s] = 1
-  for (int t = s; t + 1 < rows; ++t) {
+  for (int t = t0; t + 1 < rows; ++t) {
     const XI x = xi_shfl(b, t);
     if (lane > t) b = xi_add(b, xi_mul({Am[lane][t], Ae[lane][t]}, x));
   }
-  long long *Bm = (long long *)job.Bm[dir] + (size_t)c * TS_CHUNK * TS_CHUNK;
-  int *Be = job.Be[dir] + (size_t)c * TS_CHUNK * TS_CHUNK;
-  Bm[lane * TS_CHUNK + s] = b.m;
-  Be[lane * TS_CHUNK + s] = b.e;
+  return b;
+}
+__device__ inline void block_inv_column(int N, const TriJob &job, int dir, int c, int s,
+                                        const long long (*Am)[TS_LD], const int (*Ae)[TS_LD]) {
+  const int lane = threadIdx.x & 31;
+  const XI b = block_solve_column(lane == s ? XI{1LL << 61, 1} : XI{0, XI_NONE}, s, min(TS_CHUNK, N - c * TS_CHUNK),
+                                  Am, Ae);
+  const size_t o = (size_t)c * TS_CHUNK * TS_CHUNK + lane * TS_CHUNK + s;
+  ((long long *)job.Bm[dir])[o] = b.m;
+  job.Be[dir][o] = b.e;
 }
 
 // m 2^e for 0 <= m < 4 (a product of normalised mantissas) and e <= 1021:
@@ -830,12 +849,11 @@ __device__ inline float2 cmulf(float2 a, float2 b) {
 // each) and outputs VBN / tmpV (host)
 TriJob tri_job(int N, double *rs_f, double *rs_b, double *VBN, double *tmpV);
 
-// out[] and the kept unknowns of a solve from X_0..X_N in shared memory, by
-// the calling block
+// out[] and the kept unknowns of a solve from X_0..X_N, entries i0, i0 + step, ...
 __device__ inline void tri_solve_out(int N, double beta, const TriJob &job, int backward, const long long *Xm,
-                                     const int *Xe) {
+                                     const int *Xe, int i0, int step) {
   double *__restrict__ out = job.out[backward];
-  for (int i = threadIdx.x; i <= N; i += blockDim.x) {
+  for (int i = i0; i <= N; i += step) {
     double m;
     int e;
     xi_split({Xm[i], Xe[i]}, m, e);
@@ -946,7 +964,7 @@ __device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, in
     }
     __syncthreads();
   }
-  tri_solve_out(N, beta, job, backward, Xm, Xe);
+  tri_solve_out(N, beta, job, backward, Xm, Xe, threadIdx.x, blockDim.x);
 }
 
 

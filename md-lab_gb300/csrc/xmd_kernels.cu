@@ -849,13 +849,12 @@ __global__ void __launch_bounds__(TS_WARPS * 32) k_tri_solve(int N, double beta,
   }
 }
 
-// scratch: mantissas (ntri(N) doubles) then exponents (ntri(N) ints)
 // one direction's scratch: weights (mantissas, then exponents as ints), the
-// diagonal blocks' inverses (mantissas, exponents), the unknowns X_0..X_N
-// (mantissas, exponents)
+// diagonal blocks' inverses B and the products W (mantissas, exponents), the
+// unknowns X_0..X_N (mantissas, exponents)
 size_t rec_scratch_doubles(int N) {
   const size_t nch = (N + TS_CHUNK - 1) / TS_CHUNK;
-  return ntri(N) + (ntri(N) + 1) / 2 + 1 + nch * TS_CHUNK * TS_CHUNK * 3 / 2 + (size_t)(N + 1) + (N + 2) / 2;
+  return ntri(N) + (ntri(N) + 1) / 2 + 1 + nch * TS_CHUNK * TS_CHUNK * 3 + (size_t)(N + 1) + (N + 2) / 2;
 }
 
 // directions first .. first + count - 1 of job
@@ -871,14 +870,15 @@ size_t rec_scratch_doubles(int N) {
 
 
 // Weights and the diagonal-block inverses in one launch, so that the
-// inverses (latency-bound: a chain of 31 warp sums per column) run beside
+// inverses (latency-bound: a chain of 31 steps per column) run beside
 // the weight rows instead of after them: blocks 0..N-1 are k_weights' rows,
-// the rest take four columns of one chunk's B each and evaluate the chunk's
-// diagonal block from ENk themselves.
+// the rest take four columns of one chunk's B (groups 0..7 of the chunk) or W
+// (8..15, for the cluster solve) each and evaluate the blocks they need from
+// ENk themselves.
 __global__ void __launch_bounds__(128) k_weights_inv(int N, double beta, double vi, double lnvi,
                                                      const double *__restrict__ ENk,
                                                      const double *__restrict__ lnn, TriJob job, int first,
-                                                     int both, int nblk) {
+                                                     int both, int groups) {
   __shared__ long long Am[TS_CHUNK][TS_LD];
   __shared__ int Ae[TS_CHUNK][TS_LD];
   if ((int)blockIdx.x < N) {
@@ -887,20 +887,38 @@ __global__ void __launch_bounds__(128) k_weights_inv(int N, double beta, double 
                 blockDim.x);
     return;
   }
-  const int b = blockIdx.x - N, dir = first + b / nblk, q = b % nblk;
-  const int c = q >> 3, s0 = (q & 7) << 2, s = s0 + (threadIdx.x >> 5);
+  const int nch = (N + TS_CHUNK - 1) / TS_CHUNK;
+  const int b = blockIdx.x - N, dir = first + b / (nch * groups), c = b / groups % nch, q = b % groups;
+  const bool inv = q < 8;
+  if (!inv && c == 0) return;  // no chunk before the first
+  const int s0 = (q & 7) << 2, s = s0 + (threadIdx.x >> 5), t0 = inv ? s0 : 0;
   const int i0 = 1 + c * TS_CHUNK;
-  // columns s0.. read the block's entries t >= s0 only
+  // column s of B reads the block's entries t >= s only
   for (int e = threadIdx.x; e < TS_CHUNK * TS_CHUNK; e += blockDim.x) {
     const int r = e / TS_CHUNK, t = e % TS_CHUNK;
-    Ext w{0.0, 0};
-    if (t < r && t >= s0 && i0 + r <= N) w = weight_at(N, beta, vi, lnvi, ENk, lnn, dir, i0 + r, i0 + t);
-    const XI q = xi_from(w.m, w.e);
-    Am[r][t] = q.m;
-    Ae[r][t] = q.e;
+    XI a{0, XI_NONE};
+    if (t < r && t >= t0 && i0 + r <= N) {
+      const Ext w = weight_at(N, beta, vi, lnvi, ENk, lnn, dir, i0 + r, i0 + t);
+      a = xi_from(w.m, w.e);
+    }
+    Am[r][t] = a.m;
+    Ae[r][t] = a.e;
   }
   __syncthreads();
-  block_inv_column(N, job, dir, c, s, Am, Ae);
+  if (inv) {
+    block_inv_column(N, job, dir, c, s, Am, Ae);
+    return;
+  }
+  const int lane = threadIdx.x & 31;
+  XI u{0, XI_NONE};
+  if (i0 + lane <= N) {
+    const Ext w = weight_at(N, beta, vi, lnvi, ENk, lnn, dir, i0 + lane, i0 - TS_CHUNK + s);
+    u = xi_from(w.m, w.e);
+  }
+  u = block_solve_column(u, 0, min(TS_CHUNK, N - c * TS_CHUNK), Am, Ae);
+  const size_t o = (size_t)c * TS_CHUNK * TS_CHUNK + lane * TS_CHUNK + s;
+  ((long long *)job.Wm[dir])[o] = u.m;
+  job.We[dir][o] = u.e;
 }
 
 // One block per direction, 16 warps, three phases per chunk c:
@@ -917,18 +935,22 @@ __global__ void __launch_bounds__(TSB_WARPS * 32) k_tri_solve_b(int N, double be
   tri_solve_b_dev(N, beta, job, first + blockIdx.x, sh);
 }
 
-// The block solve spread over a thread-block cluster: one cluster of TSC_CL
-// blocks per direction.  Block 0 solves the chunks in order, as above: (U)
-// each row of chunk c adds its terms over chunk c-1's unknowns to its sum
-// over everything before, (B) X = B R.  The other blocks own the later rows'
-// running sums (chunk k >= 1 belongs to block 1 + (k-1) mod (TSC_CL-1)): in
-// iteration c each adds chunk c-1's unknowns, which block 0 wrote into its
-// shared memory, to the rows of its chunks after c, one column a lane, and
-// the owner of chunk c+1 adds up those rows' lanes and writes the completed
-// sums into block 0's shared memory.  So the long sums run on seven more SMs
-// beside block 0's solve, one cluster barrier per chunk; every block loads
-// its next weights before that barrier.
-// Bound: the chain of N/32 chunks, two warp sums and a cluster barrier each.
+// The solve spread over a thread-block cluster: one cluster of TSC_CL blocks
+// per direction.  With P_c the rows' sums of chunk c over the unknowns before
+// chunk c-1,
+//   X_c = B_c (P_c + U_c X_{c-1}) = Y_c + W_c X_{c-1},   Y_c = B_c P_c,
+// so block 0's chain is one 32 x 32 product a chunk.  The other blocks own
+// the later rows' running sums (chunk k >= 1 belongs to block
+// 1 + (k-1) mod (TSC_CL-1)): in iteration c each adds chunk c-1's unknowns,
+// which block 0 wrote into its shared memory, to the rows of its chunks after
+// c, one column a lane; the owner of chunk c+1 does that chunk's rows first,
+// adds up their lanes, forms Y_{c+1} and writes it into block 0's shared
+// memory.  Every block arrives at the iteration's cluster barrier as soon as
+// the others need nothing more of it: the bulk of the sums runs between a
+// block's arrival and its wait, with the next weights' loads in flight.
+// Bound: the chain of N/32 chunks (a product, a warp sum, a remote store and a
+// cluster barrier each); up to N = 512 it takes 8 SMs a direction off the
+// pair forces that run beside it.
 // All sums are on the integer pipe (XI): with FP64 products and a warp sum per
 // row and chunk the FP64 pipes of the summing blocks set the pace.
 constexpr int TSC_CL = 8;      // blocks per cluster (the portable cluster size)
@@ -937,8 +959,8 @@ constexpr int TSC_HB = 8;      // rows whose weights a summing warp loads ahead
 
 __host__ __device__ inline int tsc_slots(int nch) { return (nch - 1 + TSC_CL - 2) / (TSC_CL - 1); }
 static size_t tsc_smem(int N) {
-  const size_t b0 = N + 1 + 3 * TS_CHUNK + 4 * TS_CHUNK * TS_LD;
-  const size_t h = 2 * TS_CHUNK + (size_t)tsc_slots((N + TS_CHUNK - 1) / TS_CHUNK) * TS_CHUNK * 32;
+  const size_t b0 = 2 * TS_CHUNK + N + 1;
+  const size_t h = 3 * TS_CHUNK + (size_t)tsc_slots((N + TS_CHUNK - 1) / TS_CHUNK) * TS_CHUNK * 32;
   return (sizeof(long long) + sizeof(int)) * (b0 > h ? b0 : h) + 16;
 }
 
@@ -952,30 +974,38 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
   const int *__restrict__ Me = job.Me[backward];
   const long long *__restrict__ Bgm = (const long long *)job.Bm[backward];
   const int *__restrict__ Bge = job.Be[backward];
+  const long long *__restrict__ Wgm = (const long long *)job.Wm[backward];
+  const int *__restrict__ Wge = job.We[backward];
   const int nch = (N + TS_CHUNK - 1) / TS_CHUNK;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  constexpr int BLK = TS_CHUNK * TS_LD;
   constexpr int CC = TS_CHUNK * TS_CHUNK;
   extern __shared__ double sh[];
   // block 0
-  long long *Um = (long long *)sh;     // [2][TS_CHUNK][TS_LD] a chunk's weights against the chunk before it
-  long long *Bsm = Um + 2 * BLK;       // [2][TS_CHUNK][TS_LD] a chunk's B block
-  long long *Pm = Bsm + 2 * BLK;       // [2][TS_CHUNK] rows' sums over the unknowns before the previous chunk
-  long long *Rm = Pm + 2 * TS_CHUNK;   // [TS_CHUNK] right-hand sides of the chunk being solved
-  long long *Xm = Rm + TS_CHUNK;       // N+1
-  int *Ue = (int *)(Xm + N + 1);       // [2][TS_CHUNK][TS_LD]
-  int *Bse = Ue + 2 * BLK;             // [2][TS_CHUNK][TS_LD]
-  int *Pe = Bse + 2 * BLK;             // [2][TS_CHUNK]
-  int *Re = Pe + 2 * TS_CHUNK;         // [TS_CHUNK]
-  int *Xe = Re + TS_CHUNK;             // N+1
+  long long *Ym = (long long *)sh;     // [2][TS_CHUNK]
+  long long *Xm = Ym + 2 * TS_CHUNK;   // N+1
+  int *Ye = (int *)(Xm + N + 1);       // [2][TS_CHUNK]
+  int *Xe = Ye + 2 * TS_CHUNK;         // N+1
   // blocks 1..TSC_CL-1
   const int slots = tsc_slots(nch);
-  long long *Hxm = (long long *)sh;            // [2][TS_CHUNK] the last solved chunk's unknowns
-  long long *Ham = Hxm + 2 * TS_CHUNK;         // [slots][TS_CHUNK][32] the owned chunks' rows, a partial sum a lane
+  long long *Hxm = (long long *)sh;        // [2][TS_CHUNK] the last solved chunk's unknowns
+  long long *Hpm = Hxm + 2 * TS_CHUNK;     // [TS_CHUNK] a chunk's completed row sums
+  long long *Ham = Hpm + TS_CHUNK;         // [slots][TS_CHUNK][32] the owned chunks' rows, a partial sum a lane
   int *Hxe = (int *)(Ham + slots * TS_CHUNK * 32);
-  int *Hae = Hxe + 2 * TS_CHUNK;
+  int *Hpe = Hxe + 2 * TS_CHUNK;
+  int *Hae = Hpe + TS_CHUNK;
+  // two rows a warp of the 32 x 32 block of chunk c, a column a lane
+  long long bm[2];
+  int be[2];
+  auto load_block = [&](const long long *m, const int *e, int c) {
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const size_t o = (size_t)c * CC + (w + h * TSC_WARPS) * TS_CHUNK + lane;
+      bm[h] = m[o];
+      be[h] = e[o];
+    }
+  };
   // summing blocks: rows q = 0, 1, ... of the chunks after c, two a slot from
-  // slot t0(c) on; their weights against the columns from j0 on
+  // slot first_slot(c) on, and their weights against the columns from j0 on
   auto first_slot = [&](int c) { return c + 1 > rank ? (c + 1 - rank + TSC_CL - 2) / (TSC_CL - 1) : 0; };
   auto row_of = [&](int t0, int q) {
     const int k = rank + (t0 + q / 2) * (TSC_CL - 1);
@@ -988,8 +1018,9 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
     for (int u = 0; u < TSC_HB; ++u) {
       const int i = row_of(t0, qb + u);
       const bool ok = qb + u < 2 * (slots - t0) && i <= N;
-      mv[u] = ok ? Mm[moff(i, j0 + lane)] : 0.0;
-      me[u] = ok ? Me[moff(i, j0 + lane)] : 0;
+      const size_t o = ok ? moff(i, j0 + lane) : 0;
+      mv[u] = ok ? Mm[o] : 0.0;
+      me[u] = ok ? Me[o] : 0;
     }
   };
   if (rank == 0) {
@@ -997,21 +1028,19 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
       Xm[0] = 1LL << 61;  // X_0 = 1
       Xe[0] = 1;
     }
-    // chunk 0: no chunk before it; its rows' sums over column 0
-    for (int q = threadIdx.x; q < CC; q += blockDim.x) {
-      const int r = q / TS_CHUNK, o = r * TS_LD + q % TS_CHUNK;
-      const bool in = 1 + r <= N;
-      Um[o] = 0;
-      Ue[o] = XI_NONE;
-      Bsm[o] = in ? Bgm[q] : 0;
-      Bse[o] = in ? Bge[q] : XI_NONE;
+    // Y_0 = B_0 times the first rows' weights against X_0
+    const XI p = 1 + lane <= N ? xi_from(Mm[moff(1 + lane, 0)], Me[moff(1 + lane, 0)]) : XI{0, XI_NONE};
+    load_block(Bgm, Bge, 0);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const XI y = xi_warp_sum(xi_mul({bm[h], be[h]}, p));
+      if (lane == 0) {
+        Ym[w + h * TSC_WARPS] = y.m;
+        Ye[w + h * TSC_WARPS] = y.e;
+      }
     }
-    if (threadIdx.x < TS_CHUNK) {
-      const int i = 1 + threadIdx.x;
-      const XI p = i <= N ? xi_from(Mm[moff(i, 0)], Me[moff(i, 0)]) : XI{0, XI_NONE};
-      Pm[threadIdx.x] = p.m;
-      Pe[threadIdx.x] = p.e;
-    }
+    bm[0] = bm[1] = 0;
+    be[0] = be[1] = XI_NONE;  // no chunk before the first
   } else {
     for (int q = threadIdx.x; q < slots * TS_CHUNK * 32; q += blockDim.x) {
       const int k = rank + (q / (TS_CHUNK * 32)) * (TSC_CL - 1), i = 1 + k * TS_CHUNK + q / 32 % TS_CHUNK;
@@ -1019,47 +1048,19 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
       Ham[q] = p.m;
       Hae[q] = p.e;
     }
+    if (rank == 1 && nch > 1) load_block(Bgm, Bge, 1);  // chunk 1's owner
   }
   cl.sync();  // every block has started and holds its initial sums
   for (int c = 0; c < nch; ++c) {
     const int i0 = 1 + c * TS_CHUNK, buf = c & 1;
     if (rank == 0) {
-      // chunk c+1's blocks: loads issued now, stored after this chunk's solve
-      const int n0 = i0 + TS_CHUNK;
-      double su[2];
-      long long sb[2];
-      int seu[2], seb[2];
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const int rs = threadIdx.x + t * TSC_WARPS * 32;
-        const int r = rs / TS_CHUNK, k = rs % TS_CHUNK, i = n0 + r;
-        const bool in = c + 1 < nch && i <= N;
-        su[t] = in ? Mm[moff(i, i0 + k)] : 0.0;
-        seu[t] = in ? Me[moff(i, i0 + k)] : 0;
-        sb[t] = in ? Bgm[(size_t)(c + 1) * CC + rs] : 0;
-        seb[t] = in ? Bge[(size_t)(c + 1) * CC + rs] : XI_NONE;
-      }
-      // U: right-hand sides
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        const int r = w + h * TSC_WARPS, o = buf * BLK + r * TS_LD + lane;
-        XI p{Pm[buf * TS_CHUNK + r], Pe[buf * TS_CHUNK + r]};
-        if (c > 0) {
-          const int col = i0 - TS_CHUNK + lane;
-          p = xi_add(p, xi_warp_sum(xi_mul({Um[o], Ue[o]}, {Xm[col], Xe[col]})));
-        }
-        if (lane == 0) {
-          Rm[r] = p.m;
-          Re[r] = p.e;
-        }
-      }
-      __syncthreads();
-      // B: the chunk's unknowns, also into every other block's shared memory
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = w + h * TSC_WARPS, i = i0 + r, o = buf * BLK + r * TS_LD + lane;
-        if (i > N) continue;  // warp-uniform
-        const XI x = xi_warp_sum(xi_mul({Bsm[o], Bse[o]}, {Rm[lane], Re[lane]}));
+        const int r = w + h * TSC_WARPS, i = i0 + r;
+        XI x{Ym[buf * TS_CHUNK + r], Ye[buf * TS_CHUNK + r]};
+        const XI v = c > 0 ? XI{Xm[i0 - TS_CHUNK + lane], Xe[i0 - TS_CHUNK + lane]} : XI{0, XI_NONE};
+        x = xi_add(x, xi_warp_sum(xi_mul({bm[h], be[h]}, v)));
+        if (i > N) continue;
         if (lane == 0) {
           Xm[i] = x.m;
           Xe[i] = x.e;
@@ -1068,54 +1069,70 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
           *cl.map_shared_rank(Hxe + buf * TS_CHUNK + r, lane) = x.e;
         }
       }
-#pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        const int rs = threadIdx.x + t * TSC_WARPS * 32;
-        const int o = (buf ^ 1) * BLK + rs / TS_CHUNK * TS_LD + rs % TS_CHUNK;
-        const XI u = xi_from(su[t], seu[t]);
-        Um[o] = u.m;
-        Ue[o] = u.e;
-        Bsm[o] = sb[t];
-        Bse[o] = seb[t];
-      }
+      cl.barrier_arrive();
+      if (c + 1 < nch) load_block(Wgm, Wge, c + 1);
     } else {
-      if (c >= 1) {
-        // chunk c-1's unknowns into the rows of the owned chunks after c
-        const int j0 = i0 - TS_CHUNK, pb = (c - 1) & 1, t0 = first_slot(c), nq = 2 * (slots - t0);
-        const XI x{Hxm[pb * TS_CHUNK + lane], Hxe[pb * TS_CHUNK + lane]};
+      const int j0 = i0 - TS_CHUNK, pb = (c - 1) & 1, t0 = first_slot(c), nq = 2 * (slots - t0);
+      XI x{0, XI_NONE};
+      if (c >= 1) x = {Hxm[pb * TS_CHUNK + lane], Hxe[pb * TS_CHUNK + lane]};
+      // chunk c-1's unknowns into row q of the chunks after c
+      auto add_row = [&](int q, double m, int e) {
+        const int o = ((t0 + q / 2) * TS_CHUNK + w + (q & 1) * TSC_WARPS) * 32 + lane;
+        const XI a = xi_add({Ham[o], Hae[o]}, xi_mul(xi_from(m, e), x));
+        Ham[o] = a.m;
+        Hae[o] = a.e;
+      };
+      // the owner of chunk c+1 (its rows are q = 0 and 1) completes them, now
+      // over the unknowns before chunk c, and hands Y_{c+1} to block 0
+      const int kn = c + 1;
+      const bool owner = kn < nch && 1 + (kn - 1) % (TSC_CL - 1) == rank;
+      int q0 = 0;
+      if (owner) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = w + h * TSC_WARPS;
+          if (c >= 1 && row_of(t0, h) <= N) add_row(h, mv[h], me[h]);
+          const int o = (t0 * TS_CHUNK + r) * 32 + lane;
+          const XI p = xi_warp_sum({Ham[o], Hae[o]});
+          if (lane == 0) {
+            Hpm[r] = p.m;
+            Hpe[r] = p.e;
+          }
+        }
+        q0 = 2;
+        __syncthreads();
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const XI y = xi_warp_sum(xi_mul({bm[h], be[h]}, {Hpm[lane], Hpe[lane]}));
+          if (lane == 0) {
+            *cl.map_shared_rank(Ym + (kn & 1) * TS_CHUNK + w + h * TSC_WARPS, 0) = y.m;
+            *cl.map_shared_rank(Ye + (kn & 1) * TS_CHUNK + w + h * TSC_WARPS, 0) = y.e;
+          }
+        }
+      }
+      cl.barrier_arrive();
+      if (c >= 1)
         for (int qb = 0; qb < nq; qb += TSC_HB) {
           if (qb > 0) load(t0, qb, j0);
 #pragma unroll
           for (int u = 0; u < TSC_HB; ++u) {
             const int q = qb + u;
             if (q >= nq || row_of(t0, q) > N) break;  // warp-uniform
-            const int o = ((t0 + q / 2) * TS_CHUNK + w + (q & 1) * TSC_WARPS) * 32 + lane;
-            const XI a = xi_add({Ham[o], Hae[o]}, xi_mul(xi_from(mv[u], me[u]), x));
-            Ham[o] = a.m;
-            Hae[o] = a.e;
+            if (q >= q0) add_row(q, mv[u], me[u]);
           }
         }
-      }
-      // the owner of chunk c+1 hands its rows' sums (now over the unknowns
-      // before chunk c) to block 0
-      const int kn = c + 1;
-      if (kn < nch && 1 + (kn - 1) % (TSC_CL - 1) == rank) {
-        const int t = (kn - 1) / (TSC_CL - 1);
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int r = w + h * TSC_WARPS, o = (t * TS_CHUNK + r) * 32 + lane;
-          const XI p = xi_warp_sum({Ham[o], Hae[o]});
-          if (lane == 0) {
-            *cl.map_shared_rank(Pm + (kn & 1) * TS_CHUNK + r, 0) = p.m;
-            *cl.map_shared_rank(Pe + (kn & 1) * TS_CHUNK + r, 0) = p.e;
-          }
-        }
-      }
-      if (c + 1 < nch) load(first_slot(c + 1), 0, i0);
+      if (kn < nch) load(first_slot(kn), 0, i0);
+      if (kn + 1 < nch && 1 + kn % (TSC_CL - 1) == rank) load_block(Bgm, Bge, kn + 1);
     }
-    cl.sync();
+    cl.barrier_wait();
   }
-  if (rank == 0) tri_solve_out(N, beta, job, backward, Xm, Xe);
+  // V_B = -ln X / beta: an eighth of the unknowns a block, read from block 0
+  {
+    const long long *xm = cl.map_shared_rank(Xm, 0);
+    const int *xe = cl.map_shared_rank(Xe, 0);
+    tri_solve_out(N, beta, job, backward, xm, xe, rank * blockDim.x + threadIdx.x, TSC_CL * blockDim.x);
+  }
+  cl.sync();  // block 0's shared memory is read until here
 }
 
 // whether a cluster of the block solve fits on this device with `smem`
@@ -1173,18 +1190,23 @@ int solve_choice(int N) {
   return (N + TS_CHUNK - 1) / TS_CHUNK > 4 ? SOLVE_CLUSTER : SOLVE_BLOCK;
 }
 
-static cudaError_t tri_solve(int N, double beta, const TriJob &job, int first, int count, cudaStream_t st) {
+// whether the unsigned solve of N takes the cluster; *bad: it was forced, but
+// no cluster of this size fits
+static bool takes_cluster(int N, bool *bad) {
+  const bool want = solve_choice(N) == SOLVE_CLUSTER, fits = want && cluster_solve_fits(tsc_smem(N));
+  *bad = want && !fits && g_solve_force == SOLVE_CLUSTER;
+  return fits;
+}
+
+static cudaError_t tri_solve(int N, double beta, const TriJob &job, int first, int count, cudaStream_t st,
+                             bool cluster = false) {
   if (!job.sign) {
     // unsigned weights: the block solve (the diagonal-block inverses came
     // with the weights, k_weights_inv)
-    const size_t smem_c = tsc_smem(N);
-    const int path = solve_choice(N);
-    if (path == SOLVE_CLUSTER && !cluster_solve_fits(smem_c) && g_solve_force == SOLVE_CLUSTER)
-      return cudaErrorInvalidConfiguration;  // forced, but no cluster of this size fits
-    if (path == SOLVE_CLUSTER && cluster_solve_fits(smem_c)) {
+    if (cluster) {
       {
         XK_PROF(count == 2 ? "vb_tv_solve" : (first ? "tv_solve" : "vb_solve"));
-        k_tri_solve_c<<<dim3(TSC_CL, count), TSC_WARPS * 32, smem_c, st>>>(N, beta, job, first);
+        k_tri_solve_c<<<dim3(TSC_CL, count), TSC_WARPS * 32, tsc_smem(N), st>>>(N, beta, job, first);
       }
       return XK_LAUNCHED();
     }
@@ -1221,10 +1243,14 @@ TriJob tri_job(int N, double *rs_f, double *rs_b, double *VBN, double *tmpV) {
   const size_t nb = (size_t)((N + TS_CHUNK - 1) / TS_CHUNK) * TS_CHUNK * TS_CHUNK;
   double *rs[2] = {rs_f, rs_b};
   for (int d = 0; d < 2; ++d) {
-    j.Bm[d] = rs[d] ? rs[d] + boff : nullptr;
-    j.Be[d] = rs[d] ? (int *)(rs[d] + boff + nb) : nullptr;
-    j.Xm[d] = rs[d] ? rs[d] + boff + nb + nb / 2 : nullptr;
-    j.Xe[d] = rs[d] ? (int *)(rs[d] + boff + nb + nb / 2 + N + 1) : nullptr;
+    if (!rs[d]) continue;
+    double *b = rs[d] + boff;
+    j.Bm[d] = b;
+    j.Be[d] = (int *)(b + nb);
+    j.Wm[d] = b + nb + nb / 2;
+    j.We[d] = (int *)(j.Wm[d] + nb);
+    j.Xm[d] = j.Wm[d] + nb + nb / 2;
+    j.Xe[d] = (int *)(j.Xm[d] + N + 1);
   }
   j.Mm[0] = rs_f;
   j.Me[0] = (const int *)(rs_f + ntri(N));
@@ -1235,42 +1261,37 @@ TriJob tri_job(int N, double *rs_f, double *rs_b, double *VBN, double *tmpV) {
   return j;
 }
 
-// unsigned weights of directions first .. first + count - 1 and their
-// diagonal-block inverses (count = 2: first = 0)
-static cudaError_t weights_inv(int N, double beta, double vi, const double *ENk, const double *lnn,
-                               const TriJob &job, int first, int count, cudaStream_t st) {
+// unsigned weights of directions first .. first + count - 1 with their
+// diagonal blocks' inverses (count = 2: first = 0), then the solve
+static cudaError_t weights_solve(int N, double beta, double vi, const double *ENk, const double *lnn,
+                                 const TriJob &job, int first, int count, cudaStream_t st) {
   const double lnvi = vi != 0.0 ? log(vi) : 0.0;
-  const int nblk = (N + TS_CHUNK - 1) / TS_CHUNK * 8;  // four columns a block
+  bool bad;
+  const bool cluster = takes_cluster(N, &bad);
+  if (bad) return cudaErrorInvalidConfiguration;
+  const int groups = cluster ? 16 : 8, nch = (N + TS_CHUNK - 1) / TS_CHUNK;  // four columns of B or W a block
   {
     XK_PROF("weights");
-    k_weights_inv<<<N + count * nblk, 128, 0, st>>>(N, beta, vi, lnvi, ENk, lnn, job, first, count == 2 ? 1 : 0,
-                                                      nblk);
+    k_weights_inv<<<N + count * nch * groups, 128, 0, st>>>(N, beta, vi, lnvi, ENk, lnn, job, first,
+                                                           count == 2 ? 1 : 0, groups);
   }
-  return XK_LAUNCHED();
+  const cudaError_t e = XK_LAUNCHED();
+  return e == cudaSuccess ? tri_solve(N, beta, job, first, count, st, cluster) : e;
 }
 
 cudaError_t fill_vb(int N, double beta, double vi, const double *ENk, const double *lnn, double *VBN, double *rs,
                     cudaStream_t st) {
-  const TriJob j = tri_job(N, rs, nullptr, VBN, nullptr);
-  cudaError_t e = weights_inv(N, beta, vi, ENk, lnn, j, 0, 1, st);
-  if (e != cudaSuccess) return e;
-  return tri_solve(N, beta, j, 0, 1, st);
+  return weights_solve(N, beta, vi, ENk, lnn, tri_job(N, rs, nullptr, VBN, nullptr), 0, 1, st);
 }
 
 cudaError_t back_vb(int N, double beta, double vi, const double *ENk, const double *lnn, double *tmpV, double *rs,
                     cudaStream_t st) {
-  const TriJob j = tri_job(N, nullptr, rs, nullptr, tmpV);
-  cudaError_t e = weights_inv(N, beta, vi, ENk, lnn, j, 1, 1, st);
-  if (e != cudaSuccess) return e;
-  return tri_solve(N, beta, j, 1, 1, st);
+  return weights_solve(N, beta, vi, ENk, lnn, tri_job(N, nullptr, rs, nullptr, tmpV), 1, 1, st);
 }
 
 cudaError_t fill_vb_tv(int N, double beta, double vi, const double *ENk, const double *lnn, double *VBN,
                        double *tmpV, double *rs_f, double *rs_b, cudaStream_t st) {
-  const TriJob j = tri_job(N, rs_f, rs_b, VBN, tmpV);
-  cudaError_t e = weights_inv(N, beta, vi, ENk, lnn, j, 0, 2, st);
-  if (e != cudaSuccess) return e;
-  return tri_solve(N, beta, j, 0, 2, st);
+  return weights_solve(N, beta, vi, ENk, lnn, tri_job(N, rs_f, rs_b, VBN, tmpV), 0, 2, st);
 }
 
 cudaError_t fill_vb_signed(int N, double beta, double vi2, const double *ENk, const double *lnn, double *V2,
