@@ -280,15 +280,21 @@ struct Ext {
   int e;     // value = m * 2^e
 };
 
-// exp(x) in extended range for any finite x: 2^e exp(r), |r| <= ln2/2 (the
-// reduction in FP64, the exponential on the integer pipe)
-__device__ inline Ext ext_exp(double x) {
+// exp(x) for any finite x as 2^e exp(r), |r| <= ln2/2: exp(r) 2^62 from the
+// integer pipe, the reduction in FP64
+__device__ __forceinline__ long long exp_reduced(double x, int &e) {
   constexpr double MAGIC = 6755399441055744.0;  // 1.5 2^52: adding rounds to an integer, in the low word
   const double tq = fma(x, LOG2E, MAGIC), q = tq - MAGIC;
   double r = fma(-q, LN2_HI, x);
   r = fma(-q, LN2_LO, r);
   const bool large = (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFLL) >= 0x41D0000000000000LL;  // |x| >= 2^30
-  return {q62_double(exp_q62(r)), large ? (int)q : __double2loint(tq)};
+  e = large ? (int)q : __double2loint(tq);
+  return exp_q62(r);
+}
+__device__ inline Ext ext_exp(double x) {
+  Ext w;
+  w.m = q62_double(exp_reduced(x, w.e));
+  return w;
 }
 
 // exp(x) through ext_exp, the power of two put into the exponent field by
@@ -328,6 +334,82 @@ __device__ inline void ext_norm(double &m, int &e) {
   e += k;
 }
 
+// ---- extended range on the integer pipe --------------------------------
+// A non-negative number m 2^(e-62) with a 62-bit integer mantissa (2^61 <= m
+// < 2^62, or m = 0 with e = XI_NONE): nine bits more than a double's, and no
+// FP64 instruction, which on GB300 holds its pipe for 64 cycles a warp.  The
+// unsigned solves and the diagonal blocks' inverses work on these; every
+// truncation is below 2^-60 of the value.
+struct XI {
+  long long m;
+  int e;
+};
+constexpr int XI_NONE = -(1 << 29);
+
+// v 2^e of a non-negative double v
+__device__ __forceinline__ XI xi_from(double v, int e) {
+  const long long b = __double_as_longlong(v);
+  const int ex = (int)(b >> 52);
+  XI r{((b & 0xFFFFFFFFFFFFFLL) | (1LL << 52)) << 9, e + ex - 1022};
+  if (ex == 0) r = {0, XI_NONE};
+  return r;
+}
+// exp(x)
+__device__ __forceinline__ XI xi_exp(double x) {
+  int e;
+  const long long p = exp_reduced(x, e);  // 0.70 .. 1.42 times 2^62
+  return p >= (1LL << 62) ? XI{p >> 1, e + 1} : XI{p, e};
+}
+// rounded to a double (to zero below 2^-1074; e up to 1024)
+__device__ __forceinline__ double xi_double(XI a) {
+  const bool low = a.e < -1020;
+  const int e = low ? a.e + 200 : a.e;
+  if (a.m == 0 || e < -1020) return 0.0;
+  const double v = __longlong_as_double(((a.m + 256) >> 9) + ((long long)(e + 1021) << 52));
+  return low ? v * 0x1p-200 : v;
+}
+// ln of a non-zero number: y = logf of the mantissa taken to [0.7, 1.42), then
+// one Newton step against exp on the integer pipe; a handful of FP64
+// instructions where log() takes about sixty
+__device__ __forceinline__ double xi_log(XI a) {
+  const bool up = a.m < 0x2D413CCCFE779800LL;  // sqrt(1/2) 2^62: double the mantissa
+  const unsigned long long f = (unsigned long long)a.m << (up ? 2 : 1);  // mantissa 2^63
+  const int e = up ? a.e - 1 : a.e;
+  const float y = logf((float)(unsigned)(f >> 32) * 0x1p-31f);
+  const unsigned long long p = (unsigned long long)exp_q62(-(double)y);  // e^-y 2^62
+  const long long z = (long long)__umul64hi(f, p << 1) - (1LL << 62);    // (m e^-y - 1) 2^62, about 1e-7
+  const double d = (double)z * 0x1p-62;
+  return fma((double)e, LN2_HI, fma((double)e, LN2_LO, fma(-0.5 * d, d, d)) + (double)y);
+}
+__device__ __forceinline__ XI xi_mul(XI a, XI b) {
+  XI r{(long long)__umul64hi((unsigned long long)a.m << 2, (unsigned long long)b.m), a.e + b.e};
+  if (r.m < (1LL << 61)) r.m <<= 1, r.e -= 1;
+  return r;
+}
+__device__ __forceinline__ XI xi_add(XI a, XI b) {
+  XI r;
+  r.e = a.e > b.e ? a.e : b.e;
+  r.m = (a.m >> min(r.e - a.e, 63)) + (b.m >> min(r.e - b.e, 63));
+  if (r.m >= (1LL << 62)) r.m >>= 1, r.e += 1;
+  return r;
+}
+__device__ __forceinline__ XI xi_shfl(XI a, int src) {
+  return {__shfl_sync(FULL, a.m, src), __shfl_sync(FULL, a.e, src)};
+}
+// the warp's sum in every lane: aligned to the largest exponent with 57 bits,
+// in three 19-bit parts (a warp-wide integer reduction is one instruction)
+__device__ __forceinline__ XI xi_warp_sum(XI a) {
+  const int em = __reduce_max_sync(FULL, a.e);
+  const long long q = (a.m >> min(em - a.e, 63)) >> 5;
+  const unsigned p0 = __reduce_add_sync(FULL, (unsigned)q & 0x7ffffu);
+  const unsigned p1 = __reduce_add_sync(FULL, (unsigned)(q >> 19) & 0x7ffffu);
+  const unsigned p2 = __reduce_add_sync(FULL, (unsigned)(q >> 38));
+  const long long t = (long long)p0 + ((long long)p1 << 19) + ((long long)p2 << 38);
+  if (t == 0) return {0, XI_NONE};
+  const int sh = __clzll(t) - 2;
+  return {t << sh, em + 5 - sh};
+}
+
 // packed lower triangle: row i (1..N), column j (0..i-1) at tri(i) + j
 __device__ inline size_t moff(int i, int j) { return (size_t)i * (i - 1) / 2 + j; }
 
@@ -341,6 +423,8 @@ __device__ inline size_t moff(int i, int j) { return (size_t)i * (i - 1) / 2 + j
 // both = 1 (first = 0, both directions): the two triangles hold the same
 // numbers, M_{l,l-k} = M'_{N-l+k,N-l}, so block l takes row l of ENk and
 // writes each weight into both (one exponential per entry).
+// INT: the mantissas are XI's 62-bit integers (unsigned weights), else doubles.
+template <bool INT>
 __device__ inline void weights_row(int N, double beta, double vi, double lnvi, const double *__restrict__ ENk,
                                    const double *__restrict__ lnn, double *__restrict__ Mf, int *__restrict__ Ef,
                                    double *__restrict__ Mb, int *__restrict__ Eb, int first, int sgn, int both,
@@ -350,14 +434,24 @@ __device__ inline void weights_row(int N, double beta, double vi, double lnvi, c
   for (int j = t0; j < row; j += nt) {
     const int k = row - j;
     const int l = dir ? N - j : row;
-    Ext w{0.0, 0};
-    if (vi != 0.0 || k == 1) w = ext_exp(-beta * ENk[dtri(l) + k - 1] + (k - 1) * lnvi - lnn[l]);
-    if (sgn < 0 && ((k - 1) & 1)) w.m = -w.m;
-    Mm[moff(row, j)] = w.m;
-    Me[moff(row, j)] = w.e;
+    const bool on = vi != 0.0 || k == 1;
+    const double x = on ? -beta * ENk[dtri(l) + k - 1] + (k - 1) * lnvi - lnn[l] : 0.0;
+    double m;
+    int e;
+    if (INT) {
+      const XI w = on ? xi_exp(x) : XI{0, XI_NONE};
+      m = __longlong_as_double(w.m);
+      e = w.e;
+    } else {
+      const Ext w = on ? ext_exp(x) : Ext{0.0, 0};
+      m = sgn < 0 && ((k - 1) & 1) ? -w.m : w.m;
+      e = w.e;
+    }
+    Mm[moff(row, j)] = m;
+    Me[moff(row, j)] = e;
     if (both) {
-      Mb[moff(N - row + k, N - row)] = w.m;
-      Eb[moff(N - row + k, N - row)] = w.e;
+      Mb[moff(N - row + k, N - row)] = m;
+      Eb[moff(N - row + k, N - row)] = e;
     }
   }
 }
@@ -401,8 +495,9 @@ struct TriJob {
   int *Be[2];
   double *Wm[2];
   int *We[2];
-  double *Xm[2];  // optional: the unknowns X_0..X_N in extended range (unsigned
-  int *Xe[2];     // solves), kept for the connection probabilities
+  double *Sm[2];  // partial sums of the cluster solve of very long systems
+  long long *Xm[2];  // optional: the unknowns X_0..X_N as XI (unsigned solves),
+  int *Xe[2];        // kept for the connection probabilities
 };
 
 // Extended-range dot product of row i of the weights with the unknowns over
@@ -541,68 +636,13 @@ __device__ inline void ext_warp_sum(bool nz, double pm, int pe, double &sum, int
   E = Em;
 }
 
-// ---- extended range on the integer pipe --------------------------------
-// A non-negative number m 2^(e-62) with a 62-bit integer mantissa (2^61 <= m
-// < 2^62, or m = 0 with e = XI_NONE): nine bits more than a double's, and no
-// FP64 instruction, which on GB300 holds its pipe for 64 cycles a warp.  The
-// unsigned solves and the diagonal blocks' inverses work on these; every
-// truncation is below 2^-60 of the value.
-struct XI {
-  long long m;
-  int e;
-};
-constexpr int XI_NONE = -(1 << 29);
-
-// v 2^e of a non-negative double v
-__device__ __forceinline__ XI xi_from(double v, int e) {
-  const long long b = __double_as_longlong(v);
-  const int ex = (int)(b >> 52);
-  XI r{((b & 0xFFFFFFFFFFFFFLL) | (1LL << 52)) << 9, e + ex - 1022};
-  if (ex == 0) r = {0, XI_NONE};
-  return r;
-}
-// a mantissa in [0.5, 1) and its power of two (zero: 0 and 0)
-__device__ __forceinline__ void xi_split(XI a, double &m, int &e) {
-  m = __longlong_as_double(a.m == 0 ? 0LL : (((a.m >> 9) & 0xFFFFFFFFFFFFFLL) | (1022LL << 52)));
-  e = a.m == 0 ? 0 : a.e;
-}
-__device__ __forceinline__ XI xi_mul(XI a, XI b) {
-  XI r{(long long)__umul64hi((unsigned long long)a.m << 2, (unsigned long long)b.m), a.e + b.e};
-  if (r.m < (1LL << 61)) r.m <<= 1, r.e -= 1;
-  return r;
-}
-__device__ __forceinline__ XI xi_add(XI a, XI b) {
-  XI r;
-  r.e = a.e > b.e ? a.e : b.e;
-  r.m = (a.m >> min(r.e - a.e, 63)) + (b.m >> min(r.e - b.e, 63));
-  if (r.m >= (1LL << 62)) r.m >>= 1, r.e += 1;
-  return r;
-}
-__device__ __forceinline__ XI xi_shfl(XI a, int src) {
-  return {__shfl_sync(FULL, a.m, src), __shfl_sync(FULL, a.e, src)};
-}
-// the warp's sum in every lane: aligned to the largest exponent with 57 bits,
-// in three 19-bit parts (a warp-wide integer reduction is one instruction)
-__device__ __forceinline__ XI xi_warp_sum(XI a) {
-  const int em = __reduce_max_sync(FULL, a.e);
-  const long long q = (a.m >> min(em - a.e, 63)) >> 5;
-  const unsigned p0 = __reduce_add_sync(FULL, (unsigned)q & 0x7ffffu);
-  const unsigned p1 = __reduce_add_sync(FULL, (unsigned)(q >> 19) & 0x7ffffu);
-  const unsigned p2 = __reduce_add_sync(FULL, (unsigned)(q >> 38));
-  const long long t = (long long)p0 + ((long long)p1 << 19) + ((long long)p2 << 38);
-  if (t == 0) return {0, XI_NONE};
-  const int sh = __clzll(t) - 2;
-  return {t << sh, em + 5 - sh};
-}
-
 // weight M_{i,j} of direction dir (0 forward, 1 backward) from ENk, the same
-// expression k_weights evaluates (so the same number)
-__device__ inline Ext weight_at(int N, double beta, double vi, double lnvi, const double *__restrict__ ENk,
-                                const double *__restrict__ lnn, int dir, int i, int j) {
+// number weights_row stores
+__device__ inline XI weight_at(int N, double beta, double vi, double lnvi, const double *__restrict__ ENk,
+                               const double *__restrict__ lnn, int dir, int i, int j) {
   const int k = i - j, l = dir ? N - j : i;
-  Ext w{0.0, 0};
-  if (vi != 0.0 || k == 1) w = ext_exp(-beta * ENk[dtri(l) + k - 1] + (k - 1) * lnvi - lnn[l]);
-  return w;
+  if (vi == 0.0 && k != 1) return {0, XI_NONE};
+  return xi_exp(-beta * ENk[dtri(l) + k - 1] + (k - 1) * lnvi - lnn[l]);
 }
 
 // One column of B(c) = (I - A)^-1 or W(c) = (I - A)^-1 U for direction dir,
@@ -629,18 +669,6 @@ __device__ inline void block_inv_column(int N, const TriJob &job, int dir, int c
   const size_t o = (size_t)c * TS_CHUNK * TS_CHUNK + lane * TS_CHUNK + s;
   ((long long *)job.Bm[dir])[o] = b.m;
   job.Be[dir][o] = b.e;
-}
-
-// m 2^e for 0 <= m < 4 (a product of normalised mantissas) and e <= 1021:
-// one multiplication by a power of two built from its bit pattern, a second
-// one below the normal range (results under 2^-1074 round to zero)
-__device__ inline double ext_val(double m, int e) {
-  if (e < -1021) {
-    if (e < -1130) return 0.0;
-    m *= 0x1p-200;
-    e += 200;
-  }
-  return m * __longlong_as_double((long long)(e + 1023) << 52);
 }
 
 // gradient of the two springs at bead (ja, la) towards (jn, ln) and (jp, lp):
@@ -849,33 +877,33 @@ __device__ inline float2 cmulf(float2 a, float2 b) {
 // each) and outputs VBN / tmpV (host)
 TriJob tri_job(int N, double *rs_f, double *rs_b, double *VBN, double *tmpV);
 
-// out[] and the kept unknowns of a solve from X_0..X_N, entries i0, i0 + step, ...
+// out[] = -ln X / beta and the kept unknowns of a solve from X_0..X_N, entries
+// i0, i0 + step, ...
 __device__ inline void tri_solve_out(int N, double beta, const TriJob &job, int backward, const long long *Xm,
                                      const int *Xe, int i0, int step) {
   double *__restrict__ out = job.out[backward];
+  const double ib = 1.0 / beta;
   for (int i = i0; i <= N; i += step) {
-    double m;
-    int e;
-    xi_split({Xm[i], Xe[i]}, m, e);
+    const XI x{Xm[i], Xe[i]};
     if (i > 0) {
-      const double lnx = log(m) + e * LN2_HI + e * LN2_LO;
-      out[backward ? N - i : i] = -lnx / beta;
+      // the quotient, corrected by its residual
+      const double lnx = xi_log(x), q = -lnx * ib;
+      out[backward ? N - i : i] = fma(-fma(q, beta, lnx), ib, q);
     } else {
       out[backward ? N : 0] = 0.0;
     }
     if (job.Xm[backward]) {
-      job.Xm[backward][i] = m;
-      job.Xe[backward][i] = e;
+      job.Xm[backward][i] = x.m;
+      job.Xe[backward][i] = x.e;
     }
   }
 }
 
 // row i's sum over the unknowns 0 <= j < j1, by the warp
-__device__ inline XI xi_dot(const double *__restrict__ Mm, const int *__restrict__ Me, const long long *Xm,
+__device__ inline XI xi_dot(const long long *__restrict__ Mm, const int *__restrict__ Me, const long long *Xm,
                             const int *Xe, int i, int j1, int lane) {
   XI a{0, XI_NONE};
-  for (int j = lane; j < j1; j += 32)
-    a = xi_add(a, xi_mul(xi_from(Mm[moff(i, j)], Me[moff(i, j)]), {Xm[j], Xe[j]}));
+  for (int j = lane; j < j1; j += 32) a = xi_add(a, xi_mul({Mm[moff(i, j)], Me[moff(i, j)]}, {Xm[j], Xe[j]}));
   return xi_warp_sum(a);
 }
 
@@ -884,7 +912,7 @@ __device__ inline XI xi_dot(const double *__restrict__ Mm, const int *__restrict
 // row's sums inside one warp, so the result does not depend on the count).
 // sh: (8 + 4) (N + 1 + 2 TS_CHUNK + 2 TS_CHUNK TS_LD) bytes of shared memory.
 __device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, int backward, double *sh) {
-  const double *__restrict__ Mm = job.Mm[backward];
+  const long long *__restrict__ Mm = (const long long *)job.Mm[backward];
   const int *__restrict__ Me = job.Me[backward];
   const long long *__restrict__ Bgm = (const long long *)job.Bm[backward];
   const int *__restrict__ Bge = job.Be[backward];
@@ -905,9 +933,9 @@ __device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, in
     for (int q = threadIdx.x; q < TS_CHUNK * TS_CHUNK; q += blockDim.x) {
       const int r = q / TS_CHUNK, k = q % TS_CHUNK, i = n0 + r, o = r * TS_LD + k;
       const bool in = i <= N;
-      const XI u = in && c0 >= 0 ? xi_from(Mm[moff(i, c0 + k)], Me[moff(i, c0 + k)]) : XI{0, XI_NONE};
-      Um[o] = u.m;
-      Ue[o] = u.e;
+      const bool un = in && c0 >= 0;
+      Um[o] = un ? Mm[moff(i, c0 + k)] : 0;
+      Ue[o] = un ? Me[moff(i, c0 + k)] : XI_NONE;
       Bsm[o] = in ? Bgm[(size_t)cc * TS_CHUNK * TS_CHUNK + q] : 0;
       Bse[o] = in ? Bge[(size_t)cc * TS_CHUNK * TS_CHUNK + q] : XI_NONE;
     }
@@ -919,9 +947,8 @@ __device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, in
   stage(1, -1);
   // chunk 0: its rows against column 0
   for (int r = threadIdx.x; r < TS_CHUNK; r += blockDim.x) {
-    const XI p = 1 + r <= N ? xi_from(Mm[moff(1 + r, 0)], Me[moff(1 + r, 0)]) : XI{0, XI_NONE};
-    Pm[r] = p.m;
-    Pe[r] = p.e;
+    Pm[r] = 1 + r <= N ? Mm[moff(1 + r, 0)] : 0;
+    Pe[r] = 1 + r <= N ? Me[moff(1 + r, 0)] : XI_NONE;
   }
   __syncthreads();
   for (int i0 = 1, c = 0; i0 <= N; i0 += TS_CHUNK, ++c) {
@@ -1014,30 +1041,20 @@ __device__ inline void spring_interior_bead(const Geo &g, const double *__restri
   for (int d = 0; d < D; ++d) f[sidx(j, d, l, D, g.Ns)] += -gr[d];
 }
 
-// X'_{N-l} / X_N of row l (1-based) of G, as a mantissa q and an exponent qe
-__device__ inline void g_ext_row(int N, const double *__restrict__ Xfm, const int *__restrict__ Xfe,
-                                 const double *__restrict__ Xbm, const int *__restrict__ Xbe, int l, double &q,
-                                 int &qe) {
-  q = Xbm[N - l] / Xfm[N];
-  qe = Xbe[N - l] - Xfe[N];
+// 1 / X_N (its mantissa's reciprocal in FP64: one division)
+__device__ inline XI g_ext_inv(int N, const TriJob &job) {
+  const XI x{job.Xm[0][N], job.Xe[0][N]};
+  // 1 / (m 2^(e-62)) = (1 / mantissa in [1/2, 1)) 2^-e
+  return xi_from(1.0 / __longlong_as_double(((x.m + 256) >> 9) + (1021LL << 52)), -x.e);
 }
-
-// G[l][j] (1-based) from the extended-range weights and unknowns, the row's
-// factor (q, qe) from g_ext_row
-__device__ inline void g_ext_elem(int N, const double *__restrict__ Mm, const int *__restrict__ Me,
-                                  const double *__restrict__ Xfm, const int *__restrict__ Xfe, double q, int qe,
-                                  double *__restrict__ G, int l, int j) {
-  double gv;
-  if (j > l + 1) {
-    gv = 0;
-  } else if (j == l + 1) {
-    gv = 1 - ext_val(Xfm[l] * q, Xfe[l] + qe);
-  } else {
-    const size_t o = moff(l, j - 1);
-    const double w = Mm[o];
-    gv = w == 0.0 ? 0.0 : ext_val(w * Xfm[j - 1] * q, Me[o] + Xfe[j - 1] + qe);
-  }
-  G[(size_t)(l - 1) * N + (j - 1)] = gv;
+// G[l][j] (1-based) = M_{l,j-1} X_{j-1} X'_{N-l} / X_N, and 1 - X_l X'_{N-l} / X_N
+// for j = l + 1, from the recursions' numbers; q: X'_{N-l} / X_N
+__device__ inline double g_ext_elem(const TriJob &job, XI q, int l, int j) {
+  if (j > l + 1) return 0.0;
+  if (j == l + 1) return 1 - xi_double(xi_mul({job.Xm[0][l], job.Xe[0][l]}, q));
+  const size_t o = moff(l, j - 1);
+  const XI w{((const long long *)job.Mm[0])[o], job.Me[0][o]};
+  return xi_double(xi_mul(xi_mul(w, {job.Xm[0][j - 1], job.Xe[0][j - 1]}), q));
 }
 
 // FP32 phase factors e^{2 pi i n x/L}, n = 0..ns, of slot t (D = 3 layout)

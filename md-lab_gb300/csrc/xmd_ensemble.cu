@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
       const EnsSysDesc &d = E.d;
       const int N = d.g.N;
       for (long long r = ens_first(gw, sys[i].rot[R_E_W], GW); r < N; r += GW)
-        weights_row(N, d.beta, d.vi, E.lnvi, d.ENk, d.lnn, (double *)E.job.Mm[0], (int *)E.job.Me[0],
+        weights_row<true>(N, d.beta, d.vi, E.lnvi, d.ENk, d.lnn, (double *)E.job.Mm[0], (int *)E.job.Me[0],
                     (double *)E.job.Mm[1], (int *)E.job.Me[1], 0, 1, 1, (int)r + 1, 0, lane, 32);
     }
   }
@@ -453,9 +453,8 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
         __syncthreads();
         for (int e = tid; e < TS_CHUNK * TS_CHUNK; e += ENS_T) {
           const int r = e / TS_CHUNK, t = e % TS_CHUNK;
-          Ext wv{0.0, 0};
-          if (t < r && i0 + r <= N) wv = weight_at(N, d.beta, d.vi, E.lnvi, d.ENk, d.lnn, dir, i0 + r, i0 + t);
-          const XI q = xi_from(wv.m, wv.e);
+          XI q{0, XI_NONE};
+          if (t < r && i0 + r <= N) q = weight_at(N, d.beta, d.vi, E.lnvi, d.ENk, d.lnn, dir, i0 + r, i0 + t);
           Am[r][t] = q.m;
           Ae[r][t] = q.e;
         }
@@ -487,12 +486,11 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
       const EnsSys &E = sys[i];
       const int N = E.d.g.N;
       const long long n = (long long)N * N;
+      const XI iX = g_ext_inv(N, E.job);
       for (long long q = ens_first(gt, sys[i].rot[R_G], GT); q < n; q += GT) {
         const int l = (int)(q / N) + 1;
-        double qf;
-        int qe;
-        g_ext_row(N, E.job.Xm[0], E.job.Xe[0], E.job.Xm[1], E.job.Xe[1], l, qf, qe);
-        g_ext_elem(N, E.job.Mm[0], E.job.Me[0], E.job.Xm[0], E.job.Xe[0], qf, qe, E.d.G, l, (int)(q % N) + 1);
+        const XI f = xi_mul({E.job.Xm[1][N - l], E.job.Xe[1][N - l]}, iX);
+        E.d.G[q] = g_ext_elem(E.job, f, l, (int)(q % N) + 1);
       }
     }
   }

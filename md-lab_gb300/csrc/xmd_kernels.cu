@@ -676,7 +676,7 @@ __global__ void __launch_bounds__(128) k_weights(int N, double beta, double vi, 
                                                  double *__restrict__ Mf, int *__restrict__ Ef,
                                                  double *__restrict__ Mb, int *__restrict__ Eb, int first, int sgn,
                                                  int both) {
-  weights_row(N, beta, vi, lnvi, ENk, lnn, Mf, Ef, Mb, Eb, first, sgn, both, blockIdx.x + 1, first + blockIdx.y,
+  weights_row<false>(N, beta, vi, lnvi, ENk, lnn, Mf, Ef, Mb, Eb, first, sgn, both, blockIdx.x + 1, first + blockIdx.y,
               threadIdx.x, blockDim.x);
 }
 
@@ -849,12 +849,21 @@ __global__ void __launch_bounds__(TS_WARPS * 32) k_tri_solve(int N, double beta,
   }
 }
 
+// slots of the cluster solve's summing blocks (k_tri_solve_c)
+__host__ __device__ inline int tsc_slots(int nch, int CL) { return (nch - 1 + CL - 2) / (CL - 1); }
+// doubles of partial sums in memory for one direction of the SLOTS = 0 variant
+static size_t tsc_sums(int N) {
+  const int nch = (N + TS_CHUNK - 1) / TS_CHUNK;
+  return nch <= 29 ? 0 : (size_t)7 * tsc_slots(nch, 8) * TS_CHUNK * 32 * 3 / 2;
+}
+
 // one direction's scratch: weights (mantissas, then exponents as ints), the
 // diagonal blocks' inverses B and the products W (mantissas, exponents), the
-// unknowns X_0..X_N (mantissas, exponents)
+// unknowns X_0..X_N (mantissas, exponents), and the partial sums of the
+// cluster solve's memory variant
 size_t rec_scratch_doubles(int N) {
   const size_t nch = (N + TS_CHUNK - 1) / TS_CHUNK;
-  return ntri(N) + (ntri(N) + 1) / 2 + 1 + nch * TS_CHUNK * TS_CHUNK * 3 + (size_t)(N + 1) + (N + 2) / 2;
+  return ntri(N) + (ntri(N) + 1) / 2 + 1 + nch * TS_CHUNK * TS_CHUNK * 3 + (size_t)(N + 1) + (N + 2) / 2 + tsc_sums(N);
 }
 
 // directions first .. first + count - 1 of job
@@ -882,7 +891,7 @@ __global__ void __launch_bounds__(128) k_weights_inv(int N, double beta, double 
   __shared__ long long Am[TS_CHUNK][TS_LD];
   __shared__ int Ae[TS_CHUNK][TS_LD];
   if ((int)blockIdx.x < N) {
-    weights_row(N, beta, vi, lnvi, ENk, lnn, (double *)job.Mm[0], (int *)job.Me[0], (double *)job.Mm[1],
+    weights_row<true>(N, beta, vi, lnvi, ENk, lnn, (double *)job.Mm[0], (int *)job.Me[0], (double *)job.Mm[1],
                 (int *)job.Me[1], first, 1, both, blockIdx.x + 1, first, threadIdx.x,
                 blockDim.x);
     return;
@@ -897,10 +906,7 @@ __global__ void __launch_bounds__(128) k_weights_inv(int N, double beta, double 
   for (int e = threadIdx.x; e < TS_CHUNK * TS_CHUNK; e += blockDim.x) {
     const int r = e / TS_CHUNK, t = e % TS_CHUNK;
     XI a{0, XI_NONE};
-    if (t < r && t >= t0 && i0 + r <= N) {
-      const Ext w = weight_at(N, beta, vi, lnvi, ENk, lnn, dir, i0 + r, i0 + t);
-      a = xi_from(w.m, w.e);
-    }
+    if (t < r && t >= t0 && i0 + r <= N) a = weight_at(N, beta, vi, lnvi, ENk, lnn, dir, i0 + r, i0 + t);
     Am[r][t] = a.m;
     Ae[r][t] = a.e;
   }
@@ -911,10 +917,7 @@ __global__ void __launch_bounds__(128) k_weights_inv(int N, double beta, double 
   }
   const int lane = threadIdx.x & 31;
   XI u{0, XI_NONE};
-  if (i0 + lane <= N) {
-    const Ext w = weight_at(N, beta, vi, lnvi, ENk, lnn, dir, i0 + lane, i0 - TS_CHUNK + s);
-    u = xi_from(w.m, w.e);
-  }
+  if (i0 + lane <= N) u = weight_at(N, beta, vi, lnvi, ENk, lnn, dir, i0 + lane, i0 - TS_CHUNK + s);
   u = block_solve_column(u, 0, min(TS_CHUNK, N - c * TS_CHUNK), Am, Ae);
   const size_t o = (size_t)c * TS_CHUNK * TS_CHUNK + lane * TS_CHUNK + s;
   ((long long *)job.Wm[dir])[o] = u.m;
@@ -935,42 +938,39 @@ __global__ void __launch_bounds__(TSB_WARPS * 32) k_tri_solve_b(int N, double be
   tri_solve_b_dev(N, beta, job, first + blockIdx.x, sh);
 }
 
-// The solve spread over a thread-block cluster: one cluster of TSC_CL blocks
-// per direction.  With P_c the rows' sums of chunk c over the unknowns before
+// The solve spread over a thread-block cluster: one cluster of CL blocks per
+// direction.  With P_c the rows' sums of chunk c over the unknowns before
 // chunk c-1,
 //   X_c = B_c (P_c + U_c X_{c-1}) = Y_c + W_c X_{c-1},   Y_c = B_c P_c,
 // so block 0's chain is one 32 x 32 product a chunk.  The other blocks own
 // the later rows' running sums (chunk k >= 1 belongs to block
-// 1 + (k-1) mod (TSC_CL-1)): in iteration c each adds chunk c-1's unknowns,
-// which block 0 wrote into its shared memory, to the rows of its chunks after
-// c, one column a lane; the owner of chunk c+1 does that chunk's rows first,
-// adds up their lanes, forms Y_{c+1} and writes it into block 0's shared
-// memory.  Every block arrives at the iteration's cluster barrier as soon as
-// the others need nothing more of it: the bulk of the sums runs between a
-// block's arrival and its wait, with the next weights' loads in flight.
-// Bound: the chain of N/32 chunks (a product, a warp sum, a remote store and a
-// cluster barrier each); up to N = 512 it takes 8 SMs a direction off the
-// pair forces that run beside it.
-// All sums are on the integer pipe (XI): with FP64 products and a warp sum per
-// row and chunk the FP64 pipes of the summing blocks set the pace.
-constexpr int TSC_CL = 8;      // blocks per cluster (the portable cluster size)
+// 1 + (k-1) mod (CL-1), its slot (k-1) / (CL-1)): in iteration c each adds
+// chunk c-1's unknowns, which block 0 wrote into its shared memory, to the
+// rows of its chunks after c, one column a lane; the owner of chunk c+1 does
+// that chunk's rows first, adds up their lanes, forms Y_{c+1} and writes it
+// into block 0's shared memory.  Every block arrives at the iteration's
+// cluster barrier as soon as the others need nothing more of it: the bulk of
+// the sums runs between a block's arrival and its wait, with the next
+// weights' loads in flight.
+// Bound: the chain of N/32 chunks, each a product, a warp sum, a remote store
+// and a cluster barrier (about 1800 cycles), and in long systems the integer
+// instructions of the sums, which is why a row's partial sums stay in
+// registers (SLOTS > 0) and the weights come as XI.
+// Variants: 8 blocks up to 7 SLOTS + 1 = 29 chunks (N = 928; more blocks would
+// only take SMs from the pair forces beside them), 16 with 8 slots up to 121
+// chunks; beyond, or where 16 blocks do not fit, 8 with the partial sums in
+// memory (SLOTS = 0).
 constexpr int TSC_WARPS = 16;  // warps per block; warp w takes rows w and w + 16 of a chunk
-constexpr int TSC_HB = 8;      // rows whose weights a summing warp loads ahead
+constexpr int TSC_HB = 8;      // SLOTS = 0: rows whose weights a summing warp loads at a time
 
-__host__ __device__ inline int tsc_slots(int nch) { return (nch - 1 + TSC_CL - 2) / (TSC_CL - 1); }
-static size_t tsc_smem(int N) {
-  const size_t b0 = 2 * TS_CHUNK + N + 1;
-  const size_t h = 3 * TS_CHUNK + (size_t)tsc_slots((N + TS_CHUNK - 1) / TS_CHUNK) * TS_CHUNK * 32;
-  return (sizeof(long long) + sizeof(int)) * (b0 > h ? b0 : h) + 16;
-}
-
-__global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
-    k_tri_solve_c(int N, double beta, TriJob job, int first) {
+static size_t tsc_smem(int N) { return (sizeof(long long) + sizeof(int)) * (size_t)(N + 1 + 3 * TS_CHUNK) + 16; }
+template <int CL, int SLOTS>
+__global__ void __launch_bounds__(TSC_WARPS * 32) k_tri_solve_c(int N, double beta, TriJob job, int first) {
   namespace cg = cooperative_groups;
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank();
   const int backward = first + blockIdx.y;
-  const double *__restrict__ Mm = job.Mm[backward];
+  const long long *__restrict__ Mm = (const long long *)job.Mm[backward];
   const int *__restrict__ Me = job.Me[backward];
   const long long *__restrict__ Bgm = (const long long *)job.Bm[backward];
   const int *__restrict__ Bge = job.Be[backward];
@@ -980,76 +980,84 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   constexpr int CC = TS_CHUNK * TS_CHUNK;
   extern __shared__ double sh[];
-  // block 0
-  long long *Ym = (long long *)sh;     // [2][TS_CHUNK]
-  long long *Xm = Ym + 2 * TS_CHUNK;   // N+1
-  int *Ye = (int *)(Xm + N + 1);       // [2][TS_CHUNK]
-  int *Xe = Ye + 2 * TS_CHUNK;         // N+1
-  // blocks 1..TSC_CL-1
-  const int slots = tsc_slots(nch);
-  long long *Hxm = (long long *)sh;        // [2][TS_CHUNK] the last solved chunk's unknowns
-  long long *Hpm = Hxm + 2 * TS_CHUNK;     // [TS_CHUNK] a chunk's completed row sums
-  long long *Ham = Hpm + TS_CHUNK;         // [slots][TS_CHUNK][32] the owned chunks' rows, a partial sum a lane
-  int *Hxe = (int *)(Ham + slots * TS_CHUNK * 32);
-  int *Hpe = Hxe + 2 * TS_CHUNK;
-  int *Hae = Hpe + TS_CHUNK;
-  // two rows a warp of the 32 x 32 block of chunk c, a column a lane
-  long long bm[2];
-  int be[2];
+  // block 0: Y [2][TS_CHUNK], X_0..X_N; the others: the last unknowns
+  // [2][TS_CHUNK], a chunk's completed row sums [TS_CHUNK]
+  long long *Ym = (long long *)sh, *Xm = Ym + 2 * TS_CHUNK, *Hxm = Ym, *Hpm = Xm;
+  int *Ye = (int *)(Ym + N + 1 + 3 * TS_CHUNK), *Xe = Ye + 2 * TS_CHUNK, *Hxe = Ye, *Hpe = Xe;
+  // two rows a warp of the 32 x 32 block of a chunk, a column a lane
+  struct Rows {
+    long long m[2];
+    int e[2];
+  };
   auto load_block = [&](const long long *m, const int *e, int c) {
+    Rows b{{0, 0}, {XI_NONE, XI_NONE}};
+    if (c < nch)
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const size_t o = (size_t)c * CC + (w + h * TSC_WARPS) * TS_CHUNK + lane;
-      bm[h] = m[o];
-      be[h] = e[o];
-    }
+      for (int h = 0; h < 2; ++h) {
+        const size_t o = (size_t)c * CC + (w + h * TSC_WARPS) * TS_CHUNK + lane;
+        b.m[h] = m[o];
+        b.e[h] = e[o];
+      }
+    return b;
   };
-  // summing blocks: rows q = 0, 1, ... of the chunks after c, two a slot from
-  // slot first_slot(c) on, and their weights against the columns from j0 on
-  auto first_slot = [&](int c) { return c + 1 > rank ? (c + 1 - rank + TSC_CL - 2) / (TSC_CL - 1) : 0; };
-  auto row_of = [&](int t0, int q) {
-    const int k = rank + (t0 + q / 2) * (TSC_CL - 1);
-    return 1 + k * TS_CHUNK + w + (q & 1) * TSC_WARPS;
+  // summing blocks: this warp's row h of slot t
+  auto row_of = [&](int t, int h) { return 1 + (rank + t * (CL - 1)) * TS_CHUNK + w + h * TSC_WARPS; };
+  auto weight = [&](int i, int j0) {  // row i's weight against column j0 + lane
+    const size_t o = moff(i, j0 + lane);
+    return i <= N ? XI{Mm[o], Me[o]} : XI{0, XI_NONE};
   };
-  double mv[TSC_HB];
-  int me[TSC_HB];
-  auto load = [&](int t0, int qb, int j0) {
-#pragma unroll
-    for (int u = 0; u < TSC_HB; ++u) {
-      const int i = row_of(t0, qb + u);
-      const bool ok = qb + u < 2 * (slots - t0) && i <= N;
-      const size_t o = ok ? moff(i, j0 + lane) : 0;
-      mv[u] = ok ? Mm[o] : 0.0;
-      me[u] = ok ? Me[o] : 0;
-    }
+  // a + m x for a normalised x; the product may miss one bit of 62
+  auto mul_add = [&](XI a, XI m, XI x) {
+    return xi_add(a, {(long long)__umul64hi((unsigned long long)x.m << 2, (unsigned long long)m.m), m.e + x.e});
   };
+  constexpr int R = SLOTS > 0 ? 2 * SLOTS : 1;
+  XI acc[R], nxt[R];
+  const int slots = tsc_slots(nch, CL);
+  long long *Sm = nullptr;  // SLOTS = 0: partial sums [slots][TS_CHUNK][32] in memory, of this block
+  int *Se = nullptr;
+  Rows blk{{0, 0}, {XI_NONE, XI_NONE}};
   if (rank == 0) {
     if (threadIdx.x == 0) {
       Xm[0] = 1LL << 61;  // X_0 = 1
       Xe[0] = 1;
     }
     // Y_0 = B_0 times the first rows' weights against X_0
-    const XI p = 1 + lane <= N ? xi_from(Mm[moff(1 + lane, 0)], Me[moff(1 + lane, 0)]) : XI{0, XI_NONE};
-    load_block(Bgm, Bge, 0);
+    const XI p = 1 + lane <= N ? XI{Mm[moff(1 + lane, 0)], Me[moff(1 + lane, 0)]} : XI{0, XI_NONE};
+    const Rows b = load_block(Bgm, Bge, 0);
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const XI y = xi_warp_sum(xi_mul({bm[h], be[h]}, p));
+      const XI y = xi_warp_sum(xi_mul({b.m[h], b.e[h]}, p));
       if (lane == 0) {
         Ym[w + h * TSC_WARPS] = y.m;
         Ye[w + h * TSC_WARPS] = y.e;
       }
     }
-    bm[0] = bm[1] = 0;
-    be[0] = be[1] = XI_NONE;  // no chunk before the first
   } else {
-    for (int q = threadIdx.x; q < slots * TS_CHUNK * 32; q += blockDim.x) {
-      const int k = rank + (q / (TS_CHUNK * 32)) * (TSC_CL - 1), i = 1 + k * TS_CHUNK + q / 32 % TS_CHUNK;
-      const XI p = q % 32 == 0 && i <= N ? xi_from(Mm[moff(i, 0)], Me[moff(i, 0)]) : XI{0, XI_NONE};
-      Ham[q] = p.m;
-      Hae[q] = p.e;
+    // the rows' sums start with their weights against X_0, in lane 0
+    auto start = [&](int t, int h) {
+      const int i = row_of(t, h);
+      return lane == 0 && i <= N ? XI{Mm[moff(i, 0)], Me[moff(i, 0)]} : XI{0, XI_NONE};
+    };
+    if (SLOTS > 0) {
+#pragma unroll
+      for (int q = 0; q < R; ++q) {
+        acc[q] = start(q / 2, q & 1);
+        nxt[q] = {0, XI_NONE};
+      }
+    } else {
+      const size_t per = (size_t)slots * TS_CHUNK * 32;
+      Sm = (long long *)job.Sm[backward] + (rank - 1) * per;
+      Se = (int *)((long long *)job.Sm[backward] + (CL - 1) * per) + (rank - 1) * per;
+      for (int q = 0; q < 2 * slots; ++q) {
+        const XI a = start(q / 2, q & 1);
+        const size_t o = ((size_t)(q / 2) * TS_CHUNK + w + (q & 1) * TSC_WARPS) * 32 + lane;
+        Sm[o] = a.m;
+        Se[o] = a.e;
+      }
     }
-    if (rank == 1 && nch > 1) load_block(Bgm, Bge, 1);  // chunk 1's owner
+    if (rank == 1) blk = load_block(Bgm, Bge, 1);  // chunk 1's owner
   }
+  Rows blk2 = rank == 0 ? load_block(Wgm, Wge, 1) : blk;
   cl.sync();  // every block has started and holds its initial sums
   for (int c = 0; c < nch; ++c) {
     const int i0 = 1 + c * TS_CHUNK, buf = c & 1;
@@ -1057,53 +1065,55 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int r = w + h * TSC_WARPS, i = i0 + r;
-        XI x{Ym[buf * TS_CHUNK + r], Ye[buf * TS_CHUNK + r]};
+        const XI y{Ym[buf * TS_CHUNK + r], Ye[buf * TS_CHUNK + r]};
         const XI v = c > 0 ? XI{Xm[i0 - TS_CHUNK + lane], Xe[i0 - TS_CHUNK + lane]} : XI{0, XI_NONE};
-        x = xi_add(x, xi_warp_sum(xi_mul({bm[h], be[h]}, v)));
+        const XI x = xi_add(y, xi_warp_sum(xi_mul({blk.m[h], blk.e[h]}, v)));
         if (i > N) continue;
         if (lane == 0) {
           Xm[i] = x.m;
           Xe[i] = x.e;
-        } else if (lane < TSC_CL) {
+        } else if (lane < CL) {
           *cl.map_shared_rank(Hxm + buf * TS_CHUNK + r, lane) = x.m;
           *cl.map_shared_rank(Hxe + buf * TS_CHUNK + r, lane) = x.e;
         }
       }
       cl.barrier_arrive();
-      if (c + 1 < nch) load_block(Wgm, Wge, c + 1);
+      blk = blk2;  // W_{c+1}, loaded an iteration ago
+      blk2 = load_block(Wgm, Wge, c + 2);
     } else {
-      const int j0 = i0 - TS_CHUNK, pb = (c - 1) & 1, t0 = first_slot(c), nq = 2 * (slots - t0);
+      // chunk c-1's unknowns, columns j0 on
+      const int j0 = i0 - TS_CHUNK;
       XI x{0, XI_NONE};
-      if (c >= 1) x = {Hxm[pb * TS_CHUNK + lane], Hxe[pb * TS_CHUNK + lane]};
-      // chunk c-1's unknowns into row q of the chunks after c
-      auto add_row = [&](int q, double m, int e) {
-        const int o = ((t0 + q / 2) * TS_CHUNK + w + (q & 1) * TSC_WARPS) * 32 + lane;
-        const XI a = xi_add({Ham[o], Hae[o]}, xi_mul(xi_from(m, e), x));
-        Ham[o] = a.m;
-        Hae[o] = a.e;
-      };
-      // the owner of chunk c+1 (its rows are q = 0 and 1) completes them, now
-      // over the unknowns before chunk c, and hands Y_{c+1} to block 0
-      const int kn = c + 1;
-      const bool owner = kn < nch && 1 + (kn - 1) % (TSC_CL - 1) == rank;
-      int q0 = 0;
+      if (c >= 1) x = {Hxm[(buf ^ 1) * TS_CHUNK + lane], Hxe[(buf ^ 1) * TS_CHUNK + lane]};
+      // the owner of chunk c+1 completes that chunk's rows, now over the
+      // unknowns before chunk c, and hands Y_{c+1} to block 0
+      const int kn = c + 1, tn = (kn - 1) / (CL - 1);
+      const bool owner = kn < nch && kn - tn * (CL - 1) == rank;
+      // first slot whose chunk comes after c
+      const int t0 = c + 1 > rank ? (c + 1 - rank + CL - 2) / (CL - 1) : 0;
       if (owner) {
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int r = w + h * TSC_WARPS;
-          if (c >= 1 && row_of(t0, h) <= N) add_row(h, mv[h], me[h]);
-          const int o = (t0 * TS_CHUNK + r) * 32 + lane;
-          const XI p = xi_warp_sum({Ham[o], Hae[o]});
+          XI p{0, XI_NONE};
+          if (SLOTS > 0) {
+#pragma unroll
+            for (int t = 0; t < SLOTS; ++t)
+              if (t == tn) p = mul_add(acc[2 * t + h], nxt[2 * t + h], x);
+          } else {
+            const size_t o = ((size_t)tn * TS_CHUNK + w + h * TSC_WARPS) * 32 + lane;
+            p = {Sm[o], Se[o]};
+            if (c >= 1) p = mul_add(p, weight(row_of(tn, h), j0), x);
+          }
+          p = xi_warp_sum(p);
           if (lane == 0) {
-            Hpm[r] = p.m;
-            Hpe[r] = p.e;
+            Hpm[w + h * TSC_WARPS] = p.m;
+            Hpe[w + h * TSC_WARPS] = p.e;
           }
         }
-        q0 = 2;
         __syncthreads();
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const XI y = xi_warp_sum(xi_mul({bm[h], be[h]}, {Hpm[lane], Hpe[lane]}));
+          const XI y = xi_warp_sum(xi_mul({blk.m[h], blk.e[h]}, {Hpm[lane], Hpe[lane]}));
           if (lane == 0) {
             *cl.map_shared_rank(Ym + (kn & 1) * TS_CHUNK + w + h * TSC_WARPS, 0) = y.m;
             *cl.map_shared_rank(Ye + (kn & 1) * TS_CHUNK + w + h * TSC_WARPS, 0) = y.e;
@@ -1111,50 +1121,96 @@ __global__ void __cluster_dims__(TSC_CL, 1, 1) __launch_bounds__(TSC_WARPS * 32)
         }
       }
       cl.barrier_arrive();
-      if (c >= 1)
-        for (int qb = 0; qb < nq; qb += TSC_HB) {
-          if (qb > 0) load(t0, qb, j0);
+      if (SLOTS > 0) {
+#pragma unroll
+        for (int q = 0; q < R; ++q) {
+          if (q / 2 < t0) continue;
+          if (c >= 1) acc[q] = mul_add(acc[q], nxt[q], x);
+          nxt[q] = weight(row_of(q / 2, q & 1), i0);
+        }
+      } else if (c >= 1) {
+        for (int qb = 2 * (owner ? t0 + 1 : t0); qb < 2 * slots; qb += TSC_HB) {
+          XI m[TSC_HB];
+#pragma unroll
+          for (int u = 0; u < TSC_HB; ++u)
+            m[u] = qb + u < 2 * slots ? weight(row_of((qb + u) / 2, u & 1), j0) : XI{0, XI_NONE};
 #pragma unroll
           for (int u = 0; u < TSC_HB; ++u) {
             const int q = qb + u;
-            if (q >= nq || row_of(t0, q) > N) break;  // warp-uniform
-            if (q >= q0) add_row(q, mv[u], me[u]);
+            if (q >= 2 * slots) break;
+            const size_t o = ((size_t)(q / 2) * TS_CHUNK + w + (q & 1) * TSC_WARPS) * 32 + lane;
+            const XI a = mul_add({Sm[o], Se[o]}, m[u], x);
+            Sm[o] = a.m;
+            Se[o] = a.e;
           }
         }
-      if (kn < nch) load(first_slot(kn), 0, i0);
-      if (kn + 1 < nch && 1 + kn % (TSC_CL - 1) == rank) load_block(Bgm, Bge, kn + 1);
+      }
+      const int k2 = c + 2, t2 = (k2 - 1) / (CL - 1);
+      if (k2 < nch && k2 - t2 * (CL - 1) == rank) blk = load_block(Bgm, Bge, k2);
     }
     cl.barrier_wait();
   }
-  // V_B = -ln X / beta: an eighth of the unknowns a block, read from block 0
-  {
-    const long long *xm = cl.map_shared_rank(Xm, 0);
-    const int *xe = cl.map_shared_rank(Xe, 0);
-    tri_solve_out(N, beta, job, backward, xm, xe, rank * blockDim.x + threadIdx.x, TSC_CL * blockDim.x);
-  }
+  // V_B = -ln X / beta: the unknowns dealt over the blocks, read from block 0
+  tri_solve_out(N, beta, job, backward, cl.map_shared_rank(Xm, 0), cl.map_shared_rank(Xe, 0),
+                threadIdx.x * CL + rank, CL * blockDim.x);
   cl.sync();  // block 0's shared memory is read until here
 }
 
-// whether a cluster of the block solve fits on this device with `smem`
-// bytes of shared memory per block (checked once per larger size)
-static bool cluster_solve_fits(size_t smem) {
-  static size_t checked = 0;
-  static bool fits = false;
-  if (smem <= checked) return fits;
-  if (cudaFuncSetAttribute(k_tri_solve_c, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(TSC_CL, 2);
+// the variant for N that fits this device: 0 none, 1 eight blocks, 2 sixteen,
+// 3 eight with the sums in memory
+struct ClusterKernel {
+  void (*fn)(int, double, TriJob, int);
+  int cl;
+};
+static const ClusterKernel g_cluster_kernels[4] = {
+    {nullptr, 0}, {k_tri_solve_c<8, 4>, 8}, {k_tri_solve_c<16, 8>, 16}, {k_tri_solve_c<8, 0>, 8}};
+
+static void cluster_config(const ClusterKernel &k, int N, int count, cudaStream_t st, cudaLaunchConfig_t &cfg,
+                           cudaLaunchAttribute &attr) {
+  cfg = {};
+  cfg.gridDim = dim3(k.cl, count);
   cfg.blockDim = dim3(TSC_WARPS * 32);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = tsc_smem(N);
+  cfg.stream = st;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = k.cl;
+  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+}
+
+// whether two clusters of the variant fit at once with N's shared memory (the
+// largest that did and the smallest that did not are kept)
+static bool cluster_fits(int v, int N) {
+  static std::mutex mu;
+  static size_t good[4] = {0, 0, 0, 0}, bad[4] = {~(size_t)0, ~(size_t)0, ~(size_t)0, ~(size_t)0};
+  const size_t smem = tsc_smem(N);
+  std::lock_guard<std::mutex> lk(mu);
+  if (smem <= good[v]) return true;
+  if (smem >= bad[v]) return false;
+  const ClusterKernel &k = g_cluster_kernels[v];
   int n = 0;
-  const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, (void *)k_tri_solve_c, &cfg);
+  cudaError_t e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess && k.cl > 8) e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    cluster_config(k, N, 2, nullptr, cfg, attr);
+    e = cudaOccupancyMaxActiveClusters(&n, (const void *)k.fn, &cfg);
+  }
   if (e != cudaSuccess) cudaGetLastError();
-  fits = e == cudaSuccess && n >= 2;
-  checked = smem;
-  return fits;
+  if (e == cudaSuccess && n >= 2) {
+    good[v] = smem;
+    return true;
+  }
+  bad[v] = smem;
+  return false;
+}
+static int cluster_variant(int N) {
+  const int nch = (N + TS_CHUNK - 1) / TS_CHUNK;
+  if (nch <= 29) return cluster_fits(1, N) ? 1 : 0;
+  if (nch <= 121 && cluster_fits(2, N)) return 2;
+  return cluster_fits(3, N) ? 3 : 0;
 }
 
 // Which kernel solves the unsigned recursions: SOLVE_AUTO picks by size
@@ -1190,23 +1246,29 @@ int solve_choice(int N) {
   return (N + TS_CHUNK - 1) / TS_CHUNK > 4 ? SOLVE_CLUSTER : SOLVE_BLOCK;
 }
 
-// whether the unsigned solve of N takes the cluster; *bad: it was forced, but
-// no cluster of this size fits
-static bool takes_cluster(int N, bool *bad) {
-  const bool want = solve_choice(N) == SOLVE_CLUSTER, fits = want && cluster_solve_fits(tsc_smem(N));
-  *bad = want && !fits && g_solve_force == SOLVE_CLUSTER;
-  return fits;
+// the cluster variant that the unsigned solve of N takes (0: the block solve);
+// *bad: the cluster was forced, but none fits
+static int takes_cluster(int N, bool *bad) {
+  const bool want = solve_choice(N) == SOLVE_CLUSTER;
+  const int v = want ? cluster_variant(N) : 0;
+  *bad = want && !v && g_solve_force == SOLVE_CLUSTER;
+  return v;
 }
 
 static cudaError_t tri_solve(int N, double beta, const TriJob &job, int first, int count, cudaStream_t st,
-                             bool cluster = false) {
+                             int cluster = 0) {
   if (!job.sign) {
     // unsigned weights: the block solve (the diagonal-block inverses came
     // with the weights, k_weights_inv)
     if (cluster) {
       {
         XK_PROF(count == 2 ? "vb_tv_solve" : (first ? "tv_solve" : "vb_solve"));
-        k_tri_solve_c<<<dim3(TSC_CL, count), TSC_WARPS * 32, tsc_smem(N), st>>>(N, beta, job, first);
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr;
+        const ClusterKernel &k = g_cluster_kernels[cluster];
+        cluster_config(k, N, count, st, cfg, attr);
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, k.fn, N, beta, job, first);
+        if (e != cudaSuccess) return e;
       }
       return XK_LAUNCHED();
     }
@@ -1249,8 +1311,9 @@ TriJob tri_job(int N, double *rs_f, double *rs_b, double *VBN, double *tmpV) {
     j.Be[d] = (int *)(b + nb);
     j.Wm[d] = b + nb + nb / 2;
     j.We[d] = (int *)(j.Wm[d] + nb);
-    j.Xm[d] = j.Wm[d] + nb + nb / 2;
+    j.Xm[d] = (long long *)(j.Wm[d] + nb + nb / 2);
     j.Xe[d] = (int *)(j.Xm[d] + N + 1);
+    j.Sm[d] = (double *)j.Xm[d] + N + 1 + (N + 2) / 2;
   }
   j.Mm[0] = rs_f;
   j.Me[0] = (const int *)(rs_f + ntri(N));
@@ -1267,7 +1330,7 @@ static cudaError_t weights_solve(int N, double beta, double vi, const double *EN
                                  const TriJob &job, int first, int count, cudaStream_t st) {
   const double lnvi = vi != 0.0 ? log(vi) : 0.0;
   bool bad;
-  const bool cluster = takes_cluster(N, &bad);
+  const int cluster = takes_cluster(N, &bad);
   if (bad) return cudaErrorInvalidConfiguration;
   const int groups = cluster ? 16 : 8, nch = (N + TS_CHUNK - 1) / TS_CHUNK;  // four columns of B or W a block
   {
@@ -1354,15 +1417,14 @@ cudaError_t fill_g(int N, double beta, double vi, const double *ENk, const doubl
 // exp(-beta(V_B^(j-1) + E + tmpV[l] - V_B^(N))) loses beta V_B^(N) ulps to the
 // cancellation inside the exponent (up to ~1e-10 relative at N = 512).
 
-__global__ void k_fill_g_ext(int N, const double *__restrict__ Mm, const int *__restrict__ Me,
-                             const double *__restrict__ Xfm, const int *__restrict__ Xfe,
-                             const double *__restrict__ Xbm, const int *__restrict__ Xbe, double *__restrict__ G) {
+__global__ void k_fill_g_ext(int N, TriJob job, double *__restrict__ G) {
   const int l = blockIdx.y + 1;  // 1-based row
-  double q;
-  int qe;
-  g_ext_row(N, Xfm, Xfe, Xbm, Xbe, l, q, qe);
+  __shared__ XI qs;
+  if (threadIdx.x == 0) qs = xi_mul({job.Xm[1][N - l], job.Xe[1][N - l]}, g_ext_inv(N, job));
+  __syncthreads();
+  const XI q = qs;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x + 1; j <= N; j += gridDim.x * blockDim.x)
-    g_ext_elem(N, Mm, Me, Xfm, Xfe, q, qe, G, l, j);
+    G[(size_t)(l - 1) * N + (j - 1)] = g_ext_elem(job, q, l, j);
 }
 
 cudaError_t fill_g_ext(int N, const double *rs_f, const double *rs_b, double *G, cudaStream_t st) {
@@ -1370,7 +1432,7 @@ cudaError_t fill_g_ext(int N, const double *rs_f, const double *rs_b, double *G,
   dim3 grid((N + 255) / 256, N);
   {
     XK_PROF("fill_g");
-    k_fill_g_ext<<<grid, 256, 0, st>>>(N, j.Mm[0], j.Me[0], j.Xm[0], j.Xe[0], j.Xm[1], j.Xe[1], G);
+    k_fill_g_ext<<<grid, 256, 0, st>>>(N, j, G);
   }
   return XK_LAUNCHED();
 }
