@@ -1652,11 +1652,16 @@ __device__ inline void pair_eval(const PairPrm &p, const Geo &g, const double *d
       if (KIND == PAIR_PERIODIC_GAUSSIAN) t[d] = min_image(t[d], g.box[d], g.inv_box[d]);
       r2 += t[d] * t[d];
     }
-    const double s2 = p.s * p.s;
-    const double mult = (p.g / (M_PI * s2)) * exp(-r2 / s2);
+    // r^2 / s^2 by the reciprocal and one residual step (a correctly rounded
+    // quotient without an FP64 division), the exponential on the integer
+    // pipe: about 15 FP64 instructions a pair where exp() and four divisions
+    // took over a hundred
+    const double q = r2 * p.is2;
+    const double ex = exp_fast(-fma(fma(-q, p.s * p.s, r2), p.is2, q));
+    const double mult = p.g2 * ex;
 #pragma unroll
-    for (int d = 0; d < D; ++d) F[d] = mult * (2 * t[d]) / s2;
-    if (want_e) E = mult;
+    for (int d = 0; d < D; ++d) F[d] = mult * t[d];
+    if (want_e) E = p.g0 * ex;
   } else if (KIND == PAIR_COULOMB || KIND == PAIR_PERIODIC_COULOMB) {
     double t[D], r2 = 0;
 #pragma unroll
@@ -1850,20 +1855,103 @@ __device__ inline void pair_eval(const PairPrm &p, const Geo &g, const double *d
   }
 }
 
+// The Gaussian and Coulomb kinds: a warp takes one of `split` equal parts of a
+// 32 x 32 tile's rotation steps (lane l meets bead (l + s) mod 32 of the other
+// tile in step s; tiles on the diagonal visit each pair once, steps 1..16),
+// so that a small system still gives every SM sub-partition a warp: the
+// kernel is bound by the FP64 instructions' latency there, 64 cycles each in
+// a dependent chain.  Partials go to slot t * split + part of the other tile
+// t (of its own tile on the diagonal), summed by k_pair_finish.
 template <int D, int KIND, bool ENERGY>
+__global__ void __launch_bounds__(256) k_pair_split(Geo g, PairPrm p, const double *__restrict__ x,
+                                                    const double *__restrict__ m, double *__restrict__ out, int T,
+                                                    int jobs, int split) {
+  const int lane = threadIdx.x & 31, nwarps = (gridDim.x * blockDim.x) >> 5;
+  for (int w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; w < jobs * g.P * split; w += nwarps) {
+    const int part = w % split, j = w / split / jobs;
+    int job = w / split % jobs, I = 0;
+    while (job >= T - I) {
+      job -= T - I;
+      ++I;
+    }
+    const int J = I + job;
+    const bool diag = I == J;
+    const int a = I * 32 + lane, b = J * 32 + lane, nb = min(32, g.N - J * 32);
+    const bool va = a < g.N, vb = lane < nb;
+    double xa[D], xb[D], fa[D], fb[D], ea = 0;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      xa[d] = va ? x[sidx(j, d, a, D, g.Ns)] : 0.0;
+      xb[d] = vb ? x[sidx(j, d, b, D, g.Ns)] : 0.0;
+      fa[d] = fb[d] = 0.0;
+    }
+    const double ima = !ENERGY && va ? 1.0 / m[(size_t)j * g.Ns + a] : 1.0;
+    const double imb = !ENERGY && vb ? 1.0 / m[(size_t)j * g.Ns + b] : 1.0;
+    const int s0 = diag ? 1 + part * 16 / split : part * 32 / split;
+    const int s1 = diag ? 1 + (part + 1) * 16 / split : (part + 1) * 32 / split;
+    for (int s = s0; s < s1; ++s) {
+      if (diag && s >= nb && s + nb <= 32) continue;  // no pair of the tile's nb beads in this step
+      const int from = (lane + s) & 31, back = (lane - s) & 31;
+      const bool act = va && from < nb && !(diag && s == 16 && lane >= 16);
+      double dx[D], F[D], E = 0;
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        dx[d] = xa[d] - __shfl_sync(FULL, xb[d], from);
+        F[d] = 0;
+      }
+      const double im2 = __shfl_sync(FULL, imb, from);
+      if (act) pair_eval<D, KIND, ENERGY>(p, g, dx, nullptr, F, E, ENERGY, nullptr, true, nullptr, lane);
+      if constexpr (ENERGY) {
+        ea += E;
+      } else {
+        // the reference divides by the mass of the higher-index particle
+        const double inv = a > J * 32 + from ? ima : im2;
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+          F[d] *= inv;
+          fa[d] += F[d];
+          fb[d] -= __shfl_sync(FULL, F[d], back);
+        }
+      }
+    }
+    if constexpr (ENERGY) {
+      ea = warp_sum(ea);
+      if (lane == 0) out[w] = ea;
+    } else {
+      // slot layout: out[((t*P + j)*D + d)*Ns + l]
+#pragma unroll
+      for (int d = 0; d < D; ++d) {
+        if (va) out[(((size_t)(J * split + part) * g.P + j) * D + d) * g.Ns + a] = diag ? fa[d] + fb[d] : fa[d];
+        if (vb && !diag) out[(((size_t)(I * split + part) * g.P + j) * D + d) * g.Ns + b] = fb[d];
+      }
+    }
+  }
+}
+
+constexpr int PAIR_SPLIT_MAX = 8;
+// parts of a tile: enough that every SM sub-partition has two warps
+static int pair_split(const Geo &g, int jobs) {
+  int split = 1;
+  while (split < PAIR_SPLIT_MAX && (size_t)jobs * g.P * split < 2 * 4 * 152) split *= 2;
+  return split;
+}
+
+// real-space Ewald (3D): a warp per tile, partner data rotated through the lanes
+template <bool ENERGY>
 __global__ void __launch_bounds__(256, 2) k_pair_tiles(Geo g, PairPrm p,
                                                     const double *__restrict__ x,
                                                     const double *__restrict__ m,
                                                     double *__restrict__ out, int T, int jobs) {
+  constexpr int D = 3, KIND = PAIR_EWALD_REAL;
   // Ewald polynomial tables staged in shared memory (lanes index them freely)
-  extern __shared__ double stab[];  // Ewald: the two tables (EW_TAB_BYTES of dynamic shared memory)
-  if (KIND == PAIR_EWALD_REAL) {
+  extern __shared__ double stab[];  // the two tables (EW_TAB_BYTES of dynamic shared memory)
+  {
     for (int i = threadIdx.x; i < 2 * EW_NINT * (EW_DEG + 1); i += blockDim.x)
       stab[i] = i < EW_NINT * (EW_DEG + 1) ? (&c_ew_h[0][0])[i] : (&c_ew_erfc[0][0])[i - EW_NINT * (EW_DEG + 1)];
     __syncthreads();
   }
-  __shared__ EwWarp ewq[KIND == PAIR_EWALD_REAL ? 8 : 1];
-  EwWarp *ews = &ewq[KIND == PAIR_EWALD_REAL ? (threadIdx.x >> 5) : 0];
+  __shared__ EwWarp ewq[8];
+  EwWarp *ews = &ewq[threadIdx.x >> 5];
   const int lane = threadIdx.x & 31;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   // warps loop over the tile jobs (slice j, tile pair I <= J) round-robin, so
@@ -1892,7 +1980,7 @@ __global__ void __launch_bounds__(256, 2) k_pair_tiles(Geo g, PairPrm p,
     }
     // inverse masses, so that each pair multiplies instead of dividing
     // (Ewald forces: times the strength, and FP32 copies for the far images)
-    constexpr bool EWF = KIND == PAIR_EWALD_REAL && !ENERGY;
+    constexpr bool EWF = !ENERGY;
     const double ima = (!ENERGY && va) ? (EWF ? p.qs : 1.0) / m[(size_t)j * g.Ns + a] : 1.0;
     double imb = (!ENERGY && vb) ? (EWF ? p.qs : 1.0) / m[(size_t)j * g.Ns + b0] : 1.0;
     const float ima32 = EWF ? (float)ima : 0.f;
@@ -1910,10 +1998,8 @@ __global__ void __launch_bounds__(256, 2) k_pair_tiles(Geo g, PairPrm p,
         dxf[d] = xaf[d] - xbf[d];
         F[d] = 0;
       }
-      if (KIND == PAIR_EWALD_REAL) pair_eval<D, KIND, ENERGY>(p, g, dx, dxf, F, E, ENERGY, stab, act, ews, lane, G);
+      pair_eval<D, KIND, ENERGY>(p, g, dx, dxf, F, E, ENERGY, stab, act, ews, lane, G);
       if (act) {
-        if (KIND != PAIR_EWALD_REAL)
-          pair_eval<D, KIND, ENERGY>(p, g, dx, dxf, F, E, ENERGY, stab, true, nullptr, lane);
         if (ENERGY) {
           ea += E;
         } else {
@@ -1938,7 +2024,7 @@ __global__ void __launch_bounds__(256, 2) k_pair_tiles(Geo g, PairPrm p,
 #pragma unroll
       for (int d = 0; d < D; ++d) {
         xb[d] = __shfl_sync(FULL, xb[d], src);
-        if (KIND == PAIR_EWALD_REAL) xbf[d] = __shfl_sync(FULL, xbf[d], src);
+        xbf[d] = __shfl_sync(FULL, xbf[d], src);
         if (!ENERGY) fb[d] = __shfl_sync(FULL, fb[d], src);
         if (EWF) gb[d] = __shfl_sync(FULL, gb[d], src);
       }
@@ -2108,9 +2194,11 @@ size_t pair_scratch_doubles(const Geo &g) {
   // partial slots (doubles, or float2 in the FP32 form), then room for the
   // FP32 form's copies of the positions and inverse masses
   size_t a = (size_t)T * g.slots() + (g.slots() + (size_t)g.P * g.Ns + 1) / 2 + 1;
+  const int split = pair_split(g, (int)jobs);
+  if (a < (size_t)T * split * g.slots()) a = (size_t)T * split * g.slots();
   const size_t d = g.D == 3 ? (size_t)T * g.slots() + 1 + ewd_pos_doubles(g) : 0;
   if (d > a) a = d;
-  size_t b = jobs * g.P;
+  size_t b = jobs * g.P * split;
   return a > b ? a : b;
 }
 
@@ -2152,22 +2240,26 @@ int tuning(int what, int kind, int D, int N, int P) {
   return 0;
 }
 
-// the FP64 tile kernels' persistent grid: blocks per SM as tuned for this
+// the FP64 Ewald tiles' persistent grid: blocks per SM as tuned for this
 // shape (TUNE_PAIR64_BPS), else as many as stay resident
-template <int D, int KIND, bool ENERGY>
+template <bool ENERGY>
 static int pair_grid(size_t warps_needed, const Geo &g) {
   static int occ = 0, sms = 0;
-  const int full = resident_grid(k_pair_tiles<D, KIND, ENERGY>, warps_needed, occ, sms,
-                                 KIND == PAIR_EWALD_REAL ? EW_TAB_BYTES : 0);
-  const int bps = tuning(TUNE_PAIR64_BPS, KIND, D, g.N, g.P);
+  const int full = resident_grid(k_pair_tiles<ENERGY>, warps_needed, occ, sms, EW_TAB_BYTES);
+  const int bps = tuning(TUNE_PAIR64_BPS, PAIR_EWALD_REAL, 3, g.N, g.P);
   if (bps > 0 && bps < occ) return full < sms * bps ? full : sms * bps;
   return full;
 }
 
-// the Ewald kernels' derived constants (PairPrm::rc2 ... iboxf), computed
-// once per launch instead of per pair
+// the kernels' derived constants (PairPrm::rc2 ... g2), computed once per
+// launch instead of per pair
 PairPrm with_far_images(const PairPrm &p, const Geo &g) {
   PairPrm q = p;
+  if (p.s > 0) {
+    q.is2 = 1.0 / (p.s * p.s);
+    q.g0 = p.g / (M_PI * p.s * p.s);
+    q.g2 = q.g0 * 2 / (p.s * p.s);
+  }
   q.rc2 = p.rcut * p.rcut;
   q.alphaf = (float)p.alpha;
   q.rcf2 = (float)q.rc2;
@@ -2181,41 +2273,48 @@ PairPrm with_far_images(const PairPrm &p, const Geo &g) {
   return q;
 }
 
+template <int D, int KIND, bool ENERGY>
+static void launch_split(const Geo &g, const PairPrm &p, const double *x, const double *m, double *out, int T, int jobs,
+                         int split, cudaStream_t st) {
+  static int occ = 0, sms = 0;
+  const int full = resident_grid(k_pair_split<D, KIND, ENERGY>, (size_t)jobs * g.P * split, occ, sms);
+  const int bps = tuning(TUNE_PAIR64_BPS, KIND, D, g.N, g.P);
+  const int grid = bps > 0 && bps < occ && full > sms * bps ? sms * bps : full;
+  k_pair_split<D, KIND, ENERGY><<<grid, 256, 0, st>>>(g, p, x, m, out, T, jobs, split);
+}
+
+// split: parts of a tile (all but Ewald)
 template <int D, bool ENERGY>
 static cudaError_t pair_launch(const Geo &g, const PairPrm &p_in, const double *x, const double *m,
-                               double *out, int T, int jobs, cudaStream_t st) {
+                               double *out, int T, int jobs, int split, cudaStream_t st) {
   const PairPrm p = with_far_images(p_in, g);
   const size_t warps = (size_t)jobs * g.P;
   switch (p.kind) {
-    case PAIR_GAUSSIAN:
-      {
-        XK_PROF("pair_tiles_gauss");
-        k_pair_tiles<D, PAIR_GAUSSIAN, ENERGY><<<pair_grid<D, PAIR_GAUSSIAN, ENERGY>(warps, g), 256, 0, st>>>(g, p, x, m, out, T, jobs);
-      }
+    case PAIR_GAUSSIAN: {
+      XK_PROF("pair_tiles_gauss");
+      launch_split<D, PAIR_GAUSSIAN, ENERGY>(g, p, x, m, out, T, jobs, split, st);
       break;
-    case PAIR_PERIODIC_GAUSSIAN:
-      {
-        XK_PROF("pair_tiles_pgauss");
-        k_pair_tiles<D, PAIR_PERIODIC_GAUSSIAN, ENERGY><<<pair_grid<D, PAIR_PERIODIC_GAUSSIAN, ENERGY>(warps, g), 256, 0, st>>>(g, p, x, m, out, T, jobs);
-      }
+    }
+    case PAIR_PERIODIC_GAUSSIAN: {
+      XK_PROF("pair_tiles_pgauss");
+      launch_split<D, PAIR_PERIODIC_GAUSSIAN, ENERGY>(g, p, x, m, out, T, jobs, split, st);
       break;
-    case PAIR_COULOMB:
-      {
-        XK_PROF("pair_tiles_coul");
-        k_pair_tiles<D, PAIR_COULOMB, ENERGY><<<pair_grid<D, PAIR_COULOMB, ENERGY>(warps, g), 256, 0, st>>>(g, p, x, m, out, T, jobs);
-      }
+    }
+    case PAIR_COULOMB: {
+      XK_PROF("pair_tiles_coul");
+      launch_split<D, PAIR_COULOMB, ENERGY>(g, p, x, m, out, T, jobs, split, st);
       break;
-    case PAIR_PERIODIC_COULOMB:
-      {
-        XK_PROF("pair_tiles_pcoul");
-        k_pair_tiles<D, PAIR_PERIODIC_COULOMB, ENERGY><<<pair_grid<D, PAIR_PERIODIC_COULOMB, ENERGY>(warps, g), 256, 0, st>>>(g, p, x, m, out, T, jobs);
-      }
+    }
+    case PAIR_PERIODIC_COULOMB: {
+      XK_PROF("pair_tiles_pcoul");
+      launch_split<D, PAIR_PERIODIC_COULOMB, ENERGY>(g, p, x, m, out, T, jobs, split, st);
       break;
+    }
     case PAIR_EWALD_REAL:
       if (D != 3) return cudaErrorInvalidValue;
       {
         XK_PROF("pair_tiles_ewald_real");
-        k_pair_tiles<D, PAIR_EWALD_REAL, ENERGY><<<pair_grid<D, PAIR_EWALD_REAL, ENERGY>(warps, g), 256, EW_TAB_BYTES, st>>>(g, p, x, m, out, T, jobs);
+        k_pair_tiles<ENERGY><<<pair_grid<ENERGY>(warps, g), 256, EW_TAB_BYTES, st>>>(g, p, x, m, out, T, jobs);
       }
       break;
     default:
@@ -2228,13 +2327,13 @@ cudaError_t pair_force(const Geo &g, const PairPrm &p, const double *x, const do
                        double *f, double *scratch, cudaStream_t st) {
   if (p.inv_mass > 0 && ewd_applies(g, p, false)) return ewd_force(g, p, x, f, scratch, st);
   const int T = (g.N + 31) / 32;
-  const int jobs = T * (T + 1) / 2;
+  const int jobs = T * (T + 1) / 2, split = p.kind == PAIR_EWALD_REAL ? 1 : pair_split(g, jobs);
   cudaError_t e;
-  DISPATCH_D(g.D, e = (pair_launch<D, false>(g, p, x, m, scratch, T, jobs, st)));
+  DISPATCH_D(g.D, e = (pair_launch<D, false>(g, p, x, m, scratch, T, jobs, split, st)));
   if (e != cudaSuccess) return e;
   {
     XK_PROF("pair_finish");
-    k_pair_finish<<<cdiv(g.slots(), 256), 256, 0, st>>>(g, scratch, T, 1.0 / g.P, f);
+    k_pair_finish<<<cdiv(g.slots(), 256), 256, 0, st>>>(g, scratch, T * split, 1.0 / g.P, f);
   }
   return XK_LAUNCHED();
 }
@@ -2243,13 +2342,15 @@ cudaError_t pair_energy(const Geo &g, const PairPrm &p, const double *x, double 
                         double *scratch, cudaStream_t st) {
   const int T = (g.N + 31) / 32;
   const int jobs = T * (T + 1) / 2;
+  int split = 1;
   cudaError_t e;
   double unit = 1.0;
   if (ewd_applies(g, p, true)) {
     e = ewd_energy_tiles(g, p, x, scratch, st);
     unit = p.qs * p.alpha;
   } else {
-    DISPATCH_D(g.D, e = (pair_launch<D, true>(g, p, x, nullptr, scratch, T, jobs, st)));
+    if (p.kind != PAIR_EWALD_REAL) split = pair_split(g, jobs);
+    DISPATCH_D(g.D, e = (pair_launch<D, true>(g, p, x, nullptr, scratch, T, jobs, split, st)));
   }
   if (e != cudaSuccess) return e;
   // the Ewald energy carries -pi/(alpha^2 V) per pair (md_statistics_x.c:385)
@@ -2258,7 +2359,7 @@ cudaError_t pair_energy(const Geo &g, const PairPrm &p, const double *x, double 
     const double V = g.box[0] * g.box[1] * g.box[2];
     add = -p.qs * M_PI / (p.alpha * p.alpha * V) * ((double)g.N * (g.N - 1) / 2);
   }
-  return reduce_into(scratch, jobs * g.P, unit / g.P, add, acc, st);
+  return reduce_into(scratch, jobs * g.P * split, unit / g.P, add, acc, st);
 }
 
 size_t pair2_scratch_doubles(const Geo &ga, const Geo &gb) {
@@ -3451,9 +3552,9 @@ namespace xk {
 // Pair forces without any allocation (md_gb300_pair_force_noalloc_x).
 //
 // For callers that may not allocate device memory, the per-tile partial
-// forces of k_pair_tiles go to this fixed array instead of a buffer from
+// forces of k_pair_split go to this fixed array instead of a buffer from
 // the allocator.  It lives in every GPU that loads the library, until the
-// process exits.  k_pair_tiles writes every element that k_pair_finish reads,
+// process exits.  k_pair_split writes every element that k_pair_finish reads,
 // so nothing in it has to start at zero; concurrent calls share it and
 // therefore must not overlap on the GPU.
 // ===================================================================
@@ -3492,10 +3593,11 @@ cudaError_t pair_force_noalloc(const Geo &g, const PairPrm &p, const double *x, 
   const int T = (g.N + 31) / 32;
   const int jobs = T * (T + 1) / 2;
   const int nb = cdiv((size_t)jobs * g.P * 32, 256);
+  const PairPrm q = with_far_images(p, g);
   switch (g.D * 16 + p.kind) {
 #define XK_NOALLOC_CASE(DV, K)                                                                   \
   case DV * 16 + K:                                                                              \
-    k_pair_tiles<DV, K, false><<<nb, 256, 0, st>>>(g, p, x, m, scratch, T, jobs);                \
+    k_pair_split<DV, K, false><<<nb, 256, 0, st>>>(g, q, x, m, scratch, T, jobs, 1);             \
     break;
     XK_NOALLOC_CASE(1, PAIR_GAUSSIAN)
     XK_NOALLOC_CASE(1, PAIR_PERIODIC_GAUSSIAN)

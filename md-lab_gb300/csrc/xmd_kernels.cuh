@@ -187,6 +187,8 @@ struct PairPrm {
   float rcf2;           // rcut^2
   float rcf2_cull;      // rcut^2 (1 + 1e-4): the FP32 culling's margin
   float boxf[3], iboxf[3];  // box lengths and their inverses
+  // and for the Gaussian kinds
+  double is2, g0, g2;  // 1/s^2, g / (pi s^2), 2 g / (pi s^4)
 };
 // alpha R at and beyond which the FP64 kernels evaluate real-space Ewald
 // images on the FP32 pipe (every image there has h(alpha R) < 5.2e-7, and
