@@ -65,7 +65,7 @@ int md_gb300_graph_launch_x(md_gb300_graph_t_x *graph, int count);
 typedef int (*md_gb300_system_step_fn_x)(int system, void *ctx);
 int md_gb300_capture_ensemble_x(int n, md_gb300_system_step_fn_x step, void *ctx, md_gb300_graph_t_x **graph);
 /* The same ensemble step as ONE persistent kernel launch (captured into a
-   graph): the step's stages are nine phases, each holding that stage's work
+   graph): the step's stages are eight phases, each holding that stage's work
    of every system of a group of blocks spread over the group, separated by
    the group's barriers
    (a cooperative launch of exactly the blocks that fit; a barrier wait that

@@ -496,8 +496,10 @@ struct TriJob {
   double *Wm[2];
   int *We[2];
   double *Sm[2];  // partial sums of the cluster solve of very long systems
-  long long *Xm[2];  // optional: the unknowns X_0..X_N as XI (unsigned solves),
-  int *Xe[2];        // kept for the connection probabilities
+  // optional: the unknowns X_0..X_N as XI (unsigned solves) and, last, 1/X_N,
+  // kept for the connection probabilities
+  long long *Xm[2];
+  int *Xe[2];
 };
 
 // Extended-range dot product of row i of the weights with the unknowns over
@@ -688,8 +690,6 @@ __device__ inline void grad2(Geo g, const double *x, double mw2, int ja, int la,
     gr[d] = mw2 * a + mw2 * c;
   }
 }
-
-constexpr int EX_TY = 8;
 
 __device__ inline double trap_f(const TrapPrm &p, int d, double xv) {
   if (p.kind == TRAP_HARMONIC) return -p.w * p.w * (xv - p.c[d]);
@@ -895,6 +895,12 @@ __device__ inline void tri_solve_out(int N, double beta, const TriJob &job, int 
     if (job.Xm[backward]) {
       job.Xm[backward][i] = x.m;
       job.Xe[backward][i] = x.e;
+      if (i == N) {
+        // 1 / (m 2^(e-62)) = (1 / mantissa in [1/2, 1)) 2^-e
+        const XI v = xi_from(1.0 / __longlong_as_double(((x.m + 256) >> 9) + (1021LL << 52)), -x.e);
+        job.Xm[backward][N + 1] = v.m;
+        job.Xe[backward][N + 1] = v.e;
+      }
     }
   }
 }
@@ -1031,21 +1037,17 @@ __device__ inline void enk_entry(const Geo &g, const double *__restrict__ x, con
 // cancels, so w2 (x - x_n) + w2 (x - x_p) is taken directly (equal to
 // rounding; no FP64 division, the GPU's slowest FP64 operation)
 template <int D>
-__device__ inline void spring_interior_bead(const Geo &g, const double *__restrict__ x,
-                                            const double *__restrict__ m, double w2, int image,
+__device__ inline void spring_interior_bead(const Geo &g, const double *__restrict__ x, double w2, int image,
                                             double *__restrict__ f, int j, int l) {
-  (void)m;
   double gr[D];
   grad2<D>(g, x, w2, j, l, j + 1, l, j - 1, l, image, gr);
 #pragma unroll
-  for (int d = 0; d < D; ++d) f[sidx(j, d, l, D, g.Ns)] += -gr[d];
+  for (int d = 0; d < D; ++d) f[sidx(j, d, l, D, g.Ns)] = -gr[d];
 }
 
-// 1 / X_N (its mantissa's reciprocal in FP64: one division)
-__device__ inline XI g_ext_inv(int N, const TriJob &job) {
-  const XI x{job.Xm[0][N], job.Xe[0][N]};
-  // 1 / (m 2^(e-62)) = (1 / mantissa in [1/2, 1)) 2^-e
-  return xi_from(1.0 / __longlong_as_double(((x.m + 256) >> 9) + (1021LL << 52)), -x.e);
+// X'_{N-l} / X_N of row l (1-based) of G
+__device__ inline XI g_ext_row(int N, const TriJob &job, int l) {
+  return xi_mul({job.Xm[1][N - l], job.Xe[1][N - l]}, {job.Xm[0][N + 1], job.Xe[0][N + 1]});
 }
 // G[l][j] (1-based) = M_{l,j-1} X_{j-1} X'_{N-l} / X_N, and 1 - X_l X'_{N-l} / X_N
 // for j = l + 1, from the recursions' numbers; q: X'_{N-l} / X_N
@@ -1198,84 +1200,159 @@ __device__ inline void pair_tile32_job(const Geo &g, const P32 &q, const float *
   }
 }
 
-// the exchange spring forces on the end beads of particles bx*32 .. +31
-// from partners js*EX_TY + ty + k nsplit EX_TY: one 32 x EX_TY thread
-// block (tx, ty), red: EX_TY * 2D * 32 doubles of shared memory
+// ---- exchange spring forces of the end beads -----------------------------
+// Bead 1 of l meets bead P of every q with weight G[q][l], bead P of l meets
+// bead 1 of every q with weight G[l][q] (md_pimd_x.c:2674-2717): the same
+// spring vector c = xP_l - x1_q with the weight G[l][q] serves bead P of l and,
+// negated, bead 1 of q, so a 32 x 32 tile of the lower triangle serves both.  A
+// warp takes one of `parts` equal parts of a tile's rows l, a column q a lane
+// (the weights' rows and G's are then read and written whole sectors at a
+// time), forms G there and stores it (FROM_G: reads it).  The columns' sums stay
+// in the lanes; the rows' are added across them by halving exchanges, R rows
+// of (weight, weighted vector) at once: one addition a value instead of five.
+// Bound by the FP64 pipe where there are many tiles, by its latency where few.
+// The ring's own spring at an end bead does not depend on the partner: it is
+// weighted once, by the summed weights.  G is zero above the superdiagonal; an
+// element (l, l+1) in the next tile's first column goes to a corner entry.
+// scr: columns [T * parts][D+1][Ns] (slot: row tile and part), rows [T][D+1][Ns]
+// (slot: column tile), then corners [T][D+1].
+__host__ __device__ inline int exch_parts(int N) { return N <= 128 ? 8 : 4; }
+__host__ __device__ inline int exch_jobs(int N) {
+  const int T = (N + 31) / 32;
+  return T * (T + 1) / 2 * exch_parts(N);
+}
+template <int D, int R, bool FROM_G>
+__device__ inline void exch_tile_rows(const Geo &g, const double *__restrict__ x, int image, const TriJob &tj,
+                                      double *__restrict__ G, double *__restrict__ scr, int LT, int QT, int part,
+                                      int parts, int lane) {
+  constexpr int CP = D == 1 ? 2 : 4, NV = R * CP;  // padded components of a row's sums; their number
+  static_assert(NV <= 32, "a row batch's sums fill at most one value a lane");
+  const int N = g.N, T = (N + 31) / 32, q = QT * 32 + lane;
+  const bool vq = q < N;
+  double x1[D], a1[D + 1];
+#pragma unroll
+  for (int d = 0; d < D; ++d) x1[d] = vq ? x[sidx(0, d, q, D, g.Ns)] : 0.0;
+#pragma unroll
+  for (int d = 0; d <= D; ++d) a1[d] = 0.0;
+  double *rows = scr + (size_t)T * parts * (D + 1) * g.Ns;
+  for (int l0 = LT * 32 + part * 32 / parts; l0 < LT * 32 + (part + 1) * 32 / parts; l0 += R) {
+    double w[R], v[NV];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int l = l0 + r;
+      w[r] = 0.0;
+      if (l < N && vq && q <= l + 1)
+        w[r] = FROM_G ? G[(size_t)l * N + q] : g_ext_elem(tj, g_ext_row(N, tj, l + 1), l + 1, q + 1);
+    }
+    if (!FROM_G) {
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+        if (l0 + r < N && vq && q <= l0 + r + 1) G[(size_t)(l0 + r) * N + q] = w[r];
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int l = l0 + r < N ? l0 + r : N - 1;
+#pragma unroll
+      for (int d = 0; d < CP - 1; ++d) {
+        v[r * CP + d] = 0.0;
+        if (d < D) {
+          double c = x[sidx(g.P - 1, d, l, D, g.Ns)] - x1[d];
+          if (image) c = min_image(c, g.box[d], g.inv_box[d]);
+          c *= w[r];
+          v[r * CP + d] = c;
+          a1[d] -= c;
+        }
+      }
+      v[r * CP + CP - 1] = w[r];
+      a1[D] += w[r];
+    }
+#pragma unroll
+    for (int h = NV / 2, off = 16; h > 0; h /= 2, off /= 2) {
+      const bool up = lane & off;
+#pragma unroll
+      for (int i = 0; i < h; ++i) {
+        const double keep = up ? v[i + h] : v[i], send = up ? v[i] : v[i + h];
+        v[i] = keep + __shfl_xor_sync(FULL, send, off);
+      }
+    }
+#pragma unroll
+    for (int off = 16 / NV; off > 0; off /= 2) v[0] += __shfl_xor_sync(FULL, v[0], off);
+    const int i = lane / (32 / NV), l = l0 + i / CP, d = i % CP == CP - 1 ? D : i % CP;
+    if (lane % (32 / NV) == 0 && l < N && (i % CP == CP - 1 || d < D))
+      rows[((size_t)QT * (D + 1) + d) * g.Ns + l] = v[0];
+  }
+  if (vq) {
+#pragma unroll
+    for (int d = 0; d <= D; ++d) scr[((size_t)(LT * parts + part) * (D + 1) + d) * g.Ns + q] = a1[d];
+  }
+  const int l = LT * 32 + 31;
+  if (LT == QT && part == 0 && lane == 31 && l + 1 < N) {
+    double *o = G + (size_t)l * N + l + 1;
+    const double w = FROM_G ? *o : g_ext_elem(tj, g_ext_row(N, tj, l + 1), l + 1, l + 2);
+    if (!FROM_G) *o = w;
+    double *co = rows + (size_t)T * (D + 1) * g.Ns + (size_t)LT * (D + 1);
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      double c = x[sidx(g.P - 1, d, l, D, g.Ns)] - x[sidx(0, d, l + 1, D, g.Ns)];
+      if (image) c = min_image(c, g.box[d], g.inv_box[d]);
+      co[d] = c * w;
+    }
+    co[D] = w;
+  }
+}
+template <int D, bool FROM_G>
+__device__ inline void exch_tile_job(const Geo &g, const double *__restrict__ x, int image, const TriJob &tj,
+                                     double *__restrict__ G, double *__restrict__ scr, int job, int lane) {
+  const int parts = exch_parts(g.N), part = job % parts;
+  int LT = 0, QT = job / parts;
+  while (QT > LT) QT -= ++LT;
+  if (parts == 8)
+    exch_tile_rows<D, 4, FROM_G>(g, x, image, tj, G, scr, LT, QT, part, parts, lane);
+  else
+    exch_tile_rows<D, 8, FROM_G>(g, x, image, tj, G, scr, LT, QT, part, parts, lane);
+}
+
+// Share y of EX_Y of the sums of an end bead's (side 0 bead 1, side 1 bead P)
+// partial entries: of the weighted vectors' coordinate d in .x, of the weights
+// in .y.  exch_end_value adds the shares in order; the entries of a long
+// system are many and each a trip to L2, so its kernel takes a thread a share.
+constexpr int EX_Y = 8;
 template <int D>
-__device__ inline void exch_ends_block(const Geo &g, const double *__restrict__ x, const double *__restrict__ m,
-                                       double w2, int image, const double *__restrict__ G,
-                                       double *__restrict__ scratch, int nsplit, int bx, int js, int tx, int ty,
-                                       double *red) {
-  const int l = bx * 32 + tx;
-  const int N = g.N, jP = g.P - 1;
-  double a1[D], aP[D];
-#pragma unroll
-  for (int d = 0; d < D; ++d) a1[d] = aP[d] = 0;
-  if (l < N) {
-    const double m1 = m[l], mP = m[(size_t)jP * g.Ns + l];
-    // The reference adds G-weighted gradients of both springs at the end
-    // bead for every partner q; the spring inside the ring (bead 1 -> 2,
-    // bead P -> P-1) does not depend on q, so it is weighted once by the sum
-    // of the weights and only the partner spring is evaluated per q (equal
-    // to rounding).
-    double x1[D], xP[D], s1 = 0.0, sP = 0.0;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      x1[d] = x[sidx(0, d, l, D, g.Ns)];
-      xP[d] = x[sidx(jP, d, l, D, g.Ns)];
-    }
-    // partner q runs over this block's part of 0..N-1
-    for (int q = js * EX_TY + ty; q < N; q += nsplit * EX_TY) {
-      // bead 1 of l, previous bead = bead P of q, weight G[q][l]
-      const double g1 = G[(size_t)q * N + l];
-      if (g1 != 0.0) {
-        s1 += g1;
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          double c = x1[d] - x[sidx(jP, d, q, D, g.Ns)];
-          if (image) c = min_image(c, g.box[d], g.inv_box[d]);
-          a1[d] = fma(g1, c, a1[d]);
-        }
-      }
-      // bead P of l, next bead = bead 1 of q, weight G[l][q]
-      const double gP = G[(size_t)l * N + q];
-      if (gP != 0.0) {
-        sP += gP;
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          double c = xP[d] - x[sidx(0, d, q, D, g.Ns)];
-          if (image) c = min_image(c, g.box[d], g.inv_box[d]);
-          aP[d] = fma(gP, c, aP[d]);
-        }
-      }
-    }
-    const double k1 = m1 * w2, kP = mP * w2;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-      double a = x1[d] - x[sidx(1, d, l, D, g.Ns)];
-      double b = xP[d] - x[sidx(jP - 1, d, l, D, g.Ns)];
-      if (image) {
-        a = min_image(a, g.box[d], g.inv_box[d]);
-        b = min_image(b, g.box[d], g.inv_box[d]);
-      }
-      a1[d] = k1 * (s1 * a + a1[d]);
-      aP[d] = kP * (sP * b + aP[d]);
-    }
+__device__ inline double2 exch_end_share(const Geo &g, const double *__restrict__ scr, int side, int d, int l, int y) {
+  const int T = (g.N + 31) / 32, parts = exch_parts(g.N), t = l / 32;
+  const size_t row = (size_t)(D + 1) * g.Ns;
+  const double *base = scr + (side ? (size_t)T * parts * row : 0);
+  const int a = side ? 0 : t * parts, b = side ? t + 1 : T * parts;
+  double2 s = make_double2(0, 0);
+#pragma unroll 4
+  for (int k = a + y; k < b; k += EX_Y) {
+    s.x += base[k * row + (size_t)d * g.Ns + l];
+    s.y += base[k * row + (size_t)D * g.Ns + l];
   }
+  return s;
+}
+// the exchange force on the end bead, as the acceleration the step stores
+// (the bead's mass cancels, as in spring_interior_bead)
+template <int D>
+__device__ inline double exch_end_value(const Geo &g, const double *__restrict__ x, double w2, int image,
+                                        const double *__restrict__ scr, int side, int d, int l, const double2 *share,
+                                        int stride) {
+  const int T = (g.N + 31) / 32, t = (l + side) / 32;
+  double S = 0, W = 0;
 #pragma unroll
-  for (int d = 0; d < D; ++d) {
-    red[(ty * 2 * D + d) * 32 + tx] = a1[d];
-    red[(ty * 2 * D + D + d) * 32 + tx] = aP[d];
+  for (int y = 0; y < EX_Y; ++y) {
+    S += share[y * stride].x;
+    W += share[y * stride].y;
   }
-  __syncthreads();
-  if (ty == 0 && l < N) {
-#pragma unroll
-    for (int q = 0; q < 2 * D; ++q) {
-      double s = 0;
-      for (int y = 0; y < EX_TY; ++y) s += red[(y * 2 * D + q) * 32 + tx];
-      scratch[((size_t)js * 2 * D + q) * g.Ns + l] = s;
-    }
+  if (((l + side) & 31) == 0 && t > 0 && l + side < g.N) {
+    const double *co = scr + ((size_t)T * (exch_parts(g.N) + 1) * g.Ns + t - 1) * (D + 1);
+    S += side ? co[d] : -co[d];
+    W += co[D];
   }
+  const int j = side ? g.P - 1 : 0, jn = side ? g.P - 2 : 1;
+  double r = x[sidx(j, d, l, D, g.Ns)] - x[sidx(jn, d, l, D, g.Ns)];
+  if (image) r = min_image(r, g.box[d], g.inv_box[d]);
+  return -w2 * (W * r + S);
 }
 
 // ---- FP32 structure factors (mixed form) --------------------------------

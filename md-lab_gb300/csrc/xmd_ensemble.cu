@@ -6,7 +6,7 @@
 // benchmark ensemble) and one system's step is a chain of a dozen dependent
 // stages, so as separate kernels the systems keep the GPU's launch path
 // busy with about a thousand small kernels a step.  Here one launch runs
-// every stage of every system: the step is nine phases, each phase holds the
+// every stage of every system: the step is eight phases, each phase holds the
 // work of ALL systems for that stage (spread over every thread, warp or
 // block of the grid, round-robin over the systems' tasks), and the phases
 // are separated by grid barriers.  The grid is exactly the blocks that fit
@@ -37,19 +37,18 @@
 namespace xk {
 
 constexpr int ENS_T = 256;                // threads per block
-constexpr int ENS_W = ENS_T / 32;         // warps per block (the EX_TY rows of the end-bead block)
+constexpr int ENS_W = ENS_T / 32;         // warps per block
 constexpr size_t ENS_SMEM = 64 * 1024;    // dynamic shared memory per block
 constexpr int ENS_SKC = 128;              // particles per staged chunk of phase factors
 constexpr int ENS_NSMAX = 11;             // largest Ewald n_sum
 constexpr long long ENS_WAIT_LIMIT = 1LL << 31;  // clock cycles a grid-barrier wait may take (~1 s)
-static_assert(ENS_W == EX_TY, "the end-bead block is 32 x EX_TY threads");
 static_assert(ENS_SKC % SK_PB == 0, "staged chunks hold whole particle blocks");
 
 struct EnsSys {
   EnsSysDesc d;
   TriJob job;
   P32 q;
-  int T, jobs, nsplit;
+  int T, jobs;
   int ewald;  // reciprocal sums present (D = 3)
   int ns, ncol, nk;
   const int4 *cols;
@@ -76,12 +75,11 @@ enum {
   R_E_PS,    // thread: pair sums per slot
   R_E_INV,   // block: diagonal-block inverses
   R_F,       // block: solves
-  R_G,       // thread: G entries
-  R_H,       // block: end-bead exchange forces
-  R_I,       // thread: second half step per slot
+  R_G,       // warp: tile parts of G with the end beads' springs
+  R_H,       // thread: second half step per slot
   ENS_NROT
 };
-static_assert(ENS_NROT == 16, "EnsSys::rot holds every task kind");
+static_assert(ENS_NROT <= 16, "EnsSys::rot holds every task kind");
 
 // one FP32 pair tile job of the system's potential kind
 template <int D>
@@ -309,7 +307,6 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
         double f0 = 0.0;
         if (d.trap_kind) f0 += trap_f(d.tp, (int)((s / g.Ns) % D), xn) * E.pscale;
         d.f[s] = f0;
-        d.fex[s] = 0.0;
         if (d.pair_kind) E.x32[s] = (float)xn;
         if constexpr (D == 3)
           if (E.ewald) phase32_slot(g, E.ns, d.x, E.ph32, s);
@@ -328,7 +325,7 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
       const long long n = g.P > 2 ? (long long)(g.P - 2) * g.Ns : 0;
       for (long long t = ens_first(gt, sys[i].rot[R_B_SPR], GT); t < n; t += GT) {
         const int l = (int)(t % g.Ns), j = (int)(t / g.Ns) + 1;
-        if (l < g.N) spring_interior_bead<D>(g, d.x, d.m, d.w2, d.image, d.fex, j, l);
+        if (l < g.N) spring_interior_bead<D>(g, d.x, d.w2, d.image, d.fex, j, l);
       }
     }
   }
@@ -479,43 +476,21 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
   ens_grid_sync(bar, G, limit);
   ens_stamp(bar, 6);
 
-  // G: cycle probabilities G from the extended-range numbers
-  // (md_pimd_fast_fill_force_VB_x)
+  // G: cycle probabilities G from the extended-range numbers and the end beads'
+  // G-weighted springs (md_pimd_fast_fill_force_VB_x), partial sums per tile part
   {
     for (int i = i0; i < i1; ++i) {
       const EnsSys &E = sys[i];
-      const int N = E.d.g.N;
-      const long long n = (long long)N * N;
-      const XI iX = g_ext_inv(N, E.job);
-      for (long long q = ens_first(gt, sys[i].rot[R_G], GT); q < n; q += GT) {
-        const int l = (int)(q / N) + 1;
-        const XI f = xi_mul({E.job.Xm[1][N - l], E.job.Xe[1][N - l]}, iX);
-        E.d.G[q] = g_ext_elem(E.job, f, l, (int)(q % N) + 1);
-      }
+      const EnsSysDesc &d = E.d;
+      const long long n = exch_jobs(d.g.N);
+      for (long long q = ens_first(gw, sys[i].rot[R_G], GW); q < n; q += GW)
+        exch_tile_job<D, false>(d.g, d.x, d.image, E.job, d.G, d.xscr, (int)q, lane);
     }
   }
   ens_grid_sync(bar, G, limit);
   ens_stamp(bar, 7);
 
-  // H: G-weighted springs of the end beads, partial sums per partner split
-  {
-    for (int i = i0; i < i1; ++i) {
-      const EnsSys &E = sys[i];
-      const EnsSysDesc &d = E.d;
-      const Geo g = d.g;
-      const int tiles = (g.N + 31) / 32;
-      const long long n = (long long)tiles * E.nsplit;
-      for (long long tk = ens_first(gb, sys[i].rot[R_H], G); tk < n; tk += G) {
-        exch_ends_block<D>(g, d.x, d.m, d.w2, d.image, d.G, d.xscr, E.nsplit, (int)(tk % tiles), (int)(tk / tiles),
-                           lane, w, (double *)ens_sh);
-        __syncthreads();
-      }
-    }
-  }
-  ens_grid_sync(bar, G, limit);
-  ens_stamp(bar, 8);
-
-  // I: the end beads' exchange forces into fex, the second half step with
+  // H: the end beads' exchange forces into fex, the second half step with
   // f + fex (md_update_nhc_VV3_2_x), the periodic wrap
   {
     for (int i = i0; i < i1; ++i) {
@@ -523,16 +498,17 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
       const EnsSysDesc &d = E.d;
       const Geo g = d.g;
       const long long n = (long long)g.slots();
-      for (long long q = ens_first(gt, sys[i].rot[R_I], GT); q < n; q += GT) {
+      for (long long q = ens_first(gt, sys[i].rot[R_H], GT); q < n; q += GT) {
         const size_t s = (size_t)q;
         const int l = (int)(s % g.Ns);
         if (l >= g.N) continue;
         const int jd = (int)(s / g.Ns), j = jd / D, dd = jd % D;
         if (j == 0 || j == g.P - 1) {
-          const int qq = (j == g.P - 1 ? D : 0) + dd;
-          double sum = 0;
-          for (int js = 0; js < E.nsplit; ++js) sum += d.xscr[((size_t)js * 2 * D + qq) * g.Ns + l];
-          d.fex[s] += -sum / d.m[(size_t)j * g.Ns + l];
+          const int side = j == 0 ? 0 : 1;
+          double2 share[EX_Y];
+#pragma unroll
+          for (int y = 0; y < EX_Y; ++y) share[y] = exch_end_share<D>(g, d.xscr, side, dd, l, y);
+          d.fex[s] = exch_end_value<D>(g, d.x, d.w2, d.image, d.xscr, side, dd, l, share, 1);
         }
         nhc_slot<D, L>(g, 2, s, l, d.x, d.v, d.f, d.fex, d.m, d.th, d.vt, d.Q, d.iQ, d.kT, d.h);
         if (d.wrap) {
@@ -642,7 +618,6 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
     const Geo &g = E.d.g;
     if (g.D != D || g.N < 1 || g.N > ENS_MAX_N || g.P < 2) return cudaErrorInvalidValue;
     E.job = tri_job(g.N, E.d.rs_f, E.d.rs_b, E.d.VBN, E.d.tmpV);
-    E.nsplit = (int)(exch_scratch_doubles(g) / ((size_t)2 * g.D * g.Ns));
     E.T = (g.N + 31) / 32;
     E.jobs = E.T * (E.T + 1) / 2;
     if (E.d.pair_kind) E.q = make_p32(g, E.d.pp);
@@ -691,7 +666,7 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
   // group's workers of that kind
   for (int k = 0; k < K; ++k) {
     const long long stride[ENS_NROT] = {Gk * ENS_T, Gk * ENS_T, Gk * ENS_W, Gk * ENS_W, Gk, Gk, Gk * ENS_T, Gk * ENS_T,
-                                        Gk, Gk * ENS_W, Gk * ENS_T, Gk, Gk, Gk * ENS_T, Gk, Gk * ENS_T};
+                                        Gk, Gk * ENS_W, Gk * ENS_T, Gk, Gk, Gk * ENS_W, Gk * ENS_T};
     long long base[ENS_NROT] = {};
     for (int pass = 0; pass < 2; ++pass)  // the pair tiles continue E_l^(1)'s numbering
       for (int i = goff[k]; i < goff[k + 1]; ++i) {
@@ -712,9 +687,8 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
         cnt[R_E_PS] = E.d.pair_kind ? slots : 0;
         cnt[R_E_INV] = 2 * ((N + TS_CHUNK - 1) / TS_CHUNK);
         cnt[R_F] = 2;
-        cnt[R_G] = N * N;
-        cnt[R_H] = (long long)((g.N + 31) / 32) * E.nsplit;
-        cnt[R_I] = slots;
+        cnt[R_G] = exch_jobs(g.N);
+        cnt[R_H] = slots;
         for (int q = 0; q < ENS_NROT; ++q) {
           if ((q == R_B_PAIR) != (pass == 1)) continue;
           if (pass == 1 && i == goff[k]) base[R_B_PAIR] = base[R_B_EINT];

@@ -859,11 +859,11 @@ static size_t tsc_sums(int N) {
 
 // one direction's scratch: weights (mantissas, then exponents as ints), the
 // diagonal blocks' inverses B and the products W (mantissas, exponents), the
-// unknowns X_0..X_N (mantissas, exponents), and the partial sums of the
+// unknowns X_0..X_N and 1/X_N (mantissas, exponents), and the partial sums of the
 // cluster solve's memory variant
 size_t rec_scratch_doubles(int N) {
   const size_t nch = (N + TS_CHUNK - 1) / TS_CHUNK;
-  return ntri(N) + (ntri(N) + 1) / 2 + 1 + nch * TS_CHUNK * TS_CHUNK * 3 + (size_t)(N + 1) + (N + 2) / 2 + tsc_sums(N);
+  return ntri(N) + (ntri(N) + 1) / 2 + 1 + nch * TS_CHUNK * TS_CHUNK * 3 + (size_t)(N + 2) + (N + 3) / 2 + tsc_sums(N);
 }
 
 // directions first .. first + count - 1 of job
@@ -1312,8 +1312,8 @@ TriJob tri_job(int N, double *rs_f, double *rs_b, double *VBN, double *tmpV) {
     j.Wm[d] = b + nb + nb / 2;
     j.We[d] = (int *)(j.Wm[d] + nb);
     j.Xm[d] = (long long *)(j.Wm[d] + nb + nb / 2);
-    j.Xe[d] = (int *)(j.Xm[d] + N + 1);
-    j.Sm[d] = (double *)j.Xm[d] + N + 1 + (N + 2) / 2;
+    j.Xe[d] = (int *)(j.Xm[d] + N + 2);
+    j.Sm[d] = (double *)j.Xm[d] + N + 2 + (N + 3) / 2;
   }
   j.Mm[0] = rs_f;
   j.Me[0] = (const int *)(rs_f + ntri(N));
@@ -1415,106 +1415,80 @@ cudaError_t fill_g(int N, double beta, double vi, const double *ENk, const doubl
 //   G[l][l+1] = 1 - X_l X'_{N-l} / X_N
 // a product of four numbers each held to a few ulps, where the reference's
 // exp(-beta(V_B^(j-1) + E + tmpV[l] - V_B^(N))) loses beta V_B^(N) ulps to the
-// cancellation inside the exponent (up to ~1e-10 relative at N = 512).
-
-__global__ void k_fill_g_ext(int N, TriJob job, double *__restrict__ G) {
-  const int l = blockIdx.y + 1;  // 1-based row
-  __shared__ XI qs;
-  if (threadIdx.x == 0) qs = xi_mul({job.Xm[1][N - l], job.Xe[1][N - l]}, g_ext_inv(N, job));
-  __syncthreads();
-  const XI q = qs;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x + 1; j <= N; j += gridDim.x * blockDim.x)
-    G[(size_t)(l - 1) * N + (j - 1)] = g_ext_elem(job, q, l, j);
-}
-
-cudaError_t fill_g_ext(int N, const double *rs_f, const double *rs_b, double *G, cudaStream_t st) {
-  const TriJob j = tri_job(N, (double *)rs_f, (double *)rs_b, nullptr, nullptr);
-  dim3 grid((N + 255) / 256, N);
-  {
-    XK_PROF("fill_g");
-    k_fill_g_ext<<<grid, 256, 0, st>>>(N, j, G);
-  }
-  return XK_LAUNCHED();
-}
+// cancellation inside the exponent (up to ~1e-10 relative at N = 512); k_exch
+// below forms it where the springs need it.
 
 // ===================================================================
 // exchange-weighted spring forces: md_pimd_x.c:2674-2717
 // ===================================================================
 
 
-// interior beads j = 2..P-1 (1-based): plain springs
-template <int D>
-__global__ void k_spring_interior(Geo g, const double *__restrict__ x,
-                                  const double *__restrict__ m, double w2, int image,
-                                  double *__restrict__ f) {
-  const int P2 = g.P - 2;
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (P2 <= 0 || t >= (size_t)P2 * g.Ns) return;
-  const int l = (int)(t % g.Ns), j = (int)(t / g.Ns) + 1;  // 0-based bead index 1..P-2
-  if (l >= g.N) return;
-  spring_interior_bead<D>(g, x, m, w2, image, f, j, l);
-}
-
-// bead 1 and bead P of every particle, weighted by G.  Block (32 x 8)
-// covers 32 particles and one slice of the partner index range; partial
-// sums go to scratch[js][side][d][l] and are added to f by k_exch_finish.
-
-template <int D>
-__global__ void k_exch_ends(Geo g, const double *__restrict__ x, const double *__restrict__ m,
-                            double w2, int image, const double *__restrict__ G,
-                            double *__restrict__ scratch, int nsplit) {
-  __shared__ double red[EX_TY * 2 * D * 32];
-  exch_ends_block<D>(g, x, m, w2, image, G, scratch, nsplit, blockIdx.x, blockIdx.y, threadIdx.x, threadIdx.y, red);
-}
-
-template <int D>
-__global__ void k_exch_finish(Geo g, const double *__restrict__ m,
-                              const double *__restrict__ scratch, int nsplit,
-                              double *__restrict__ f) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 2 * D * g.Ns) return;
-  const int l = t % g.Ns, q = t / g.Ns;  // q = side*D + d
-  if (l >= g.N) return;
-  const int side = q / D, d = q % D;
-  const int j = side ? g.P - 1 : 0;
-  double s = 0;
-  for (int js = 0; js < nsplit; ++js) s += scratch[((size_t)js * 2 * D + q) * g.Ns + l];
-  f[sidx(j, d, l, D, g.Ns)] += -s / m[(size_t)j * g.Ns + l];
-}
-
-static int exch_split(const Geo &g) {
-  const int tiles = (g.N + 31) / 32;
-  int ns = (2 * 152 + tiles - 1) / tiles;
-  const int maxs = (g.N + EX_TY - 1) / EX_TY;
-  if (ns > maxs) ns = maxs;
-  if (ns < 1) ns = 1;
-  return ns;
-}
-
-size_t exch_scratch_doubles(const Geo &g) { return (size_t)exch_split(g) * 2 * g.D * g.Ns; }
-
-cudaError_t exch_force(const Geo &g, const double *x, const double *m, double w2, int image,
-                       const double *G, double *f, double *scratch, cudaStream_t st) {
-  if (g.P > 2) {
-    const size_t n = (size_t)(g.P - 2) * g.Ns;
-    {
-      XK_PROF("spring_interior");
-      DISPATCH_D(g.D, k_spring_interior<D><<<cdiv(n, 256), 256, 0, st>>>(g, x, m, w2, image, f));
-    }
-    cudaError_t e = XK_LAUNCHED();
-    if (e != cudaSuccess) return e;
+// One launch for G and the springs that do not wait for its sums: warps of
+// the first `nt` blocks take the tile parts of exch_tile_job (four a block: one
+// a scheduler, spread over the SMs), the threads of the others the interior
+// beads j = 2..P-1 (1-based).  With k_exch_finish two launches where G, a fill
+// of f, the interior, the ends (each spring vector formed once a side) and
+// their sums were five: 34 us against 48 (sums of launches timed apart, with
+// some 4 us a launch) at N = 512, P = 64, a whole step of N = 64, P = 64 51 us
+// against 57; at N = 1600 the FP64 pipe bounds both, 71 and 70 us.  R = 8 rows
+// a batch and four parts a tile: two parts 65 us, four 58 at N = 1600.
+constexpr int EX_W = 4;
+template <int D, bool FROM_G>
+__global__ void __launch_bounds__(32 * EX_W) k_exch(Geo g, const double *__restrict__ x, double w2, int image,
+                                                    TriJob tj, double *__restrict__ G, double *__restrict__ f,
+                                                    double *__restrict__ scr, int nt, int jobs) {
+  if ((int)blockIdx.x < nt) {
+    const int job = blockIdx.x * EX_W + (threadIdx.x >> 5);
+    if (job < jobs) exch_tile_job<D, FROM_G>(g, x, image, tj, G, scr, job, threadIdx.x & 31);
+    return;
   }
-  const int ns = exch_split(g);
-  dim3 grid((g.N + 31) / 32, ns), blk(32, EX_TY);
+  const size_t t = (size_t)(blockIdx.x - nt) * blockDim.x + threadIdx.x;
+  const int l = (int)(t % g.Ns), j = (int)(t / g.Ns) + 1;  // 0-based bead index 1..P-2
+  if (j >= g.P - 1) return;
+  if (l < g.N) {
+    spring_interior_bead<D>(g, x, w2, image, f, j, l);
+  } else {
+    for (int d = 0; d < D; ++d) f[sidx(j, d, l, D, g.Ns)] = 0.0;
+  }
+}
+
+// the end beads, from the tiles' partial sums: 32 x EX_Y threads take 32 beads'
+// sums in one coordinate
+template <int D>
+__global__ void __launch_bounds__(32 * EX_Y) k_exch_finish(Geo g, const double *__restrict__ x, double w2, int image,
+                                                           const double *__restrict__ scr, double *__restrict__ f) {
+  __shared__ double2 share[EX_Y][32];
+  const int t = blockIdx.x * 32 + threadIdx.x, l = t % g.Ns, side = t / g.Ns, d = blockIdx.y;
+  if (side < 2 && l < g.N) share[threadIdx.y][threadIdx.x] = exch_end_share<D>(g, scr, side, d, l, threadIdx.y);
+  __syncthreads();
+  if (threadIdx.y != 0 || side >= 2) return;
+  f[sidx(side ? g.P - 1 : 0, d, l, D, g.Ns)] =
+      l < g.N ? exch_end_value<D>(g, x, w2, image, scr, side, d, l, &share[0][threadIdx.x], 32) : 0.0;
+}
+
+size_t exch_scratch_doubles(const Geo &g) {
+  const size_t T = (g.N + 31) / 32;
+  return (T * (exch_parts(g.N) + 1) * g.Ns + T) * (g.D + 1);
+}
+
+cudaError_t exch_force(const Geo &g, const double *x, double w2, int image, const double *rs_f, const double *rs_b,
+                       double *G, double *f, double *scratch, cudaStream_t st) {
+  const int jobs = exch_jobs(g.N), nt = cdiv(jobs, EX_W);
+  const int ni = g.P > 2 ? cdiv((size_t)(g.P - 2) * g.Ns, 32 * EX_W) : 0;
   {
     XK_PROF("exch_ends");
-    DISPATCH_D(g.D, k_exch_ends<D><<<grid, blk, 0, st>>>(g, x, m, w2, image, G, scratch, ns));
+    if (rs_f) {
+      const TriJob tj = tri_job(g.N, (double *)rs_f, (double *)rs_b, nullptr, nullptr);
+      DISPATCH_D(g.D, (k_exch<D, false><<<nt + ni, 32 * EX_W, 0, st>>>(g, x, w2, image, tj, G, f, scratch, nt, jobs)));
+    } else {
+      DISPATCH_D(g.D, (k_exch<D, true><<<nt + ni, 32 * EX_W, 0, st>>>(g, x, w2, image, TriJob{}, G, f, scratch, nt, jobs)));
+    }
   }
   cudaError_t e = XK_LAUNCHED();
   if (e != cudaSuccess) return e;
   {
     XK_PROF("exch_finish");
-    DISPATCH_D(g.D, k_exch_finish<D><<<cdiv(2 * g.D * g.Ns, 256), 256, 0, st>>>(g, m, scratch, ns, f));
+    DISPATCH_D(g.D, k_exch_finish<D><<<dim3(cdiv(2 * g.Ns, 32), g.D), dim3(32, EX_Y), 0, st>>>(g, x, w2, image, scratch, f));
   }
   return XK_LAUNCHED();
 }

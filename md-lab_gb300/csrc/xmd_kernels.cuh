@@ -139,14 +139,15 @@ cudaError_t fill_vb_signed(int N, double beta, double vi2, const double *ENk, co
 // lnn: the host table of ln l then 1/l (2 (N+1) doubles)
 cudaError_t fill_g(int N, double beta, double vi, const double *ENk, const double *VBN,
                    const double *tmpV, const double *lnn, double *G, cudaStream_t st);
-// G from the extended-range weights and unknowns that fill_vb_tv left in
-// its scratch (rs_f, rs_b): valid only while that call's ENk, beta and xi
-// are current; a few ulps where fill_g loses up to beta V_B^(N) ulps
-cudaError_t fill_g_ext(int N, const double *rs_f, const double *rs_b, double *G, cudaStream_t st);
-// scratch: at least exch_scratch_doubles(g) doubles
+// the exchange spring forces f (every slot written, the padding zero).
+// With rs_f and rs_b, the scratch of a fill_vb_tv whose ENk, beta and xi are
+// current, G comes from the extended-range numbers left there (a few ulps,
+// where fill_g loses up to beta V_B^(N) ulps) and is stored below and on the
+// superdiagonal (zero above, which the caller keeps); with rs_f null it is
+// read.  scratch: at least exch_scratch_doubles(g) doubles
 size_t exch_scratch_doubles(const Geo &g);
-cudaError_t exch_force(const Geo &g, const double *x, const double *m, double w2, int image,
-                       const double *G, double *f, double *scratch, cudaStream_t st);
+cudaError_t exch_force(const Geo &g, const double *x, double w2, int image, const double *rs_f, const double *rs_b,
+                       double *G, double *f, double *scratch, cudaStream_t st);
 
 // ---- external forces ----
 enum TrapKind { TRAP_HARMONIC = 1, TRAP_HARMONIC_2 = 2, TRAP_NEG_HARMONIC = 3 };
@@ -407,7 +408,7 @@ cudaError_t ensemble_launch(const EnsLaunch &e, cudaStream_t st);
 // the last one at block 0's own end), block 0's own time in phase B for its
 // springs, E_l^(1), pair tiles and structure factors, then each group's
 // step time (its first block's start to end).  Synchronous.
-constexpr int ENS_PHASES = 9;
+constexpr int ENS_PHASES = 8;
 cudaError_t ensemble_status(const EnsLaunch &e, int *failed, double *phase_us = nullptr);
 void ensemble_free(EnsLaunch &e);
 // the supported shapes: N <= ENS_MAX_N, L in {4, 8}, D in 1..3, n_sum <= 11

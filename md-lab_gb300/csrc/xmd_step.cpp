@@ -343,17 +343,17 @@ int md_pimd_fast_fill_force_VB_x(md_pimd_t_x *pimd, int image) {
   if (pd->tmpv_fresh && pd->tmpv_beta == pimd->beta && pd->tmpv_vi == pimd->vi) {
     // both recursions of the current ENk are in pd->rec: G from their
     // extended-range numbers
-    double *rs = pd->rec.as<double>();
-    XMD_CUDA(xk::fill_g_ext(N, rs, rs + xk::rec_scratch_doubles(N), pd->G.as<double>(), st));
+    const double *rs = pd->rec.as<double>();
+    XMD_CUDA(xk::exch_force(sd->geo, sd->x.as<double>(), pimd->omegaP * pimd->omegaP, image, rs,
+                            rs + xk::rec_scratch_doubles(N), pd->G.as<double>(), sd->fex.as<double>(), scr, st));
   } else {
     XMD_CUDA(xk::back_vb(N, pimd->beta, pimd->vi, pd->ENk.as<double>(), pd->lnn.as<double>(),
                          pd->tmpV.as<double>(), pd->rec.as<double>(), st));
     XMD_CUDA(xk::fill_g(N, pimd->beta, pimd->vi, pd->ENk.as<double>(), pd->VBN.as<double>(),
                         pd->tmpV.as<double>(), pd->lnn.as<double>(), pd->G.as<double>(), st));
+    XMD_CUDA(xk::exch_force(sd->geo, sd->x.as<double>(), pimd->omegaP * pimd->omegaP, image, nullptr, nullptr,
+                            pd->G.as<double>(), sd->fex.as<double>(), scr, st));
   }
-  XMD_CUDA(cudaMemsetAsync(sd->fex.p, 0, sd->geo.slots() * sizeof(double), st));
-  XMD_CUDA(xk::exch_force(sd->geo, sd->x.as<double>(), sd->m.as<double>(), pimd->omegaP * pimd->omegaP, image,
-                          pd->G.as<double>(), sd->fex.as<double>(), scr, st));
   XMD_TRY(side_end(sd));
   pd->g_fresh = true;
   pd->g_beta = pimd->beta;
