@@ -630,7 +630,7 @@ def ensemble_form(lib, R, args):
     nph = lib.md_gb300_ensemble_phase_times_x(gp, ph, 44)
     group_us = [round(v, 1) for v in ph[12:nph]]
     phase_us = {nm: round(v, 1) for nm, v in zip(
-        ("VV3_1", "springs_Eint_tiles_Sk", "prefix_tables", "ENk_recip", "weights_inverses_pairsum", "solves",
+        ("VV3_1", "springs_Eint_tiles_Sk", "prefix_recip", "ENk", "weights_inverses_pairsum", "solves",
          "G_exch_ends", "VV3_2", "block0_springs", "block0_Eint", "block0_tiles", "block0_Sk"), ph)}
     lib.md_gb300_graph_free_x(gp)
     for _, s, _ in systems:

@@ -1059,54 +1059,22 @@ __device__ inline double g_ext_elem(const TriJob &job, XI q, int l, int j) {
   return xi_double(xi_mul(xi_mul(w, {job.Xm[0][j - 1], job.Xe[0][j - 1]}), q));
 }
 
-// FP32 phase factors e^{2 pi i n x/L}, n = 0..ns, of slot t (D = 3 layout)
-__device__ inline void phase32_slot(const Geo &g, int ns, const double *__restrict__ x, float2 *__restrict__ ph32,
-                                    size_t t) {
-  const int l = (int)(t % g.Ns);
-  const int jd = (int)(t / g.Ns);  // j*3 + d
-  const int d = jd % 3;
+// FP32 phase factor e^{2 pi i x/L} of slot t (D = 3): the fraction of x/L in
+// FP64 (exact), the sine and cosine of the reduced angle in FP32.  The sums
+// form the harmonics where they use them (phase32_next): a slice's eleven rows
+// a coordinate are ten times the reads, and cost more than nine products.
+__device__ inline float2 phase32_slot(const Geo &g, const double *__restrict__ x, size_t t) {
+  const int l = (int)(t % g.Ns), d = (int)(t / g.Ns) % 3;
   float s1 = 0.f, c1 = 1.f;
   if (l < g.N) {
     double u = x[t] * g.inv_box[d];
     u -= rint(u);  // in [-1/2, 1/2]
     sincospif((float)(2.0 * u), &s1, &c1);
   }
-  float re = 1.f, im = 0.f;
-  float2 *o = ph32 + (size_t)jd * (ns + 1) * g.Ns + l;
-  o[0] = make_float2(1.f, 0.f);
-  for (int n = 1; n <= ns; ++n) {
-    const float r2 = fmaf(re, c1, -im * s1), i2 = fmaf(re, s1, im * c1);
-    re = r2;
-    im = i2;
-    o[(size_t)n * g.Ns] = make_float2(re, im);
-  }
+  return make_float2(c1, s1);
 }
-
-// entry n (0..ns) of column ci's FP32 force table of slice j, in FP32
-// from the FP32 structure factors S and coefficients coef32
-__device__ inline void recip_table32_entry(const int4 *__restrict__ cols, int ncol, const float2 *__restrict__ S,
-                                           const float *__restrict__ coef32, int nk, float2 *__restrict__ T, int ns,
-                                           int j, int ci, int n) {
-  const int NT = 4 * ns + 1;
-  const int4 c = cols[ci];
-  auto W = [&](int nz) {
-    if (nz < c.z) return make_float2(0.f, 0.f);
-    const int k = c.w + (nz - c.z);
-    const float2 s = S[(size_t)j * nk + k];
-    return make_float2(coef32[k] * s.x, -coef32[k] * s.y);
-  };
-  float2 *o = T + ((size_t)j * ncol + ci) * NT;
-  if (n == 0) {
-    o[0] = W(0);
-  } else {
-    const float2 wp = W(n), wm = W(-n);
-    const float Ar = wp.x + wm.x, Ai = wp.y + wm.y, Br = wp.x - wm.x, Bi = wp.y - wm.y;
-    const float fn = (float)n;
-    o[4 * n - 3] = make_float2(Ar, Ai);
-    o[4 * n - 2] = make_float2(Br, Bi);
-    o[4 * n - 1] = make_float2(fn * Ar, fn * Ai);
-    o[4 * n] = make_float2(fn * Br, fn * Bi);
-  }
+__device__ __forceinline__ float2 phase32_next(float2 e, float2 e1) {
+  return make_float2(fmaf(e.x, e1.x, __fmul_rn(-e.y, e1.y)), fmaf(e.x, e1.y, __fmul_rn(e.y, e1.x)));
 }
 
 // tile job wi (slice wi / jobs, tile pair I <= J) of the FP32 pair forces,
@@ -1355,65 +1323,28 @@ __device__ inline double exch_end_value(const Geo &g, const double *__restrict__
   return -w2 * (W * r + S);
 }
 
-// ---- FP32 structure factors (mixed form) --------------------------------
-// An item is one kept wave-vector column (nx, ny) and SK_NG harmonics
-// nz = n0+1 .. n0+SK_NG (and nz = 0 when n0 = 0) of one bead slice.  The
-// particles' phase products are summed in FP32 over SK_PB particles at a
-// time, and each partial sum is added into double-float accumulators: the FP32
-// partial of at most 16 unit-size terms carries an error of ~1e-7 of a
-// term, the size of the FP32 phase factors' own rounding, at a sixth of
-// the arithmetic of a double-float addition per particle.
-constexpr int SK_NG = 4;   // harmonics per item
-constexpr int SK_PB = 16;  // particles per FP32 partial sum
+// ---- FP32 reciprocal sums (mixed form) ------------------------------------
+// Both kernels' bodies for a block of SK_W warps, shared with the persistent
+// ensemble step, whose results are the same bits: the order of every sum
+// depends on N, the columns and SK_W alone.
+constexpr int SK_NG = 8;                // harmonics of one structure-factor item
+static_assert(SK_NG % 2 == 0, "z factors are read two at a time, 16 bytes aligned");
+constexpr int SK_W = 8, SK_T = 32 * SK_W;
+constexpr int SK_CH = 128;              // particles staged at a time
+constexpr int SK_NC = 4 * SK_NG + 2;    // sums of one item
 
-struct SkAcc {
-  DF s0r, s0i, P[SK_NG][2], Q[SK_NG][2];
-};
-
-// the item's sums over the staged particles 0 .. cnt-1 of a chunk (sp:
-// [3][ns+1][stride] phase factors; stride padded so that rows fall in
-// different banks): thread g of gr sharing the item takes particles
-// b + g, b + g + gr, ... (SK_PB of them) of each block b of SK_PB * gr
-// consecutive particles, blocks b0, b0 + SK_PB gr, ... (one thread: every
-// block of SK_PB particles in order)
-__device__ inline void sk_item_blocks(SkAcc &A, const float2 *__restrict__ sp, int stride, int ns, int ax, int ay,
-                                      bool cy, int n0, int cnt, int g, int gr) {
-  for (int b = 0; b < cnt; b += SK_PB * gr) {
-    float s0r = 0.f, s0i = 0.f, p[SK_NG][2], q[SK_NG][2];
-#pragma unroll
-    for (int u = 0; u < SK_NG; ++u) p[u][0] = p[u][1] = q[u][0] = q[u][1] = 0.f;
-    for (int k = 0; k < SK_PB; ++k) {
-      const int l = b + g + k * gr;
-      if (l >= cnt) break;
-      float2 ey = sp[((ns + 1) + ay) * stride + l];
-      if (cy) ey.y = -ey.y;
-      const float2 exy = cmulf(sp[ax * stride + l], ey);
-      s0r += exy.x;
-      s0i += exy.y;
-#pragma unroll
-      for (int u = 0; u < SK_NG; ++u) {
-        const int n = n0 + u + 1;
-        if (n > ns) break;
-        const float2 ez = sp[(2 * (ns + 1) + n) * stride + l];
-        p[u][0] = fmaf(exy.x, ez.x, p[u][0]);
-        p[u][1] = fmaf(exy.y, ez.x, p[u][1]);
-        q[u][0] = fmaf(exy.x, ez.y, q[u][0]);
-        q[u][1] = fmaf(exy.y, ez.y, q[u][1]);
-      }
-    }
-    if (n0 == 0) {
-      A.s0r.add(s0r);
-      A.s0i.add(s0i);
-    }
-#pragma unroll
-    for (int u = 0; u < SK_NG; ++u) {
-      if (n0 + u + 1 > ns) break;
-      A.P[u][0].add(p[u][0]);
-      A.P[u][1].add(p[u][1]);
-      A.Q[u][0].add(q[u][0]);
-      A.Q[u][1].add(q[u][1]);
-    }
-  }
+// staged phase factors of one particle, in float2: z harmonics 1.., x and y
+// harmonics 0..; the stride is an odd number of 16-byte units, so that lanes
+// writing 16 bytes each of different particles meet different banks
+__host__ __device__ inline int sk32_z(int ns) { return (ns + 1) & ~1; }
+__host__ __device__ inline int sk32_x(int ns) { return (ns + 2) & ~1; }
+__host__ __device__ inline int sk32_stride(int ns) {
+  const int s = sk32_z(ns) + 2 * sk32_x(ns);
+  return s / 2 % 2 ? s : s + 2;
+}
+__host__ __device__ inline size_t sk32_smem(int ns) {
+  const size_t a = sizeof(float2) * SK_CH * sk32_stride(ns), b = sizeof(float2) * SK_W / 2 * SK_NC * 32;
+  return a > b ? a : b;
 }
 
 // a + b and a - b of two double-float values, rounded to FP32 (TwoSum of
@@ -1429,57 +1360,233 @@ __device__ inline float df_diff(const DF &a, const DF &b) {
   return s + ((e + a.lo) - b.lo);
 }
 
-// S(k) of the item's wave vectors in FP32 (the FP32 force tables are all
-// that reads it): Sj is the slice's row S + j nk
-__device__ inline void sk_item_store(const SkAcc &A, float2 *Sj, int4 c, int ns, int n0) {
-  float2 *o = Sj + c.w - c.z;
-  if (n0 == 0 && c.z <= 0) o[0] = make_float2(A.s0r.hi + A.s0r.lo, A.s0i.hi + A.s0i.lo);
+// Structure factors of 32 items of slice j and from them their entries of the
+// force tables, T[column][0..ns]: W(0), then (A, B) = W(n) +- W(-n) with
+// W = c(n) conj(S(n)).  Item i: column i's harmonics nz = 0..SK_NG for
+// i < ncol, above that column i - ncol's further ones (the nlong columns that
+// have them; columns are sorted longest first).  An item is a lane, the warps
+// take every SK_W-th particle: the particle's z factors are then read at one
+// address, its x and y factors at different banks, and a column's
+// exp(i(x + y)) is formed once for its harmonics.  Each product is added in
+// FP32, at most SK_CH / SK_W = 16 particles at a time (an error of ~1e-7 of a
+// term, the size of the phase factors' own rounding), each partial sum in
+// double-float.  Bound by FP32 issue, four multiply-adds a harmonic, at 60 to
+// 70% of the issue slots.  37 us and no tables kernel (8 us) at N = 512, P = 64,
+// |n| <= 10, against 72 with a thread per four harmonics of a column, whose
+// lanes read scattered rows of staged harmonics; items of 6, 8 and 10 harmonics
+// 38, 37 and 42 us (blocks an SM: 3, 2, 2), in the ensemble step 509, 492, 507.
+// sh: sk32_smem(ns) bytes; every thread of the block calls.
+__device__ inline void sk32_group(const Geo &g, int ns, int ncol, int nlong, const int4 *__restrict__ cols,
+                                  const float *__restrict__ coef32, const float2 *__restrict__ ph1,
+                                  float4 *__restrict__ T, int j, int group, float2 *sh) {
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5, item = group * 32 + lane;
+  const bool live = item < ncol + nlong, more = item >= ncol;
+  const int ci = live ? (more ? item - ncol : item) : 0, n0 = more ? SK_NG : 0;
+  const int4 c = cols[ci];
+  const int top = live ? min(col_nz(c) - n0, SK_NG) : 0;
+  const int zs = sk32_z(ns), xs = sk32_x(ns), stride = sk32_stride(ns);
+  const int ox = zs + col_nx(c), oy = zs + xs + abs(c.y);
+  const float sy = c.y < 0 ? -1.f : 1.f;
+  float h[SK_NC], lo[SK_NC];  // s0 (re, im), then per harmonic P (re, im), Q (re, im)
 #pragma unroll
-  for (int u = 0; u < SK_NG; ++u) {
-    const int n = n0 + u + 1;
-    if (n > ns) break;
-    const DF &Pr = A.P[u][0], &Pi = A.P[u][1], &Qr = A.Q[u][0], &Qi = A.Q[u][1];
-    o[n] = make_float2(df_diff(Pr, Qi), df_sum(Pi, Qr));
-    if (c.z < 0) o[-n] = make_float2(df_sum(Pr, Qi), df_diff(Pi, Qr));
+  for (int k = 0; k < SK_NC; ++k) h[k] = lo[k] = 0.f;
+  auto flush = [&](int k) {
+    DF a{h[k], 0.f};
+    a.add(lo[k]);
+    h[k] = a.hi;
+    lo[k] = a.lo;
+  };
+  // a thread's first factors of a chunk, read while the one before is summed
+  constexpr int NQ = (3 * SK_CH + SK_T - 1) / SK_T;
+  float2 first[NQ];
+  auto fetch = [&](int l0) {
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+      const int q = tid + k * SK_T, li = l0 + q % SK_CH, d = q / SK_CH;
+      if (d < 3 && li < g.N) first[k] = ph1[((size_t)j * 3 + d) * g.Ns + li];
+    }
+  };
+  fetch(0);
+  for (int l0 = 0; l0 < g.N; l0 += SK_CH) {
+    const int cnt = min(g.N - l0, SK_CH);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) {
+      const int q = tid + k * SK_T, li = q % SK_CH, d = q / SK_CH;
+      if (d >= 3 || li >= cnt) continue;
+      const float2 e1 = first[k];
+      float2 e = d == 2 ? e1 : make_float2(1.f, 0.f);
+      float4 *o = (float4 *)(sh + li * stride + (d == 2 ? 0 : zs + d * xs));
+      for (int n = d == 2 ? 1 : 0; n <= ns; n += 2) {
+        const float2 f = phase32_next(e, e1);
+        *o++ = make_float4(e.x, e.y, f.x, f.y);
+        e = phase32_next(f, e1);
+      }
+    }
+    fetch(l0 + SK_CH);
+    __syncthreads();
+    if (l0 > 0) {
+#pragma unroll
+      for (int k = 0; k < SK_NC; ++k)
+        if (k < 2 + 4 * top) flush(k);
+    }
+    if (live) {
+#pragma unroll 2
+      for (int li = w; li < cnt; li += SK_W) {
+        const float2 *row = sh + li * stride;
+        const float2 ex = row[ox], ey = row[oy];
+        const float yi = sy * ey.y;
+        const float er = fmaf(ex.x, ey.x, __fmul_rn(-ex.y, yi)), ei = fmaf(ex.x, yi, __fmul_rn(ex.y, ey.x));
+        lo[0] = __fadd_rn(lo[0], er);
+        lo[1] = __fadd_rn(lo[1], ei);
+#pragma unroll
+        for (int u = 0; u < SK_NG; u += 2) {
+          if (u >= top) break;
+          const float4 z = *(const float4 *)(row + n0 + u);
+          float *a = lo + 2 + 4 * u;
+          a[0] = fmaf(er, z.x, a[0]);
+          a[1] = fmaf(ei, z.x, a[1]);
+          a[2] = fmaf(er, z.y, a[2]);
+          a[3] = fmaf(ei, z.y, a[3]);
+          a[4] = fmaf(er, z.z, a[4]);
+          a[5] = fmaf(ei, z.z, a[5]);
+          a[6] = fmaf(er, z.w, a[6]);
+          a[7] = fmaf(ei, z.w, a[7]);
+        }
+      }
+    }
+  }
+  // the warps' sums meet in shared memory, the upper half's in the lower half's
+  // first; warp u mod SK_W finishes harmonic u of each item
+  constexpr int HW = SK_W / 2;
+  float2 *mine = sh + (w % HW) * SK_NC * 32 + lane;
+  __syncthreads();
+  if (w >= HW) {
+#pragma unroll
+    for (int k = 0; k < SK_NC; ++k)
+      if (k < 2 + 4 * top) mine[k * 32] = make_float2(h[k], lo[k]);
+  }
+  __syncthreads();
+  if (w < HW) {
+#pragma unroll
+    for (int k = 0; k < SK_NC; ++k)
+      if (k < 2 + 4 * top) {
+        const float2 p = mine[k * 32];
+        DF a{h[k], lo[k]};
+        a.add(p.x);
+        mine[k * 32] = make_float2(a.hi, __fadd_rn(a.lo, p.y));
+      }
+  }
+  __syncthreads();
+  for (int u = w; u <= top; u += SK_W) {
+    if (!live || (more && u == 0)) continue;
+    DF v[4];
+    const int k0 = u == 0 ? 0 : 4 * u - 2, nk = u == 0 ? 2 : 4;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (k >= nk) break;
+#pragma unroll
+      for (int i = 0; i < HW; ++i) {
+        const float2 p = sh[(i * SK_NC + k0 + k) * 32 + lane];
+        v[k].add(p.x);
+        v[k].add(p.y);
+      }
+    }
+    float4 *o = T + ((size_t)j * ncol + ci) * (ns + 1);
+    const float *cf = coef32 + c.w - c.z;  // cf[nz], nz >= c.z
+    if (u == 0) {
+      const float c0 = c.z <= 0 ? cf[0] : 0.f;
+      o[0] = make_float4(c0 * (v[0].hi + v[0].lo), -c0 * (v[1].hi + v[1].lo), 0.f, 0.f);
+    } else {
+      // S(+-n) = (P_r -+ Q_i, P_i +- Q_r)
+      const int n = n0 + u;
+      const float cp = cf[n], cm = c.z < 0 ? cf[-n] : 0.f;
+      const float pr = __fmul_rn(cp, df_diff(v[0], v[3])), pi = __fmul_rn(-cp, df_sum(v[1], v[2]));
+      const float mr = __fmul_rn(cm, df_sum(v[0], v[3])), mi = __fmul_rn(-cm, df_diff(v[1], v[2]));
+      o[n] = make_float4(__fadd_rn(pr, mr), __fadd_rn(pi, mi), __fsub_rn(pr, mr), __fsub_rn(pi, mi));
+      // the forces take harmonics two at a time
+      if (n == col_nz(c) && n % 2 && n < ns) o[n + 1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
   }
 }
+__host__ __device__ inline int sk32_groups(int ncol, int nlong) { return (ncol + nlong + 31) / 32; }
 
-constexpr int RF_PB = 128;  // particles per block of the FP32 reciprocal forces (two threads each)
+// a column as the forces read it: rows of its x and y factors, nzmax, unused;
+// nx, ny, sign of ny
+struct RecipCol {
+  int ox, oy, nz, pad;
+  float fx, fy, sy, pad2;
+};
+__device__ inline RecipCol recip_col32(int4 c, int ns) {
+  return {col_nx(c) * 32, (ns + 1 + abs(c.y)) * 32, col_nz(c), 0, (float)col_nx(c), (float)c.y, c.y < 0 ? -1.f : 1.f, 0.f};
+}
 
-// One particle's reciprocal force sums over cc kept columns (k_recip_force32's
-// arithmetic): cols and the columns' FP32 force tables sT (4 ns + 1 entries
-// each) in shared memory, the particle's x and y phase factors at
-// pxy[(d (ns+1) + n) * stride + li] (shared), its z factors in ez[1..ns]
+// Reciprocal forces on 32 particles of slice j, one a lane, by a block of SK_W warps: warp w sums columns w, w + SK_W, ..., so that
+// the lanes read each table entry at one address; Kahan sums, the warps' added
+// in double-float.  sc, sT: columns (recip_col32) and force tables; pxy: [2][ns+1][32]
+// float2, red: [SK_W][3][32] float2, of these warps alone (red may lie over
+// sT).  NSM: the largest ns.  Bound by FP32 issue, eight multiply-adds a
+// harmonic: 36 us at N = 512, P = 64, |n| <= 10, 57 with two threads a particle,
+// each on half the columns with its own reads of the tables.
 template <int NSM>
-__device__ inline void recip_cols32(Kahan &Fx, Kahan &Fy, Kahan &Fz, const int4 *__restrict__ cols, int cc,
-                                    const float2 *__restrict__ sT, int ns, const float2 *__restrict__ pxy, int stride,
-                                    int li, const float2 *ez) {
-  const int NT = 4 * ns + 1;
-  for (int ci = 0; ci < cc; ++ci) {
-    const int4 c = cols[ci];
-    const int nzc = col_nz(c);
-    float2 ey = pxy[((ns + 1) + (c.y < 0 ? -c.y : c.y)) * stride + li];
-    if (c.y < 0) ey.y = -ey.y;
-    const float2 exy = cmulf(pxy[col_nx(c) * stride + li], ey);
-    const float2 *t = sT + ci * NT;
-    float Ur = t[0].x, Ui = t[0].y, Vr = 0.f, Vi = 0.f;
-#pragma unroll
-    for (int n = 1; n <= NSM; ++n) {
-      if (n > ns || n > nzc) break;
-      const float2 A = t[4 * n - 3], B = t[4 * n - 2], nA = t[4 * n - 1], nB = t[4 * n];
-      const float cz = ez[n].x, sz = ez[n].y;
-      Ur = fmaf(cz, A.x, fmaf(-sz, B.y, Ur));
-      Ui = fmaf(cz, A.y, fmaf(sz, B.x, Ui));
-      Vr = fmaf(cz, nB.x, fmaf(-sz, nA.y, Vr));
-      Vi = fmaf(cz, nB.y, fmaf(sz, nA.x, Vi));
+__device__ inline void recip_tile32(const Geo &g, int ns, int ncol, const RecipCol *sc, const float4 *sT, float2 *pxy,
+                                    float2 *red, const float2 *__restrict__ ph1, double scale, double *__restrict__ f,
+                                    int j, int l0, int w, int lane) {
+  const int l = min(l0 + lane, g.N - 1);  // lanes past the end repeat the last particle
+  const float2 *p1 = ph1 + (size_t)j * 3 * g.Ns + l;
+  if (w < 2) {
+    const float2 e1 = p1[(size_t)w * g.Ns];
+    float2 e = make_float2(1.f, 0.f);
+    for (int n = 0; n <= ns; ++n) {
+      pxy[(w * (ns + 1) + n) * 32 + lane] = e;
+      e = phase32_next(e, e1);
     }
-    const float Tm = fmaf(exy.x, Ui, exy.y * Ur);
-    const float Zm = fmaf(exy.x, Vi, exy.y * Vr);
-    Fx.add((float)col_nx(c) * Tm);
-    Fy.add((float)c.y * Tm);
-    Fz.add(Zm);
+  }
+  float2 ez[NSM], nz[NSM];  // e^{i n z}, and n times it
+  ez[0] = nz[0] = p1[(size_t)2 * g.Ns];
+#pragma unroll
+  for (int n = 1; n < NSM; ++n) {
+    ez[n] = phase32_next(ez[n - 1], ez[0]);
+    nz[n] = make_float2(__fmul_rn((float)(n + 1), ez[n].x), __fmul_rn((float)(n + 1), ez[n].y));
+  }
+  __syncthreads();
+  Kahan F[3];
+  for (int ci = w; ci < ncol; ci += SK_W) {
+    const RecipCol c = sc[ci];
+    const float4 *t = sT + ci * (ns + 1);
+    const float2 vx = pxy[c.ox + lane], vy = pxy[c.oy + lane];
+    const float yi = c.sy * vy.y;
+    const float er = fmaf(vx.x, vy.x, __fmul_rn(-vx.y, yi)), ei = fmaf(vx.x, yi, __fmul_rn(vx.y, vy.x));
+    const float4 w0 = t[0];
+    float ur = w0.x, ui = w0.y, vr = 0.f, vi = 0.f;
+#pragma unroll
+    for (int n = 0; n < NSM; ++n) {  // harmonic n + 1; an odd nzmax is followed by a zero entry
+      if (n % 2 == 0 && n >= c.nz) break;
+      const float4 ab = t[n + 1];
+      ur = fmaf(ez[n].x, ab.x, fmaf(-ez[n].y, ab.w, ur));
+      ui = fmaf(ez[n].x, ab.y, fmaf(ez[n].y, ab.z, ui));
+      vr = fmaf(nz[n].x, ab.z, fmaf(-nz[n].y, ab.y, vr));
+      vi = fmaf(nz[n].x, ab.w, fmaf(nz[n].y, ab.x, vi));
+    }
+    const float Tm = fmaf(er, ui, __fmul_rn(ei, ur));
+    F[0].add(__fmul_rn(c.fx, Tm));
+    F[1].add(__fmul_rn(c.fy, Tm));
+    F[2].add(fmaf(er, vi, __fmul_rn(ei, vr)));
+  }
+  __syncthreads();  // the tables are no longer read
+#pragma unroll
+  for (int d = 0; d < 3; ++d) red[(w * 3 + d) * 32 + lane] = make_float2(F[d].s, -F[d].c);
+  __syncthreads();
+  if (w < 3 && l0 + lane < g.N) {
+    DF s;
+    for (int i = 0; i < SK_W; ++i) {
+      const float2 p = red[(i * 3 + w) * 32 + lane];
+      s.add(p.x);
+      s.add(p.y);
+    }
+    const double ib = w == 0 ? g.inv_box[0] : (w == 1 ? g.inv_box[1] : g.inv_box[2]);
+    f[sidx(j, w, l, 3, g.Ns)] += scale * s.value() * ib;
   }
 }
 
 }  // namespace xk
-

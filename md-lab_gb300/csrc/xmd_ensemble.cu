@@ -18,7 +18,7 @@
 // of the exchange recursions and their block solve, the cycle probabilities
 // G, the exchange spring forces, the FP32 pair tiles and their FP64
 // finishing sums, and the FP32 Ewald reciprocal sums (structure factors
-// per column in double-float, force tables, Kahan-compensated forces).
+// per column in double-float with their force tables, Kahan-compensated forces).
 // The forces add up in the order of the per-system calls (trap, reciprocal,
 // real space; the exchange forces with the second half step), so one
 // persistent step reproduces one step of the per-system calls.
@@ -39,10 +39,9 @@ namespace xk {
 constexpr int ENS_T = 256;                // threads per block
 constexpr int ENS_W = ENS_T / 32;         // warps per block
 constexpr size_t ENS_SMEM = 64 * 1024;    // dynamic shared memory per block
-constexpr int ENS_SKC = 128;              // particles per staged chunk of phase factors
 constexpr int ENS_NSMAX = 11;             // largest Ewald n_sum
 constexpr long long ENS_WAIT_LIMIT = 1LL << 31;  // clock cycles a grid-barrier wait may take (~1 s)
-static_assert(ENS_SKC % SK_PB == 0, "staged chunks hold whole particle blocks");
+static_assert(ENS_T == SK_T, "the FP32 reciprocal sums take SK_W warps");
 
 struct EnsSys {
   EnsSysDesc d;
@@ -50,11 +49,11 @@ struct EnsSys {
   P32 q;
   int T, jobs;
   int ewald;  // reciprocal sums present (D = 3)
-  int ns, ncol, nk;
+  int ns, ncol, nlong;
   const int4 *cols;
   const float *coef32;
-  float2 *ph32, *T32;
-  float2 *S;
+  float2 *ph1;
+  float4 *T32;
   float *part, *x32;
   double lnvi, rscale, pscale;
   int rot[16];  // per task kind: (the kind's tasks before this system) mod (workers of that kind)
@@ -66,11 +65,10 @@ enum {
   R_B_SPR,   // thread: interior springs
   R_B_EINT,  // warp: E_l^(1) per particle (the pair tiles continue its numbering)
   R_B_PAIR,  // warp: FP32 pair tile jobs
-  R_B_SK,    // block: structure factors per slice
+  R_B_SK,    // block: structure factors and force tables per slice and 32 items
   R_C_PRE,   // block: prefix sums per system
-  R_C_TAB,   // thread: force-table entries
+  R_C_REC,   // block: reciprocal forces per slice
   R_D_ENK,   // thread: cycle energies E_l^(k), k >= 2
-  R_D_REC,   // block: reciprocal forces per slice
   R_E_W,     // warp: weight rows
   R_E_PS,    // thread: pair sums per slot
   R_E_INV,   // block: diagonal-block inverses
@@ -104,89 +102,22 @@ __device__ inline void ens_pair_job(const EnsSys &E, int wi, int lane) {
   }
 }
 
-// Structure factors of bead slice j by the calling block: one thread per
-// item (kept column, SK_NG harmonics), every particle block in order, as
-// k_sk32 with one thread per item computes them; the particles' phase
-// factors staged in shared memory ENS_SKC at a time.
-__device__ inline void ens_sk_slice(const EnsSys &E, int j, float2 *sp) {
-  const Geo &g = E.d.g;
-  const int ns = E.ns, N = g.N, tid = threadIdx.x;
-  const int ngr = (ns + SK_NG - 1) / SK_NG;
-  const int items = E.ncol * ngr;
-  const float2 *base = E.ph32 + (size_t)j * 3 * (ns + 1) * g.Ns;
-  const int rows = 3 * (ns + 1);
-  for (int b0 = 0; b0 < items; b0 += ENS_T) {
-    const int item = b0 + tid;
-    const bool live = item < items;
-    const int ci = live ? item / ngr : 0, n0 = live ? (item % ngr) * SK_NG : 0;
-    const int4 c = live ? E.cols[ci] : make_int4(0, 0, 1, 0);
-    const int ax = col_nx(c), ay = c.y < 0 ? -c.y : c.y;
-    const bool cy = c.y < 0;
-    SkAcc A;
-    for (int l0 = 0; l0 < N; l0 += ENS_SKC) {
-      const int cnt = N - l0 < ENS_SKC ? N - l0 : ENS_SKC;
-      __syncthreads();
-      for (int q = tid; q < rows * ENS_SKC; q += ENS_T) {
-        const int l = q % ENS_SKC, row = q / ENS_SKC;
-        sp[row * (ENS_SKC + 1) + l] = l < cnt ? base[(size_t)row * g.Ns + l0 + l] : make_float2(0.f, 0.f);
-      }
-      __syncthreads();
-      if (live) sk_item_blocks(A, sp, ENS_SKC + 1, ns, ax, ay, cy, n0, cnt, 0, 1);
-    }
-    if (live) sk_item_store(A, E.S + (size_t)j * E.nk, c, ns, n0);
-  }
-}
-
-// Reciprocal forces on the particles of bead slice j by the calling block,
-// as k_recip_force32 computes them (two threads per particle, each summing
-// its half of the columns in order with recip_cols32, the halves added in
-// double), 128 particles at a time; the columns, the particles' x and y
-// phase factors and as many columns' force tables as fit are staged in
-// shared memory.
+// Reciprocal forces on the particles of bead slice j by the calling block, 32
+// at a time, as k_recip_force32 computes them; the columns and force tables
+// staged once.
 __device__ inline void ens_recip_slice(const EnsSys &E, int j, unsigned char *sh) {
   const Geo &g = E.d.g;
-  const int ns = E.ns, NT = 4 * ns + 1, ncol = E.ncol, N = g.N, tid = threadIdx.x;
-  int4 *sc = (int4 *)sh;
-  float2 *pxy = (float2 *)(sc + ncol);
-  float2 *sT = pxy + 2 * (ns + 1) * 128;
-  const int ccap = (int)((ENS_SMEM - sizeof(int4) * ncol - sizeof(float2) * 2 * (ns + 1) * 128) / (sizeof(float2) * NT));
-  const float2 *Tj = E.T32 + (size_t)j * ncol * NT;
-  const float2 *pj = E.ph32 + (size_t)j * 3 * (ns + 1) * g.Ns;
-  const int li = tid >> 1, h = tid & 1;
-  const int half = (ncol + 1) / 2, ca = h ? half : 0, cb = h ? ncol : half;
+  const int ns = E.ns, ncol = E.ncol, tid = threadIdx.x;
+  float4 *sT = (float4 *)sh;
+  RecipCol *sc = (RecipCol *)(sT + ncol * (ns + 1));
+  float2 *pxy = (float2 *)(sc + ncol), *red = pxy + 2 * (ns + 1) * 32;
+  const float4 *Tj = E.T32 + (size_t)j * ncol * (ns + 1);
   __syncthreads();
-  for (int q = tid; q < ncol; q += ENS_T) sc[q] = E.cols[q];
-  for (int lb = 0; lb < N; lb += 128) {
-    const int l = lb + li;
-    const bool live = l < N;
-    __syncthreads();
-    for (int q = tid; q < 2 * (ns + 1) * 128; q += ENS_T) {
-      const int r = q / 128, lq = q % 128;
-      pxy[q] = lb + lq < N ? pj[(size_t)r * g.Ns + lb + lq] : make_float2(0.f, 0.f);
-    }
-    float2 ez[ENS_NSMAX + 1];
-#pragma unroll
-    for (int n = 1; n <= ENS_NSMAX; ++n)
-      ez[n] = (live && n <= ns) ? pj[((size_t)2 * (ns + 1) + n) * g.Ns + l] : make_float2(0.f, 0.f);
-    Kahan Fx, Fy, Fz;
-    for (int c0 = 0; c0 < ncol; c0 += ccap) {
-      const int cc = ncol - c0 < ccap ? ncol - c0 : ccap;
-      __syncthreads();
-      for (int q = tid; q < cc * NT; q += ENS_T) sT[q] = Tj[(size_t)c0 * NT + q];
-      __syncthreads();
-      const int a = ca > c0 ? ca : c0, b = cb < c0 + cc ? cb : c0 + cc;
-      if (live && a < b) recip_cols32<ENS_NSMAX>(Fx, Fy, Fz, sc + a, b - a, sT + (size_t)(a - c0) * NT, ns, pxy, 128, li, ez);
-    }
-    double fx = Fx.value(), fy = Fy.value(), fz = Fz.value();
-    fx += __shfl_xor_sync(FULL, fx, 1);
-    fy += __shfl_xor_sync(FULL, fy, 1);
-    fz += __shfl_xor_sync(FULL, fz, 1);
-    if (live && !h) {
-      double *f = E.d.f;
-      f[sidx(j, 0, l, 3, g.Ns)] += E.rscale * fx * g.inv_box[0];
-      f[sidx(j, 1, l, 3, g.Ns)] += E.rscale * fy * g.inv_box[1];
-      f[sidx(j, 2, l, 3, g.Ns)] += E.rscale * fz * g.inv_box[2];
-    }
+  for (int q = tid; q < ncol * (ns + 1); q += ENS_T) sT[q] = Tj[q];
+  for (int q = tid; q < ncol; q += ENS_T) sc[q] = recip_col32(E.cols[q], ns);
+  for (int l0 = 0; l0 < g.N; l0 += 32) {
+    if (l0 > 0) __syncthreads();
+    recip_tile32<ENS_NSMAX>(g, ns, ncol, sc, sT, pxy, red, E.ph1, E.rscale, E.d.f, j, l0, tid >> 5, tid & 31);
   }
 }
 
@@ -309,7 +240,7 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
         d.f[s] = f0;
         if (d.pair_kind) E.x32[s] = (float)xn;
         if constexpr (D == 3)
-          if (E.ewald) phase32_slot(g, E.ns, d.x, E.ph32, s);
+          if (E.ewald) E.ph1[s] = phase32_slot(g, d.x, s);
       }
     }
   }
@@ -350,7 +281,10 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
     for (int i = i0; i < i1; ++i) {
       const EnsSys &E = sys[i];
       if (!E.ewald) continue;
-      for (long long j = ens_first(gb, sys[i].rot[R_B_SK], G); j < E.d.g.P; j += G) ens_sk_slice(E, (int)j, (float2 *)ens_sh);
+      const long long n = (long long)E.d.g.P * sk32_groups(E.ncol, E.nlong);
+      for (long long q = ens_first(gb, sys[i].rot[R_B_SK], G); q < n; q += G)
+        sk32_group(E.d.g, E.ns, E.ncol, E.nlong, E.cols, E.coef32, E.ph1, E.T32, (int)(q % E.d.g.P),
+                   (int)(q / E.d.g.P), (float2 *)ens_sh);
     }
   }
   ens_sub(bar, 3);
@@ -358,7 +292,7 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
   ens_stamp(bar, 2);
 
   // C: prefix sums of the increments (a block per system, the block size of
-  // k_enk_direct's own scan, into gl[N ..]); the FP32 force tables
+  // k_enk_direct's own scan, into gl[N ..]); reciprocal forces
   {
     for (int i = i0; i < i1; ++i) {
       const EnsSysDesc &d = sys[i].d;
@@ -373,19 +307,13 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
     for (int i = i0; i < i1; ++i) {
       const EnsSys &E = sys[i];
       if (!E.ewald) continue;
-      const int per = E.ns + 1;
-      const long long n = (long long)E.d.g.P * E.ncol * per;
-      for (long long q = ens_first(gt, sys[i].rot[R_C_TAB], GT); q < n; q += GT) {
-        const long long r = q / per;
-        recip_table32_entry(E.cols, E.ncol, E.S, E.coef32, E.nk, E.T32, E.ns, (int)(r / E.ncol), (int)(r % E.ncol),
-                            (int)(q % per));
-      }
+      for (long long j = ens_first(gb, sys[i].rot[R_C_REC], G); j < E.d.g.P; j += G) ens_recip_slice(E, (int)j, ens_sh);
     }
   }
   ens_grid_sync(bar, G, limit);
   ens_stamp(bar, 3);
 
-  // D: the cycle energies E_l^(k), k >= 2; reciprocal forces
+  // D: the cycle energies E_l^(k), k >= 2
   {
     for (int i = i0; i < i1; ++i) {
       const EnsSysDesc &d = sys[i].d;
@@ -399,13 +327,6 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
         const int k = 2 + (int)(q - (long long)r * (r - 1) / 2);
         enk_entry<D>(g, d.x, d.m, d.w2, d.image, d.Eint, d.gl + g.N, d.ENk, r + 1, k);
       }
-    }
-  }
-  if constexpr (D == 3) {
-    for (int i = i0; i < i1; ++i) {
-      const EnsSys &E = sys[i];
-      if (!E.ewald) continue;
-      for (long long j = ens_first(gb, sys[i].rot[R_D_REC], G); j < E.d.g.P; j += G) ens_recip_slice(E, (int)j, ens_sh);
     }
   }
   ens_grid_sync(bar, G, limit);
@@ -627,12 +548,11 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
       if (r.nsum < 1 || r.nsum > ENS_NSMAX) return cudaErrorInvalidValue;
       E.ns = r.nsum;
       E.ncol = r.ncol;
-      E.nk = r.nk;
+      E.nlong = r.nlong;
       E.cols = (const int4 *)r.kvec;
       E.coef32 = (const float *)(r.coef + r.nk);
-      E.ph32 = (float2 *)(r.phase + recip_phase_doubles(g, r.nsum));
-      E.T32 = (float2 *)r.T;
-      E.S = (float2 *)r.S;
+      E.ph1 = (float2 *)(r.phase + recip_phase_doubles(g, r.nsum));
+      E.T32 = (float4 *)r.T;
       E.rscale = 4 * M_PI * E.d.inv_mP;
     }
     E.lnvi = E.d.vi != 0.0 ? log(E.d.vi) : 0.0;
@@ -665,8 +585,8 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
   // the kernel's loops number them); rot = tasks before the system, mod the
   // group's workers of that kind
   for (int k = 0; k < K; ++k) {
-    const long long stride[ENS_NROT] = {Gk * ENS_T, Gk * ENS_T, Gk * ENS_W, Gk * ENS_W, Gk, Gk, Gk * ENS_T, Gk * ENS_T,
-                                        Gk, Gk * ENS_W, Gk * ENS_T, Gk, Gk, Gk * ENS_W, Gk * ENS_T};
+    const long long stride[ENS_NROT] = {Gk * ENS_T, Gk * ENS_T, Gk * ENS_W, Gk * ENS_W, Gk, Gk, Gk, Gk * ENS_T, Gk * ENS_W,
+                                        Gk * ENS_T, Gk, Gk, Gk * ENS_W, Gk * ENS_T};
     long long base[ENS_NROT] = {};
     for (int pass = 0; pass < 2; ++pass)  // the pair tiles continue E_l^(1)'s numbering
       for (int i = goff[k]; i < goff[k + 1]; ++i) {
@@ -678,11 +598,10 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
         cnt[R_B_SPR] = P > 2 ? (P - 2) * g.Ns : 0;
         cnt[R_B_EINT] = N;
         cnt[R_B_PAIR] = E.d.pair_kind ? (long long)E.jobs * P : 0;
-        cnt[R_B_SK] = E.ewald ? P : 0;
+        cnt[R_B_SK] = E.ewald ? P * sk32_groups(E.ncol, E.nlong) : 0;
         cnt[R_C_PRE] = N >= 2 ? 1 : 0;
-        cnt[R_C_TAB] = E.ewald ? P * E.ncol * (E.ns + 1) : 0;
+        cnt[R_C_REC] = E.ewald ? P : 0;
         cnt[R_D_ENK] = N * (N - 1) / 2;
-        cnt[R_D_REC] = E.ewald ? P : 0;
         cnt[R_E_W] = N;
         cnt[R_E_PS] = E.d.pair_kind ? slots : 0;
         cnt[R_E_INV] = 2 * ((N + TS_CHUNK - 1) / TS_CHUNK);

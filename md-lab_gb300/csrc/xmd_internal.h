@@ -108,6 +108,7 @@ struct PimdDev {
   double rc_alpha = 0, rc_qs = 0, rc_box[3] = {0, 0, 0};
   int rc_nk = 0;
   int rc_ncol = 0;  // kept wave-vector columns
+  int rc_nlong = 0; // of those, with a second FP32 structure-factor item
   int rc_tsz = 0;   // entries of their compact force tables
   int rc_df_items = 0, rc_items = 0, rc_tdf = 0;  // the double-float kernels' tables (xk::Recip)
   double rc_csum = 0;

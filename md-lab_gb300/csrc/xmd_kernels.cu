@@ -2739,6 +2739,8 @@ cudaError_t recip_setup(const Geo &g, int ns, double alpha, double qs, Recip &r,
   r.nsum = ns;
   r.nk = nk;
   r.ncol = (int)cd.size();
+  r.nlong = 0;
+  for (const auto &k : kept) r.nlong += k.first > SK_NG;
   r.tsz = toff.back();
   r.csum = 0;
   for (double c : coef) r.csum += c;
@@ -3778,184 +3780,79 @@ cudaError_t pair_force32(const Geo &g, const PairPrm &p, const double *x, const 
 }
 
 // ---- reciprocal space, mixed ----------------------------------------
-// FP32 copies of the FP64 phase factors: ph32[((j*3 + d)*(NS+1) + n)*Ns + l]
-// FP32 phases straight from the positions (the layout of k_phase): the
-// fraction of x/L is taken in FP64 (exact), the sine and cosine of the
-// reduced angle in FP32, the harmonics by FP32 complex products; the
-// results match k_phase's rounded to FP32 to a few FP32 units, without the
-// FP64 sine and cosine.
-__global__ void k_phase32(Geo g, int ns, const double *__restrict__ x, float2 *__restrict__ ph32) {
+// first phase factors of the positions: ph1[(j*3 + d)*Ns + l]
+__global__ void __launch_bounds__(256) k_phase32(Geo g, const double *__restrict__ x, float2 *__restrict__ ph1) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= (size_t)g.P * 3 * g.Ns) return;
-  phase32_slot(g, ns, x, ph32, t);
+  if (t < (size_t)g.P * 3 * g.Ns) ph1[t] = phase32_slot(g, x, t);
 }
 
-
-// structure factors of the mixed form: block (items, slice j) of 256
-// threads, GR threads per item (GR = 1: each item's particles in order,
-// the persistent ensemble's arithmetic; GR = 4 or 16 for large slices with
-// few items: the GR threads take interleaved particles and their
-// accumulators are combined pairwise in a fixed order).  The staged rows
-// are padded by one entry so that the lanes' different rows fall in
-// different banks.
-template <int NS, int GR>
-__global__ void __launch_bounds__(256) k_sk32(Geo g, const float2 *__restrict__ ph, const int4 *__restrict__ cols,
-                                              int ncol, float2 *__restrict__ S, int nk) {
-  constexpr int NGR = (NS + SK_NG - 1) / SK_NG;
-  constexpr int CH = GR == 16 ? 256 : 64, LD = CH + 1;  // particles per staged chunk (whole blocks of SK_PB GR)
-  static_assert(CH % (SK_PB * GR) == 0, "staged chunks hold whole particle blocks");
-  __shared__ float2 sp[3 * (NS + 1) * LD];
-  const int j = blockIdx.y;
-  const int gq = threadIdx.x % GR;
-  const int item = blockIdx.x * (256 / GR) + threadIdx.x / GR;
-  const bool live = item < ncol * NGR;
-  const int ci = live ? item / NGR : 0, n0 = live ? (item % NGR) * SK_NG : 0;
-  const int4 c = live ? cols[ci] : make_int4(0, 0, 1, 0);
-  const int ax = col_nx(c), ay = c.y < 0 ? -c.y : c.y;
-  const bool cy = c.y < 0;
-  SkAcc A;
-  const float2 *base = ph + (size_t)j * 3 * (NS + 1) * g.Ns;
-  for (int l0 = 0; l0 < g.N; l0 += CH) {
-    const int cnt = g.N - l0 < CH ? g.N - l0 : CH;
-    __syncthreads();
-    for (int q = threadIdx.x; q < 3 * (NS + 1) * CH; q += 256) {
-      const int l = q % CH, row = q / CH;
-      sp[row * LD + l] = l < cnt ? base[(size_t)row * g.Ns + l0 + l] : make_float2(0.f, 0.f);
-    }
-    __syncthreads();
-    if (live) sk_item_blocks(A, sp, LD, NS, ax, ay, cy, n0, cnt, gq, GR);
-  }
-  if (GR > 1) {
-    auto comb = [](DF &v, int o) {
-      const float h = __shfl_xor_sync(FULL, v.hi, o), lo = __shfl_xor_sync(FULL, v.lo, o);
-      v.add(h);
-      v.lo += lo;
-    };
-#pragma unroll
-    for (int o = 1; o < GR; o <<= 1) {
-      comb(A.s0r, o);
-      comb(A.s0i, o);
-#pragma unroll
-      for (int u = 0; u < SK_NG; ++u) {
-        comb(A.P[u][0], o);
-        comb(A.P[u][1], o);
-        comb(A.Q[u][0], o);
-        comb(A.Q[u][1], o);
-      }
-    }
-  }
-  if (!live || gq != 0) return;
-  sk_item_store(A, S + (size_t)j * nk, c, NS, n0);
+// a block per (slice, 32 items), the longest items' blocks first
+__global__ void __launch_bounds__(SK_T, 2) k_sk32(Geo g, int ns, int ncol, int nlong, const int4 *__restrict__ cols,
+                                                  const float *__restrict__ coef32, const float2 *__restrict__ ph1,
+                                                  float4 *__restrict__ T) {
+  extern __shared__ __align__(16) float2 sk32_sh[];
+  sk32_group(g, ns, ncol, nlong, cols, coef32, ph1, T, blockIdx.x, blockIdx.y, sk32_sh);
 }
 
-// force tables as k_recip_tables, stored in FP32
+// a block per slice and 32 of its particles (recip_tile32); four blocks an SM
+// (64 registers) or three (80) at N = 512, P = 64 36 us each, four better where
+// the columns are few
 template <int NS>
-__global__ void k_recip_tables32(const int4 *__restrict__ cols, int ncol, const float2 *__restrict__ S,
-                                 const float *__restrict__ coef32, int nk, float2 *__restrict__ T) {
+__global__ void __launch_bounds__(SK_T, 4) k_recip_force32(Geo g, int ncol, const int4 *__restrict__ cols,
+                                                           const float2 *__restrict__ ph1,
+                                                           const float4 *__restrict__ T, double scale,
+                                                           double *__restrict__ f) {
+  extern __shared__ __align__(16) float4 rf32_sh[];
+  float4 *sT = rf32_sh;
+  RecipCol *sc = (RecipCol *)(sT + ncol * (NS + 1));
   const int j = blockIdx.y;
-  const int ci = blockIdx.x * blockDim.y + threadIdx.y;
-  const int n = threadIdx.x;
-  if (ci >= ncol || n > NS) return;
-  recip_table32_entry(cols, ncol, S, coef32, nk, T, NS, j, ci, n);
+  const float4 *Tj = T + (size_t)j * ncol * (NS + 1);
+  for (int q = threadIdx.x; q < ncol * (NS + 1); q += SK_T) sT[q] = Tj[q];
+  for (int q = threadIdx.x; q < ncol; q += SK_T) sc[q] = recip_col32(cols[q], NS);
+  recip_tile32<NS>(g, NS, ncol, sc, sT, (float2 *)(sc + ncol), (float2 *)rf32_sh, ph1, scale, f, j, blockIdx.x * 32,
+                   threadIdx.x >> 5, threadIdx.x & 31);
 }
 
-// Two threads per particle, RF_PB particles a block: thread h of a pair
-// sums the columns of its half (recip_cols32, the columns in order), and the
-// two compensated sums are added in double.
-template <int NS>
-__global__ void __launch_bounds__(2 * RF_PB) k_recip_force32(Geo g, const float2 *__restrict__ ph,
-                                                       const int4 *__restrict__ cols, int ncol,
-                                                       const float2 *__restrict__ T, double scale,
-                                                       double *__restrict__ f) {
-  constexpr int NT = 4 * NS + 1;
-  extern __shared__ __align__(16) float smf[];
-  // the columns (16-byte records first, so that they stay aligned), the x
-  // and y phase factors of the block's 64 particles, and the slice's force
-  // tables, all staged
-  int4 *sc = (int4 *)smf;
-  float2 *pxy = (float2 *)(sc + ncol);
-  float2 *sT = pxy + 2 * (NS + 1) * RF_PB;
-  const int j = blockIdx.y;
-  const float2 *Tj = T + (size_t)j * ncol * NT;
-  for (int q = threadIdx.x; q < ncol * NT; q += blockDim.x) sT[q] = Tj[q];
-  for (int q = threadIdx.x; q < ncol; q += blockDim.x) sc[q] = cols[q];
-  const int l0 = blockIdx.x * RF_PB, li = threadIdx.x >> 1, h = threadIdx.x & 1, l = l0 + li;
-  const float2 *pj = ph + (size_t)j * 3 * (NS + 1) * g.Ns;
-  for (int q = threadIdx.x; q < 2 * (NS + 1) * RF_PB; q += blockDim.x) {
-    const int r = q / RF_PB, lq = l0 + q % RF_PB;
-    pxy[q] = lq < g.N ? pj[(size_t)r * g.Ns + lq] : make_float2(0.f, 0.f);
-  }
-  __syncthreads();
-  const bool live = l < g.N;
-  float2 ez[NS + 1];
-#pragma unroll
-  for (int n = 1; n <= NS; ++n) ez[n] = live ? pj[((size_t)2 * (NS + 1) + n) * g.Ns + l] : make_float2(0.f, 0.f);
-  const int half = (ncol + 1) / 2, ca = h ? half : 0, cb = h ? ncol : half;
-  Kahan Fx, Fy, Fz;
-  if (live) recip_cols32<NS>(Fx, Fy, Fz, sc + ca, cb - ca, sT + (size_t)ca * NT, NS, pxy, RF_PB, li, ez);
-  double fx = Fx.value(), fy = Fy.value(), fz = Fz.value();
-  fx += __shfl_xor_sync(FULL, fx, 1);
-  fy += __shfl_xor_sync(FULL, fy, 1);
-  fz += __shfl_xor_sync(FULL, fz, 1);
-  if (!live || h) return;
-  f[sidx(j, 0, l, 3, g.Ns)] += scale * fx * g.inv_box[0];
-  f[sidx(j, 1, l, 3, g.Ns)] += scale * fy * g.inv_box[1];
-  f[sidx(j, 2, l, 3, g.Ns)] += scale * fz * g.inv_box[2];
-}
-
-// phases, structure factors, tables and forces in FP32 for all kept columns
+// phases, structure factors with their force tables, and forces in FP32 for
+// all kept columns; the tables use the FP64 form's buffer, the phases lie
+// behind the FP64 ones
 cudaError_t recip_force32(const Geo &g, const Recip &r, const double *x, double inv_mP, double *f,
                           cudaStream_t st) {
   if (g.D != 3) return cudaErrorInvalidValue;
-  const int4 *cols = (const int4 *)r.kvec;
-  const int nc = r.ncol;
-  // the FP32 structure factors and tables use the FP64 form's buffers
-  float2 *S32 = (float2 *)r.S, *T32 = (float2 *)r.T;
-  const size_t n = (size_t)g.P * 3 * g.Ns;
-  // FP32 phases live behind the FP64 ones in the same buffer
-  float2 *ph32 = (float2 *)(r.phase + recip_phase_doubles(g, r.nsum));
+  if (r.ncol <= 0) return cudaSuccess;
+  float2 *ph1 = (float2 *)(r.phase + recip_phase_doubles(g, r.nsum));
   {
     XK_PROF("phase32");
-    k_phase32<<<cdiv(n, 256), 256, 0, st>>>(g, r.nsum, x, ph32);
+    k_phase32<<<cdiv((size_t)g.P * 3 * g.Ns, 256), 256, 0, st>>>(g, x, ph1);
   }
   cudaError_t e = XK_LAUNCHED();
   if (e != cudaSuccess) return e;
-  if (nc <= 0) return cudaSuccess;
-  dim3 tgrid((nc + 7) / 8, g.P), tblk(r.nsum + 1, 8);
-  dim3 grid((g.N + RF_PB - 1) / RF_PB, g.P);
-  const size_t smem =
-      sizeof(float2) * nc * (4 * r.nsum + 1) + sizeof(int4) * nc + sizeof(float2) * 2 * (r.nsum + 1) * RF_PB;
+  {
+    XK_PROF("sk32");
+    static bool opted = false;
+    if (!opted) {
+      e = cudaFuncSetAttribute(k_sk32, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      if (e != cudaSuccess) return e;
+      opted = true;
+    }
+    k_sk32<<<dim3(g.P, sk32_groups(r.ncol, r.nlong)), SK_T, sk32_smem(r.nsum), st>>>(
+        g, r.nsum, r.ncol, r.nlong, (const int4 *)r.kvec, (const float *)(r.coef + r.nk), ph1, (float4 *)r.T);
+  }
+  e = XK_LAUNCHED();
+  if (e != cudaSuccess) return e;
+  XK_PROF("recip_force32");
   DISPATCH_NS(r.nsum, {
-    {
-      // one thread per item for slices below SK_BIG_N particles; above,
-      // 4 or (few items) 16 threads share an item's particle blocks
-      XK_PROF("sk32");
-      const int items = nc * ((NS + SK_NG - 1) / SK_NG);
-      if (g.N < SK_BIG_N)
-        k_sk32<NS, 1><<<dim3((items + 255) / 256, g.P), 256, 0, st>>>(g, ph32, cols, nc,
-                                                                     S32, r.nk);
-      else if (items > 64 || NS > 6)
-        k_sk32<NS, 4><<<dim3((items + 63) / 64, g.P), 256, 0, st>>>(g, ph32, cols, nc, S32, r.nk);
-      else
-        k_sk32<(NS <= 6 ? NS : 6), 16><<<dim3((items + 15) / 16, g.P), 256, 0, st>>>(
-            g, ph32, cols, nc, S32, r.nk);
-    }
-    {
-      XK_PROF("recip_tables32");
-      k_recip_tables32<NS><<<tgrid, tblk, 0, st>>>(cols, nc, S32, (const float *)(r.coef + r.nk),
-                                                  r.nk, T32);
-    }
     auto kf = k_recip_force32<NS>;
     static bool opted = false;
     if (!opted) {
-      cudaError_t ea = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
-      if (ea != cudaSuccess) return ea;
+      e = cudaFuncSetAttribute(kf, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      if (e != cudaSuccess) return e;
       opted = true;
     }
-    {
-      XK_PROF("recip_force32");
-      kf<<<grid, 2 * RF_PB, smem, st>>>(g, ph32, cols, nc, T32, 4 * M_PI * inv_mP, f);
-    }
+    const size_t tab = (sizeof(float4) * (NS + 1) + sizeof(RecipCol)) * r.ncol + sizeof(float2) * 2 * (NS + 1) * 32;
+    const size_t red = sizeof(float2) * SK_W * 3 * 32;
+    kf<<<dim3((g.N + 31) / 32, g.P), SK_T, tab > red ? tab : red, st>>>(
+        g, r.ncol, (const int4 *)r.kvec, ph1, (const float4 *)r.T, 4 * M_PI * inv_mP, f);
   });
   return XK_LAUNCHED();
 }

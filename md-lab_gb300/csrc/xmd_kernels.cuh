@@ -260,6 +260,7 @@ struct Recip {
   int nsum;
   int nk;              // half-space wave vectors of the cube
   int ncol;            // kept columns (set by recip_setup)
+  int nlong;           // of those, with more harmonics than one FP32 structure-factor item has (likewise)
   int tsz;             // entries of the kept columns' force tables (compact, set by recip_setup)
   int df_items, items; // structure-factor items of the double-float kernels: with double-float harmonics, all
   int tdf;             // float4 entries of their compact force tables (all three set by recip_setup)
@@ -323,7 +324,7 @@ cudaError_t pair_force32(const Geo &g, const PairPrm &p, const double *x, const 
 // FP32 pair kernel for a system shape; 8 unless set
 void set_pair32_warps(int kind, int D, int N, int P, int warps);
 int pair32_warps(int kind, int D, int N, int P);
-// needs r.phase sized recip_phase_doubles(g, nsum) * 3 / 2 (FP32 copy behind)
+// needs r.phase sized recip_phase_doubles(g, nsum) * 3 / 2 (FP32 phases behind)
 cudaError_t recip_force32(const Geo &g, const Recip &r, const double *x, double inv_mP, double *f,
                           cudaStream_t st);
 

@@ -403,6 +403,7 @@ int xmd::ewald_tables(md_pimd_t_x *pimd, SimDev *sd, PimdDev *pd) {
   r.S = pd->rc_S.as<double>();
   XMD_CUDA(xk::recip_setup(g, ns, a, qs, r, stream()));
   pd->rc_ncol = r.ncol;
+  pd->rc_nlong = r.nlong;
   pd->rc_tsz = r.tsz;
   pd->rc_df_items = r.df_items;
   pd->rc_items = r.items;
@@ -425,6 +426,7 @@ xk::Recip xmd::recip_of(PimdDev *pd) {
   r.nsum = pd->rc_nsum;
   r.nk = pd->rc_nk;
   r.ncol = pd->rc_ncol;
+  r.nlong = pd->rc_nlong;
   r.tsz = pd->rc_tsz;
   r.df_items = pd->rc_df_items;
   r.items = pd->rc_items;
