@@ -208,7 +208,11 @@ constexpr size_t ewd_smem() {
 // 218 us; energies of the latter 57 and 325 us; 256 x 256 cross pairs 145 and
 // 667 us).  The forces' error against 64-bit sums, set by the cut-off at
 // alpha R = 5.2, is 3.6e-13 of the forces' norm (4.1e-13 with the FP64 tiles
-// and their FP32 far images), 12 to 512 electrons alike.
+// and their FP32 far images), 12 to 512 electrons alike.  Energies take three
+// limbs: in two, images below the sum's last bit were lost and biased it by
+// -5e-16 of the pair energies; now 0.6e-15 (128 electrons, 32 beads, rms of 16
+// states) and 0.5e-15 (512, 64) of the energy against 64 bits, 1.3e-15 and
+// 2.6e-15 with the FP64 tiles, for 61 us at the former instead of 59.
 template <bool CROSS, bool ENERGY>
 __global__ void __launch_bounds__(32 * EWD_WARPS, 2)
     k_ewd_tiles(EwdPrm q, int P, EwdSide A, EwdSide B, float2 *__restrict__ outa, float2 *__restrict__ outb,
@@ -263,6 +267,7 @@ __global__ void __launch_bounds__(32 * EWD_WARPS, 2)
     const bool test_cube = !q.cube || __any_sync(ALL, wrapped);
     __syncwarp();
     df fa[3], fb[3], en = {0.f, 0.f};
+    float enc = 0.f;  // third limb of the energy: far images are smaller than the pair's last bit
 #pragma unroll
     for (int d = 0; d < 3; ++d) fa[d] = fb[d] = {0.f, 0.f};
     const int s0 = diag ? 1 : 0, s1 = diag ? 16 : 31;
@@ -325,10 +330,13 @@ __global__ void __launch_bounds__(32 * EWD_WARPS, 2)
       for (int r = lane; r < total; r += 32) {
         const float2 v = ws->q[r];
         const df f = ewd_image<ENERGY>({v.x, v.y}, tab);
-        if (ENERGY)
-          en = df_norm(df_add(en, f));
-        else
+        if (ENERGY) {
+          const df s0 = two_sum(en.h, f.h), s1 = two_sum(en.l, f.l), s2 = two_sum(s0.l, s1.h);
+          en = fast_two_sum(s0.h, s2.h);
+          enc = __fadd_rn(enc, __fadd_rn(s1.l, s2.l));
+        } else {
           ws->q[r] = make_float2(f.h, f.l);
+        }
       }
       __syncwarp();
       if constexpr (ENERGY) {
@@ -344,7 +352,7 @@ __global__ void __launch_bounds__(32 * EWD_WARPS, 2)
               const float R2 = R0.h + q.Sh[d] + q.Th[d] * m[d].h + ((c & 1) ? Ad[0].h : 0.f) +
                                ((c & 2) ? Ad[1].h : 0.f) + ((c & 4) ? Ad[2].h : 0.f);
               const float na = d == 0 ? a2.y - b2v.y : (d == 1 ? a2.z - b2v.z : a2.w - b2v.w);
-              if (R2 < q.rc2 && ((okm >> c) & 1u) && fabsf(na + sh[d] - sg[d]) <= q.nsum) en.l += ewd_erfc32(R2);
+              if (R2 < q.rc2 && ((okm >> c) & 1u) && fabsf(na + sh[d] - sg[d]) <= q.nsum) enc += ewd_erfc32(R2);
             }
         }
       } else {
@@ -376,7 +384,7 @@ __global__ void __launch_bounds__(32 * EWD_WARPS, 2)
       }
     }
     if constexpr (ENERGY) {
-      double e = df_value(en);
+      double e = df_value(en) + (double)enc;
 #pragma unroll
       for (int o = 16; o; o >>= 1) e += __shfl_down_sync(ALL, e, o);
       if (lane == 0) eout[w] = e;
