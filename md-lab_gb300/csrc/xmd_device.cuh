@@ -10,6 +10,7 @@
 #include <cmath>
 #include <cstddef>
 #include <cstdint>
+#include <type_traits>
 
 #include "xmd_ewald_tables.h"
 #include "xmd_kernels.cuh"
@@ -733,18 +734,36 @@ struct DF {
 // 2.32 to 1.11.
 constexpr float EW32_XCUT = 3.6f;
 
+// The approximate unit's operations without the code around them for
+// subnormal numbers, which cannot matter here: 1/R^3 overflows for such an R^2,
+// and the other arguments are within [1, 3] and above -19.
+__device__ __forceinline__ float rsqrt_ftz(float v) {
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float rcp_ftz(float v) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float ex2_ftz(float v) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
 // h(alpha R) / R^3 in FP32 without tables: h(x) = exp(-x^2) (2x/sqrt(pi) +
 // erfcx(x)), erfcx(x) ~ t P(t), t = 1/(1 + x/2) (fit in xmd_ewald_tables.h,
 // relative error 2e-8 on [0, 4.7]); 1/R from rsqrt, exp from ex2
 __device__ __forceinline__ float ew_h32(float R2, float alpha) {
   const float cc[EW32_DEG + 1] = EW32_ERFCX_INIT;
-  const float ri = rsqrtf(R2);
+  const float ri = rsqrt_ftz(R2);
   const float x = alpha * (R2 * ri);
-  const float t = __fdividef(1.f, fmaf((float)EW32_C, x, 1.f));
+  const float t = rcp_ftz(fmaf((float)EW32_C, x, 1.f));
   float q = cc[EW32_DEG];
 #pragma unroll
   for (int k = EW32_DEG - 1; k >= 0; --k) q = fmaf(q, t, cc[k]);
-  const float e = __expf(-x * x);
+  const float e = ex2_ftz(-x * x * 1.4426950408889634f);
   return e * fmaf(x, 1.1283791670955126f, q * t) * (ri * ri * ri);
 }
 
@@ -757,6 +776,7 @@ struct P32 {
   float qs;          // Coulomb / Ewald strength
   float alpha, rc2;  // Ewald: splitting, FP32 cut-off squared
   int kmax;          // Ewald: 0 = 8-image search, else |k_d| <= kmax
+  int single;        // Ewald: no image shifted along two axes lies inside the cut-off
   int nsum;          // Ewald: the reference's image cube |n_d| <= nsum
   int uniform;       // all beads of the system have one mass (1/m = im0)
   float im0;
@@ -765,7 +785,7 @@ struct P32 {
 // the FP32 pair kernel's constants for a system and potential (host)
 P32 make_p32(const Geo &g, const PairPrm &p);
 
-template <int D, int KIND>
+template <int D, int KIND, bool SINGLE>
 __device__ inline void pair_eval32(const P32 &q, const float *dx, float *F) {
   if (KIND == PAIR_GAUSSIAN || KIND == PAIR_PERIODIC_GAUSSIAN) {
     float t[D], r2 = 0.f;
@@ -806,7 +826,42 @@ __device__ inline void pair_eval32(const P32 &q, const float *dx, float *F) {
     }
     const float ns = (float)q.nsum;
     float F0 = 0.f, F1 = 0.f, F2 = 0.f;
-    if (q.kmax == 0) {
+    if (SINGLE) {
+      // A component shifted by a box edge is at least half the edge long, so
+      // below sqrt(L_d^2 + L_e^2) / 2 (0.707 L; alpha L > 5.1) only the minimum
+      // image and the three shifted along one axis are left: the first is
+      // evaluated by every lane together, the others, 0.23 a pair at alpha L =
+      // 5.6, as many rounds as the busiest lane has (see k_pair_tiles32 for
+      // what this gives).
+      const float R0 = fmaf(m[2], m[2], fmaf(m[1], m[1], m[0] * m[0]));
+      bool in = R0 < q.rc2;
+      unsigned mask = 0u;
+#pragma unroll
+      for (int d = 0; d < 3; ++d)
+        if (R0 + q.L[d] * fmaf(-2.f, fabsf(m[d]), q.L[d]) < q.rc2) mask |= 1u << d;
+      if (q.nsum < 2) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          if (!(fabsf(r[d]) <= ns)) in = false, mask &= 1u << d;
+          if (!(fabsf(r[d] + sg[d]) <= ns)) mask &= ~(1u << d);
+        }
+      }
+      const float mult0 = in ? ew_h32(R0, q.alpha) : 0.f;
+      F0 = m[0] * mult0;
+      F1 = m[1] * mult0;
+      F2 = m[2] * mult0;
+      while (mask) {
+        const unsigned low = mask & (0u - mask);
+        mask ^= low;
+        const float t0 = (low & 1) ? m[0] - copysignf(q.L[0], m[0]) : m[0];
+        const float t1 = (low & 2) ? m[1] - copysignf(q.L[1], m[1]) : m[1];
+        const float t2 = (low & 4) ? m[2] - copysignf(q.L[2], m[2]) : m[2];
+        const float mult = ew_h32(fmaf(t2, t2, fmaf(t1, t1, t0 * t0)), q.alpha);
+        F0 = fmaf(t0, mult, F0);
+        F1 = fmaf(t1, mult, F1);
+        F2 = fmaf(t2, mult, F2);
+      }
+    } else if (q.kmax == 0) {
       // With a_d = |m_d| the shifted component has length L_d - a_d, so an
       // image's squared distance is |m|^2 plus dl_d = L_d (L_d - 2 a_d) for
       // each shifted axis: the 8 candidates are tested with a few adds.  The
@@ -1077,6 +1132,8 @@ __device__ __forceinline__ float2 phase32_next(float2 e, float2 e1) {
   return make_float2(fmaf(e.x, e1.x, __fmul_rn(-e.y, e1.y)), fmaf(e.x, e1.y, __fmul_rn(e.y, e1.x)));
 }
 
+constexpr int P32_UNROLL = 2;  // steps of the single-shift Ewald tiles evaluated side by side
+
 // tile job wi (slice wi / jobs, tile pair I <= J) of the FP32 pair forces,
 // one warp: per-tile sums into out (see k_pair_tiles32)
 template <int D, int KIND>
@@ -1099,57 +1156,54 @@ __device__ inline void pair_tile32_job(const Geo &g, const P32 &q, const float *
     xb[d] = vb ? x[sidx(j, d, b0, D, g.Ns)] : 0.f;
     fa[d] = fb[d] = 0.f;
   }
-  const int src = (lane + 1) & 31;
-  if (q.uniform) {
-    for (int s = 0; s < 32; ++s) {
-      const int bi = J * 32 + ((lane + s) & 31);
-      if (va && bi < g.N && (I != J || a > bi)) {
-        float dx[D], F[D];
+  // a diagonal tile visits each pair once in 16 steps (the last by half the lanes)
+  const bool diag = I == J;
+  const int src = (lane + 1) & 31, s0 = diag ? 1 : 0, s1 = diag ? 16 : 31;
+  const float ima = !q.uniform && va ? im[(size_t)j * g.Ns + a] : 1.f;
+  float imb = !q.uniform && vb ? im[(size_t)j * g.Ns + b0] : 1.f;
+  if (diag) {
 #pragma unroll
-        for (int d = 0; d < D; ++d) dx[d] = xa[d] - xb[d];
-        pair_eval32<D, KIND>(q, dx, F);
+    for (int d = 0; d < D; ++d) xb[d] = __shfl_sync(FULL, xb[d], src);
+    imb = __shfl_sync(FULL, imb, src);
+  }
+  auto step = [&](int s, auto single) {
+    const int bi = J * 32 + ((lane + s) & 31);
+    if (va && bi < g.N && !(diag && s == 16 && lane >= 16)) {
+      float dx[D], F[D];
 #pragma unroll
-        for (int d = 0; d < D; ++d) {
-          fa[d] += F[d];
-          fb[d] -= F[d];
-        }
+      for (int d = 0; d < D; ++d) dx[d] = xa[d] - xb[d];
+      pair_eval32<D, KIND, decltype(single)::value>(q, dx, F);
+      // the reference divides by the mass of the higher-index particle; with
+      // one mass for all the sums are multiplied by its inverse
+      if (!q.uniform) {
+        const float inv = a > bi ? ima : imb;
+#pragma unroll
+        for (int d = 0; d < D; ++d) F[d] *= inv;
       }
 #pragma unroll
       for (int d = 0; d < D; ++d) {
-        xb[d] = __shfl_sync(FULL, xb[d], src);
-        fb[d] = __shfl_sync(FULL, fb[d], src);
+        fa[d] += F[d];
+        fb[d] -= F[d];
       }
     }
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-      fa[d] *= q.im0;
-      fb[d] *= q.im0;
+      xb[d] = __shfl_sync(FULL, xb[d], src);
+      fb[d] = __shfl_sync(FULL, fb[d], src);
     }
+    if (!q.uniform) imb = __shfl_sync(FULL, imb, src);
+  };
+  if (KIND == PAIR_EWALD_REAL && q.single) {
+#pragma unroll P32_UNROLL
+    for (int s = s0; s <= s1; ++s) step(s, std::true_type{});
   } else {
-    const float ima = va ? im[(size_t)j * g.Ns + a] : 1.f;
-    float imb = vb ? im[(size_t)j * g.Ns + b0] : 1.f;
-    for (int s = 0; s < 32; ++s) {
-      const int bi = J * 32 + ((lane + s) & 31);
-      if (va && bi < g.N && (I != J || a > bi)) {
-        float dx[D], F[D];
+    for (int s = s0; s <= s1; ++s) step(s, std::false_type{});
+  }
+  const int home = (lane - s1 - 1) & 31;  // b's sums are s1 + 1 lanes away
 #pragma unroll
-        for (int d = 0; d < D; ++d) dx[d] = xa[d] - xb[d];
-        pair_eval32<D, KIND>(q, dx, F);
-        // the reference divides by the mass of the higher-index particle
-        const float inv = a > bi ? ima : imb;
-#pragma unroll
-        for (int d = 0; d < D; ++d) {
-          fa[d] = fmaf(F[d], inv, fa[d]);
-          fb[d] = fmaf(-F[d], inv, fb[d]);
-        }
-      }
-#pragma unroll
-      for (int d = 0; d < D; ++d) {
-        xb[d] = __shfl_sync(FULL, xb[d], src);
-        fb[d] = __shfl_sync(FULL, fb[d], src);
-      }
-      imb = __shfl_sync(FULL, imb, src);
-    }
+  for (int d = 0; d < D; ++d) {
+    fb[d] = __shfl_sync(FULL, fb[d], home);
+    if (q.uniform) fa[d] *= q.im0, fb[d] *= q.im0;
   }
   if (I == J) {
     if (va) {

@@ -3622,6 +3622,12 @@ namespace xk {
 // rounding of the FP32 positions); the per-tile partials are added in double
 // by k_pair_finish32.  With one mass for all beads (q.uniform) the inverse
 // mass is applied to the partials instead of to every pair.
+// Bound by instruction issue (200 a step before the last of the changes here,
+// 78% of the slots).  Ewald at N = 512, P = 64, alpha L = 5.6: 83 us with eight
+// candidates a pair and 32 steps on the diagonal, 69 with the minimum image
+// and single shifts only, where no other can lie inside the cut-off, and 16
+// steps, 65 with two steps unrolled, 59 without the subnormal handling of
+// rsqrtf, division and __expf.
 template <int D, int KIND>
 __global__ void __launch_bounds__(256, 3) k_pair_tiles32(Geo g, P32 q, const float *__restrict__ x,
                                                       const float *__restrict__ im,
@@ -3721,6 +3727,15 @@ P32 make_p32(const Geo &g, const PairPrm &p) {
   q.kmax = p.kmax[0] > p.kmax[1] ? (p.kmax[0] > p.kmax[2] ? p.kmax[0] : p.kmax[2])
                                  : (p.kmax[1] > p.kmax[2] ? p.kmax[1] : p.kmax[2]);
   if (p.kind == PAIR_EWALD_REAL && rc32 <= fmin(g.box[0], fmin(g.box[1], g.box[2]))) q.kmax = 0;
+  if (q.kmax == 0 && p.kind == PAIR_EWALD_REAL) {
+    // (1e-5: the FP32 rounding of the separations)
+    double two = 1e300;
+    for (int d = 0; d < 3; ++d) {
+      const double e = g.box[(d + 1) % 3];
+      two = fmin(two, (g.box[d] * g.box[d] + e * e) / 4);
+    }
+    q.single = rc32 * rc32 < two * (1 - 1e-5);
+  }
   q.uniform = p.inv_mass > 0;
   q.im0 = (float)p.inv_mass;
   return q;
