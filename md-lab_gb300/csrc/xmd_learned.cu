@@ -139,6 +139,16 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
                : "memory");
 }
 
+// shared to global memory (both addresses and the size multiples of 16 bytes);
+// bulk_wait_all waits for all of the thread's
+__device__ __forceinline__ void bulk_s2g(void *dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_wait_all() {
+  asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   const uint32_t lo = __bfloat16_as_ushort(__float2bfloat16_rn(a));
   const uint32_t hi = __bfloat16_as_ushort(__float2bfloat16_rn(b));
@@ -377,11 +387,17 @@ constexpr uint32_t W1 = 0, W2 = 16384, W3 = 49152, X = 53248, H1 = 69632, H2 = 1
 constexpr uint32_t WBYTES = 16384 + 32768 + 4096;
 }  // namespace fw
 
-// layer epilogue: h = tanh(acc + bias) of this thread's row, written as BF16
-// into a K = 128 image at dst
-__device__ __forceinline__ void epi_hidden(uint32_t taddr, const float *bias, uint8_t *dst, int row) {
+// Threads of the network kernels: four warpgroups, each of which reaches all 128
+// TMEM lanes (a lane is a row), so that four threads share a row, a quarter of
+// its columns each.  With one warpgroup a scheduler had one warp, and the
+// kernel waited for the latency of every tanh and TMEM read.
+constexpr int MLP_T = 512;
+
+// layer epilogue: h = tanh(acc + bias) of this thread's row and quarter, written
+// as BF16 into a K = 128 image at dst
+__device__ __forceinline__ void epi_hidden(uint32_t taddr, const float *bias, uint8_t *dst, int row, int quarter) {
 #pragma unroll 1
-  for (int c0 = 0; c0 < 128; c0 += 16) {
+  for (int c0 = quarter * 32; c0 < quarter * 32 + 32; c0 += 16) {
     float v[16];
     tc::tmem_ld16(taddr + c0, v);
     uint32_t pk[8];
@@ -413,13 +429,13 @@ __device__ __forceinline__ void issue_layer(uint32_t s0, int layer, uint32_t tm)
   }
 }
 
-__global__ void __launch_bounds__(128, 1) k_mlp_fwd(MlpDev w, const uint8_t *__restrict__ ximg, int ntiles,
+__global__ void __launch_bounds__(MLP_T, 1) k_mlp_fwd(MlpDev w, const uint8_t *__restrict__ ximg, int ntiles,
                                                   float4 *__restrict__ Y, int *err, long long wait) {
   extern __shared__ __align__(1024) uint8_t sm[];
   float *sb1 = (float *)(sm + fw::B), *sb2 = sb1 + 128, *sb3 = sb2 + 128;
   uint64_t *bars = (uint64_t *)(sm + fw::BAR);
   uint32_t *slot = (uint32_t *)(sm + fw::SLOT);
-  const int tid = threadIdx.x, warp = tid >> 5, row = tid;
+  const int tid = threadIdx.x, warp = tid >> 5, row = tid & 127, quarter = tid >> 7;
   const uint32_t s0 = tc::saddr(sm);
   const uint32_t bar_w = tc::saddr(&bars[0]), bar_x = tc::saddr(&bars[1]), bar_m = tc::saddr(&bars[2]);
   if (tid == 0) {
@@ -428,15 +444,17 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(MlpDev w, const uint8_t *__r
     tc::mbar_init(bar_m, 1);
     tc::mbar_fence_init();
   }
-  sb1[tid] = w.b1[tid];
-  sb2[tid] = w.b2[tid];
+  if (tid < 128) {
+    sb1[tid] = w.b1[tid];
+    sb2[tid] = w.b2[tid];
+  }
   if (tid < 4) sb3[tid] = w.b3[tid];
   if (warp == 0) tc::tmem_alloc(tc::saddr(slot), 512);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
   const uint32_t tm = *slot;
-  const uint32_t tl = tm + ((uint32_t)(warp * 32) << 16);  // this warp's TMEM lanes
+  const uint32_t tl = tm + ((uint32_t)((warp & 3) * 32) << 16);  // this warp's TMEM lanes
   if (tid == 0) {
     tc::mbar_expect_tx(bar_w, fw::WBYTES);
     tc::bulk_g2s(s0 + fw::W1, w.w1img, 16384, bar_w);
@@ -463,10 +481,10 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(MlpDev w, const uint8_t *__r
       if (!ok) break;
       tc::fence_after();
       if (layer == 1) {
-        epi_hidden(tl, sb1, sm + fw::H1, row);
+        epi_hidden(tl, sb1, sm + fw::H1, row, quarter);
       } else if (layer == 2) {
-        epi_hidden(tl + 128, sb2, sm + fw::H2, row);
-      } else {
+        epi_hidden(tl + 128, sb2, sm + fw::H2, row, quarter);
+      } else if (quarter == 0) {
         float v[4];
         tc::tmem_ld4(tl + 256, v);
         Y[(size_t)tile * MLP_TILE + row] = make_float4(v[0] + sb3[0], v[1] + sb3[1], v[2] + sb3[2], v[3] + sb3[3]);
@@ -485,8 +503,12 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(MlpDev w, const uint8_t *__r
 
 // ===================================================================
 // MLP training step: forward, loss, backward; weight gradients accumulate in
-// TMEM over all tiles of the CTA and go to global memory once
+// TMEM over all tiles of the CTA and go to global memory once.  A step of 128
+// tiles with the optimiser: 71 us with one warpgroup and scalar atomics, 30 with
+// rows copied out in bulk, 25 with four warpgroups (MLP_T) as well; bound by the
+// chain of five dependent products with their epilogues on one tile a CTA
 // ===================================================================
+static_assert(128 * (528 + 272) <= 167936 - 53248, "the padded gradient rows fit over X .. DZ2");
 // Shared memory: W1 16 K | W2 32 K | W3 4 K | X 16 K | H1 32 K | H2 32 K (later
 // dZ1) | dZ2 32 K | dY 4 K (rows x 16 outputs) | W3 FP32 | biases | bias
 // gradients | loss | mbarriers | TMEM slot.
@@ -497,7 +519,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_fwd(MlpDev w, const uint8_t *__r
 namespace tr {
 constexpr uint32_t W1 = 0, W2 = 16384, W3 = 49152, X = 53248, H1 = 69632, H2 = 102400, DZ2 = 135168,
                    DY = 167936, W3F = 172032, B1 = W3F + 2048, B2 = B1 + 512, B3 = B2 + 512, GB1 = B3 + 16,
-                   GB2 = GB1 + 512, GB3 = GB2 + 512, BAR = GB3 + 32, SLOT = BAR + 24, SMEM = SLOT + 16;
+                   GB2 = GB1 + 2048, GB3 = GB2 + 2048, BAR = GB3 + 128, SLOT = BAR + 24, SMEM = SLOT + 16;
 constexpr uint32_t T_Z1 = 0, T_Z2 = 128, T_Y = 256, T_W3 = 272, T_W1 = 288, T_W2 = 384;
 }  // namespace tr
 
@@ -521,7 +543,7 @@ XK_HD inline int batch_tile(uint32_t seed, int i, int ntiles) {
 }
 
 template <int MNV>
-__global__ void __launch_bounds__(128, 1) k_mlp_train(MlpDev w, const uint8_t *__restrict__ ximg,
+__global__ void __launch_bounds__(MLP_T, 1) k_mlp_train(MlpDev w, const uint8_t *__restrict__ ximg,
                                                     const float *__restrict__ V, const float4 *__restrict__ T,
                                                     int ntiles_data, int batch_tiles, uint32_t seed, MlpLoss loss,
                                                     float *__restrict__ grad, float *__restrict__ lossacc, int *err,
@@ -532,7 +554,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_train(MlpDev w, const uint8_t *_
   float *gb1 = (float *)(sm + tr::GB1), *gb2 = (float *)(sm + tr::GB2), *gb3 = (float *)(sm + tr::GB3);
   uint64_t *bars = (uint64_t *)(sm + tr::BAR);
   uint32_t *slot = (uint32_t *)(sm + tr::SLOT);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row = tid;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row = tid & 127, quarter = tid >> 7;
   const uint32_t s0 = tc::saddr(sm);
   const uint32_t bar_w = tc::saddr(&bars[0]), bar_x = tc::saddr(&bars[1]), bar_m = tc::saddr(&bars[2]);
   if (tid == 0) {
@@ -541,19 +563,21 @@ __global__ void __launch_bounds__(128, 1) k_mlp_train(MlpDev w, const uint8_t *_
     tc::mbar_init(bar_m, 1);
     tc::mbar_fence_init();
   }
-  for (int i = tid; i < 512; i += 128) w3f[i] = w.w3f[i];
-  sb1[tid] = w.b1[tid];
-  sb2[tid] = w.b2[tid];
+  for (int i = tid; i < 512; i += MLP_T) w3f[i] = w.w3f[i];
+  if (tid < 128) {
+    sb1[tid] = w.b1[tid];
+    sb2[tid] = w.b2[tid];
+  }
   gb1[tid] = 0.f;
   gb2[tid] = 0.f;
-  if (tid < 8) gb3[tid] = 0.f;  // db3[0..3], loss terms [4], [5]
+  if (tid < 32) gb3[tid] = 0.f;  // per warp of quarter 0: db3[0..3], loss terms [4], [5]
   if (tid < 4) sb3[tid] = w.b3[tid];
   if (warp == 0) tc::tmem_alloc(tc::saddr(slot), 512);
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
   const uint32_t tm = *slot;
-  const uint32_t tl = tm + ((uint32_t)(warp * 32) << 16);
+  const uint32_t tl = tm + ((uint32_t)((warp & 3) * 32) << 16);
   if (tid == 0) {
     tc::mbar_expect_tx(bar_w, fw::WBYTES);
     tc::bulk_g2s(s0 + tr::W1, w.w1img, 16384, bar_w);
@@ -599,7 +623,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_train(MlpDev w, const uint8_t *_
     }
     mma_wait();
     if (!ok) break;
-    epi_hidden(tl + tr::T_Z1, sb1, sm + tr::H1, row);
+    epi_hidden(tl + tr::T_Z1, sb1, sm + tr::H1, row, quarter);
     to_tensor();
     if (tid == 0) {
       tc::fence_after();
@@ -611,7 +635,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_train(MlpDev w, const uint8_t *_
     }
     mma_wait();
     if (!ok) break;
-    epi_hidden(tl + tr::T_Z2, sb2, sm + tr::H2, row);
+    epi_hidden(tl + tr::T_Z2, sb2, sm + tr::H2, row, quarter);
     to_tensor();
     if (tid == 0) {
       tc::fence_after();
@@ -641,24 +665,25 @@ __global__ void __launch_bounds__(128, 1) k_mlp_train(MlpDev w, const uint8_t *_
 #pragma unroll
     for (int m = 0; m < 3; ++m)
       dy[1 + m] = 2.f * loss.wf * (dF[0] * v[3 * m] + dF[1] * v[3 * m + 1] + dF[2] * v[3 * m + 2]) * wr * loss.inv_rows;
-    {
+    if (quarter == 0) {
       const float s0e = tc::warp_sumf(Le), s0f = tc::warp_sumf(Lf);
       float s[4];
 #pragma unroll
       for (int o = 0; o < 4; ++o) s[o] = tc::warp_sumf(dy[o]);
       if (lane == 0) {
-        atomicAdd(&gb3[4], s0e);
-        atomicAdd(&gb3[5], s0f);
+        float *b = gb3 + warp * 8;
+        b[4] += s0e;
+        b[5] += s0f;
 #pragma unroll
-        for (int o = 0; o < 4; ++o) atomicAdd(&gb3[o], s[o]);
+        for (int o = 0; o < 4; ++o) b[o] += s[o];
       }
+      *(uint4 *)(sm + tr::DY + kmaj_off(row, 0, 16)) =
+          make_uint4(tc::pack_bf16(dy[0], dy[1]), tc::pack_bf16(dy[2], dy[3]), 0u, 0u);
+      *(uint4 *)(sm + tr::DY + kmaj_off(row, 8, 16)) = make_uint4(0u, 0u, 0u, 0u);
     }
-    *(uint4 *)(sm + tr::DY + kmaj_off(row, 0, 16)) =
-        make_uint4(tc::pack_bf16(dy[0], dy[1]), tc::pack_bf16(dy[2], dy[3]), 0u, 0u);
-    *(uint4 *)(sm + tr::DY + kmaj_off(row, 8, 16)) = make_uint4(0u, 0u, 0u, 0u);
-    // dZ2 = (dY W3) * (1 - h2^2), in groups of 32 columns for the bias sums
-#pragma unroll 1
-    for (int g0 = 0; g0 < 128; g0 += 32) {
+    // dZ2 = (dY W3) * (1 - h2^2), a warp's 32 rows and columns for the bias sums
+    const int g0 = quarter * 32;
+    {
       float dz[32];
 #pragma unroll
       for (int c8 = 0; c8 < 32; c8 += 8) {
@@ -682,7 +707,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_train(MlpDev w, const uint8_t *_
         *(uint4 *)(sm + tr::DZ2 + kmaj_off(row, g0 + c8, 128)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
       }
       const float s = tc::transpose_sum(dz);
-      atomicAdd(&gb2[g0 + lane], s);
+      gb2[(warp & 3) * 128 + g0 + lane] += s;
     }
     to_tensor();
     // ---- backward MMAs: dW3^T += H2^T dY, dH1 = dZ2 W2, dW2 += dZ2^T H1 ----
@@ -703,8 +728,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_train(MlpDev w, const uint8_t *_
     mma_wait();
     if (!ok) break;
     // dZ1 = dH1 * (1 - h1^2) into the H2 region
-#pragma unroll 1
-    for (int g0 = 0; g0 < 128; g0 += 32) {
+    {
       float dz[32];
 #pragma unroll
       for (int c16 = 0; c16 < 32; c16 += 16) {
@@ -728,7 +752,7 @@ __global__ void __launch_bounds__(128, 1) k_mlp_train(MlpDev w, const uint8_t *_
         }
       }
       const float s = tc::transpose_sum(dz);
-      atomicAdd(&gb1[g0 + lane], s);
+      gb1[(warp & 3) * 128 + g0 + lane] += s;
     }
     to_tensor();
     // dW1 += dZ1^T X
@@ -748,34 +772,49 @@ __global__ void __launch_bounds__(128, 1) k_mlp_train(MlpDev w, const uint8_t *_
   }
   if (!ok) tc_fail(err, 3);
   if (ok && done > 0) {
-    // weight gradients out of TMEM: lane = output row o (dW1, dW2) or hidden
-    // unit c (dW3^T)
+    // The CTA's gradients, added up by the optimiser in the CTAs' order, so that
+    // the same data train to the same bits.
+    // Weight gradients out of TMEM, lane = output row o (dW1, dW2) or hidden
+    // unit c (dW3^T), over the activations' shared memory into rows padded by 16
+    // bytes (lanes then write different banks), each row by one bulk copy.
+    // Scalar atomics of 128 CTAs on one copy, each lane at its own row, took two
+    // thirds of the kernel's time.
+    float *part = grad + (size_t)blockIdx.x * MLP_NPARAM;
     const int o = row;
-#pragma unroll 1
-    for (int c0 = 0; c0 < 128; c0 += 16) {
-      float g[16];
-      tc::tmem_ld16(tl + tr::T_W2 + c0, g);
+    uint8_t *r2 = sm + tr::X + o * 528, *r1 = sm + tr::X + 128 * 528 + o * 272;
 #pragma unroll
-      for (int i = 0; i < 16; ++i) atomicAdd(&grad[MLP_W2 + o * 128 + c0 + i], g[i]);
-    }
-#pragma unroll 1
-    for (int c0 = 0; c0 < 64; c0 += 16) {
+    for (int k = 0; k < 3; ++k) {  // 32 columns of dW2, 16 of dW1
+      const int c0 = k < 2 ? quarter * 32 + k * 16 : quarter * 16;
       float g[16];
-      tc::tmem_ld16(tl + tr::T_W1 + c0, g);
+      tc::tmem_ld16(tl + (k < 2 ? tr::T_W2 : tr::T_W1) + c0, g);
+      float4 *d = (float4 *)((k < 2 ? r2 : r1) + c0 * 4);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) atomicAdd(&grad[MLP_W1 + o * 64 + c0 + i], g[i]);
+      for (int i = 0; i < 4; ++i) d[i] = make_float4(g[4 * i], g[4 * i + 1], g[4 * i + 2], g[4 * i + 3]);
     }
-    {
+    if (quarter == 0) {
       float g[4];
       tc::tmem_ld4(tl + tr::T_W3, g);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) atomicAdd(&grad[MLP_W3 + i * 128 + o], g[i]);
+      for (int i = 0; i < 4; ++i) w3f[i * 128 + o] = g[i];
     }
+    // the warps' bias sums, into the first warp's
+    if (tid < 256) {
+      float *gb = tid < 128 ? gb1 + tid : gb2 + tid - 128;
+      gb[0] = (gb[0] + gb[128]) + (gb[256] + gb[384]);
+    } else if (tid < 262) {
+      float *gb = gb3 + tid - 256;
+      gb[0] = (gb[0] + gb[8]) + (gb[16] + gb[24]);
+    }
+    tc::fence_async_smem();
     __syncthreads();
-    atomicAdd(&grad[MLP_B1 + tid], gb1[tid]);
-    atomicAdd(&grad[MLP_B2 + tid], gb2[tid]);
-    if (tid < 4) atomicAdd(&grad[MLP_B3 + tid], gb3[tid]);
+    if (quarter == 0) tc::bulk_s2g(part + MLP_W2 + o * 128, tc::saddr(r2), 512);
+    if (quarter == 1) tc::bulk_s2g(part + MLP_W1 + o * 64, tc::saddr(r1), 256);
+    if (tid < 4) tc::bulk_s2g(part + MLP_W3 + tid * 128, s0 + tr::W3F + tid * 512, 512);
+    if (tid == 4) tc::bulk_s2g(part + MLP_B1, s0 + tr::GB1, 512);
+    if (tid == 5) tc::bulk_s2g(part + MLP_B2, s0 + tr::GB2, 512);
+    if (tid == 6) tc::bulk_s2g(part + MLP_B3, s0 + tr::GB3, 16);
     if (tid < 2) atomicAdd(&lossacc[tid], gb3[4 + tid]);
+    tc::bulk_wait_all();
   }
   tc::fence_before();
   __syncthreads();
@@ -802,19 +841,53 @@ __device__ __forceinline__ void pack_param(int i, float p, uint8_t *w1img, uint8
   }
 }
 
-__global__ void k_mlp_adam(float *__restrict__ p, float *__restrict__ g, float *__restrict__ m1,
-                           float *__restrict__ m2, AdamPrm a, uint8_t *w1img, uint8_t *w2img, uint8_t *w3img,
-                           float *w3f) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= MLP_NPARAM) return;
-  const float gi = g[i];
+// Parameter 128 blockIdx.x + t of this block's threads t < 128: the sum of the
+// CTAs' parts, in a fixed order.  The parts of 128 CTAs are 13 MB: a thread sums
+// every eighth part of four parameters, so that all are in flight at once
+// (eight loads in flight a thread and parameter: 6 us a step more).
+static_assert(MLP_NPARAM % 4 == 0, "parts are read 16 bytes at a time");
+constexpr int AD_T = 256;
+__device__ __forceinline__ float part_sum(const float *__restrict__ part, int n) {
+  __shared__ float4 sh[AD_T / 32][32];
+  const int t = threadIdx.x, tx = t & 31, ty = t >> 5, q = blockIdx.x * 32 + tx;
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (q < MLP_NPARAM / 4) {
+#pragma unroll 8
+    for (int c = ty; c < n; c += AD_T / 32) {
+      const float4 v = ((const float4 *)part)[(size_t)c * (MLP_NPARAM / 4) + q];
+      s.x += v.x, s.y += v.y, s.z += v.z, s.w += v.w;
+    }
+  }
+  sh[ty][tx] = s;
+  __syncthreads();
+  float r = 0.f;
+  if (t < 128) {
+#pragma unroll
+    for (int k = 0; k < AD_T / 32; ++k) r += ((const float *)sh[k])[t];
+  }
+  return r;
+}
+
+__global__ void __launch_bounds__(AD_T) k_mlp_adam(float *__restrict__ p, const float *__restrict__ part, int nparts,
+                                                   float *__restrict__ m1, float *__restrict__ m2, AdamPrm a,
+                                                   uint8_t *w1img, uint8_t *w2img, uint8_t *w3img, float *w3f) {
+  const float gi = part_sum(part, nparts);
+  const int i = blockIdx.x * 128 + threadIdx.x;
+  if (threadIdx.x >= 128 || i >= MLP_NPARAM) return;
   const float m = a.b1 * m1[i] + (1.f - a.b1) * gi, v = a.b2 * m2[i] + (1.f - a.b2) * gi * gi;
   m1[i] = m;
   m2[i] = v;
   const float pi = p[i] - a.lr * (m * a.c1) / (sqrtf(v * a.c2) + a.eps);
   p[i] = pi;
-  g[i] = 0.f;
   pack_param(i, pi, w1img, w2img, w3img, w3f);
+}
+
+// the summed gradients
+__global__ void __launch_bounds__(AD_T) k_mlp_grad_sum(const float *__restrict__ part, int nparts,
+                                                       float *__restrict__ grad) {
+  const float gi = part_sum(part, nparts);
+  const int i = blockIdx.x * 128 + threadIdx.x;
+  if (threadIdx.x < 128 && i < MLP_NPARAM) grad[i] = gi;
 }
 
 __global__ void k_mlp_pack(const float *__restrict__ p, uint8_t *w1img, uint8_t *w2img, uint8_t *w3img, float *w3f) {
@@ -822,12 +895,17 @@ __global__ void k_mlp_pack(const float *__restrict__ p, uint8_t *w1img, uint8_t 
   if (i < MLP_NPARAM) pack_param(i, p[i], w1img, w2img, w3img, w3f);
 }
 
-cudaError_t mlp_adam(float *param, float *grad, float *m1, float *m2, AdamPrm a, uint8_t *w1img, uint8_t *w2img,
-                     uint8_t *w3img, float *w3f, cudaStream_t st) {
+cudaError_t mlp_adam(float *param, const float *part, int nparts, float *m1, float *m2, AdamPrm a, uint8_t *w1img,
+                     uint8_t *w2img, uint8_t *w3img, float *w3f, cudaStream_t st) {
   {
     XK_PROF("mlp_adam");
-    k_mlp_adam<<<(MLP_NPARAM + 255) / 256, 256, 0, st>>>(param, grad, m1, m2, a, w1img, w2img, w3img, w3f);
+    k_mlp_adam<<<(MLP_NPARAM + 127) / 128, AD_T, 0, st>>>(param, part, nparts, m1, m2, a, w1img, w2img, w3img, w3f);
   }
+  return XK_LAUNCHED();
+}
+
+cudaError_t mlp_grad_sum(const float *part, int nparts, float *grad, cudaStream_t st) {
+  k_mlp_grad_sum<<<(MLP_NPARAM + 127) / 128, AD_T, 0, st>>>(part, nparts, grad);
   return XK_LAUNCHED();
 }
 
@@ -862,10 +940,12 @@ cudaError_t mlp_forward(const MlpDev &w, const uint8_t *ximg, int ntiles, float4
   const int grid = ntiles < sm_count() ? ntiles : sm_count();
   {
     XK_PROF("mlp_forward");
-    k_mlp_fwd<<<grid, 128, fw::SMEM, st>>>(w, ximg, ntiles, Y, err, wait_limit());
+    k_mlp_fwd<<<grid, MLP_T, fw::SMEM, st>>>(w, ximg, ntiles, Y, err, wait_limit());
   }
   return XK_LAUNCHED();
 }
+
+int mlp_train_parts(int batch_tiles) { return batch_tiles < sm_count() ? batch_tiles : sm_count(); }
 
 cudaError_t mlp_train_grad(const MlpDev &w, const uint8_t *ximg, const float *V, const float4 *T, int ntiles_data,
                            int batch_tiles, uint32_t seed, MlpLoss loss, float *grad, float *lossacc, int mn_variant,
@@ -879,10 +959,10 @@ cudaError_t mlp_train_grad(const MlpDev &w, const uint8_t *ximg, const float *V,
     if (e != cudaSuccess) return e;
     opted = true;
   }
-  const int grid = batch_tiles < sm_count() ? batch_tiles : sm_count();
+  const int grid = mlp_train_parts(batch_tiles);
   {
     XK_PROF("mlp_train");
-    kf<<<grid, 128, tr::SMEM, st>>>(w, ximg, V, T, ntiles_data, batch_tiles, seed, loss, grad, lossacc, err,
+    kf<<<grid, MLP_T, tr::SMEM, st>>>(w, ximg, V, T, ntiles_data, batch_tiles, seed, loss, grad, lossacc, err,
                                     wait_limit());
   }
   return XK_LAUNCHED();
@@ -967,7 +1047,9 @@ __global__ void __launch_bounds__(SH_T) k_sk_shells(Geo g, DescPrm p, const doub
       sr += part[q][kl].x;
       si += part[q][kl].y;
     }
-    atomicAdd(&p.shell[j * DESC_SHELLS + kv.w], (sr * sr + si * si) * p.shell_norm[kv.w]);
+    // fixed point: the sum does not depend on the order of its blocks
+    atomicAdd(&p.shell[j * DESC_SHELLS + kv.w],
+              (unsigned long long)__float2ull_rn((sr * sr + si * si) * p.shell_norm[kv.w] * SHELL_ONE));
   }
 }
 
@@ -1106,7 +1188,10 @@ __global__ void __launch_bounds__(DS_T, 2) k_desc(Geo g, DescPrm p, const double
   }
   const int lr = l0 + rr;
   if (lr >= g.N) return;
-  const float4 sh = *(const float4 *)(p.shell + j * DESC_SHELLS + f0);
+  const ulonglong2 sh01 = *(const ulonglong2 *)(p.shell + j * DESC_SHELLS + f0),
+                   sh23 = *(const ulonglong2 *)(p.shell + j * DESC_SHELLS + f0 + 2);
+  const float4 sh = make_float4(__ull2float_rn(sh01.x) * (1.f / SHELL_ONE), __ull2float_rn(sh01.y) * (1.f / SHELL_ONE),
+                                __ull2float_rn(sh23.x) * (1.f / SHELL_ONE), __ull2float_rn(sh23.y) * (1.f / SHELL_ONE));
   const float sv[4] = {sqrtf(sh.x), sqrtf(sh.y), sqrtf(sh.z), sqrtf(sh.w)};
   const size_t grow = (size_t)j * g.N + lr;
   if (RAW) {
@@ -1160,7 +1245,7 @@ cudaError_t desc_build(const Geo &g, const DescPrm &p, const double *x, uint8_t 
     }
     opted[2] = smem_sh;
   }
-  cudaError_t e = cudaMemsetAsync(p.shell, 0, sizeof(float) * DESC_SHELLS * g.P, st);
+  cudaError_t e = cudaMemsetAsync(p.shell, 0, sizeof(*p.shell) * DESC_SHELLS * g.P, st);
   if (e != cudaSuccess) return e;
   {
     XK_PROF("desc_shells");

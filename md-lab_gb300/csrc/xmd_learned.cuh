@@ -45,6 +45,7 @@ struct MlpDev {
   const float *w3f;      // [4][128] the BF16 values of W3 as FP32
 };
 
+constexpr float SHELL_ONE = 1099511627776.f;  // 2^40: fixed point, up to 2^24 particles
 // descriptor constants (host-computed from the box)
 struct DescPrm {
   float rc, inv_h;             // cut-off radius (half the smallest box length), bins per unit
@@ -59,7 +60,7 @@ struct DescPrm {
   const int4 *kvec;            // half-space wave vectors of the lowest shells: (nx >= 0, ny, nz, shell)
   int nkvec, nmax;             // their count and largest |n_i|
   const float *shell_norm;     // [DESC_SHELLS] 1 / (N x half-space vectors of the shell)
-  float *shell;                // [P][DESC_SHELLS] scratch: each slice's shell features (squared)
+  unsigned long long *shell;   // [P][DESC_SHELLS] scratch: each slice's shell features (squared), times SHELL_ONE
   const float *fmean, *fistd;  // feature normalisation
 };
 
@@ -78,22 +79,25 @@ struct MlpLoss {
   float we, wf;      // weights of the energy and force terms
   float inv_rows;    // 1 / rows in the batch
 };
-// one training step's gradients: grad (MLP_NPARAM floats, accumulated with
-// atomics, zeroed by the caller) and loss[2] (energy, force terms).  tiles:
+// one training step's gradients: mlp_train_parts(batch_tiles) parts of
+// MLP_NPARAM floats each, one a CTA, which mlp_adam or mlp_grad_sum adds up in a
+// fixed order, and loss[2] (energy, force terms, accumulated).  tiles:
 // batch tiles drawn from [0, ntiles_data) by a hash of (seed, index); seed 0
 // takes tiles 0 .. batch_tiles-1 in order (batch_tiles <= ntiles_data).
 // mn_variant: descriptor reading of MN-major operands; only 0 (the one
 // tc_selftest confirms) is accepted.
+int mlp_train_parts(int batch_tiles);
 cudaError_t mlp_train_grad(const MlpDev &w, const uint8_t *ximg, const float *V, const float4 *T,
                            int ntiles_data, int batch_tiles, uint32_t seed, MlpLoss loss, float *grad,
                            float *lossacc, int mn_variant, int *err, cudaStream_t st);
 
-// Adam on the FP32 master parameters, then repack the images; zeroes grad
+// Adam on the FP32 master parameters, then repack the images
 struct AdamPrm {
   float lr, b1, b2, eps, c1, c2;  // c1 = 1/(1-b1^t), c2 = 1/(1-b2^t)
 };
-cudaError_t mlp_adam(float *param, float *grad, float *m1, float *m2, AdamPrm a, uint8_t *w1img,
+cudaError_t mlp_adam(float *param, const float *part, int nparts, float *m1, float *m2, AdamPrm a, uint8_t *w1img,
                      uint8_t *w2img, uint8_t *w3img, float *w3f, cudaStream_t st);
+cudaError_t mlp_grad_sum(const float *part, int nparts, float *grad, cudaStream_t st);
 // images from the master parameters without an update
 cudaError_t mlp_pack(const float *param, uint8_t *w1img, uint8_t *w2img, uint8_t *w3img, float *w3f,
                      cudaStream_t st);

@@ -445,7 +445,7 @@ int md_gb300_ewald_model_create_x(md_gb300_ewald_model_t_x **out, md_pimd_t_x *p
     if (!rc && cudaMemsetAsync(b.p, 0, bytes, stream()) != cudaSuccess) rc = fail(MD_GB_ERR_CUDA, "memset");
   };
   res(M->par, 4 * xk::MLP_NPARAM);
-  res(M->grad, 4 * xk::MLP_NPARAM);
+  res(M->grad, 4 * (size_t)xk::MLP_NPARAM * (1 + xk::mlp_train_parts(1 << 30)));  // the CTAs' parts, their sum
   res(M->m1, 4 * xk::MLP_NPARAM);
   res(M->m2, 4 * xk::MLP_NPARAM);
   res(M->w1, 16384);
@@ -460,7 +460,7 @@ int md_gb300_ewald_model_create_x(md_gb300_ewald_model_t_x **out, md_pimd_t_x *p
   shell_vectors(kvh, kcount, kmax);
   res(M->dkv, sizeof(int) * kvh.size());
   res(M->dsn, 4 * xk::DESC_SHELLS);
-  res(M->dsh, 4 * (size_t)xk::DESC_SHELLS * g.P);
+  res(M->dsh, 8 * (size_t)xk::DESC_SHELLS * g.P);
   res(M->fmean, 4 * 64);
   res(M->fistd, 4 * 64);
   res(M->dsx, (size_t)capacity_cfg * (rows / xk::MLP_TILE) * tile_bytes);
@@ -507,7 +507,7 @@ int md_gb300_ewald_model_create_x(md_gb300_ewald_model_t_x **out, md_pimd_t_x *p
   M->dp.nkvec = (int)(kvh.size() / 4);
   M->dp.nmax = kmax;
   M->dp.shell_norm = M->dsn.as<float>();
-  M->dp.shell = M->dsh.as<float>();
+  M->dp.shell = M->dsh.as<unsigned long long>();
   M->dp.rc = (float)rcut;
   M->dp.inv_h = (float)(xk::DESC_BINS / rcut);
   for (int d = 0; d < 3; ++d) {
@@ -596,7 +596,7 @@ int md_gb300_ewald_model_train_x(md_gb300_ewald_model_t_x *M, int steps, int bat
                                 M->err.as<int>(), st));
     xk::AdamPrm a{(float)lr, 0.9f, 0.999f, 1e-8f, (float)(1.0 / (1.0 - pow(0.9, M->adam_t))),
                   (float)(1.0 / (1.0 - pow(0.999, M->adam_t)))};
-    XMD_CUDA(xk::mlp_adam(M->par.as<float>(), M->grad.as<float>(), M->m1.as<float>(), M->m2.as<float>(), a,
+    XMD_CUDA(xk::mlp_adam(M->par.as<float>(), M->grad.as<float>(), xk::mlp_train_parts(batch_tiles), M->m1.as<float>(), M->m2.as<float>(), a,
                           M->w1.as<uint8_t>(), M->w2.as<uint8_t>(), M->w3.as<uint8_t>(), M->w3f.as<float>(), st));
   }
   float la[2] = {0, 0};
@@ -722,6 +722,7 @@ int md_gb300_mlp_grad_x(md_gb300_ewald_model_t_x *M, const float *X, const float
   cudaError_t e = cudaSuccess;
   if (!rc) {
     xk::MlpLoss L{(float)we, (float)wf, (float)(1.0 / rows)};
+    float *sum = M->grad.as<float>() + (size_t)xk::MLP_NPARAM * xk::mlp_train_parts(1 << 30);
     int kerr = 0;
     if ((e = cudaMemsetAsync(dv.p, 0, rp * xk::DESC_VSTRIDE * 4, st)) == cudaSuccess &&
         (e = cudaMemsetAsync(dt.p, 0, rp * 16, st)) == cudaSuccess &&
@@ -729,15 +730,14 @@ int md_gb300_mlp_grad_x(md_gb300_ewald_model_t_x *M, const float *X, const float
         (e = cudaMemcpyAsync(dv.p, V, (size_t)rows * xk::DESC_VSTRIDE * 4, cudaMemcpyHostToDevice, st)) ==
             cudaSuccess &&
         (e = cudaMemcpyAsync(dt.p, T, (size_t)rows * 16, cudaMemcpyHostToDevice, st)) == cudaSuccess &&
-        (e = cudaMemsetAsync(M->grad.p, 0, 4 * xk::MLP_NPARAM, st)) == cudaSuccess &&
         (e = cudaMemsetAsync(M->lossacc.p, 0, 8, st)) == cudaSuccess &&
         (e = xk::mlp_train_grad(dev_view(M), dx.as<uint8_t>(), dv.as<float>(), dt.as<float4>(), nt, nt, 0u, L,
                                 M->grad.as<float>(), M->lossacc.as<float>(), mnv, M->err.as<int>(), st)) ==
             cudaSuccess &&
-        (e = cudaMemcpyAsync(grad, M->grad.p, 4 * xk::MLP_NPARAM, cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
+        (e = xk::mlp_grad_sum(M->grad.as<float>(), xk::mlp_train_parts(nt), sum, st)) == cudaSuccess &&
+        (e = cudaMemcpyAsync(grad, sum, 4 * xk::MLP_NPARAM, cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
         (!loss || (e = cudaMemcpyAsync(loss, M->lossacc.p, 8, cudaMemcpyDeviceToHost, st)) == cudaSuccess) &&
-        (e = cudaMemcpyAsync(&kerr, M->err.p, sizeof(int), cudaMemcpyDeviceToHost, st)) == cudaSuccess &&
-        (e = cudaMemsetAsync(M->grad.p, 0, 4 * xk::MLP_NPARAM, st)) == cudaSuccess)
+        (e = cudaMemcpyAsync(&kerr, M->err.p, sizeof(int), cudaMemcpyDeviceToHost, st)) == cudaSuccess)
       e = cudaStreamSynchronize(st);
     if (e != cudaSuccess)
       rc = cuda_fail(e, "network gradient");
