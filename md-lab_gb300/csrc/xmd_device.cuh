@@ -1575,17 +1575,29 @@ __device__ inline RecipCol recip_col32(int4 c, int ns) {
   return {col_nx(c) * 32, (ns + 1 + abs(c.y)) * 32, col_nz(c), 0, (float)col_nx(c), (float)c.y, c.y < 0 ? -1.f : 1.f, 0.f};
 }
 
+// the FP32 pair tiles' partial sums of slot s, in double
+__device__ inline double pair_sum32(const Geo &g, const float *__restrict__ part, int T, size_t s) {
+  const size_t S = g.slots();
+  double acc = 0;
+#pragma unroll 4
+  for (int t = 0; t < T; ++t) acc += (double)part[(size_t)t * S + s];
+  return acc;
+}
+
 // Reciprocal forces on 32 particles of slice j, one a lane, by a block of SK_W warps: warp w sums columns w, w + SK_W, ..., so that
 // the lanes read each table entry at one address; Kahan sums, the warps' added
 // in double-float.  sc, sT: columns (recip_col32) and force tables; pxy: [2][ns+1][32]
 // float2, red: [SK_W][3][32] float2, of these warps alone (red may lie over
-// sT).  NSM: the largest ns.  Bound by FP32 issue, eight multiply-adds a
+// sT).  The real space's tile sums (part, T tiles, pscale) are added here too:
+// their loads pass beside other blocks' sums, and the reciprocal forces' own
+// trip to f serves both.  NSM: the largest ns.  Bound by FP32 issue, eight multiply-adds a
 // harmonic: 36 us at N = 512, P = 64, |n| <= 10, 57 with two threads a particle,
 // each on half the columns with its own reads of the tables.
 template <int NSM>
 __device__ inline void recip_tile32(const Geo &g, int ns, int ncol, const RecipCol *sc, const float4 *sT, float2 *pxy,
                                     float2 *red, const float2 *__restrict__ ph1, double scale, double *__restrict__ f,
-                                    int j, int l0, int w, int lane) {
+                                    int j, int l0, int w, int lane, const float *__restrict__ part, int T,
+                                    double pscale) {
   const int l = min(l0 + lane, g.N - 1);  // lanes past the end repeat the last particle
   const float2 *p1 = ph1 + (size_t)j * 3 * g.Ns + l;
   if (w < 2) {
@@ -1639,7 +1651,8 @@ __device__ inline void recip_tile32(const Geo &g, int ns, int ncol, const RecipC
       s.add(p.y);
     }
     const double ib = w == 0 ? g.inv_box[0] : (w == 1 ? g.inv_box[1] : g.inv_box[2]);
-    f[sidx(j, w, l, 3, g.Ns)] += scale * s.value() * ib;
+    const size_t o = sidx(j, w, l, 3, g.Ns);
+    f[o] = (f[o] + scale * s.value() * ib) + pair_sum32(g, part, T, o) * pscale;
   }
 }
 

@@ -117,7 +117,8 @@ __device__ inline void ens_recip_slice(const EnsSys &E, int j, unsigned char *sh
   for (int q = tid; q < ncol; q += ENS_T) sc[q] = recip_col32(E.cols[q], ns);
   for (int l0 = 0; l0 < g.N; l0 += 32) {
     if (l0 > 0) __syncthreads();
-    recip_tile32<ENS_NSMAX>(g, ns, ncol, sc, sT, pxy, red, E.ph1, E.rscale, E.d.f, j, l0, tid >> 5, tid & 31);
+    recip_tile32<ENS_NSMAX>(g, ns, ncol, sc, sT, pxy, red, E.ph1, E.rscale, E.d.f, j, l0, tid >> 5, tid & 31,
+                            E.part, E.T, E.pscale);
   }
 }
 
@@ -347,15 +348,12 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
   {
     for (int i = i0; i < i1; ++i) {
       const EnsSys &E = sys[i];
-      if (!E.d.pair_kind) continue;
+      if (!E.d.pair_kind || E.ewald) continue;  // (Ewald's: with the reciprocal forces)
       const Geo g = E.d.g;
       const long long n = (long long)g.slots();
       for (long long q = ens_first(gt, sys[i].rot[R_E_PS], GT); q < n; q += GT) {
         const size_t s = (size_t)q;
-        if ((int)(s % g.Ns) >= g.N) continue;
-        double acc = 0;
-        for (int t = 0; t < E.T; ++t) acc += (double)E.part[(size_t)t * n + s];
-        E.d.f[s] += acc * E.pscale;
+        if ((int)(s % g.Ns) < g.N) E.d.f[s] += pair_sum32(g, E.part, E.T, s) * E.pscale;
       }
     }
   }
@@ -603,7 +601,7 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
         cnt[R_C_REC] = E.ewald ? P : 0;
         cnt[R_D_ENK] = N * (N - 1) / 2;
         cnt[R_E_W] = N;
-        cnt[R_E_PS] = E.d.pair_kind ? slots : 0;
+        cnt[R_E_PS] = E.d.pair_kind && !E.ewald ? slots : 0;
         cnt[R_E_INV] = 2 * ((N + TS_CHUNK - 1) / TS_CHUNK);
         cnt[R_F] = 2;
         cnt[R_G] = exch_jobs(g.N);

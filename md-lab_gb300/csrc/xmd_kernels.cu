@@ -3644,11 +3644,13 @@ __global__ void __launch_bounds__(256, 3) k_pair_tiles32(Geo g, P32 q, const flo
 // FP32 copies of the positions and inverse masses for the FP32 pair kernel
 // FP32 positions and (im32 non-null: beads of different masses) inverse
 // masses; with one mass for all beads the tiles apply it to their sums and
-// no division is taken here
+// no division is taken here; ph1 (non-null, D = 3): first phase factors,
+// ph1[(j*3 + d)*Ns + l]
 __global__ void k_to32(Geo g, const double *__restrict__ x, const double *__restrict__ m, float *__restrict__ x32,
-                       float *__restrict__ im32) {
+                       float *__restrict__ im32, float2 *__restrict__ ph1) {
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t < g.slots()) x32[t] = (float)x[t];
+  if (ph1 && t < g.slots()) ph1[t] = phase32_slot(g, x, t);
   if (im32 && t < (size_t)g.P * g.Ns) im32[t] = (float)(1.0 / m[t]);
 }
 
@@ -3656,11 +3658,8 @@ __global__ void k_to32(Geo g, const double *__restrict__ x, const double *__rest
 __global__ void k_pair_finish32(Geo g, const float *__restrict__ part, int T, double scale,
                                 double *__restrict__ f) {
   const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const size_t S = g.slots();
-  if (s >= S || (int)(s % g.Ns) >= g.N) return;
-  double acc = 0;
-  for (int t = 0; t < T; ++t) acc += (double)part[(size_t)t * S + s];
-  f[s] += acc * scale;
+  if (s >= g.slots() || (int)(s % g.Ns) >= g.N) return;
+  f[s] += pair_sum32(g, part, T, s) * scale;
 }
 
 // Tile shape of the FP32 pair kernel: warps (32 x 32 pair tiles) per block,
@@ -3741,66 +3740,67 @@ P32 make_p32(const Geo &g, const PairPrm &p) {
   return q;
 }
 
-cudaError_t pair_force32(const Geo &g, const PairPrm &p, const double *x, const double *m, double *f,
-                         double *scratch, cudaStream_t st) {
+// scratch of the FP32 pair forces: T * slots float partials (room for twice
+// that is reserved), then the FP32 positions and inverse masses
+struct P32Bufs {
+  int T;
+  float *part, *x32, *im32;
+};
+static P32Bufs p32_bufs(const Geo &g, double *scratch) {
   const int T = (g.N + 31) / 32;
-  const int jobs = T * (T + 1) / 2;
+  float *x32 = (float *)(scratch + (size_t)T * g.slots());
+  return {T, (float *)scratch, x32, x32 + g.slots()};
+}
+static cudaError_t pair_tiles32(const Geo &g, const PairPrm &p, const P32 &q, const P32Bufs &b, cudaStream_t st) {
+  const int jobs = b.T * (b.T + 1) / 2;
   int wpb = pair32_warps(p.kind, g.D, g.N, g.P);
   if (wpb != 1 && wpb != 2 && wpb != 4 && wpb != 8) wpb = 8;
-  const P32 q = make_p32(g, p);
-  // scratch: T * slots float partials (room for twice that is reserved),
-  // then the FP32 positions and inverse masses
-  float *part = (float *)scratch;
-  float *x32 = (float *)(scratch + (size_t)T * g.slots());
-  float *im32 = x32 + g.slots();
-  {
-    XK_PROF("to32");
-    k_to32<<<cdiv(g.slots(), 256), 256, 0, st>>>(g, x, m, x32, q.uniform ? nullptr : im32);
-  }
-  cudaError_t le = XK_LAUNCHED();
-  if (le != cudaSuccess) return le;
-  {
-    XK_PROF(p.kind == PAIR_EWALD_REAL ? "pair_tiles32_ewald_real" : "pair_tiles32");
-    switch (g.D * 16 + p.kind) {
+  cudaError_t le = cudaSuccess;
+  XK_PROF(p.kind == PAIR_EWALD_REAL ? "pair_tiles32_ewald_real" : "pair_tiles32");
+  switch (g.D * 16 + p.kind) {
 #define XK_P32_CASE(DV, K) \
   case DV * 16 + K:        \
-    le = launch_pair32<DV, K>(g, q, x32, im32, part, T, jobs, wpb, st); \
+    le = launch_pair32<DV, K>(g, q, b.x32, b.im32, b.part, b.T, jobs, wpb, st); \
     break;
-      XK_P32_CASE(1, PAIR_GAUSSIAN)
-      XK_P32_CASE(1, PAIR_PERIODIC_GAUSSIAN)
-      XK_P32_CASE(1, PAIR_COULOMB)
-      XK_P32_CASE(1, PAIR_PERIODIC_COULOMB)
-      XK_P32_CASE(2, PAIR_GAUSSIAN)
-      XK_P32_CASE(2, PAIR_PERIODIC_GAUSSIAN)
-      XK_P32_CASE(2, PAIR_COULOMB)
-      XK_P32_CASE(2, PAIR_PERIODIC_COULOMB)
-      XK_P32_CASE(3, PAIR_GAUSSIAN)
-      XK_P32_CASE(3, PAIR_PERIODIC_GAUSSIAN)
-      XK_P32_CASE(3, PAIR_COULOMB)
-      XK_P32_CASE(3, PAIR_PERIODIC_COULOMB)
-      XK_P32_CASE(3, PAIR_EWALD_REAL)
+    XK_P32_CASE(1, PAIR_GAUSSIAN)
+    XK_P32_CASE(1, PAIR_PERIODIC_GAUSSIAN)
+    XK_P32_CASE(1, PAIR_COULOMB)
+    XK_P32_CASE(1, PAIR_PERIODIC_COULOMB)
+    XK_P32_CASE(2, PAIR_GAUSSIAN)
+    XK_P32_CASE(2, PAIR_PERIODIC_GAUSSIAN)
+    XK_P32_CASE(2, PAIR_COULOMB)
+    XK_P32_CASE(2, PAIR_PERIODIC_COULOMB)
+    XK_P32_CASE(3, PAIR_GAUSSIAN)
+    XK_P32_CASE(3, PAIR_PERIODIC_GAUSSIAN)
+    XK_P32_CASE(3, PAIR_COULOMB)
+    XK_P32_CASE(3, PAIR_PERIODIC_COULOMB)
+    XK_P32_CASE(3, PAIR_EWALD_REAL)
 #undef XK_P32_CASE
-      default:
-        return cudaErrorInvalidValue;
-    }
+    default:
+      return cudaErrorInvalidValue;
   }
-  if (le != cudaSuccess) return le;
+  return le != cudaSuccess ? le : XK_LAUNCHED();
+}
+
+cudaError_t pair_force32(const Geo &g, const PairPrm &p, const double *x, const double *m, double *f,
+                         double *scratch, cudaStream_t st) {
+  const P32 q = make_p32(g, p);
+  const P32Bufs b = p32_bufs(g, scratch);
+  {
+    XK_PROF("to32");
+    k_to32<<<cdiv(g.slots(), 256), 256, 0, st>>>(g, x, m, b.x32, q.uniform ? nullptr : b.im32, nullptr);
+  }
   cudaError_t e = XK_LAUNCHED();
+  if (e == cudaSuccess) e = pair_tiles32(g, p, q, b, st);
   if (e != cudaSuccess) return e;
   {
     XK_PROF("pair_finish");
-    k_pair_finish32<<<cdiv(g.slots(), 256), 256, 0, st>>>(g, part, T, 1.0 / g.P, f);
+    k_pair_finish32<<<cdiv(g.slots(), 256), 256, 0, st>>>(g, b.part, b.T, 1.0 / g.P, f);
   }
   return XK_LAUNCHED();
 }
 
 // ---- reciprocal space, mixed ----------------------------------------
-// first phase factors of the positions: ph1[(j*3 + d)*Ns + l]
-__global__ void __launch_bounds__(256) k_phase32(Geo g, const double *__restrict__ x, float2 *__restrict__ ph1) {
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t < (size_t)g.P * 3 * g.Ns) ph1[t] = phase32_slot(g, x, t);
-}
-
 // a block per (slice, 32 items), the longest items' blocks first
 __global__ void __launch_bounds__(SK_T, 2) k_sk32(Geo g, int ns, int ncol, int nlong, const int4 *__restrict__ cols,
                                                   const float *__restrict__ coef32, const float2 *__restrict__ ph1,
@@ -3816,7 +3816,8 @@ template <int NS>
 __global__ void __launch_bounds__(SK_T, 4) k_recip_force32(Geo g, int ncol, const int4 *__restrict__ cols,
                                                            const float2 *__restrict__ ph1,
                                                            const float4 *__restrict__ T, double scale,
-                                                           double *__restrict__ f) {
+                                                           double *__restrict__ f, const float *__restrict__ part,
+                                                           int ntile, double pscale) {
   extern __shared__ __align__(16) float4 rf32_sh[];
   float4 *sT = rf32_sh;
   RecipCol *sc = (RecipCol *)(sT + ncol * (NS + 1));
@@ -3825,20 +3826,26 @@ __global__ void __launch_bounds__(SK_T, 4) k_recip_force32(Geo g, int ncol, cons
   for (int q = threadIdx.x; q < ncol * (NS + 1); q += SK_T) sT[q] = Tj[q];
   for (int q = threadIdx.x; q < ncol; q += SK_T) sc[q] = recip_col32(cols[q], NS);
   recip_tile32<NS>(g, NS, ncol, sc, sT, (float2 *)(sc + ncol), (float2 *)rf32_sh, ph1, scale, f, j, blockIdx.x * 32,
-                   threadIdx.x >> 5, threadIdx.x & 31);
+                   threadIdx.x >> 5, threadIdx.x & 31, part, ntile, pscale);
 }
 
-// phases, structure factors with their force tables, and forces in FP32 for
-// all kept columns; the tables use the FP64 form's buffer, the phases lie
-// behind the FP64 ones
-cudaError_t recip_force32(const Geo &g, const Recip &r, const double *x, double inv_mP, double *f,
-                          cudaStream_t st) {
+// The mixed form's Ewald forces: FP32 positions and phases, real-space tiles,
+// structure factors with their force tables, and the forces of both sums in
+// four launches (separate copies, phases and a finishing kernel for the tiles
+// were six: 199 us a step of N = 512, P = 64 then, 196 now).  The tiles, which fill
+// the GPU, come after the structure factors: beside a learned residual, its own
+// stream's chain then starts early (222 us a step with the tiles first, 211).  The tables use
+// the FP64 form's buffer, the phases lie behind the FP64 ones.
+cudaError_t ewald_force32(const Geo &g, const PairPrm &p, const Recip &r, const double *x, const double *m,
+                          double inv_mP, double *f, double *scratch, cudaStream_t st) {
   if (g.D != 3) return cudaErrorInvalidValue;
-  if (r.ncol <= 0) return cudaSuccess;
+  if (r.ncol <= 0) return pair_force32(g, p, x, m, f, scratch, st);
+  const P32 q = make_p32(g, p);
+  const P32Bufs b = p32_bufs(g, scratch);
   float2 *ph1 = (float2 *)(r.phase + recip_phase_doubles(g, r.nsum));
   {
-    XK_PROF("phase32");
-    k_phase32<<<cdiv((size_t)g.P * 3 * g.Ns, 256), 256, 0, st>>>(g, x, ph1);
+    XK_PROF("to32");
+    k_to32<<<cdiv(g.slots(), 256), 256, 0, st>>>(g, x, m, b.x32, q.uniform ? nullptr : b.im32, ph1);
   }
   cudaError_t e = XK_LAUNCHED();
   if (e != cudaSuccess) return e;
@@ -3854,6 +3861,7 @@ cudaError_t recip_force32(const Geo &g, const Recip &r, const double *x, double 
         g, r.nsum, r.ncol, r.nlong, (const int4 *)r.kvec, (const float *)(r.coef + r.nk), ph1, (float4 *)r.T);
   }
   e = XK_LAUNCHED();
+  if (e == cudaSuccess) e = pair_tiles32(g, p, q, b, st);
   if (e != cudaSuccess) return e;
   XK_PROF("recip_force32");
   DISPATCH_NS(r.nsum, {
@@ -3867,7 +3875,7 @@ cudaError_t recip_force32(const Geo &g, const Recip &r, const double *x, double 
     const size_t tab = (sizeof(float4) * (NS + 1) + sizeof(RecipCol)) * r.ncol + sizeof(float2) * 2 * (NS + 1) * 32;
     const size_t red = sizeof(float2) * SK_W * 3 * 32;
     kf<<<dim3((g.N + 31) / 32, g.P), SK_T, tab > red ? tab : red, st>>>(
-        g, r.ncol, (const int4 *)r.kvec, ph1, (const float4 *)r.T, 4 * M_PI * inv_mP, f);
+        g, r.ncol, (const int4 *)r.kvec, ph1, (const float4 *)r.T, 4 * M_PI * inv_mP, f, b.part, b.T, 1.0 / g.P);
   });
   return XK_LAUNCHED();
 }

@@ -325,8 +325,8 @@ cudaError_t pair_force32(const Geo &g, const PairPrm &p, const double *x, const 
 void set_pair32_warps(int kind, int D, int N, int P, int warps);
 int pair32_warps(int kind, int D, int N, int P);
 // needs r.phase sized recip_phase_doubles(g, nsum) * 3 / 2 (FP32 phases behind)
-cudaError_t recip_force32(const Geo &g, const Recip &r, const double *x, double inv_mP, double *f,
-                          cudaStream_t st);
+cudaError_t ewald_force32(const Geo &g, const PairPrm &p, const Recip &r, const double *x, const double *m,
+                          double inv_mP, double *f, double *scratch, cudaStream_t st);
 
 // static structure factor of slices ja, jb for nq wave vectors qis[3q..]:
 // out[q] = (sum_l cos q.x_a)(sum_l cos q.x_b)/N + (sin)(sin)/N

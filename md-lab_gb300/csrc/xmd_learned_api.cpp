@@ -324,8 +324,7 @@ int learned_pair_force(md_pimd_t_x *pimd, SimDev *sd, PimdDev *pd, const xk::Pai
   // timing each kernel alone: the network's branch is joined at once
   if (xk::profiling() && !capturing()) XMD_CUDA(cudaStreamWaitEvent(st, M->mdone, 0));
   if (md_gb300_get_precision_x() == MD_GB_PRECISION_MIXED) {
-    XMD_CUDA(xk::recip_force32(sd->geo, M->cheap, x, inv_mP, f, st));
-    XMD_CUDA(xk::pair_force32(sd->geo, prm, x, sd->m.as<double>(), f, scr, st));
+    XMD_CUDA(xk::ewald_force32(sd->geo, prm, M->cheap, x, sd->m.as<double>(), inv_mP, f, scr, st));
   } else {
     XMD_CUDA(xk::recip_force(sd->geo, M->cheap, x, inv_mP, f, st));
     XMD_CUDA(xk::pair_force(sd->geo, prm, x, sd->m.as<double>(), f, scr, st));

@@ -501,15 +501,16 @@ int md_pimd_calc_pair_force_x(md_pimd_t_x *pimd, md_pair_force_t_x pf) {
     if (learned == 1) return learned_pair_force(pimd, sd, pd, prm, scr);
     const double inv_mP = 1.0 / (sd->mass0 * pimd->P);
     if (mixed)
-      XMD_CUDA(xk::recip_force32(sd->geo, recip_of(pd), sd->x.as<double>(), inv_mP, sd->f.as<double>(), st));
+      XMD_CUDA(xk::ewald_force32(sd->geo, prm, recip_of(pd), sd->x.as<double>(), sd->m.as<double>(), inv_mP,
+                                 sd->f.as<double>(), scr, st));
     else
       XMD_CUDA(xk::recip_force(sd->geo, recip_of(pd), sd->x.as<double>(), inv_mP, sd->f.as<double>(), st,
                                g_precision != MD_GB_PRECISION_FP64_STRICT));
   }
-  if (mixed)
-    XMD_CUDA(xk::pair_force32(sd->geo, prm, sd->x.as<double>(), sd->m.as<double>(), sd->f.as<double>(), scr, st));
-  else
+  if (!mixed)
     XMD_CUDA(xk::pair_force(sd->geo, prm, sd->x.as<double>(), sd->m.as<double>(), sd->f.as<double>(), scr, st));
+  else if (kind != xk::PAIR_EWALD_REAL)
+    XMD_CUDA(xk::pair_force32(sd->geo, prm, sd->x.as<double>(), sd->m.as<double>(), sd->f.as<double>(), scr, st));
   if (learned == 2) XMD_TRY(learned_judge_step(pimd, sd, pd));
   return 0;
 }
