@@ -82,7 +82,7 @@ int md_gb300_capture_ensemble_x(int n, md_gb300_system_step_fn_x step, void *ctx
    Other calls are refused (MD_GB_ERR_UNSUPPORTED).  The results equal those
    of the per-system calls.  The grid is the shape that
    md_gb300_autotune_ensemble_x chose for this ensemble's shapes, else 2
-   blocks per SM in 4 groups. */
+   blocks per SM in 16 groups. */
 int md_gb300_capture_ensemble_persistent_x(int n, md_gb300_system_step_fn_x step, void *ctx,
                                            md_gb300_graph_t_x **graph);
 /* 0 when every launch of a persistent ensemble graph so far completed its

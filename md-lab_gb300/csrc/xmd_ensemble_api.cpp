@@ -283,8 +283,13 @@ int md_gb300_capture_ensemble_persistent_x(int n, md_gb300_system_step_fn_x step
   XMD_TRY(plan(n, step, ctx, descs, pimds));
   EnsChoice shape = chosen_shape(signature(descs));
   if (!shape.bps) {
+    // untuned: two blocks an SM in 16 groups of systems (fewer where there are
+    // fewer systems).  Groups run in different phases, one's FP64 and latency
+    // beside another's FP32 sums; 1, 4, 8, 16 groups: 647, 478, 449, 446 us a step
+    // of 64 systems of 16 to 128 electrons, 414, 311, 276, 278 of 49, 173, 148,
+    // 150, 149 of 7; three blocks an SM spill registers: 496 with 16 groups
     shape.bps = std::min(2, xk::ensemble_max_blocks_per_sm(D, MD_NHC_LENGTH_X));
-    shape.groups = 4;
+    shape.groups = 16;
   }
   if (shape.bps < 1) return fail(MD_GB_ERR_UNSUPPORTED, "the persistent ensemble kernel does not fit on an SM");
   xk::EnsLaunch *e = new xk::EnsLaunch();
