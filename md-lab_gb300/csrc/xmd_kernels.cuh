@@ -105,8 +105,9 @@ cudaError_t set_value(double *p, double v, cudaStream_t st);
 // gl: scratch of 2N doubles (the row increments and their prefix sums)
 cudaError_t fill_enk(const Geo &g, const double *x, const double *m, double w2, int image,
                      double *Eint, double *ENk, double *gl, cudaStream_t st);
+// (H: 2N doubles of scratch)
 cudaError_t fill_enk2(const Geo &g, const double *x, const double *m, double w2, int image,
-                      double *ENk2, cudaStream_t st);
+                      double *ENk2, double *H, cudaStream_t st);
 // the cubic path's table (md_pimd_fill_ENk2_x), a different quantity
 cudaError_t fill_enk2_cubic(const Geo &g, const double *x, const double *m, double w2, int image,
                             double *ENk2, cudaStream_t st);

@@ -918,7 +918,7 @@ int md_pimd_fast_fill_ENk2_x(md_pimd_t_x *pimd, int image) {
   XMD_TRY(check_plain(pimd));
   XMD_TRY(check_image(sd, image));
   XMD_CUDA(xk::fill_enk2(sd->geo, sd->x.as<double>(), sd->m.as<double>(), pimd->omegaP * pimd->omegaP, image,
-                         pd->ENk2.as<double>(), stream()));
+                         pd->ENk2.as<double>(), pd->linkt.as<double>(), stream()));
   return 0;
 }
 
