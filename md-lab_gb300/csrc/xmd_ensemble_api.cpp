@@ -304,6 +304,7 @@ int md_gb300_capture_ensemble_persistent_x(int n, md_gb300_system_step_fn_x step
       GRAPH_ENSEMBLE, out);
   if (rc) return rc;
   mark_fresh(pimds);
+  mark_graph(*out, pimds);
   return 0;
 }
 

@@ -12,6 +12,7 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <vector>
 
 #include "md_gb300_x.h"
 #include "xmd_kernels.cuh"
@@ -63,6 +64,8 @@ void release(DevBuf &b);
 void *host_alloc(size_t bytes);
 void host_free(void *p);
 
+unsigned long long next_id();
+
 struct SimDev {
   bool valid = false;  // device copy authoritative
   // the layout whose padding lanes were last zeroed (re-uploads of the same
@@ -87,6 +90,7 @@ struct SimDev {
 };
 
 struct PimdDev {
+  const unsigned long long id = next_id();  // not an address: states come and go at the same one
   bool valid = false;  // ENk / ENk2 / VBN / Eint on the device authoritative
   DevBuf ENk, ENk2, Eint, VBN, tmpV, G;
   DevBuf linkt;  // 2N doubles: ENk increments and their prefix sums (scratch of the ENk and ENk2 fills)
@@ -96,6 +100,8 @@ struct PimdDev {
   DevBuf rec;  // weights of the forward and backward recursions (two halves)
   // tmpV (backward recursion) computed by the last md_pimd_fill_VB_x from
   // the current ENk with these beta and vi
+  // (both flags describe the calls issued so far; a replayed graph restores
+  // those its own calls left, GraphMarks)
   bool tmpv_fresh = false;
   double tmpv_beta = 0, tmpv_vi = 0;
   // G (the cycle probabilities) belongs to the stored ENk, VBN and tmpV at
@@ -113,6 +119,26 @@ struct PimdDev {
   int rc_df_items = 0, rc_items = 0, rc_tdf = 0;  // the double-float kernels' tables (xk::Recip)
   double rc_csum = 0;
 };
+
+// What the exchange calls of a graph leave when it is replayed: for each state
+// they touched, whether the recursions and G are those of its cycle energies,
+// and for which beta and xi.  A replay without them would leave the flags of
+// the last call made by hand: an estimator after it would take the recursion
+// although G is there (ten steps of 1600 ideal bosons and their estimator 4870
+// us, now 4054; the mixed 512-electron gas 2440, now 2311), or a G that the replay
+// has outdated.
+struct GraphMark {
+  const md_pimd_t_x *pimd;
+  unsigned long long id;
+  bool partial;  // only the forces, from recursions that the graph does not hold: G counts as unknown
+  bool tmpv, g;
+  double tmpv_beta, tmpv_vi, g_beta, g_vi;
+};
+// an exchange call touches pd; whole: the call replaces the recursions or
+// outdates them, so that what follows does not depend on what was before
+void mark_exchange(const md_pimd_t_x *pimd, const PimdDev *pd, bool whole);
+// the graph leaves the flags that the states have now
+void mark_graph(md_gb300_graph_t_x *g, const std::vector<md_pimd_t_x *> &pimds);
 
 struct StatsDev {
   bool valid = false;

@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstdlib>
@@ -611,9 +612,61 @@ struct md_gb300_graph {
   void (*release)(void *) = nullptr;  // frees what the graph's kernels read (owned)
   void *owned = nullptr;
   int kind = 0;  // what owned is (capture_single's caller)
+  std::vector<GraphMark> marks;  // what a replay leaves of the exchange state
 };
 
 namespace xmd {
+
+unsigned long long next_id() {
+  static std::atomic<unsigned long long> n{0};
+  return ++n;
+}
+
+// the states touched by this thread's capture in progress
+static thread_local std::vector<GraphMark> t_marks;
+
+void mark_exchange(const md_pimd_t_x *pimd, const PimdDev *pd, bool whole) {
+  if (!capturing()) return;
+  for (GraphMark &m : t_marks)
+    if (m.id == pd->id) {
+      if (whole) m.partial = false;
+      return;
+    }
+  t_marks.push_back({pimd, pd->id, !whole, false, false, 0, 0, 0, 0});
+}
+
+// the flags as they are now, of the states that are still there
+static void take_flags(std::vector<GraphMark> &marks) {
+  for (GraphMark &m : marks) {
+    const PimdDev *pd = lookup(g_pimd, m.pimd, false);
+    if (!pd || pd->id != m.id) continue;
+    m.tmpv = pd->tmpv_fresh, m.tmpv_beta = pd->tmpv_beta, m.tmpv_vi = pd->tmpv_vi;
+    m.g = pd->g_fresh && !m.partial, m.g_beta = pd->g_beta, m.g_vi = pd->g_vi;
+  }
+}
+
+static void capture_marks(md_gb300_graph *gr) {
+  take_flags(t_marks);
+  gr->marks.swap(t_marks);
+  t_marks.clear();
+}
+
+void mark_graph(md_gb300_graph_t_x *gr, const std::vector<md_pimd_t_x *> &pimds) {
+  gr->marks.clear();
+  for (const md_pimd_t_x *p : pimds)
+    if (const PimdDev *pd = lookup(g_pimd, p, false)) gr->marks.push_back({p, pd->id, false, false, false, 0, 0, 0, 0});
+  take_flags(gr->marks);
+}
+
+static void replay_marks(const md_gb300_graph *gr) {
+  for (const GraphMark &m : gr->marks) {
+    PimdDev *pd = lookup(g_pimd, m.pimd, false);
+    if (!pd || pd->id != m.id) continue;
+    mark_exchange(m.pimd, pd, !m.partial);  // a replay that is itself captured
+    if (!m.partial) pd->tmpv_fresh = m.tmpv, pd->tmpv_beta = m.tmpv_beta, pd->tmpv_vi = m.tmpv_vi;
+    pd->g_fresh = m.g, pd->g_beta = m.g_beta, pd->g_vi = m.g_vi;
+  }
+}
 
 void *graph_owned(md_gb300_graph_t_x *g, int kind) { return g && g->kind == kind ? g->owned : nullptr; }
 
@@ -703,6 +756,7 @@ int md_gb300_capture_begin_x(void) {
   if (capturing()) return fail(MD_GB_ERR_CAPTURE, "already capturing");
   XMD_TRY(join_side());  // no side-stream work from before the capture stays open
   XMD_CUDA(cudaStreamBeginCapture(stream(), cudaStreamCaptureModeThreadLocal));
+  t_marks.clear();
   return 0;
 }
 
@@ -722,6 +776,7 @@ int md_gb300_capture_end_x(md_gb300_graph_t_x **out) {
     delete gr;
     return cuda_fail(e, "cudaGraphInstantiate");
   }
+  capture_marks(gr);
   *out = gr;
   return 0;
 }
@@ -745,6 +800,7 @@ int md_gb300_capture_ensemble_x(int n, md_gb300_system_step_fn_x step, void *ctx
   std::vector<cudaEvent_t> ev(n + 1, nullptr);
   for (auto &e : ev) XMD_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   int rc = 0;
+  t_marks.clear();
   cudaError_t ce = cudaStreamBeginCapture(main, cudaStreamCaptureModeThreadLocal);
   if (ce == cudaSuccess) ce = cudaEventRecord(ev[n], main);
   // every system's calls go to its own branch, forked from and joined to
@@ -780,6 +836,7 @@ int md_gb300_capture_ensemble_x(int n, md_gb300_system_step_fn_x step, void *ctx
     delete gr;
     return cuda_fail(ie, "cudaGraphInstantiate");
   }
+  capture_marks(gr);
   *out = gr;
   return 0;
 }
@@ -788,6 +845,7 @@ int md_gb300_graph_launch_x(md_gb300_graph_t_x *gr, int count) {
   if (!gr || count < 0) return fail(MD_GB_ERR_ARG, "invalid graph launch");
   XMD_TRY(join_side());
   for (int i = 0; i < count; ++i) XMD_CUDA(cudaGraphLaunch(gr->e, stream()));
+  if (count) replay_marks(gr);
   return 0;
 }
 

@@ -286,6 +286,7 @@ int md_pimd_fast_fill_ENk_x(md_pimd_t_x *pimd, int image) {
   XMD_TRY(check_image(sd, image));
   XMD_CUDA(xk::fill_enk(sd->geo, sd->x.as<double>(), sd->m.as<double>(), pimd->omegaP * pimd->omegaP, image,
                         pd->Eint.as<double>(), pd->ENk.as<double>(), pd->linkt.as<double>(), stream()));
+  mark_exchange(pimd, pd, true);
   pd->tmpv_fresh = false;
   pd->g_fresh = false;
   return 0;
@@ -311,6 +312,7 @@ int md_pimd_fill_VB_x(md_pimd_t_x *pimd) {
   XMD_CUDA(xk::fill_vb_tv(pimd->N, pimd->beta, pimd->vi, pd->ENk.as<double>(), pd->lnn.as<double>(),
                           pd->VBN.as<double>(), pd->tmpV.as<double>(), rs, rs + xk::rec_scratch_doubles(pimd->N), s2));
   XMD_TRY(side_end(nullptr));
+  mark_exchange(pimd, pd, true);
   pd->tmpv_fresh = true;
   pd->tmpv_beta = pimd->beta;
   pd->tmpv_vi = pimd->vi;
@@ -355,6 +357,7 @@ int md_pimd_fast_fill_force_VB_x(md_pimd_t_x *pimd, int image) {
                             pd->G.as<double>(), sd->fex.as<double>(), scr, st));
   }
   XMD_TRY(side_end(sd));
+  mark_exchange(pimd, pd, false);
   pd->g_fresh = true;
   pd->g_beta = pimd->beta;
   pd->g_vi = pimd->vi;
