@@ -188,10 +188,11 @@ constexpr size_t ewd_smem() {
   return sizeof(float4) * 2 * (ENERGY ? EWD_ERFC_NINT : EWD_H_NINT) + sizeof(EwdWarp) * EWD_WARPS;
 }
 
-// One warp per 32 x 32 tile of a slice, as in k_pair_tiles: a's beads in the
-// lanes, b's rotating by, accumulated with Newton's third law, partials into
-// slots summed by k_ewd_finish (no atomics).  Tiles on the diagonal visit
-// each pair once (16 steps) and come last.
+// One warp per 32 x 32 tile of a slice, as in k_pair_tiles, or per part of its
+// steps (ewd_split): a's beads in the lanes, b's rotating by, accumulated with
+// Newton's third law, partials into slots summed by k_ewd_finish (no
+// atomics).  Tiles on the diagonal visit each pair once (16 steps) and come
+// last.
 //
 // Per step the lane's pair gives the squared lengths of its 8 candidates in
 // pairs: |m|^2 plus A_d = L_d^2 - 2 L_d |m_d| per shifted axis.  Those inside
@@ -204,19 +205,19 @@ constexpr size_t ewd_smem() {
 //
 // Bound: FP32 issue, about 650 operations a pair and step.  Measured on the
 // 512-electron, 64-bead gas (alpha L = 5.6, 3.35 images a pair, 8.4 M pairs):
-// 257 us where the FP64 tiles took 1352 (128 electrons, 32 beads: 51 and
-// 218 us; energies of the latter 57 and 325 us; 256 x 256 cross pairs 145 and
-// 667 us).  The forces' error against 64-bit sums, set by the cut-off at
+// 257 us where the FP64 tiles took 1352 (256 x 256 cross pairs 145 and 667
+// us); in parts 128 electrons, 32 beads take 24 us (51 with whole tiles, 218 in
+// FP64) and their energies less than half of the 61 us of whole tiles (325).  The forces' error against 64-bit sums, set by the cut-off at
 // alpha R = 5.2, is 3.6e-13 of the forces' norm (4.1e-13 with the FP64 tiles
 // and their FP32 far images), 12 to 512 electrons alike.  Energies take three
 // limbs: in two, images below the sum's last bit were lost and biased it by
 // -5e-16 of the pair energies; now 0.6e-15 (128 electrons, 32 beads, rms of 16
 // states) and 0.5e-15 (512, 64) of the energy against 64 bits, 1.3e-15 and
-// 2.6e-15 with the FP64 tiles, for 61 us at the former instead of 59.
+// 2.6e-15 with the FP64 tiles, for 3% more time.
 template <bool CROSS, bool ENERGY>
 __global__ void __launch_bounds__(32 * EWD_WARPS, 2)
     k_ewd_tiles(EwdPrm q, int P, EwdSide A, EwdSide B, float2 *__restrict__ outa, float2 *__restrict__ outb,
-                double *__restrict__ eout, int TA, int TB) {
+                double *__restrict__ eout, int TA, int TB, int split) {
   extern __shared__ __align__(16) float4 ewd_sm[];
   constexpr int NROW = 2 * (ENERGY ? EWD_ERFC_NINT : EWD_H_NINT);
   float4 *tab = ewd_sm;
@@ -230,8 +231,9 @@ __global__ void __launch_bounds__(32 * EWD_WARPS, 2)
   const unsigned lt = (1u << lane) - 1u;
   const int nwarps = gridDim.x * EWD_WARPS;
   const int full = CROSS ? TA * TB : TA * (TA - 1) / 2;
-  const int njobs = (full + (CROSS ? 0 : TA)) * P;
-  for (int w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; w < njobs; w += nwarps) {
+  const int njobs = (full + (CROSS ? 0 : TA)) * P * split;
+  for (int u = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; u < njobs; u += nwarps) {
+    const int w = u / split, part = u % split;
     int j, I, J;
     const bool diag = !CROSS && w >= full * P;
     if (CROSS) {
@@ -270,7 +272,8 @@ __global__ void __launch_bounds__(32 * EWD_WARPS, 2)
     float enc = 0.f;  // third limb of the energy: far images are smaller than the pair's last bit
 #pragma unroll
     for (int d = 0; d < 3; ++d) fa[d] = fb[d] = {0.f, 0.f};
-    const int s0 = diag ? 1 : 0, s1 = diag ? 16 : 31;
+    const int steps = (diag ? 16 : 32) / split;
+    const int s0 = (diag ? 1 : 0) + part * steps, s1 = s0 + steps - 1;
     for (int s = s0; s <= s1; ++s) {
       const int bl = (lane + s) & 31;
       const bool act = va && J * 32 + bl < B.N && !(diag && s == 16 && lane >= 16);
@@ -387,7 +390,7 @@ __global__ void __launch_bounds__(32 * EWD_WARPS, 2)
       double e = df_value(en) + (double)enc;
 #pragma unroll
       for (int o = 16; o; o >>= 1) e += __shfl_down_sync(ALL, e, o);
-      if (lane == 0) eout[w] = e;
+      if (lane == 0) eout[u] = e;
     } else {
       // b's sums back to their home lanes
 #pragma unroll
@@ -401,7 +404,7 @@ __global__ void __launch_bounds__(32 * EWD_WARPS, 2)
 #pragma unroll
           for (int d = 0; d < 3; ++d) {
             const df f = df_norm(df_add(fa[d], fb[d]));
-            outa[(((size_t)I * P + j) * 3 + d) * A.Ns + a] = make_float2(f.h, f.l);
+            outa[(((size_t)(I * split + part) * P + j) * 3 + d) * A.Ns + a] = make_float2(f.h, f.l);
           }
         continue;
       }
@@ -410,13 +413,13 @@ __global__ void __launch_bounds__(32 * EWD_WARPS, 2)
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
           const df f = df_norm(fa[d]);
-          outa[(((size_t)J * P + j) * 3 + d) * A.Ns + a] = make_float2(f.h, f.l);
+          outa[(((size_t)(J * split + part) * P + j) * 3 + d) * A.Ns + a] = make_float2(f.h, f.l);
         }
       if (vb)
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
           const df f = df_norm(fb[d]);
-          ob[(((size_t)I * P + j) * 3 + d) * B.Ns + b0] = make_float2(f.h, f.l);
+          ob[(((size_t)(I * split + part) * P + j) * 3 + d) * B.Ns + b0] = make_float2(f.h, f.l);
         }
     }
   }
@@ -428,6 +431,7 @@ __global__ void k_ewd_finish(int N, int Ns, size_t S, const float2 *__restrict__
   const size_t s = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= S || (int)(s % Ns) >= N) return;
   df acc = {0.f, 0.f};
+#pragma unroll 8
   for (int t = 0; t < T; ++t) {
     const float2 v = part[(size_t)t * S + s];
     acc = df_norm(df_add(acc, {v.x, v.y}));
@@ -435,9 +439,25 @@ __global__ void k_ewd_finish(int N, int Ns, size_t S, const float2 *__restrict__
   f[s] += scale * df_value(acc);
 }
 
+// Parts of a tile's rotation steps.  With a warp a tile, 128 electrons and 32
+// beads kept 320 of the 2432 warps that fit on 152 SMs, and a large system ended
+// on a round that few warps had work in.  So up to four parts until there are
+// four rounds of warps; eight only where four leave most SM sub-partitions idle
+// (a part costs a slot of partials).  A step of N x P electrons (|n| <= 4) with
+// whole tiles, and with 2, 4 and 8 parts, * taken: 16 x 4 63, 53* (8); 64 x 32
+// 96, 64* (8); 128 x 32 109, 85, 80*, 87; 128 x 64 119, 106, 94*, 96; 200 x 48
+// 160, 138, 133*, 134; 300 x 64 234, 222, 221*; 512 x 64 435, 433*; 256 + 256 x
+// 64 614, -, 612* us.
+int ewd_split(size_t jobs) {
+  if (jobs * 4 < 8 * 152) return 8;
+  int split = 1;
+  while (split < 4 && jobs * split < 4 * 2432) split *= 2;
+  return split;
+}
+
 template <bool CROSS, bool ENERGY>
 static cudaError_t launch_tiles(const EwdPrm &q, int P, const EwdSide &A, const EwdSide &B, float2 *oa, float2 *ob,
-                                double *eo, int TA, int TB, int bps, cudaStream_t st) {
+                                double *eo, int TA, int TB, int split, int bps, cudaStream_t st) {
   static int occ = 0, sms = 0;
   if (!occ) {
     int dev = 0;
@@ -453,11 +473,14 @@ static cudaError_t launch_tiles(const EwdPrm &q, int P, const EwdSide &A, const 
     if (e != cudaSuccess) return e;
     occ = n > 0 ? n : 1;
   }
-  const size_t jobs = (size_t)(CROSS ? TA * TB : TA * (TA + 1) / 2) * P;
-  const size_t need = (jobs + EWD_WARPS - 1) / EWD_WARPS;
+  const size_t jobs = (size_t)(CROSS ? TA * TB : TA * (TA + 1) / 2) * P * split;
   const size_t room = (size_t)sms * (bps > 0 && bps < occ ? bps : occ);
-  k_ewd_tiles<CROSS, ENERGY><<<(int)(need < room ? need : room), 32 * EWD_WARPS, ewd_smem<ENERGY>(), st>>>(
-      q, P, A, B, oa, ob, eo, TA, TB);
+  // fewer jobs than warps: over as many SMs as there are jobs
+  size_t grid = (jobs + EWD_WARPS - 1) / EWD_WARPS;
+  if (grid < jobs && grid < (size_t)sms) grid = jobs < (size_t)sms ? jobs : sms;
+  if (grid > room) grid = room;
+  k_ewd_tiles<CROSS, ENERGY><<<(int)grid, 32 * EWD_WARPS, ewd_smem<ENERGY>(), st>>>(
+      q, P, A, B, oa, ob, eo, TA, TB, split);
   return XK_LAUNCHED();
 }
 
@@ -476,39 +499,42 @@ static cudaError_t finish(const Geo &g, const float2 *part, int T, double scale,
 // scratch: T slots of partials (8 bytes each), then the split positions
 cudaError_t ewd_force(const Geo &g, const PairPrm &p, const double *x, double *f, double *scratch, cudaStream_t st) {
   const EwdPrm q = make_ewd(g, p);
-  const int T = (g.N + 31) / 32;
-  double *pos = scratch + (((size_t)T * g.slots() + 1) & ~(size_t)1);
+  const int T = (g.N + 31) / 32, split = ewd_split((size_t)T * (T + 1) / 2 * g.P);
+  double *pos = scratch + (((size_t)T * split * g.slots() + 1) & ~(size_t)1);
   cudaError_t e = split_positions(g, q, x, pos, st);
   if (e != cudaSuccess) return e;
   const EwdSide A{(const float4 *)pos, g.N, g.Ns};
   {
     XK_PROF("pair_tiles_ewald_real");
-    e = launch_tiles<false, false>(q, g.P, A, A, (float2 *)scratch, nullptr, nullptr, T, T,
+    e = launch_tiles<false, false>(q, g.P, A, A, (float2 *)scratch, nullptr, nullptr, T, T, split,
                                    tuning(TUNE_PAIR64_BPS, PAIR_EWALD_REAL, 3, g.N, g.P), st);
   }
   if (e != cudaSuccess) return e;
   // unit charges and scaled lengths inside: F = s alpha^2 / (m P) sum
-  return finish(g, (const float2 *)scratch, T, p.qs * p.alpha * p.alpha * p.inv_mass / g.P, f, st);
+  return finish(g, (const float2 *)scratch, T * split, p.qs * p.alpha * p.alpha * p.inv_mass / g.P, f, st);
 }
 
-// per-tile energies erfc(x)/x (jobs * P doubles, T (T + 1) / 2 jobs a slice)
-cudaError_t ewd_energy_tiles(const Geo &g, const PairPrm &p, const double *x, double *scratch, cudaStream_t st) {
+// energies erfc(x)/x of the tiles' parts (jobs * P * *parts doubles, T (T + 1) / 2 jobs a slice)
+cudaError_t ewd_energy_tiles(const Geo &g, const PairPrm &p, const double *x, double *scratch, int *parts,
+                             cudaStream_t st) {
   const EwdPrm q = make_ewd(g, p);
-  const int T = (g.N + 31) / 32;
-  double *pos = scratch + (((size_t)T * g.slots() + 1) & ~(size_t)1);
+  const int T = (g.N + 31) / 32, split = ewd_split((size_t)T * (T + 1) / 2 * g.P);
+  double *pos = scratch + (((size_t)T * split * g.slots() + 1) & ~(size_t)1);
   cudaError_t e = split_positions(g, q, x, pos, st);
   if (e != cudaSuccess) return e;
   const EwdSide A{(const float4 *)pos, g.N, g.Ns};
+  *parts = split;
   XK_PROF("pair_tiles_ewald_real");
-  return launch_tiles<false, true>(q, g.P, A, A, nullptr, nullptr, scratch, T, T, 0, st);
+  return launch_tiles<false, true>(q, g.P, A, A, nullptr, nullptr, scratch, T, T, split, 0, st);
 }
 
 cudaError_t ewd_force_2(const Geo &ga, const Geo &gb, const PairPrm &p, const double *xa, double inv_ma,
                         const double *xb, double inv_mb, double *fa, double *fb, double *scratch, cudaStream_t st) {
   const EwdPrm q = make_ewd(ga, p);
   const int TA = (ga.N + 31) / 32, TB = (gb.N + 31) / 32;
-  double *oa = scratch, *ob = oa + (size_t)TB * ga.slots();
-  double *pa = scratch + (((size_t)TB * ga.slots() + (size_t)TA * gb.slots() + 1) & ~(size_t)1);
+  const int split = ewd_split((size_t)TA * TB * ga.P);
+  double *oa = scratch, *ob = oa + (size_t)TB * split * ga.slots();
+  double *pa = scratch + ((((size_t)TB * ga.slots() + (size_t)TA * gb.slots()) * split + 1) & ~(size_t)1);
   double *pb = pa + ewd_pos_doubles(ga);
   cudaError_t e = split_positions(ga, q, xa, pa, st);
   if (e == cudaSuccess) e = split_positions(gb, q, xb, pb, st);
@@ -516,13 +542,13 @@ cudaError_t ewd_force_2(const Geo &ga, const Geo &gb, const PairPrm &p, const do
   {
     XK_PROF("pair_cross");
     e = launch_tiles<true, false>(q, ga.P, {(const float4 *)pa, ga.N, ga.Ns}, {(const float4 *)pb, gb.N, gb.Ns},
-                                  (float2 *)oa, (float2 *)ob, nullptr, TA, TB, 0, st);
+                                  (float2 *)oa, (float2 *)ob, nullptr, TA, TB, split, 0, st);
   }
   if (e != cudaSuccess) return e;
   const double s = p.qs * p.alpha * p.alpha / ga.P;
-  e = finish(ga, (const float2 *)oa, TB, s * inv_ma, fa, st);
+  e = finish(ga, (const float2 *)oa, TB * split, s * inv_ma, fa, st);
   if (e != cudaSuccess) return e;
-  return finish(gb, (const float2 *)ob, TA, s * inv_mb, fb, st);
+  return finish(gb, (const float2 *)ob, TA * split, s * inv_mb, fb, st);
 }
 
 }  // namespace xk

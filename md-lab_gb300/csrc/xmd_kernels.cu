@@ -2225,7 +2225,7 @@ size_t pair_scratch_doubles(const Geo &g) {
   size_t a = (size_t)T * g.slots() + (g.slots() + (size_t)g.P * g.Ns + 1) / 2 + 1;
   const int split = pair_split(g, (int)jobs);
   if (a < (size_t)T * split * g.slots()) a = (size_t)T * split * g.slots();
-  const size_t d = g.D == 3 ? (size_t)T * g.slots() + 1 + ewd_pos_doubles(g) : 0;
+  const size_t d = g.D == 3 ? (size_t)T * ewd_split(jobs * g.P) * g.slots() + 1 + ewd_pos_doubles(g) : 0;
   if (d > a) a = d;
   size_t b = jobs * g.P * split;
   return a > b ? a : b;
@@ -2375,7 +2375,7 @@ cudaError_t pair_energy(const Geo &g, const PairPrm &p, const double *x, double 
   cudaError_t e;
   double unit = 1.0;
   if (ewd_applies(g, p, true)) {
-    e = ewd_energy_tiles(g, p, x, scratch, st);
+    e = ewd_energy_tiles(g, p, x, scratch, &split, st);
     unit = p.qs * p.alpha;
   } else {
     if (p.kind != PAIR_EWALD_REAL) split = pair_split(g, jobs);
@@ -2394,7 +2394,7 @@ cudaError_t pair_energy(const Geo &g, const PairPrm &p, const double *x, double 
 size_t pair2_scratch_doubles(const Geo &ga, const Geo &gb) {
   const int TA = (ga.N + 31) / 32, TB = (gb.N + 31) / 32;
   size_t forces = (size_t)TB * ga.slots() + (size_t)TA * gb.slots();
-  if (ga.D == 3) forces += 1 + ewd_pos_doubles(ga) + ewd_pos_doubles(gb);
+  if (ga.D == 3) forces = forces * ewd_split((size_t)TA * TB * ga.P) + 1 + ewd_pos_doubles(ga) + ewd_pos_doubles(gb);
   const size_t energy = (size_t)TA * TB * ga.P;
   return forces > energy ? forces : energy;
 }

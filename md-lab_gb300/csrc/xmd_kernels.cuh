@@ -216,9 +216,11 @@ cudaError_t pair_energy(const Geo &g, const PairPrm &p, const double *x, double 
 // the scratch, and the launches pair_force and pair_force_2 hand over
 bool ewd_applies(const Geo &g, const PairPrm &p, bool energy);
 size_t ewd_pos_doubles(const Geo &g);
+int ewd_split(size_t jobs);  // parts of a tile, of jobs tiles in all
 cudaError_t ewd_force(const Geo &g, const PairPrm &p, const double *x, double *f, double *scratch, cudaStream_t st);
-// the real-space energies of the tile jobs, in units of s alpha, into scratch
-cudaError_t ewd_energy_tiles(const Geo &g, const PairPrm &p, const double *x, double *scratch, cudaStream_t st);
+// the real-space energies of the tile jobs' *parts parts, in units of s alpha, into scratch
+cudaError_t ewd_energy_tiles(const Geo &g, const PairPrm &p, const double *x, double *scratch, int *parts,
+                             cudaStream_t st);
 cudaError_t ewd_force_2(const Geo &ga, const Geo &gb, const PairPrm &p, const double *xa, double inv_ma,
                         const double *xb, double inv_mb, double *fa, double *fb, double *scratch, cudaStream_t st);
 
