@@ -440,18 +440,18 @@ __global__ void k_ewd_finish(int N, int Ns, size_t S, const float2 *__restrict__
 }
 
 // Parts of a tile's rotation steps.  With a warp a tile, 128 electrons and 32
-// beads kept 320 of the 2432 warps that fit on 152 SMs, and a large system ended
-// on a round that few warps had work in.  So up to four parts until there are
-// four rounds of warps; eight only where four leave most SM sub-partitions idle
-// (a part costs a slot of partials).  A step of N x P electrons (|n| <= 4) with
-// whole tiles, and with 2, 4 and 8 parts, * taken: 16 x 4 63, 53* (8); 64 x 32
-// 96, 64* (8); 128 x 32 109, 85, 80*, 87; 128 x 64 119, 106, 94*, 96; 200 x 48
-// 160, 138, 133*, 134; 300 x 64 234, 222, 221*; 512 x 64 435, 433*; 256 + 256 x
-// 64 614, -, 612* us.
+// beads kept 320 of the 2432 warps that fit on 152 SMs.  So up to four parts
+// until there are two rounds of warps (beyond, the last round costs less than
+// the parts' slots of partials); eight only where four leave most SM
+// sub-partitions idle.  A step of N x P electrons (|n| <= 4) with whole tiles,
+// and with 2, 4 and 8 parts, * taken: 16 x 4 63, 53* (8); 64 x 32 96, 64* (8);
+// 128 x 32 109, 85, 80*, 87; 128 x 64 119, 106, 94*, 96; 200 x 48 160, 138,
+// 133*, 134; 300 x 64 234, 222*, 221; 512 x 33 282, 281*, 280; 512 x 64 435*,
+// 433; 256 + 256 x 64 614, 610* (2 a cross tile) us.
 int ewd_split(size_t jobs) {
   if (jobs * 4 < 8 * 152) return 8;
   int split = 1;
-  while (split < 4 && jobs * split < 4 * 2432) split *= 2;
+  while (split < 4 && jobs * split < 2 * 2432) split *= 2;
   return split;
 }
 

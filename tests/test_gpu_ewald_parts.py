@@ -10,7 +10,7 @@ from test_gpu_ewald_df import TOL_E, TOL_F, _energy, _forces, _system
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("P", [2, 102, 810, 1620, 1622, 3250])  # 3 tiles a bead slice
+@pytest.mark.parametrize("P", [2, 101, 102, 810, 811, 1621, 1622])  # 3 tiles a bead slice
 def test_forces_and_energy(P):
     lib = xmd_x.load(3, 4)
     N, L = 40, 5.0
@@ -25,7 +25,7 @@ def test_forces_and_energy(P):
         s.free()
 
 
-@pytest.mark.parametrize("P", [3, 77, 1217, 2433])  # 4 cross tiles a bead slice
+@pytest.mark.parametrize("P", [3, 77, 609, 1215, 1216])  # 4 cross tiles a bead slice
 def test_cross_pairs(P):
     lib = xmd_x.load(3, 4)
     xmd_x.set_potentials(lib, coul_s=1.0, alpha=5.6 / 5.0, nsum=4)
