@@ -90,9 +90,10 @@ int md_gb300_capture_ensemble_persistent_x(int n, md_gb300_system_step_fn_x step
 int md_gb300_ensemble_status_x(md_gb300_graph_t_x *graph);
 /* The last launch's phase durations in microseconds (up to n of them: the
    thermostat's first half and force reset; springs, cycle-energy increments,
-   pair tiles and structure factors; prefix sums and force tables; cycle
-   energies and reciprocal forces; recursion weights, block inverses and the
-   pair sums; the two solves; G; the end-bead exchange forces; the second
+   pair tiles and structure factors; prefix sums and reciprocal forces; cycle
+   energies and pair sums; recursion weights and block inverses; the two
+   solves; G (0: formed within the next); G and the end-bead exchange forces;
+   the second
    half step), as one block saw them, then that block's own time in the
    second phase for its springs, cycle-energy increments, pair tiles and
    structure factors, then each group's step time; returns the number of
@@ -165,15 +166,12 @@ int md_gb300_pair_force_noalloc_x(md_pair_force_t_x pf, const double *x, const d
 
 /* Arithmetic of the pair forces (md_pimd_calc_pair_force_x), including
    both Ewald parts.  MD_GB_PRECISION_FP64 (default) reproduces MD-Lab to
-   1e-10: every term is FP64 except two groups of small ones, evaluated on
-   the FP32 pipe: the real-space Ewald images at alpha R >= 4 (each below
-   5.2e-7 of the pair strength over R^2; added to the FP64 sum per pair),
-   and the reciprocal wave-vector columns (nx, ny) whose every vector has a
-   force weight |G| c(n) below 1e-7 of the largest (FP32 structure factors,
-   tables and compensated column sums).  Against
-   MD_GB_PRECISION_FP64_STRICT, which evaluates those in FP64 too, the
-   forces of the 512-electron, 64-bead electron gas (Ewald |n| <= 10) differ
-   by 2.4e-16 of the largest and by at most 6.8e-12 of any bead's own.
+   1e-10: FP64 except the Ewald sums, which run in double-float (unevaluated
+   sums of two FP32 values, 48 significant bits; wave vectors of a force
+   weight |G| c(n) below 1e-8 of the largest in FP32).  Forces are 3.6e-13 of
+   their norm from 64-bit sums (set by the cut-off at alpha R = 5.2), and
+   within 2e-12 of the largest from MD_GB_PRECISION_FP64_STRICT, which
+   evaluates every term in FP64.
    MD_GB_PRECISION_MIXED evaluates pair and real-space Ewald forces in
    FP32: each lane adds at most 32 FP32 pair terms (one 32 x 32 tile), and
    the tile partials are added in FP64; the reciprocal sum builds its

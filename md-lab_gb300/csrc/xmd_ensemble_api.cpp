@@ -324,8 +324,10 @@ int md_gb300_ensemble_phase_times_x(md_gb300_graph_t_x *graph, double *us, int n
   int failed = 0;
   double t[xk::ENS_PHASES + 4 + xk::ENS_MAX_GROUPS];
   XMD_CUDA(xk::ensemble_status(*e, &failed, t));
-  const int m = xk::ENS_PHASES + 4 + e->groups;
-  for (int k = 0; k < n && k < m; ++k) us[k] = t[k];
+  // nine phases to the caller: G, its own phase once, is formed within the next
+  constexpr int G_AT = 6;
+  const int m = xk::ENS_PHASES + 5 + e->groups;
+  for (int k = 0; k < n && k < m; ++k) us[k] = k < G_AT ? t[k] : (k == G_AT ? 0.0 : t[k - 1]);
   return m;
 }
 
