@@ -1626,8 +1626,8 @@ __device__ inline void recip_tile32(const Geo &g, int ns, int ncol, const RecipC
     const float4 w0 = t[0];
     float ur = w0.x, ui = w0.y, vr = 0.f, vi = 0.f;
 #pragma unroll
-    for (int n = 0; n < NSM; ++n) {  // harmonic n + 1; an odd nzmax is followed by a zero entry
-      if (n % 2 == 0 && n >= c.nz) break;
+    for (int n = 0; n < NSM; ++n) {  // harmonic n + 1; an odd nzmax below ns is followed by a zero entry
+      if (n % 2 == 0 ? n >= c.nz : n >= ns) break;
       const float4 ab = t[n + 1];
       ur = fmaf(ez[n].x, ab.x, fmaf(-ez[n].y, ab.w, ur));
       ui = fmaf(ez[n].x, ab.y, fmaf(ez[n].y, ab.z, ui));
