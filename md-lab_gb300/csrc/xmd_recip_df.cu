@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(128) k_df_phase(Geo g, int ns, const double *_
   }
 }
 
-// Structure factors: DF_GR threads share an item (column and DF_NG harmonics)
+// Structure factors: GR threads share an item (column and DF_NG harmonics)
 // of a slice, particles interleaved; phases staged DF_CH particles at a time,
 // the next chunk copied asynchronously while one is summed.  With
 // P = sum e_xy cos(nz theta_z), Q = sum e_xy sin(nz theta_z):
@@ -150,21 +150,23 @@ __global__ void __launch_bounds__(128) k_df_phase(Geo g, int ns, const double *_
 // inside the sphere a column has at most seven, so e_xy is formed once a
 // column, and no group is padded (142 -> 83 us at 512 x 64 with the
 // asynchronous copies).  Blocks of the double-float items, the longest, start
-// first.
-constexpr int DF_CH = 64, DF_SK_T = 512, DF_GR = 8;
+// first.  Two blocks of 256 threads an SM and not one of 512, which left a
+// third of the chip idle in the last round: 512 x 33, |n| <= 10, 82 -> 63 us;
+// 700 x 20, |n| <= 9, 109 -> 80; 512 x 64 83 -> 82.
+constexpr int DF_CH = 64, DF_SK_T = 256;
 
 __device__ __forceinline__ void copy16(float4 *dst, const float4 *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
 }
 
-template <int NS>
-__global__ void __launch_bounds__(DF_SK_T, 1)
+template <int NS, int GR>
+__global__ void __launch_bounds__(DF_SK_T, 2)
     k_df_sk(int N, int Ns, const float4 *__restrict__ ph, const int4 *__restrict__ cols, const int *__restrict__ items,
             int ndf, int nitems, float4 *__restrict__ S, int nk) {
   constexpr int LD = DF_CH + 1, STAGE = 3 * (NS + 1) * LD, NG = NS < DF_NG ? NS : DF_NG;
   extern __shared__ __align__(16) float4 df_sp[];  // two stages of [3][NS + 1][LD]
-  const int j = blockIdx.x, gq = threadIdx.x % DF_GR;
-  const int it = blockIdx.y * (DF_SK_T / DF_GR) + threadIdx.x / DF_GR;
+  const int j = blockIdx.x, gq = threadIdx.x % GR;
+  const int it = blockIdx.y * (DF_SK_T / GR) + threadIdx.x / GR;
   const bool live = it < nitems;
   const int item = live ? items[it] : 0;
   const int4 c = cols[item & 0xffff];
@@ -196,7 +198,7 @@ __global__ void __launch_bounds__(DF_SK_T, 1)
     const float4 *sp = df_sp + (k & 1) * STAGE;
     const int cnt = min(N - k * DF_CH, DF_CH);
     if (nd >= 0) {
-      for (int l = gq; l < cnt; l += DF_GR) {
+      for (int l = gq; l < cnt; l += GR) {
         const dfc ex = unpack(sp[ox + l]);
         dfc ey = unpack(sp[oy + l]);
         ey.i.h *= sy, ey.i.l *= sy;
@@ -222,7 +224,7 @@ __global__ void __launch_bounds__(DF_SK_T, 1)
         }
       }
     } else {
-      for (int l = gq; l < cnt; l += DF_GR) {
+      for (int l = gq; l < cnt; l += GR) {
         const float4 ex = sp[ox + l], ey = sp[oy + l];
         const float yi = sy * ey.y;
         const float er = fmaf(ex.x, ey.x, -ex.y * yi), ei = fmaf(ex.x, yi, ex.y * ey.x);
@@ -252,7 +254,7 @@ __global__ void __launch_bounds__(DF_SK_T, 1)
     }
   }
 #pragma unroll
-  for (int o = 1; o < DF_GR; o <<= 1) {
+  for (int o = 1; o < GR; o <<= 1) {
     s0r = df_add(s0r, shfl_xor(ALL, s0r, o));
     s0i = df_add(s0i, shfl_xor(ALL, s0i, o));
 #pragma unroll
@@ -466,6 +468,22 @@ constexpr size_t sk_smem() {
   return 2 * sizeof(float4) * 3 * (NS + 1) * (DF_CH + 1);
 }
 
+template <int NS, int GR>
+static cudaError_t launch_sk(const Geo &g, const Recip &r, cudaStream_t st) {
+  static bool opted = false;
+  if (!opted) {
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_df_sk<NS, GR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sk_smem<NS>());
+    if (e != cudaSuccess) return e;
+    opted = true;
+  }
+  const dim3 grid(g.P, cdivz(r.items, DF_SK_T / GR));
+  k_df_sk<NS, GR><<<grid, DF_SK_T, sk_smem<NS>(), st>>>(g.N, g.Ns, (const float4 *)r.phase, df_cols(r),
+                                                       df_base(r) + items_at(r.nsum), r.df_items, r.items,
+                                                       (float4 *)r.S, r.nk);
+  return XK_LAUNCHED();
+}
+
 cudaError_t recip_df_sk(const Geo &g, const Recip &r, const double *x, cudaStream_t st) {
   {
     XK_PROF("phase");
@@ -474,19 +492,12 @@ cudaError_t recip_df_sk(const Geo &g, const Recip &r, const double *x, cudaStrea
   cudaError_t e = XK_LAUNCHED();
   if (e != cudaSuccess || r.items <= 0) return e;
   XK_PROF("sk");
-  const dim3 grid(g.P, cdivz(r.items, DF_SK_T / DF_GR));
-  DF_NS(r.nsum, {
-    static bool opted = false;
-    if (!opted) {
-      e = cudaFuncSetAttribute(k_df_sk<NS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sk_smem<NS>());
-      if (e != cudaSuccess) return e;
-      opted = true;
-    }
-    k_df_sk<NS><<<grid, DF_SK_T, sk_smem<NS>(), st>>>(g.N, g.Ns, (const float4 *)r.phase, df_cols(r),
-                                                     df_base(r) + items_at(r.nsum), r.df_items, r.items, (float4 *)r.S,
-                                                     r.nk);
-  });
-  return XK_LAUNCHED();
+  // 16 threads an item where 8 would give four SMs seven blocks at most:
+  // 700 x 20, |n| <= 9, 80 -> 53 us; 512 x 33, |n| <= 10 (264 blocks), 63 -> 55;
+  // 128 x 32, |n| <= 8 (160), 22.0 -> 20.7; 200 x 48, |n| <= 9 (288), keeps 38 (43)
+  const bool few = (size_t)g.P * cdivz(r.items, DF_SK_T / 8) * 4 <= 7 * 152;
+  DF_NS(r.nsum, { return few ? launch_sk<NS, 16>(g, r, st) : launch_sk<NS, 8>(g, r, st); });
+  return cudaSuccess;
 }
 
 cudaError_t recip_df_tables_of(const Geo &g, const Recip &r, cudaStream_t st) {
