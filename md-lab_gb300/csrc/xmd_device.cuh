@@ -1353,12 +1353,18 @@ __device__ inline double2 exch_end_share(const Geo &g, const double *__restrict_
   }
   return s;
 }
+// the spring vector of end bead `side` (0: bead 1, 1: bead P) along its own
+// ring, coordinate d
+__device__ inline double exch_own_spring(const Geo &g, const double *__restrict__ x, int image, int side, int d, int l) {
+  const int j = side ? g.P - 1 : 0, jn = side ? g.P - 2 : 1;
+  const double r = x[sidx(j, d, l, g.D, g.Ns)] - x[sidx(jn, d, l, g.D, g.Ns)];
+  return image ? min_image(r, g.box[d], g.inv_box[d]) : r;
+}
 // the exchange force on the end bead, as the acceleration the step stores
-// (the bead's mass cancels, as in spring_interior_bead)
+// (the bead's mass cancels, as in spring_interior_bead); r: exch_own_spring
 template <int D>
-__device__ inline double exch_end_value(const Geo &g, const double *__restrict__ x, double w2, int image,
-                                        const double *__restrict__ scr, int side, int d, int l, const double2 *share,
-                                        int stride) {
+__device__ inline double exch_end_value(const Geo &g, double r, double w2, const double *__restrict__ scr, int side,
+                                        int d, int l, const double2 *share, int stride) {
   const int T = (g.N + 31) / 32, t = (l + side) / 32;
   double S = 0, W = 0;
 #pragma unroll
@@ -1371,9 +1377,6 @@ __device__ inline double exch_end_value(const Geo &g, const double *__restrict__
     S += side ? co[d] : -co[d];
     W += co[D];
   }
-  const int j = side ? g.P - 1 : 0, jn = side ? g.P - 2 : 1;
-  double r = x[sidx(j, d, l, D, g.Ns)] - x[sidx(jn, d, l, D, g.Ns)];
-  if (image) r = min_image(r, g.box[d], g.inv_box[d]);
   return -w2 * (W * r + S);
 }
 

@@ -62,7 +62,7 @@ struct EnsSys {
 // task kinds of the step's phases (threads, warps or blocks, as noted)
 enum {
   R_A,       // thread: first half step per slot
-  R_B_SPR,   // thread: interior springs
+  R_B_SPR,   // thread: ring springs
   R_B_EINT,  // warp: E_l^(1) per particle (the pair tiles continue its numbering)
   R_B_PAIR,  // warp: FP32 pair tile jobs
   R_B_SK,    // block: structure factors and force tables per slice and 32 items
@@ -248,16 +248,25 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
   ens_grid_sync(bar, G, limit);
   ens_stamp(bar, 1);
 
-  // B: interior ring springs into fex; E_l^(1) and the prefix-sum increments
-  // (md_pimd_fast_fill_ENk_x); FP32 pair tiles; structure factors
+  // B: interior ring springs into fex, and for the end beads the spring vector
+  // along their own ring (phase H moves the beads it would be formed from); E_l^(1)
+  // and the prefix-sum increments (md_pimd_fast_fill_ENk_x); FP32 pair tiles;
+  // structure factors
   {
     for (int i = i0; i < i1; ++i) {
       const EnsSysDesc &d = sys[i].d;
       const Geo g = d.g;
-      const long long n = g.P > 2 ? (long long)(g.P - 2) * g.Ns : 0;
+      const long long n = (long long)g.P * g.Ns;
       for (long long t = ens_first(gt, sys[i].rot[R_B_SPR], GT); t < n; t += GT) {
-        const int l = (int)(t % g.Ns), j = (int)(t / g.Ns) + 1;
-        if (l < g.N) spring_interior_bead<D>(g, d.x, d.w2, d.image, d.fex, j, l);
+        const int l = (int)(t % g.Ns), j = (int)(t / g.Ns);
+        if (l >= g.N) continue;
+        if (j > 0 && j < g.P - 1) {
+          spring_interior_bead<D>(g, d.x, d.w2, d.image, d.fex, j, l);
+        } else {
+#pragma unroll
+          for (int dd = 0; dd < D; ++dd)
+            d.fex[sidx(j, dd, l, D, g.Ns)] = exch_own_spring(g, d.x, d.image, j > 0, dd, l);
+        }
       }
     }
   }
@@ -410,7 +419,8 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
   ens_stamp(bar, 7);
 
   // H: the end beads' exchange forces into fex, the second half step with
-  // f + fex (md_update_nhc_VV3_2_x), the periodic wrap
+  // f + fex (md_update_nhc_VV3_2_x), the periodic wrap.  A thread reads and moves
+  // its own slot's position only
   {
     for (int i = i0; i < i1; ++i) {
       const EnsSys &E = sys[i];
@@ -427,7 +437,7 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
           double2 share[EX_Y];
 #pragma unroll
           for (int y = 0; y < EX_Y; ++y) share[y] = exch_end_share<D>(g, d.xscr, side, dd, l, y);
-          d.fex[s] = exch_end_value<D>(g, d.x, d.w2, d.image, d.xscr, side, dd, l, share, 1);
+          d.fex[s] = exch_end_value<D>(g, d.fex[s], d.w2, d.xscr, side, dd, l, share, 1);
         }
         nhc_slot<D, L>(g, 2, s, l, d.x, d.v, d.f, d.fex, d.m, d.th, d.vt, d.Q, d.iQ, d.kT, d.h);
         if (d.wrap) {
@@ -593,7 +603,7 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
         const long long slots = (long long)g.slots(), N = g.N, P = g.P;
         long long cnt[ENS_NROT] = {};
         cnt[R_A] = slots;
-        cnt[R_B_SPR] = P > 2 ? (P - 2) * g.Ns : 0;
+        cnt[R_B_SPR] = P * g.Ns;
         cnt[R_B_EINT] = N;
         cnt[R_B_PAIR] = E.d.pair_kind ? (long long)E.jobs * P : 0;
         cnt[R_B_SK] = E.ewald ? P * sk32_groups(E.ncol, E.nlong) : 0;

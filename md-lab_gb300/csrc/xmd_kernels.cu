@@ -1518,7 +1518,9 @@ __global__ void __launch_bounds__(32 * EX_Y) k_exch_finish(Geo g, const double *
   __syncthreads();
   if (threadIdx.y != 0 || side >= 2) return;
   f[sidx(side ? g.P - 1 : 0, d, l, D, g.Ns)] =
-      l < g.N ? exch_end_value<D>(g, x, w2, image, scr, side, d, l, &share[0][threadIdx.x], 32) : 0.0;
+      l < g.N ? exch_end_value<D>(g, exch_own_spring(g, x, image, side, d, l), w2, scr, side, d, l,
+                                  &share[0][threadIdx.x], 32)
+              : 0.0;
 }
 
 size_t exch_scratch_doubles(const Geo &g) {
