@@ -674,6 +674,19 @@ __device__ inline void block_inv_column(int N, const TriJob &job, int dir, int c
   job.Be[dir][o] = b.e;
 }
 
+// one column of W(c) likewise, c >= 1
+__device__ inline void block_w_column(int N, double beta, double vi, double lnvi, const double *__restrict__ ENk,
+                                      const double *__restrict__ lnn, const TriJob &job, int dir, int c, int s,
+                                      const long long (*Am)[TS_LD], const int (*Ae)[TS_LD]) {
+  const int lane = threadIdx.x & 31, i0 = 1 + c * TS_CHUNK;
+  XI u{0, XI_NONE};
+  if (i0 + lane <= N) u = weight_at(N, beta, vi, lnvi, ENk, lnn, dir, i0 + lane, i0 - TS_CHUNK + s);
+  u = block_solve_column(u, 0, min(TS_CHUNK, N - c * TS_CHUNK), Am, Ae);
+  const size_t o = (size_t)c * TS_CHUNK * TS_CHUNK + lane * TS_CHUNK + s;
+  ((long long *)job.Wm[dir])[o] = u.m;
+  job.We[dir][o] = u.e;
+}
+
 // gradient of the two springs at bead (ja, la) towards (jn, ln) and (jp, lp):
 // m w2 (x - x_n) + m w2 (x - x_p), md_pimd_x.c:2344-2367
 template <int D>
@@ -968,16 +981,26 @@ __device__ inline XI xi_dot(const long long *__restrict__ Mm, const int *__restr
   return xi_warp_sum(a);
 }
 
+// a + m x for a normalised x; the product may miss one bit of 62
+__device__ __forceinline__ XI xi_mul_add(XI a, XI m, XI x) {
+  return xi_add(a, {(long long)__umul64hi((unsigned long long)x.m << 2, (unsigned long long)m.m), m.e + x.e});
+}
+
 // The block solve of direction `backward` by the calling thread block (any
 // whole number of warps; rows of a chunk go round-robin over the warps, each
 // row's sums inside one warp, so the result does not depend on the count).
+// viaw: by the products W, X_c = B_c P_c + W_c X_{c-1}, with the sums in the order
+// of the cluster solve (k_tri_solve_c), whose bits it then gives.
 // sh: (8 + 4) (N + 1 + 2 TS_CHUNK + 2 TS_CHUNK TS_LD) bytes of shared memory.
-__device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, int backward, double *sh) {
+__device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, int backward, double *sh,
+                                       bool viaw = false) {
   const long long *__restrict__ Mm = (const long long *)job.Mm[backward];
   const int *__restrict__ Me = job.Me[backward];
   const long long *__restrict__ Bgm = (const long long *)job.Bm[backward];
   const int *__restrict__ Bge = job.Be[backward];
-  long long *Um = (long long *)sh;          // [TS_CHUNK][TS_LD] next chunk vs the chunk before it
+  const long long *__restrict__ Wgm = (const long long *)job.Wm[backward];
+  const int *__restrict__ Wge = job.We[backward];
+  long long *Um = (long long *)sh;          // [TS_CHUNK][TS_LD] next chunk vs the chunk before it (viaw: its W block)
   long long *Bsm = Um + TS_CHUNK * TS_LD;   // [TS_CHUNK][TS_LD] the chunk's B block
   long long *Pm = Bsm + TS_CHUNK * TS_LD;   // [TS_CHUNK] sums over the unknowns before the previous chunk
   long long *Rm = Pm + TS_CHUNK;            // [TS_CHUNK] right-hand sides of the chunk
@@ -988,15 +1011,16 @@ __device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, in
   int *Re = Pe + TS_CHUNK;                  // [TS_CHUNK]
   int *Xe = Re + TS_CHUNK;                  // N+1
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  // stage chunk n0's B block and its rows' weights against columns c0..c0+31
+  // stage chunk n0's B block and its rows' weights against columns c0..c0+31, or W
   auto stage = [&](int n0, int c0) {
     const int cc = (n0 - 1) / TS_CHUNK;
     for (int q = threadIdx.x; q < TS_CHUNK * TS_CHUNK; q += blockDim.x) {
       const int r = q / TS_CHUNK, k = q % TS_CHUNK, i = n0 + r, o = r * TS_LD + k;
       const bool in = i <= N;
       const bool un = in && c0 >= 0;
-      Um[o] = un ? Mm[moff(i, c0 + k)] : 0;
-      Ue[o] = un ? Me[moff(i, c0 + k)] : XI_NONE;
+      const size_t uo = viaw ? (size_t)cc * TS_CHUNK * TS_CHUNK + q : un ? moff(i, c0 + k) : 0;
+      Um[o] = un ? (viaw ? Wgm : Mm)[uo] : 0;
+      Ue[o] = un ? (viaw ? Wge : Me)[uo] : XI_NONE;
       Bsm[o] = in ? Bgm[(size_t)cc * TS_CHUNK * TS_CHUNK + q] : 0;
       Bse[o] = in ? Bge[(size_t)cc * TS_CHUNK * TS_CHUNK + q] : XI_NONE;
     }
@@ -1013,11 +1037,14 @@ __device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, in
   }
   __syncthreads();
   for (int i0 = 1, c = 0; i0 <= N; i0 += TS_CHUNK, ++c) {
-    // U: right-hand sides
+    // U: right-hand sides (viaw: B_c P_c)
     for (int r = w; r < TS_CHUNK; r += nw) {
+      const int o = r * TS_LD + lane;
       XI p{Pm[r], Pe[r]};
-      if (c > 0) {
-        const int col = i0 - TS_CHUNK + lane, o = r * TS_LD + lane;
+      if (viaw) {
+        p = xi_warp_sum(xi_mul({Bsm[o], Bse[o]}, {Pm[lane], Pe[lane]}));
+      } else if (c > 0) {
+        const int col = i0 - TS_CHUNK + lane;
         p = xi_add(p, xi_warp_sum(xi_mul({Um[o], Ue[o]}, {Xm[col], Xe[col]})));
       }
       if (lane == 0) {
@@ -1028,9 +1055,15 @@ __device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, in
     __syncthreads();
     // B: the chunk's unknowns
     for (int r = w; r < TS_CHUNK; r += nw) {
-      const int i = i0 + r, o = r * TS_LD + lane;
+      const int i = i0 + r, o = r * TS_LD + lane, col = i0 - TS_CHUNK + lane;
       if (i > N) break;  // warp-uniform
-      const XI x = xi_warp_sum(xi_mul({Bsm[o], Bse[o]}, {Rm[lane], Re[lane]}));
+      XI x;
+      if (!viaw)
+        x = xi_warp_sum(xi_mul({Bsm[o], Bse[o]}, {Rm[lane], Re[lane]}));
+      else if (c > 0)
+        x = xi_add({Rm[r], Re[r]}, xi_warp_sum(xi_mul({Um[o], Ue[o]}, {Xm[col], Xe[col]})));
+      else
+        x = {Rm[r], Re[r]};
       if (lane == 0) {
         Xm[i] = x.m;
         Xe[i] = x.e;
@@ -1044,7 +1077,17 @@ __device__ inline void tri_solve_b_dev(int N, double beta, const TriJob &job, in
     stage(n0, i0);
     for (int r = w; r < TS_CHUNK; r += nw) {
       const int i = n0 + r;
-      const XI p = i <= N ? xi_dot(Mm, Me, Xm, Xe, i, i0, lane) : XI{0, XI_NONE};
+      XI p{0, XI_NONE};
+      if (i <= N && !viaw) {
+        p = xi_dot(Mm, Me, Xm, Xe, i, i0, lane);
+      } else if (i <= N) {
+        if (lane == 0) p = {Mm[moff(i, 0)], Me[moff(i, 0)]};
+        for (int j = 1 + lane; j < i0; j += TS_CHUNK) {
+          const size_t q = moff(i, j);
+          p = xi_mul_add(p, {Mm[q], Me[q]}, {Xm[j], Xe[j]});
+        }
+        p = xi_warp_sum(p);
+      }
       if (lane == 0) {
         Pm[r] = p.m;
         Pe[r] = p.e;

@@ -48,6 +48,7 @@ struct EnsSys {
   TriJob job;
   P32 q;
   int T, jobs;
+  int viaw;   // the per-system calls take the cluster solve: its arithmetic (tri_solve_b_dev)
   int ewald;  // reciprocal sums present (D = 3)
   int ns, ncol, nlong;
   const int4 *cols;
@@ -373,8 +374,11 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
       const EnsSys &E = sys[i];
       const EnsSysDesc &d = E.d;
       const int N = d.g.N, nch = (N + TS_CHUNK - 1) / TS_CHUNK;
-      for (long long tk = ens_first(gb, sys[i].rot[R_E_INV], G); tk < 2 * nch; tk += G) {
-        const int dir = (int)tk / nch, c = (int)tk % nch, i0 = 1 + c * TS_CHUNK;
+      const int kinds = E.viaw ? 2 : 1;  // B, and W for the cluster's arithmetic
+      for (long long tk = ens_first(gb, sys[i].rot[R_E_INV], G); tk < 2 * nch * kinds; tk += G) {
+        const int dir = (int)tk / (nch * kinds), c = (int)tk % nch, i0 = 1 + c * TS_CHUNK;
+        const bool inv = (int)tk / nch % kinds == 0;
+        if (!inv && c == 0) continue;  // no chunk before the first
         __syncthreads();
         for (int e = tid; e < TS_CHUNK * TS_CHUNK; e += ENS_T) {
           const int r = e / TS_CHUNK, t = e % TS_CHUNK;
@@ -384,7 +388,12 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
           Ae[r][t] = q.e;
         }
         __syncthreads();
-        for (int sc = w; sc < TS_CHUNK; sc += ENS_W) block_inv_column(N, E.job, dir, c, sc, Am, Ae);
+        for (int sc = w; sc < TS_CHUNK; sc += ENS_W) {
+          if (inv)
+            block_inv_column(N, E.job, dir, c, sc, Am, Ae);
+          else
+            block_w_column(N, d.beta, d.vi, E.lnvi, d.ENk, d.lnn, E.job, dir, c, sc, Am, Ae);
+        }
       }
     }
   }
@@ -397,7 +406,7 @@ __global__ void __launch_bounds__(ENS_T, MINB) k_ensemble_step(const EnsSys *__r
       const EnsSys &E = sys[i];
       for (long long dir = ens_first(gb, sys[i].rot[R_F], G); dir < 2; dir += G) {
         __syncthreads();
-        tri_solve_b_dev(E.d.g.N, E.d.beta, E.job, (int)dir, (double *)ens_sh);
+        tri_solve_b_dev(E.d.g.N, E.d.beta, E.job, (int)dir, (double *)ens_sh, E.viaw);
       }
     }
   }
@@ -547,6 +556,7 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
     const Geo &g = E.d.g;
     if (g.D != D || g.N < 1 || g.N > ENS_MAX_N || g.P < 2) return cudaErrorInvalidValue;
     E.job = tri_job(g.N, E.d.rs_f, E.d.rs_b, E.d.VBN, E.d.tmpV);
+    E.viaw = solve_by_cluster(g.N);
     E.T = (g.N + 31) / 32;
     E.jobs = E.T * (E.T + 1) / 2;
     if (E.d.pair_kind) E.q = make_p32(g, E.d.pp);
@@ -612,7 +622,7 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
         cnt[R_D_ENK] = N * (N - 1) / 2;
         cnt[R_E_W] = N;
         cnt[R_E_PS] = E.d.pair_kind && !E.ewald ? slots : 0;
-        cnt[R_E_INV] = 2 * ((N + TS_CHUNK - 1) / TS_CHUNK);
+        cnt[R_E_INV] = 2 * ((N + TS_CHUNK - 1) / TS_CHUNK) * (E.viaw ? 2 : 1);
         cnt[R_F] = 2;
         cnt[R_G] = exch_jobs(g.N);
         cnt[R_H] = slots;

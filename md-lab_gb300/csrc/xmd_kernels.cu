@@ -970,13 +970,7 @@ __global__ void __launch_bounds__(128) k_weights_inv(int N, double beta, double 
     block_inv_column(N, job, dir, c, s, Am, Ae);
     return;
   }
-  const int lane = threadIdx.x & 31;
-  XI u{0, XI_NONE};
-  if (i0 + lane <= N) u = weight_at(N, beta, vi, lnvi, ENk, lnn, dir, i0 + lane, i0 - TS_CHUNK + s);
-  u = block_solve_column(u, 0, min(TS_CHUNK, N - c * TS_CHUNK), Am, Ae);
-  const size_t o = (size_t)c * TS_CHUNK * TS_CHUNK + lane * TS_CHUNK + s;
-  ((long long *)job.Wm[dir])[o] = u.m;
-  job.We[dir][o] = u.e;
+  block_w_column(N, beta, vi, lnvi, ENk, lnn, job, dir, c, s, Am, Ae);
 }
 
 // One block per direction, 16 warps, three phases per chunk c:
@@ -1060,10 +1054,6 @@ __global__ void __launch_bounds__(TSC_WARPS * 32) k_tri_solve_c(int N, double be
   auto weight = [&](int i, int j0) {  // row i's weight against column j0 + lane
     const size_t o = moff(i, j0 + lane);
     return i <= N ? XI{Mm[o], Me[o]} : XI{0, XI_NONE};
-  };
-  // a + m x for a normalised x; the product may miss one bit of 62
-  auto mul_add = [&](XI a, XI m, XI x) {
-    return xi_add(a, {(long long)__umul64hi((unsigned long long)x.m << 2, (unsigned long long)m.m), m.e + x.e});
   };
   constexpr int R = SLOTS > 0 ? 2 * SLOTS : 1;
   XI acc[R], nxt[R];
@@ -1153,11 +1143,11 @@ __global__ void __launch_bounds__(TSC_WARPS * 32) k_tri_solve_c(int N, double be
           if (SLOTS > 0) {
 #pragma unroll
             for (int t = 0; t < SLOTS; ++t)
-              if (t == tn) p = mul_add(acc[2 * t + h], nxt[2 * t + h], x);
+              if (t == tn) p = xi_mul_add(acc[2 * t + h], nxt[2 * t + h], x);
           } else {
             const size_t o = ((size_t)tn * TS_CHUNK + w + h * TSC_WARPS) * 32 + lane;
             p = {Sm[o], Se[o]};
-            if (c >= 1) p = mul_add(p, weight(row_of(tn, h), j0), x);
+            if (c >= 1) p = xi_mul_add(p, weight(row_of(tn, h), j0), x);
           }
           p = xi_warp_sum(p);
           if (lane == 0) {
@@ -1180,7 +1170,7 @@ __global__ void __launch_bounds__(TSC_WARPS * 32) k_tri_solve_c(int N, double be
 #pragma unroll
         for (int q = 0; q < R; ++q) {
           if (q / 2 < t0) continue;
-          if (c >= 1) acc[q] = mul_add(acc[q], nxt[q], x);
+          if (c >= 1) acc[q] = xi_mul_add(acc[q], nxt[q], x);
           nxt[q] = weight(row_of(q / 2, q & 1), i0);
         }
       } else if (c >= 1) {
@@ -1194,7 +1184,7 @@ __global__ void __launch_bounds__(TSC_WARPS * 32) k_tri_solve_c(int N, double be
             const int q = qb + u;
             if (q >= 2 * slots) break;
             const size_t o = ((size_t)(q / 2) * TS_CHUNK + w + (q & 1) * TSC_WARPS) * 32 + lane;
-            const XI a = mul_add({Sm[o], Se[o]}, m[u], x);
+            const XI a = xi_mul_add({Sm[o], Se[o]}, m[u], x);
             Sm[o] = a.m;
             Se[o] = a.e;
           }
@@ -1308,6 +1298,11 @@ static int takes_cluster(int N, bool *bad) {
   const int v = want ? cluster_variant(N) : 0;
   *bad = want && !v && g_solve_force == SOLVE_CLUSTER;
   return v;
+}
+
+bool solve_by_cluster(int N) {
+  bool bad;
+  return takes_cluster(N, &bad) != 0;
 }
 
 static cudaError_t tri_solve(int N, double beta, const TriJob &job, int first, int count, cudaStream_t st,

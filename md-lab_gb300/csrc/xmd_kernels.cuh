@@ -135,6 +135,7 @@ int solve_path();
 // record the path for one N (the solve autotuner) and read the path used for N
 void set_solve_choice(int N, int path);
 int solve_choice(int N);
+bool solve_by_cluster(int N);  // whether the unsigned solve of N runs on a cluster now
 cudaError_t fill_vb_signed(int N, double beta, double vi2, const double *ENk, const double *lnn, double *V2,
                            double *sign, double *rs, cudaStream_t st);
 // lnn: the host table of ln l then 1/l (2 (N+1) doubles)
