@@ -1632,18 +1632,20 @@ __device__ inline double pair_sum32(const Geo &g, const float *__restrict__ part
 
 // Reciprocal forces on 32 particles of slice j, one a lane, by a block of SK_W warps: warp w sums columns w, w + SK_W, ..., so that
 // the lanes read each table entry at one address; Kahan sums, the warps' added
-// in double-float.  sc, sT: columns (recip_col32) and force tables; pxy: [2][ns+1][32]
+// in double-float.  sc, sT: columns (recip_col32) and force tables, of all columns
+// or (PARTS, cap < ncol) of cap at a time, a multiple of SK_W, which stage(c0, n)
+// brings there; pxy: [2][ns+1][32]
 // float2, red: [SK_W][3][32] float2, of these warps alone (red may lie over
 // sT).  The real space's tile sums (part, T tiles, pscale) are added here too:
 // their loads pass beside other blocks' sums, and the reciprocal forces' own
 // trip to f serves both.  NSM: the largest ns.  Bound by FP32 issue, eight multiply-adds a
 // harmonic: 36 us at N = 512, P = 64, |n| <= 10, 57 with two threads a particle,
 // each on half the columns with its own reads of the tables.
-template <int NSM>
-__device__ inline void recip_tile32(const Geo &g, int ns, int ncol, const RecipCol *sc, const float4 *sT, float2 *pxy,
-                                    float2 *red, const float2 *__restrict__ ph1, double scale, double *__restrict__ f,
-                                    int j, int l0, int w, int lane, const float *__restrict__ part, int T,
-                                    double pscale) {
+template <int NSM, bool PARTS, class Stage>
+__device__ inline void recip_tile32(const Geo &g, int ns, int ncol, int cap, Stage stage, const RecipCol *sc,
+                                    const float4 *sT, float2 *pxy, float2 *red, const float2 *__restrict__ ph1,
+                                    double scale, double *__restrict__ f, int j, int l0, int w, int lane,
+                                    const float *__restrict__ part, int T, double pscale) {
   const int l = min(l0 + lane, g.N - 1);  // lanes past the end repeat the last particle
   const float2 *p1 = ph1 + (size_t)j * 3 * g.Ns + l;
   if (w < 2) {
@@ -1663,7 +1665,7 @@ __device__ inline void recip_tile32(const Geo &g, int ns, int ncol, const RecipC
   }
   __syncthreads();
   Kahan F[3];
-  for (int ci = w; ci < ncol; ci += SK_W) {
+  auto column = [&](int ci) {
     const RecipCol c = sc[ci];
     const float4 *t = sT + ci * (ns + 1);
     const float2 vx = pxy[c.ox + lane], vy = pxy[c.oy + lane];
@@ -1684,6 +1686,17 @@ __device__ inline void recip_tile32(const Geo &g, int ns, int ncol, const RecipC
     F[0].add(__fmul_rn(c.fx, Tm));
     F[1].add(__fmul_rn(c.fy, Tm));
     F[2].add(fmaf(er, vi, __fmul_rn(ei, vr)));
+  };
+  if (PARTS && cap < ncol) {
+    for (int c0 = 0; c0 < ncol; c0 += cap) {
+      const int n = min(cap, ncol - c0);
+      if (c0 > 0) __syncthreads();  // the part before is no longer read
+      stage(c0, n);
+      __syncthreads();
+      for (int ci = w; ci < n; ci += SK_W) column(ci);
+    }
+  } else {
+    for (int ci = w; ci < ncol; ci += SK_W) column(ci);
   }
   __syncthreads();  // the tables are no longer read
 #pragma unroll

@@ -32,16 +32,15 @@
 #include <vector>
 
 #include "xmd_device.cuh"
+#include "xmd_ens_layout.h"
 #include "xmd_kernels.cuh"
 
 namespace xk {
 
-constexpr int ENS_T = 256;                // threads per block
-constexpr int ENS_W = ENS_T / 32;         // warps per block
-constexpr size_t ENS_SMEM = 64 * 1024;    // dynamic shared memory per block
-constexpr int ENS_NSMAX = 11;             // largest Ewald n_sum
+constexpr int ENS_T = 32 * ENS_W;         // threads per block
 constexpr long long ENS_WAIT_LIMIT = 1LL << 31;  // clock cycles a grid-barrier wait may take (~1 s)
 static_assert(ENS_T == SK_T, "the FP32 reciprocal sums take SK_W warps");
+static_assert(sizeof(RecipCol) == 32, "ens_recip_column counts a record of 32 bytes");
 
 struct EnsSys {
   EnsSysDesc d;
@@ -51,6 +50,7 @@ struct EnsSys {
   int viaw;   // the per-system calls take the cluster solve: its arithmetic (tri_solve_b_dev)
   int ewald;  // reciprocal sums present (D = 3)
   int ns, ncol, nlong;
+  int cap;    // columns of the reciprocal forces staged at a time
   const int4 *cols;
   const float *coef32;
   float2 *ph1;
@@ -105,21 +105,25 @@ __device__ inline void ens_pair_job(const EnsSys &E, int wi, int lane) {
 
 // Reciprocal forces on the particles of bead slice j by the calling block, 32
 // at a time, as k_recip_force32 computes them; the columns and force tables
-// staged once.
+// staged once, or in parts for each 32 particles where not all fit
+// (ens_recip_columns).
 __device__ inline void ens_recip_slice(const EnsSys &E, int j, unsigned char *sh) {
   const Geo &g = E.d.g;
-  const int ns = E.ns, ncol = E.ncol, tid = threadIdx.x;
+  const int ns = E.ns, ncol = E.ncol, cap = E.cap, tid = threadIdx.x;
   float4 *sT = (float4 *)sh;
-  RecipCol *sc = (RecipCol *)(sT + ncol * (ns + 1));
-  float2 *pxy = (float2 *)(sc + ncol), *red = pxy + 2 * (ns + 1) * 32;
+  RecipCol *sc = (RecipCol *)(sT + cap * (ns + 1));
+  float2 *pxy = (float2 *)(sc + cap), *red = pxy + 2 * (ns + 1) * 32;
   const float4 *Tj = E.T32 + (size_t)j * ncol * (ns + 1);
+  auto stage = [&](int c0, int n) {
+    for (int q = tid; q < n * (ns + 1); q += ENS_T) sT[q] = Tj[(size_t)c0 * (ns + 1) + q];
+    for (int q = tid; q < n; q += ENS_T) sc[q] = recip_col32(E.cols[c0 + q], ns);
+  };
   __syncthreads();
-  for (int q = tid; q < ncol * (ns + 1); q += ENS_T) sT[q] = Tj[q];
-  for (int q = tid; q < ncol; q += ENS_T) sc[q] = recip_col32(E.cols[q], ns);
+  if (cap >= ncol) stage(0, ncol);
   for (int l0 = 0; l0 < g.N; l0 += 32) {
     if (l0 > 0) __syncthreads();
-    recip_tile32<ENS_NSMAX>(g, ns, ncol, sc, sT, pxy, red, E.ph1, E.rscale, E.d.f, j, l0, tid >> 5, tid & 31,
-                            E.part, E.T, E.pscale);
+    recip_tile32<ENS_NSMAX, true>(g, ns, ncol, cap, stage, sc, sT, pxy, red, E.ph1, E.rscale, E.d.f, j, l0, tid >> 5,
+                                  tid & 31, E.part, E.T, E.pscale);
   }
 }
 
@@ -555,6 +559,7 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
     E.d = sd[i];
     const Geo &g = E.d.g;
     if (g.D != D || g.N < 1 || g.N > ENS_MAX_N || g.P < 2) return cudaErrorInvalidValue;
+    if (ens_solve_bytes(g.N, TS_CHUNK) > ENS_SMEM) return cudaErrorInvalidValue;
     E.job = tri_job(g.N, E.d.rs_f, E.d.rs_b, E.d.VBN, E.d.tmpV);
     E.viaw = solve_by_cluster(g.N);
     E.T = (g.N + 31) / 32;
@@ -567,6 +572,8 @@ cudaError_t ensemble_prepare(const EnsSysDesc *sd, int n, int D, int L, int bloc
       E.ns = r.nsum;
       E.ncol = r.ncol;
       E.nlong = r.nlong;
+      E.cap = ens_recip_columns(r.nsum, r.ncol);
+      if (std::max(ens_recip_bytes(r.nsum, r.ncol), sk32_smem(r.nsum)) > ENS_SMEM) return cudaErrorInvalidValue;
       E.cols = (const int4 *)r.kvec;
       E.coef32 = (const float *)(r.coef + r.nk);
       E.ph1 = (float2 *)(r.phase + recip_phase_doubles(g, r.nsum));

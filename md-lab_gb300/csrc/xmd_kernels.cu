@@ -3877,8 +3877,8 @@ __global__ void __launch_bounds__(SK_T, 4) k_recip_force32(Geo g, int ncol, cons
   const float4 *Tj = T + (size_t)j * ncol * (NS + 1);
   for (int q = threadIdx.x; q < ncol * (NS + 1); q += SK_T) sT[q] = Tj[q];
   for (int q = threadIdx.x; q < ncol; q += SK_T) sc[q] = recip_col32(cols[q], NS);
-  recip_tile32<NS>(g, NS, ncol, sc, sT, (float2 *)(sc + ncol), (float2 *)rf32_sh, ph1, scale, f, j, blockIdx.x * 32,
-                   threadIdx.x >> 5, threadIdx.x & 31, part, ntile, pscale);
+  recip_tile32<NS, false>(g, NS, ncol, ncol, [](int, int) {}, sc, sT, (float2 *)(sc + ncol), (float2 *)rf32_sh, ph1,
+                          scale, f, j, blockIdx.x * 32, threadIdx.x >> 5, threadIdx.x & 31, part, ntile, pscale);
 }
 
 // The mixed form's Ewald forces: FP32 positions and phases, real-space tiles,
