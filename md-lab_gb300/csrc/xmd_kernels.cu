@@ -2281,7 +2281,7 @@ static int pair_grid(size_t warps_needed, const Geo &g) {
 // launch instead of per pair
 PairPrm with_far_images(const PairPrm &p, const Geo &g) {
   PairPrm q = p;
-  if (p.s > 0) {
+  if (p.kind == PAIR_GAUSSIAN || p.kind == PAIR_PERIODIC_GAUSSIAN) {  // (the range enters squared: any sign)
     q.is2 = 1.0 / (p.s * p.s);
     q.g0 = p.g / (M_PI * p.s * p.s);
     q.g2 = q.g0 * 2 / (p.s * p.s);
@@ -3768,8 +3768,8 @@ P32 make_p32(const Geo &g, const PairPrm &p) {
     q.L[d] = (float)g.box[d];
     q.iL[d] = (float)g.inv_box[d];
   }
-  q.igs2 = p.s > 0 ? (float)(1.0 / (p.s * p.s)) : 0.f;
-  q.gpre = p.s > 0 ? (float)(p.g / (M_PI * p.s * p.s) * (2.0 / (p.s * p.s))) : 0.f;
+  q.igs2 = p.s != 0 ? (float)(1.0 / (p.s * p.s)) : 0.f;
+  q.gpre = p.s != 0 ? (float)(p.g / (M_PI * p.s * p.s) * (2.0 / (p.s * p.s))) : 0.f;
   q.qs = (float)p.qs;
   q.alpha = (float)p.alpha;
   q.nsum = p.nsum;
