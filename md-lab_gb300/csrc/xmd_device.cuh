@@ -282,29 +282,36 @@ struct Ext {
 };
 
 // exp(x) for any finite x as 2^e exp(r), |r| <= ln2/2: exp(r) 2^62 from the
-// integer pipe, the reduction in FP64
+// integer pipe, the reduction in FP64.  The series reads r's bits, so an x that
+// is infinite or no number is told by its own exponent, EXP_BAD; from 2^30 on e
+// is held to +-2^29.
+constexpr int EXP_BAD = 0x7fffffff;
 __device__ __forceinline__ long long exp_reduced(double x, int &e) {
   constexpr double MAGIC = 6755399441055744.0;  // 1.5 2^52: adding rounds to an integer, in the low word
   const double tq = fma(x, LOG2E, MAGIC), q = tq - MAGIC;
   double r = fma(-q, LN2_HI, x);
   r = fma(-q, LN2_LO, r);
-  const bool large = (__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFLL) >= 0x41D0000000000000LL;  // |x| >= 2^30
-  e = large ? (int)q : __double2loint(tq);
+  const int hi = __double2hiint(x) & 0x7fffffff;
+  e = __double2loint(tq);
+  if (hi >= 0x41d00000)  // |x| >= 2^30
+    e = hi >= 0x7ff00000 ? EXP_BAD : x < 0 ? -(1 << 29) : 1 << 29;
   return exp_q62(r);
 }
 __device__ inline Ext ext_exp(double x) {
   Ext w;
   w.m = q62_double(exp_reduced(x, w.e));
+  if (w.e == EXP_BAD) w = {x - x, 0};  // (not a number)
   return w;
 }
 
-// exp(x) through ext_exp, the power of two put into the exponent field by
+// exp(x) as ext_exp forms it, the power of two put into the exponent field by
 // integer arithmetic; results near or beyond the ends of the normal range
-// (|x| > 700) are left to exp()
+// (|x| > 700) and anything that is no finite number are left to exp()
 __device__ inline double exp_fast(double x) {
-  const Ext w = ext_exp(x);
-  if (w.e <= -1020 || w.e >= 1020) return exp(x);
-  return __longlong_as_double(__double_as_longlong(w.m) + ((long long)w.e << 52));
+  int e;
+  const double m = q62_double(exp_reduced(x, e));
+  if (e <= -1020 || e >= 1020) return exp(x);
+  return __longlong_as_double(__double_as_longlong(m) + ((long long)e << 52));
 }
 
 // m * 2^d for d <= 0 (0 once the result would drop below the subnormals)
@@ -341,11 +348,16 @@ __device__ inline void ext_norm(double &m, int &e) {
 // FP64 instruction, which on GB300 holds its pipe for 64 cycles a warp.  The
 // unsigned solves and the diagonal blocks' inverses work on these; every
 // truncation is below 2^-60 of the value.
+// A number that is none (from an infinite or NaN energy) is one of exponent
+// XI_BAD: products hold exponents to it, sums take the largest, so that whatever
+// contains it has an exponent above XI_TOP, which no number reaches (weights
+// are at most xi^N), and becomes NaN where it leaves these forms; a zero times it
+// is a zero still, whose exponent stays far below any number's.
 struct XI {
   long long m;
   int e;
 };
-constexpr int XI_NONE = -(1 << 29);
+constexpr int XI_NONE = -(1 << 30) + (1 << 25), XI_BAD = 1 << 28, XI_TOP = 1 << 26;
 
 // v 2^e of a non-negative double v
 __device__ __forceinline__ XI xi_from(double v, int e) {
@@ -359,10 +371,12 @@ __device__ __forceinline__ XI xi_from(double v, int e) {
 __device__ __forceinline__ XI xi_exp(double x) {
   int e;
   const long long p = exp_reduced(x, e);  // 0.70 .. 1.42 times 2^62
+  if (e >= XI_BAD || e <= -(1 << 29)) return {1LL << 61, min(e, XI_BAD)};
   return p >= (1LL << 62) ? XI{p >> 1, e + 1} : XI{p, e};
 }
-// rounded to a double (to zero below 2^-1074; e up to 1024)
+// rounded to a double (to zero below 2^-1074; e up to 1024, or above XI_TOP)
 __device__ __forceinline__ double xi_double(XI a) {
+  if (a.e > XI_TOP) return __longlong_as_double(0x7ff8000000000000LL);
   const bool low = a.e < -1020;
   const int e = low ? a.e + 200 : a.e;
   if (a.m == 0 || e < -1020) return 0.0;
@@ -383,7 +397,7 @@ __device__ __forceinline__ double xi_log(XI a) {
   return fma((double)e, LN2_HI, fma((double)e, LN2_LO, fma(-0.5 * d, d, d)) + (double)y);
 }
 __device__ __forceinline__ XI xi_mul(XI a, XI b) {
-  XI r{(long long)__umul64hi((unsigned long long)a.m << 2, (unsigned long long)b.m), a.e + b.e};
+  XI r{(long long)__umul64hi((unsigned long long)a.m << 2, (unsigned long long)b.m), __viaddmin_s32(a.e, b.e, XI_BAD)};
   if (r.m < (1LL << 61)) r.m <<= 1, r.e -= 1;
   return r;
 }
@@ -955,7 +969,7 @@ __device__ inline void tri_solve_out(int N, double beta, const TriJob &job, int 
     const XI x{Xm[i], Xe[i]};
     if (i > 0) {
       // the quotient, corrected by its residual
-      const double lnx = xi_log(x), q = -lnx * ib;
+      const double lnx = x.e > XI_TOP ? xi_double(x) : xi_log(x), q = -lnx * ib;
       out[backward ? N - i : i] = fma(-fma(q, beta, lnx), ib, q);
     } else {
       out[backward ? N : 0] = 0.0;
@@ -965,7 +979,8 @@ __device__ inline void tri_solve_out(int N, double beta, const TriJob &job, int 
       job.Xe[backward][i] = x.e;
       if (i == N) {
         // 1 / (m 2^(e-62)) = (1 / mantissa in [1/2, 1)) 2^-e
-        const XI v = xi_from(1.0 / __longlong_as_double(((x.m + 256) >> 9) + (1021LL << 52)), -x.e);
+        XI v = xi_from(1.0 / __longlong_as_double(((x.m + 256) >> 9) + (1021LL << 52)), -x.e);
+        if (x.e > XI_TOP) v.e = XI_BAD;
         job.Xm[backward][N + 1] = v.m;
         job.Xe[backward][N + 1] = v.e;
       }
@@ -983,7 +998,8 @@ __device__ inline XI xi_dot(const long long *__restrict__ Mm, const int *__restr
 
 // a + m x for a normalised x; the product may miss one bit of 62
 __device__ __forceinline__ XI xi_mul_add(XI a, XI m, XI x) {
-  return xi_add(a, {(long long)__umul64hi((unsigned long long)x.m << 2, (unsigned long long)m.m), m.e + x.e});
+  return xi_add(a, {(long long)__umul64hi((unsigned long long)x.m << 2, (unsigned long long)m.m),
+                    __viaddmin_s32(m.e, x.e, XI_BAD)});
 }
 
 // The block solve of direction `backward` by the calling thread block (any

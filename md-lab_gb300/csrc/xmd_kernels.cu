@@ -1683,7 +1683,9 @@ __device__ inline void pair_eval(const PairPrm &p, const Geo &g, const double *d
     // pipe: about 15 FP64 instructions a pair where exp() and four divisions
     // took over a hundred
     const double q = r2 * p.is2;
-    const double ex = exp_fast(-fma(fma(-q, p.s * p.s, r2), p.is2, q));
+    double a = fma(fma(-q, p.s * p.s, r2), p.is2, q);
+    if ((__double2hiint(a) & 0x7ff00000) == 0x7ff00000) a = q;  // r^2 or s^2 beyond the range: no residual
+    const double ex = exp_fast(-a);
     const double mult = p.g2 * ex;
 #pragma unroll
     for (int d = 0; d < D; ++d) F[d] = mult * t[d];
