@@ -346,8 +346,11 @@ __device__ inline void ext_norm(double &m, int &e) {
 // A non-negative number m 2^(e-62) with a 62-bit integer mantissa (2^61 <= m
 // < 2^62, or m = 0 with e = XI_NONE): nine bits more than a double's, and no
 // FP64 instruction, which on GB300 holds its pipe for 64 cycles a warp.  The
-// unsigned solves and the diagonal blocks' inverses work on these; every
-// truncation is below 2^-60 of the value.
+// unsigned solves and the diagonal blocks' inverses work on these: a product or
+// a sum of two drops less than 2^-60 of its value, a warp's sum rounds to 2^-57
+// of its largest term.  G is within 3 to 5e-16 of 128-bit recursions' (N = 512 and
+// 1000; 5 to 8e-16 when warp sums dropped five bits of every lane, 7e-15 in FP64
+// with sums of 57 bits).
 // A number that is none (from an infinite or NaN energy) is one of exponent
 // XI_BAD: products hold exponents to it, sums take the largest, so that whatever
 // contains it has an exponent above XI_TOP, which no number reaches (weights
@@ -411,15 +414,17 @@ __device__ __forceinline__ XI xi_add(XI a, XI b) {
 __device__ __forceinline__ XI xi_shfl(XI a, int src) {
   return {__shfl_sync(FULL, a.m, src), __shfl_sync(FULL, a.e, src)};
 }
-// the warp's sum in every lane: aligned to the largest exponent with 57 bits,
-// in three 19-bit parts (a warp-wide integer reduction is one instruction)
+// the warp's sum in every lane: aligned to the largest exponent, in parts of 21,
+// 21 and 20 bits (a warp-wide integer reduction is one 32-bit instruction), and
+// rounded once, to a 2^-57th of the largest term (32 terms need five bits more)
 __device__ __forceinline__ XI xi_warp_sum(XI a) {
   const int em = __reduce_max_sync(FULL, a.e);
-  const long long q = (a.m >> min(em - a.e, 63)) >> 5;
-  const unsigned p0 = __reduce_add_sync(FULL, (unsigned)q & 0x7ffffu);
-  const unsigned p1 = __reduce_add_sync(FULL, (unsigned)(q >> 19) & 0x7ffffu);
-  const unsigned p2 = __reduce_add_sync(FULL, (unsigned)(q >> 38));
-  const long long t = (long long)p0 + ((long long)p1 << 19) + ((long long)p2 << 38);
+  const long long q = a.m >> min(em - a.e, 63);
+  const unsigned p0 = __reduce_add_sync(FULL, (unsigned)q & 0x1fffffu);
+  const unsigned p1 = __reduce_add_sync(FULL, (unsigned)(q >> 21) & 0x1fffffu);
+  const unsigned p2 = __reduce_add_sync(FULL, (unsigned)(q >> 42));
+  const long long low = (long long)p0 + ((long long)p1 << 21);
+  const long long t = ((long long)p2 << 37) + ((low + 16) >> 5);  // below 2^62
   if (t == 0) return {0, XI_NONE};
   const int sh = __clzll(t) - 2;
   return {t << sh, em + 5 - sh};
