@@ -1048,9 +1048,17 @@ __global__ void __launch_bounds__(SH_T) k_sk_shells(Geo g, DescPrm p, const doub
       si += part[q][kl].y;
     }
     // fixed point: the sum does not depend on the order of its blocks
-    atomicAdd(&p.shell[j * DESC_SHELLS + kv.w],
-              (unsigned long long)__float2ull_rn((sr * sr + si * si) * p.shell_norm[kv.w] * SHELL_ONE));
+    const float v = (sr * sr + si * si) * p.shell_norm[kv.w];
+    unsigned long long *o = &p.shell[j * DESC_SHELLS + kv.w];
+    if (v <= 3.4028235e38f)
+      atomicAdd(o, __float2ull_rn(v * p.shell_one));
+    else
+      atomicOr(o, 1ULL << 63);
   }
+}
+// a shell's sum as a number
+__device__ __forceinline__ float shell_value(unsigned long long s, float inv_one) {
+  return (long long)s < 0 ? __int_as_float(0x7fffffff) : __ull2float_rn(s) * inv_one;
 }
 
 // Radial and vector features.  Block = 32 particles of one bead slice (the
@@ -1190,8 +1198,9 @@ __global__ void __launch_bounds__(DS_T, 2) k_desc(Geo g, DescPrm p, const double
   if (lr >= g.N) return;
   const ulonglong2 sh01 = *(const ulonglong2 *)(p.shell + j * DESC_SHELLS + f0),
                    sh23 = *(const ulonglong2 *)(p.shell + j * DESC_SHELLS + f0 + 2);
-  const float4 sh = make_float4(__ull2float_rn(sh01.x) * (1.f / SHELL_ONE), __ull2float_rn(sh01.y) * (1.f / SHELL_ONE),
-                                __ull2float_rn(sh23.x) * (1.f / SHELL_ONE), __ull2float_rn(sh23.y) * (1.f / SHELL_ONE));
+  const float io = 1.f / p.shell_one;
+  const float4 sh = make_float4(shell_value(sh01.x, io), shell_value(sh01.y, io), shell_value(sh23.x, io),
+                                shell_value(sh23.y, io));
   const float sv[4] = {sqrtf(sh.x), sqrtf(sh.y), sqrtf(sh.z), sqrtf(sh.w)};
   const size_t grow = (size_t)j * g.N + lr;
   if (RAW) {

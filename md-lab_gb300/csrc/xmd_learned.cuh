@@ -45,7 +45,15 @@ struct MlpDev {
   const float *w3f;      // [4][128] the BF16 values of W3 as FP32
 };
 
-constexpr float SHELL_ONE = 1099511627776.f;  // 2^40: fixed point, up to 2^24 particles
+// Shell features are added in 64-bit fixed point: a shell's sum is N at most (every
+// particle at one point), which the largest power of two below it takes to
+// 2^62; a part that is no number sets the top bit.  At N = 512 the unit is 2^-53, below
+// the square of what FP32 sums of N phases resolve, over N.
+inline float shell_one(int N) {
+  int b = 0;
+  while ((1LL << b) < N) ++b;
+  return (float)(1ULL << (62 - b));
+}
 // descriptor constants (host-computed from the box)
 struct DescPrm {
   float rc, inv_h;             // cut-off radius (half the smallest box length), bins per unit
@@ -60,7 +68,8 @@ struct DescPrm {
   const int4 *kvec;            // half-space wave vectors of the lowest shells: (nx >= 0, ny, nz, shell)
   int nkvec, nmax;             // their count and largest |n_i|
   const float *shell_norm;     // [DESC_SHELLS] 1 / (N x half-space vectors of the shell)
-  unsigned long long *shell;   // [P][DESC_SHELLS] scratch: each slice's shell features (squared), times SHELL_ONE
+  unsigned long long *shell;   // [P][DESC_SHELLS] scratch: each slice's shell features (squared), times shell_one
+  float shell_one;             // (shell_one(N))
   const float *fmean, *fistd;  // feature normalisation
 };
 

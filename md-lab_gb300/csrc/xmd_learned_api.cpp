@@ -507,6 +507,7 @@ int md_gb300_ewald_model_create_x(md_gb300_ewald_model_t_x **out, md_pimd_t_x *p
   M->dp.nmax = kmax;
   M->dp.shell_norm = M->dsn.as<float>();
   M->dp.shell = M->dsh.as<unsigned long long>();
+  M->dp.shell_one = xk::shell_one(g.N);
   M->dp.rc = (float)rcut;
   M->dp.inv_h = (float)(xk::DESC_BINS / rcut);
   for (int d = 0; d < 3; ++d) {
