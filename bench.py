@@ -232,9 +232,8 @@ def kept_nz_pairs(nsum, part=None):
     |nz|: the library leaves out vectors whose force weight |G| c(n) is
     below 1e-17 of the largest (RECIP_KEEP), so the column kernels run
     this many +-nz pairs instead of ncol * nsum (cubic box, alpha L = ALPHA_L).
-    part "fp64" / "fp32": only the columns the FP64 form's split keeps in
-    FP64 / sends to the FP32 kernels (largest weight in the column at or
-    above / below 1e-7 of the largest, RECIP_SPLIT)"""
+    part "fp64" / "fp32": only the columns whose largest force weight is at
+    or above / below 1e-7 of the largest of all"""
     w = {}
     for nx in range(nsum + 1):
         for ny in range(-nsum, nsum + 1):
@@ -271,9 +270,10 @@ def shell_vectors(count=32):
 
 
 def kernel_flops(name, nsum=NSUM, split=False):
-    """split: the FP64 form's kernels with their FP32 parts split off (real-
-    space images at alpha R >= 4 and the small-weight wave-vector columns
-    on the FP32 pipe): the FP64 work of the FP64 kernels"""
+    """split: without the terms that FP32 holds to 1e-12 of a force: real-
+    space images at alpha R >= 4 (the FP64 tiles of a box shorter than the
+    cut-off take them in FP32) and the small-weight wave-vector columns.  No
+    form measured here has that split"""
     part = "fp64" if split else None
     if name in ("recip_force", "recip_force32"):
         # 17.7 flop per +-nz pair of a kept column per particle and slice

@@ -166,12 +166,17 @@ int md_gb300_pair_force_noalloc_x(md_pair_force_t_x pf, const double *x, const d
 
 /* Arithmetic of the pair forces (md_pimd_calc_pair_force_x), including
    both Ewald parts.  MD_GB_PRECISION_FP64 (default) reproduces MD-Lab to
-   1e-10: FP64 except the Ewald sums, which run in double-float (unevaluated
-   sums of two FP32 values, 48 significant bits; wave vectors of a force
-   weight |G| c(n) below 1e-8 of the largest in FP32).  Forces are 3.6e-13 of
-   their norm from 64-bit sums (set by the cut-off at alpha R = 5.2), and
-   within 2e-12 of the largest from MD_GB_PRECISION_FP64_STRICT, which
-   evaluates every term in FP64.
+   1e-10: FP64 except the Ewald sums of forces and energies, which run in
+   double-float (unevaluated sums of two FP32 values, 48 significant bits;
+   wave vectors of a force weight |G| c(n) below 1e-8 of the largest in
+   FP32).  Forces are 3.6e-13 of their norm from 64-bit sums (set by the
+   cut-off at alpha R = 5.2), and within 2e-12 of the largest from
+   MD_GB_PRECISION_FP64_STRICT, which evaluates every term in FP64.  Measured
+   against that form on electron gases of 16 to 512 electrons (alpha L = 5.6):
+   3.3e-14 of the norm, 2.6e-12 of any bead's own force (that bead's is 0.3% of
+   the rms force; 2.2e-13 for 61 electrons).  Energies are 0.6e-15 of the pair
+   energy from 64-bit sums and 2.2e-15 from the strict form's; the cross
+   energies of two species are summed in FP64.
    MD_GB_PRECISION_MIXED evaluates pair and real-space Ewald forces in
    FP32: each lane adds at most 32 FP32 pair terms (one 32 x 32 tile), and
    the tile partials are added in FP64; the reciprocal sum builds its
@@ -179,7 +184,8 @@ int md_gb300_pair_force_noalloc_x(md_pair_force_t_x pf, const double *x, const d
    particles at a time and those partial sums in double-float (two-sum),
    then FP32 force tables and compensated (Kahan) column sums per particle.
    Positions, the exchange recursion, springs, the thermostat and every
-   estimator stay FP64.  The force error against the FP64 form, measured as
+   estimator stay FP64, but for the Ewald energies, which are the
+   double-float ones of MD_GB_PRECISION_FP64.  The force error against the FP64 form, measured as
    max |f32 - f64| / max |f64| over all beads of the 512-electron, 64-bead
    electron gas (Ewald |n| <= 10), is 1.1e-5 and set mainly by the FP32
    rounding of the pair separations; the library's tests bound it by 5e-5
@@ -208,8 +214,9 @@ int md_gb300_autotune_fp64_x(md_pimd_t_x *pimd, md_pair_force_t_x pf, int repeat
 
 /* Which kernel solves the exchange recursions (V_B and the backward tmpV,
    md_pimd_fill_VB_x and the force call): MD_GB_SOLVE_BLOCK runs one thread
-   block per direction, MD_GB_SOLVE_CLUSTER one cluster of eight blocks per
-   direction (distributed shared memory), MD_GB_SOLVE_AUTO (default) picks
+   block per direction, MD_GB_SOLVE_CLUSTER one cluster of eight blocks
+   (sixteen for N = 929 to 3872) per direction (distributed shared memory),
+   MD_GB_SOLVE_AUTO (default) picks
    per N: a choice recorded by md_gb300_autotune_solve_x, else the cluster
    from N = 129 on.  All paths give the same values to rounding.  Forcing
    the cluster where none of its size fits makes the recursion calls fail

@@ -3,10 +3,9 @@
 //
 // The FP64 pipe holds a warp's instruction for 64 cycles on GB300, and the
 // FP64 sums' results carry an error of about 1e-12 of a bead's force anyway
-// (cut-offs, FP32 far images and small columns); double-float rounding,
-// about 1e-14, is far below that.  The strict form (every term FP64) and
-// geometries these kernels do not take stay on the kernels of
-// xmd_kernels.cu.
+// (the cut-off); double-float rounding, about 1e-14, is far below that.  The
+// strict form (every term FP64) and geometries these kernels do not take stay
+// on the kernels of xmd_kernels.cu.
 #include <cfloat>
 #include <cmath>
 
@@ -207,10 +206,10 @@ constexpr size_t ewd_smem() {
 // 512-electron, 64-bead gas (alpha L = 5.6, 3.35 images a pair, 8.4 M pairs):
 // 257 us where the FP64 tiles took 1352 (256 x 256 cross pairs 145 and 667
 // us); in parts 128 electrons, 32 beads take 24 us (51 with whole tiles, 218 in
-// FP64) and their energies less than half of the 61 us of whole tiles (325).  The forces' error against 64-bit sums, set by the cut-off at
-// alpha R = 5.2, is 3.6e-13 of the forces' norm (4.1e-13 with the FP64 tiles
-// and their FP32 far images), 12 to 512 electrons alike.  Energies take three
-// limbs: in two, images below the sum's last bit were lost and biased it by
+// FP64) and their energies 24 (61 and 325).  The forces' error against 64-bit
+// sums, set by the cut-off at alpha R = 5.2, is 3.6e-13 of the forces' norm
+// (4.1e-13 with the FP64 tiles and their FP32 far images), 12 to 512 electrons
+// alike.  Energies take three limbs: in two, images below the sum's last bit were lost and biased it by
 // -5e-16 of the pair energies; now 0.6e-15 (128 electrons, 32 beads, rms of 16
 // states) and 0.5e-15 (512, 64) of the energy against 64 bits, 1.3e-15 and
 // 2.6e-15 with the FP64 tiles, for 3% more time.
@@ -443,8 +442,9 @@ __global__ void k_ewd_finish(int N, int Ns, size_t S, const float2 *__restrict__
 // beads kept 320 of the 2432 warps that fit on 152 SMs.  So up to four parts
 // until there are two rounds of warps (beyond, the last round costs less than
 // the parts' slots of partials); eight only where four leave most SM
-// sub-partitions idle.  A step of N x P electrons (|n| <= 4) with whole tiles,
-// and with 2, 4 and 8 parts, * taken: 16 x 4 63, 53* (8); 64 x 32 96, 64* (8);
+// sub-partitions idle.  The parts set the order of the sums, so the line counts
+// 152 SMs and not the device's: the same system gives the same bits.  A step of
+// N x P electrons (|n| <= 4) with whole tiles, and with 2, 4 and 8 parts, * taken: 16 x 4 63, 53* (8); 64 x 32 96, 64* (8);
 // 128 x 32 109, 85, 80*, 87; 128 x 64 119, 106, 94*, 96; 200 x 48 160, 138,
 // 133*, 134; 300 x 64 234, 222*, 221; 512 x 33 282, 281*, 280; 512 x 64 435*,
 // 433; 256 + 256 x 64 614, 610* (2 a cross tile) us.

@@ -1957,7 +1957,8 @@ __global__ void __launch_bounds__(256) k_pair_split(Geo g, PairPrm p, const doub
 }
 
 constexpr int PAIR_SPLIT_MAX = 8;
-// parts of a tile: enough that every SM sub-partition has two warps
+// parts of a tile: enough that every SM sub-partition has two warps (of 152 SMs,
+// not the device's: the parts set the order of the sums)
 static int pair_split(const Geo &g, int jobs) {
   int split = 1;
   while (split < PAIR_SPLIT_MAX && (size_t)jobs * g.P * split < 2 * 4 * 152) split *= 2;

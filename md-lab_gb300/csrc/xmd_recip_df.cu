@@ -492,7 +492,8 @@ cudaError_t recip_df_sk(const Geo &g, const Recip &r, const double *x, cudaStrea
   cudaError_t e = XK_LAUNCHED();
   if (e != cudaSuccess || r.items <= 0) return e;
   XK_PROF("sk");
-  // 16 threads an item where 8 would give four SMs seven blocks at most:
+  // 16 threads an item where 8 would give four SMs seven blocks at most (152
+  // SMs by number: the threads set the order of the sums):
   // 700 x 20, |n| <= 9, 80 -> 53 us; 512 x 33, |n| <= 10 (264 blocks), 63 -> 55;
   // 128 x 32, |n| <= 8 (160), 22.0 -> 20.7; 200 x 48, |n| <= 9 (288), keeps 38 (43)
   const bool few = (size_t)g.P * cdivz(r.items, DF_SK_T / 8) * 4 <= 7 * 152;
